@@ -28,6 +28,7 @@ UNITS = [
     ("mapping.cu", ["--fmad=false"]),
     ("psf.cu", ["--fmad=false"]),
     ("linalg.cu", []),
+    ("ozaki.cu", []),
     ("sparseops.cu", []),
     ("noalloc.cu", []),
     ("mixed.cu", []),
@@ -41,7 +42,8 @@ UNITS = [
     ("fitparam.cpp", []),
     ("qlpix_api.cpp", []),
 ]
-HEADERS = ["qlpix_internal.h", "qlpix_ctx.h", "lens_device.cuh", "nfw_device.cuh", "patterson_rule.h", "chol.cuh", "chol128.cuh", "tc_common.cuh", "tc_syrk.cuh", "brent.h"]
+HEADERS = ["qlpix_internal.h", "qlpix_ctx.h", "lens_device.cuh", "nfw_device.cuh", "patterson_rule.h", "chol.cuh", "chol128.cuh", "tc_common.cuh", "tc_syrk.cuh",
+           "ozaki.cuh", "tma_map.h", "brent.h"]
 
 
 def _newer(src, obj, deps):

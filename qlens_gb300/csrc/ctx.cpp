@@ -48,8 +48,9 @@ static void free_work(Work& w)
     void* ptrs[] = {w.spx, w.spy, w.cx, w.cy, w.ccx, w.ccy, w.cell3, w.w3, w.mapped, w.active_index, w.pixmaps,
                     w.rowidx, w.pixindex, w.rowpix, w.rowptr, w.Lidx, w.Lval, w.cidx, w.cval, w.ccnt, w.Lpsf,
                     w.dvec, w.cvec, w.D, w.F, w.R, w.s, w.tmp, w.model, w.partial, w.linv, w.gs, w.out, w.ep,
-                    w.fb_ray, w.fb_xy, w.fb_count, w.F0, w.gpart, w.gpart_cnt, w.cpart, w.lnz, w.sur_eps, w.xlist, w.xcount, w.nfw_xy};
+                    w.fb_ray, w.fb_xy, w.fb_count, w.F0, w.gpart, w.gpart_cnt, w.cpart, w.sur_eps, w.xlist, w.xcount, w.nfw_xy};
     for (void* p : ptrs) if (p) cudaFree(p);
+    oz_free(w.oz);
     memset(&w, 0, sizeof(w));
 }
 
@@ -128,12 +129,16 @@ static int alloc_work(qlp_ctx* c, Slot& s, int n_mask, int nsub, int Mcells, int
 static int ensure_fp64_mats(Slot& s)
 {
     if (s.fp64_mats) return QLP_OK;
-    CK(dalloc(&s.w.Lpsf, (size_t)s.N_cap * s.M_cap), "alloc L'");
-    CK(cudaMemset(s.w.Lpsf, 0, sizeof(double) * (size_t)s.N_cap * s.M_cap), "memset");
-    s.w.lnz_chunks = (s.N_cap + 15) / 16;
-    CK(dalloc(&s.w.lnz, (size_t)s.w.lnz_chunks * (s.M_cap / 64)), "alloc L' flags");
-    CK(dalloc(&s.w.F, (size_t)s.M_cap * s.M_cap), "alloc F");
-    CK(dalloc(&s.w.R, (size_t)s.M_cap * s.M_cap), "alloc R");
+    if (!s.w.Lpsf) {
+        CK(dalloc(&s.w.Lpsf, (size_t)s.N_cap * s.M_cap), "alloc L'");
+        CK(cudaMemset(s.w.Lpsf, 0, sizeof(double) * (size_t)s.N_cap * s.M_cap), "memset");
+    }
+    if (!s.w.oz) {
+        const int r = oz_alloc(&s.w.oz, s.N_cap, s.M_cap);
+        if (r != QLP_OK) return r;
+    }
+    if (!s.w.F) CK(dalloc(&s.w.F, (size_t)s.M_cap * s.M_cap), "alloc F");
+    if (!s.w.R) CK(dalloc(&s.w.R, (size_t)s.M_cap * s.M_cap), "alloc R");
     s.fp64_mats = true;
     return QLP_OK;
 }
@@ -704,7 +709,7 @@ int ctx_eval_batch(qlp_ctx* c, const double* params, const double* regparams, co
     int S = std::min(n, std::max(1, std::min(c->max_slots, QLP_MAX_SLOTS)));
     for (int k = 0; k < S; k++) {
         int r = ensure_slot(c, k, nmask_max, cells_max, std::max(snx_max, 2), std::max(sny_max, 2));
-        if (r == QLP_OK && c->precision == QLP_MIXED) r = mixed_init(c->slots[k]);
+        if (r == QLP_OK) r = (c->precision == QLP_MIXED) ? mixed_init(c->slots[k]) : ensure_fp64_mats(c->slots[k]);
         if (r != QLP_OK) {
             if (k == 0) return r;
             free_slot(c->slots[k]);

@@ -22,6 +22,7 @@
 #include "qlpix_ctx.h"
 #include "chol.cuh"
 #include "tc_syrk.cuh"
+#include "tma_map.h"
 #include "chol128.cuh"
 
 namespace qlpix {
@@ -76,39 +77,10 @@ struct MixedWork {
 
 static MixedWork* mw_of(Slot& s) { return reinterpret_cast<MixedWork*>(s.mixed); }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn get_encode()
-{
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    }
-    return fn;
-}
-
 // 128-row boxes of 128 bytes (32 FP32 or 64 F16 values), 128-byte swizzle
 static int make_map(CUtensorMap* map, void* base, int rows, int cols, bool half)
 {
-    EncodeTiledFn enc = get_encode();
-    if (!enc) return QLP_ERR_CUDA;
-    const size_t esz = half ? 2 : 4;
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * esz};
-    cuuint32_t box[2] = {(cuuint32_t)(128 / esz), TC_TILE};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(map, half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims,
-                     strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? QLP_OK : QLP_ERR_CUDA;
+    return make_map_box(map, base, rows, cols, half, TC_TILE, half ? 64 : 32);
 }
 
 // ---------------------------------------------------------------------------

@@ -1,0 +1,339 @@
+// ozaki.cu -- the plain path's FP64 contraction F = L'^T C^-1 L' on the tensor
+// cores: L' cut into digits (k_oz_scan, k_oz_slice), the digit products
+// (k_oz_syrk, ozaki.cuh) and the integers turned into F (k_oz_finish).
+// Reference: QLens::create_lensing_matrices_from_Lmatrix_dense
+// (pixelgrid.cpp:15590-15736).
+#include <cuda_fp16.h>
+#include <algorithm>
+#include "qlpix_ctx.h"
+#include "ozaki.cuh"
+#include "tma_map.h"
+
+namespace qlpix {
+
+// Digits of L' kept at a time: a larger L' goes in chunks of image pixels, the
+// integer sums of the chunks adding up.
+#define OZ_CHUNK_BYTES ((size_t)1 << 30)
+// Digit products in flight: with fewer tiles than this the pixels of each tile
+// are split over several CTAs (one CTA per SM; two rounds even out the sparsity)
+#define OZ_WANT_CTAS (2 * 152)
+
+struct OzWork {
+    __half* xs = nullptr;              // [OZ_S][M128][Kc] digits of L'^T sqrt(C^-1)
+    unsigned long long* part = nullptr; // [tile][hi, lo][64 columns][128 rows], zero between evaluations
+    int* emax = nullptr;               // [M128] largest biased exponent of each source cell's column of L'
+    unsigned char* nz = nullptr;       // [M128 / 64][nst] 32-pixel stages where 64 cells have a nonzero
+    int M128 = 0, Kc = 0, nst = 0, ntiles = 0;
+    CUtensorMap map_a, map_b;
+};
+
+// Tile t of the lower triangle: 128-row block I, 64-column block j <= 2 I + 1.
+__device__ __forceinline__ void oz_tile(int t, int& I, int& j)
+{
+    int i = (int)((sqrtf(4.0f * t + 1.0f) - 1.0f) * 0.5f);
+    while ((i + 1) * (i + 2) <= t) i++;
+    while (i * (i + 1) > t) i--;
+    I = i;
+    j = t - i * (i + 1);
+}
+
+// Each source cell's largest biased exponent and the 32-pixel stages of each
+// 64 cells that hold a nonzero.  Reads the dense L' once (memory bound); the
+// tests are on the bits, FP64 compares would bound it instead.  A CTA takes
+// 64 cells x 128 pixels.
+__global__ void __launch_bounds__(256) k_oz_scan(const GridState* __restrict__ gs, const double* __restrict__ L,
+                                                 int ldL, int* __restrict__ emax, unsigned char* __restrict__ nz,
+                                                 int nst)
+{
+    __shared__ int se[4][64];
+    __shared__ int any[4];
+    const int N = gs->N, M = gs->M;
+    const int cb = blockIdx.y, p0 = blockIdx.x * 128;
+    if (cb * 64 >= M || p0 >= N) return;
+    const int c = threadIdx.x & 63, q = threadIdx.x >> 6;      // pixels [32 q, 32 q + 32) of the chunk: one stage
+    const int cell = cb * 64 + c;
+    if (threadIdx.x < 4) any[threadIdx.x] = 0;
+    int e = 0;
+    if (cell < M) {
+        const int r0 = p0 + 32 * q, r1 = min(r0 + 32, N);
+        const double* col = L + cell;
+        #pragma unroll 8
+        for (int r = r0; r < r1; r++) e = max(e, oz_exponent(col[(size_t)r * ldL]));
+    }
+    __syncthreads();
+    se[q][c] = e;
+    if (__any_sync(0xffffffffu, e != 0) && (threadIdx.x & 31) == 0) any[q] = 1;
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        const int m = max(max(se[0][c], se[1][c]), max(se[2][c], se[3][c]));
+        if (m > 0) atomicMax(&emax[cell], m);
+    }
+    if (threadIdx.x < 4 && p0 + 32 * (int)threadIdx.x < N)
+        nz[(size_t)cb * nst + (p0 >> 5) + threadIdx.x] = any[threadIdx.x] ? 1 : 0;
+}
+
+// With a noise map the operand is L' sqrt(C^-1): the exponent of the largest
+// sqrt(C^-1) is added to every cell's bound (an upper bound of the product's).
+__global__ void __launch_bounds__(1024) k_oz_noise_exp(const GridState* __restrict__ gs,
+                                                       const double* __restrict__ cvec, int* __restrict__ emax)
+{
+    __shared__ int top;
+    if (threadIdx.x == 0) top = 0;
+    __syncthreads();
+    int e = 0;
+    for (int r = threadIdx.x; r < gs->N; r += blockDim.x) e = max(e, oz_exponent(sqrt(cvec[r])));
+    atomicMax(&top, e);
+    __syncthreads();
+    const int add = top - 1022;                                // sqrt(C^-1) < 2^add
+    for (int c = threadIdx.x; c < gs->M; c += blockDim.x) {
+        const int m = emax[c];
+        if (m > 0 && m < 2047) emax[c] = (top >= 2047) ? 2047 : min(2046, max(1, m + add));
+    }
+}
+
+// The digits of 64 cells x 32 pixels of L'^T (sqrt(C^-1)): L' is read along the
+// cells (512-byte rows), transposed through shared memory as integers and
+// written along the pixels, 16 bytes a thread and digit.  Stages without a
+// nonzero in the cells' 128-row block are never loaded by the products, so they
+// are skipped.  14 bytes written per 8 read: memory bound.
+__global__ void __launch_bounds__(256) k_oz_slice(const GridState* __restrict__ gs, const double* __restrict__ L,
+                                                  int ldL, const double* __restrict__ cvec, int use_noise_map,
+                                                  const int* __restrict__ emax, const unsigned char* __restrict__ nz,
+                                                  int nst, int st0, __half* __restrict__ xs, int M128, int Kc)
+{
+    __shared__ unsigned long long sq[64][33];
+    const int N = gs->N, M = gs->M;
+    const int cb = blockIdx.y, st = st0 + blockIdx.x, p0 = st * 32;
+    const int ncb = (M + 63) / 64;
+    if (cb >= ((ncb + 1) & ~1) || p0 >= N) return;
+    const int other = cb ^ 1;
+    if (!((cb < ncb && nz[(size_t)cb * nst + st]) || (other < ncb && nz[(size_t)other * nst + st]))) return;
+    {
+        const int c = threadIdx.x & 63, q = threadIdx.x >> 6;
+        const int cell = cb * 64 + c;
+        const int em = (cell < M) ? emax[cell] : 0;
+        #pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int k = q + 4 * u, r = p0 + k;
+            double x = 0;
+            if (cell < M && r < N) {
+                x = L[(size_t)r * ldL + cell];
+                if (use_noise_map && x != 0) x *= sqrt(cvec[r]);
+            }
+            sq[c][k] = oz_bias(em > 0 && em < 2047 ? oz_fixed(x, em) : 0);
+        }
+    }
+    __syncthreads();
+    const int c = threadIdx.x >> 2, k0 = (threadIdx.x & 3) * 8;
+    unsigned long long q[8];
+    #pragma unroll
+    for (int u = 0; u < 8; u++) q[u] = sq[c][k0 + u];
+    __half* out = xs + (size_t)(cb * 64 + c) * Kc + (size_t)blockIdx.x * 32 + k0;
+    #pragma unroll
+    for (int d = 0; d < OZ_S; d++) {
+        uint4 v;
+        v.x = oz_digits(q[0], q[1], d);
+        v.y = oz_digits(q[2], q[3], d);
+        v.z = oz_digits(q[4], q[5], d);
+        v.w = oz_digits(q[6], q[7], d);
+        *reinterpret_cast<uint4*>(out + (size_t)d * M128 * Kc) = v;
+    }
+}
+
+// What bounds it: the tensor pipe where a stage is live, 28 digit products of
+// 128 x 64 x 32 each (an N = 64 MMA reads 6 KB of shared memory per 32 clocks of
+// arithmetic, so it runs at about two thirds of the pipe), and the reading of
+// the accumulators beside it.  The FP64 pipe's SYRK that it replaces (64x64
+// tiles, the same zero blocks skipped) was at 99 % of that pipe: F of 2,934
+// cells x 11,772 pixels 23.5 -> 1.10 ms, 738 x 6,220 4.29 -> 0.13 ms, 96 x 448
+// 0.48 -> 0.05 ms, everything of launch_syrk_fp64 included.
+// The digit products of one tile over its share of the chunk's live stages
+// (both blocks have a nonzero among the stage's 32 pixels): grid (tiles,
+// splits).  The tile's integers are added into `part` by 64-bit reductions, lanes
+// along the rows.
+__global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_syrk(const __grid_constant__ CUtensorMap map_a,
+                                                          const __grid_constant__ CUtensorMap map_b, GridState* gs,
+                                                          const unsigned char* __restrict__ nz, int nst, int st0,
+                                                          int st1, int M128, unsigned long long* __restrict__ part)
+{
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ OzPipe pipe;
+    __shared__ int n_live;
+    int I, j;
+    oz_tile(blockIdx.x, I, j);
+    const int ncb = (gs->M + 63) / 64;
+    if (j >= ncb || 2 * I >= ncb) return;
+    const unsigned char* fa = nz + (size_t)(2 * I) * nst;
+    const unsigned char* fb = (2 * I + 1 < ncb) ? fa + nst : fa;      // the block's second 64 rows, if there are any
+    const unsigned char* fj = nz + (size_t)j * nst;
+    const int e = min(st1, (gs->N + 31) >> 5);
+    if (threadIdx.x == 0) n_live = 0;
+    __syncthreads();
+    int cnt = 0;
+    for (int k = st0 + threadIdx.x; k < e; k += blockDim.x) cnt += ((fa[k] | fb[k]) & fj[k]) ? 1 : 0;
+    if (cnt) atomicAdd(&n_live, cnt);
+    __syncthreads();
+    const int total = n_live;
+    const int s0 = (int)((long long)total * blockIdx.y / gridDim.y);
+    const int n = (int)((long long)total * (blockIdx.y + 1) / gridDim.y) - s0;     // this CTA's live stages
+    if (n == 0) return;
+
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    oz_begin(pipe);
+    long long hi[32];
+    int lo[32];
+    bool ok = true;
+    if (warp == OZ_EPI) {
+        // TMA: 32 stages' flags at a time, the live ones in order
+        int seen = 0, it = 0;
+        bool good = true;
+        for (int k0 = st0; k0 < e && it < n && good; k0 += 32) {
+            const int k = k0 + lane;
+            unsigned live = __ballot_sync(0xffffffffu, k < e && ((fa[k] | fb[k]) & fj[k]));
+            const int c = __popc(live);
+            if (seen + c <= s0) { seen += c; continue; }
+            for (; live && it < n; live &= live - 1) {
+                if (seen++ < s0) continue;
+                const int st = k0 + __ffs(live) - 1;
+                if (lane == 0) {
+                    good = good && oz_load_stage(pipe, smem, it, &map_a, &map_b, M128, (st - st0) * 32, I * OZ_TM,
+                                                 j * OZ_TN);
+                    if (good) pipe.n_issued = it + 1;
+                }
+                it++;
+            }
+            good = __shfl_sync(0xffffffffu, good, 0);
+        }
+    } else if (warp == OZ_EPI + 1) {
+        if (lane == 0) oz_mma_loop(pipe, smem, n);
+    } else {
+        #pragma unroll
+        for (int c = 0; c < 32; c++) hi[c] = lo[c] = 0;
+        ok = oz_accumulate(pipe, n, hi, lo);
+    }
+    __syncwarp();
+    oz_end(pipe);
+    if (pipe.abort) {
+        if (threadIdx.x == 0) atomicExch(&gs->status, QLP_ERR_TIMEOUT);
+        return;
+    }
+    if (warp < OZ_EPI && ok) {
+        unsigned long long* out = part + (size_t)blockIdx.x * 2 * OZ_TM * OZ_TN + (size_t)(warp >> 2) * 32 * OZ_TM +
+                                  (warp & 3) * 32 + lane;
+        #pragma unroll
+        for (int c = 0; c < 32; c++) {
+            atomicAdd(out + c * OZ_TM, (unsigned long long)hi[c]);
+            atomicAdd(out + OZ_TM * OZ_TN + c * OZ_TM, (unsigned long long)lo[c]);
+        }
+    }
+}
+
+// F from the integers: (hi 2^24 + lo) 2^(Ea + Eb - 60) times the uniform C^-1,
+// and the integers set back to zero.  A CTA takes 32 columns of a tile, through
+// shared memory so that both sides move whole rows.
+__global__ void __launch_bounds__(256) k_oz_finish(const GridState* __restrict__ gs,
+                                                   unsigned long long* __restrict__ part,
+                                                   const int* __restrict__ emax, double scale,
+                                                   double* __restrict__ F, int ldF)
+{
+    __shared__ double s[32][OZ_TM + 1];
+    int I, j;
+    oz_tile(blockIdx.x >> 1, I, j);
+    const int h = blockIdx.x & 1;
+    const int M = gs->M, Mp = (M + 63) & ~63;
+    if (I * OZ_TM >= Mp || j * OZ_TN >= Mp) return;
+    unsigned long long* in = part + (size_t)(blockIdx.x >> 1) * 2 * OZ_TM * OZ_TN + (size_t)h * 32 * OZ_TM;
+    const int r = threadIdx.x & 127, a = I * OZ_TM + r;
+    const double sa = (a < M) ? oz_scale(emax[a]) : 0.0;
+    for (int c = threadIdx.x >> 7; c < 32; c += 2) {
+        const long long hi = (long long)in[c * OZ_TM + r], lo = (long long)in[OZ_TM * OZ_TN + c * OZ_TM + r];
+        in[c * OZ_TM + r] = 0;
+        in[OZ_TM * OZ_TN + c * OZ_TM + r] = 0;
+        const int b = j * OZ_TN + h * 32 + c;
+        const double sb = (b < M) ? oz_scale(emax[b]) : 0.0;
+        // 2^-60 split over the two scales' products: no overflow on the way
+        s[c][r] = ((fma((double)hi, 16777216.0, (double)lo) * 0x1p-60 * sa) * sb) * scale;
+    }
+    __syncthreads();
+    const int c = threadIdx.x & 31;
+    for (int row = threadIdx.x >> 5; row < OZ_TM; row += 8)
+        if (I * OZ_TM + row < Mp) F[(size_t)(I * OZ_TM + row) * ldF + j * OZ_TN + h * 32 + c] = s[c][row];
+}
+
+void oz_free(OzWork* z)
+{
+    if (!z) return;
+    void* ptrs[] = {z->xs, z->part, z->emax, z->nz};
+    for (void* p : ptrs) if (p) cudaFree(p);
+    delete z;
+}
+
+// Workspace for N_cap image pixels and M_cap source cells.
+int oz_alloc(OzWork** out, int N_cap, int M_cap)
+{
+    OzWork* z = new OzWork();
+    z->M128 = (M_cap + OZ_TM - 1) / OZ_TM * OZ_TM;
+    const int nI = z->M128 / OZ_TM;
+    z->ntiles = nI * (nI + 1);
+    z->nst = (std::max(N_cap, 1) + 31) / 32;
+    const int fit = (int)std::min<size_t>(1u << 20, OZ_CHUNK_BYTES / ((size_t)OZ_S * 2 * z->M128)) / 128 * 128;
+    z->Kc = std::min(z->nst * 32, std::max(128, fit));
+    cudaError_t e = cudaSuccess;
+    auto A = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes); };
+    const size_t pbytes = (size_t)z->ntiles * 2 * OZ_TM * OZ_TN * sizeof(long long);
+    A((void**)&z->xs, (size_t)OZ_S * z->M128 * z->Kc * sizeof(__half));
+    A((void**)&z->part, pbytes);
+    A((void**)&z->emax, sizeof(int) * z->M128);
+    A((void**)&z->nz, (size_t)(z->M128 / 64) * z->nst);
+    if (e == cudaSuccess) e = cudaMemset(z->part, 0, pbytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_oz_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
+    int rc = QLP_OK;
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_error("%s (%d)", "FP64 contraction workspace", (int)e);
+        rc = (e == cudaErrorMemoryAllocation) ? QLP_ERR_NOMEM : QLP_ERR_CUDA;
+    } else if (make_map_box(&z->map_a, z->xs, (size_t)OZ_S * z->M128, z->Kc, true, OZ_TM, OZ_KS) != QLP_OK ||
+               make_map_box(&z->map_b, z->xs, (size_t)OZ_S * z->M128, z->Kc, true, OZ_TN, OZ_KS) != QLP_OK) {
+        set_error("%s (%d)", "cuTensorMapEncodeTiled unavailable or failed", 0);
+        rc = QLP_ERR_CUDA;
+    }
+    if (rc != QLP_OK) { oz_free(z); return rc; }
+    *out = z;
+    return QLP_OK;
+}
+
+void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st)
+{
+    OzWork* z = w.oz;
+    const int nI = (M_max + OZ_TM - 1) / OZ_TM, tiles = nI * (nI + 1), ncb = 2 * nI;
+    int n = 0;
+    cudaMemsetAsync(z->emax, 0, sizeof(int) * z->M128, st);
+    if (N_max > 0) {
+        k_oz_scan<<<dim3((N_max + 127) / 128, ncb), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, z->emax, z->nz, z->nst);
+        n++;
+        if (sd.use_noise_map) {
+            k_oz_noise_exp<<<1, 1024, 0, st>>>(w.gs, w.cvec, z->emax);
+            n++;
+        }
+    }
+    const int nst = (N_max + 31) / 32, per = z->Kc / 32;
+    for (int s0 = 0; s0 < nst; s0 += per) {
+        const int cnt = std::min(per, nst - s0);
+        // pixels split so that a small problem's few tiles still fill the GPU,
+        // but no finer than one read of the accumulators per CTA
+        const int split = std::max(1, std::min({(OZ_WANT_CTAS + tiles - 1) / tiles, (cnt + OZ_FLUSH - 1) / OZ_FLUSH,
+                                                64}));
+        k_oz_slice<<<dim3(cnt, ncb), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, w.cvec, sd.use_noise_map, z->emax, z->nz,
+                                                   z->nst, s0, z->xs, z->M128, z->Kc);
+        k_oz_syrk<<<dim3(tiles, split), OZ_THREADS, OZ_SMEM, st>>>(z->map_a, z->map_b, w.gs, z->nz, z->nst, s0,
+                                                                   s0 + cnt, z->M128, z->part);
+        n += 2;
+    }
+    k_oz_finish<<<2 * tiles, 256, 0, st>>>(w.gs, z->part, z->emax, sd.use_noise_map ? 1.0 : sd.cov_inverse, w.F,
+                                           w.ldF);
+    count_launches(n + 1);
+}
+
+}  // namespace qlpix

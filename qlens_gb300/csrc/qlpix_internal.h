@@ -158,6 +158,8 @@ __device__ __forceinline__ SrcOpts eval_grid(SrcOpts o, const StaticData& s)
 }
 #endif
 
+struct OzWork;
+
 // Per-evaluation device workspace (sized for the largest case at creation).
 struct Work {
     double* spx;  double* spy;         // n_sub source points
@@ -174,8 +176,7 @@ struct Work {
     int* Lidx;    double* Lval;        // pre-PSF L, CSR
     int* cidx;    double* cval; int* ccnt;   // compressed rows (duplicates summed), same capacity
     double* Lpsf;                      // N x ldL, FP64
-    unsigned char* lnz;                // plain path: nonzero flags of L' per (64-column block, 16-row chunk)
-    int lnz_chunks;                    // row chunks per column block in lnz
+    OzWork* oz;                        // plain path: workspace of the FP64 contraction (ozaki.cu)
     int ldL;                           // leading dimension of Lpsf (>= M_max)
     double* dvec; double* cvec;        // N: data and C^-1 per active row
     double* D;                         // M
@@ -219,6 +220,8 @@ void op_conv(const StaticData& sd, Work& w, int N_cap, bool transpose, const dou
 void launch_dvec(const StaticData& sd, Work& w, int N_max, cudaStream_t st);
 void launch_D(Work& w, int N_max, int M_max, cudaStream_t st);
 void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st);
+int oz_alloc(OzWork** out, int N_cap, int M_cap);
+void oz_free(OzWork* z);
 // parts: REG_F adds lambda R to F, REG_R writes R (both: the plain evaluation)
 #define REG_F 1
 #define REG_R 2
