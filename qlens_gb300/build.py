@@ -29,6 +29,7 @@ UNITS = [
     ("psf.cu", ["--fmad=false"]),
     ("linalg.cu", []),
     ("ozaki.cu", []),
+    ("cholfp64.cu", []),
     ("sparseops.cu", []),
     ("noalloc.cu", []),
     ("mixed.cu", []),

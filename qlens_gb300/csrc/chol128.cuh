@@ -550,18 +550,6 @@ __global__ void __launch_bounds__(128, 3) k_chol_upd16(const __grid_constant__ C
 // single-pass GPU scans), and every wait is bounded by ~1 s of %globaltimer,
 // after which the CTA raises QLP_ERR_TIMEOUT and stops.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int ld_acquire(const int* p)
-{
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release(int* p, int v)
-{
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 // Thread 0 waits until flags[j] is set, then counts how many of the flags
 // j .. jend-1 are set in a row; the count (0 on timeout) is broadcast.
 __device__ __forceinline__ int wait_ready(const int* flags, int j, int jend, int step, GridState* gs, int* sh)

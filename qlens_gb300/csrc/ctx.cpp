@@ -12,7 +12,6 @@
 namespace qlpix {
 
 void psf_init_attributes();
-void linalg_init_attributes();
 void sparseops_init_attributes();
 void sur_exact_init_attributes();
 
@@ -50,6 +49,8 @@ static void free_work(Work& w)
                     w.dvec, w.cvec, w.D, w.F, w.R, w.s, w.tmp, w.model, w.partial, w.linv, w.gs, w.out, w.ep,
                     w.fb_ray, w.fb_xy, w.fb_count, w.F0, w.gpart, w.gpart_cnt, w.cpart, w.sur_eps, w.xlist, w.xcount, w.nfw_xy};
     for (void* p : ptrs) if (p) cudaFree(p);
+    chol64_free(w.cholF);
+    chol64_free(w.cholR);
     oz_free(w.oz);
     memset(&w, 0, sizeof(w));
 }
@@ -135,6 +136,14 @@ static int ensure_fp64_mats(Slot& s)
     }
     if (!s.w.oz) {
         const int r = oz_alloc(&s.w.oz, s.N_cap, s.M_cap);
+        if (r != QLP_OK) return r;
+    }
+    if (!s.w.cholF) {
+        const int r = chol64_alloc(&s.w.cholF, s.M_cap, oz_buffer(s.w.oz));
+        if (r != QLP_OK) return r;
+    }
+    if (!s.w.cholR) {
+        const int r = chol64_alloc(&s.w.cholR, s.M_cap, nullptr);
         if (r != QLP_OK) return r;
     }
     if (!s.w.F) CK(dalloc(&s.w.F, (size_t)s.M_cap * s.M_cap), "alloc F");
@@ -238,7 +247,6 @@ int ctx_init(qlp_ctx* c, const qlp_image* im, const qlp_psf* psf, const qlp_srcg
     so.regparam = opts->regparam;
 
     psf_init_attributes();
-    linalg_init_attributes();
     sparseops_init_attributes();
     sur_exact_init_attributes();
     int snx = std::max(so.snx, 2), sny = std::max(so.sny, 2);
@@ -298,6 +306,13 @@ static bool model_has_nfw(const qlp_ctx* c)
     return false;
 }
 
+// CTAs of one factorisation on the plain path: the whole GPU for an evaluation
+// alone, its share in a batch.  A CTA holds its SM while it waits, so the
+// factorisations in flight must fit side by side; at least 8 each, so that the
+// digit products (~25 SM ms at 3,000 cells) stay within the chain of pivot
+// blocks (~4 ms).
+static int chol64_ctas(const qlp_ctx* c) { return std::max(8, 148 / std::max(1, c->in_flight)); }
+
 // The launch sequence of one evaluation on stream st with the workspace of
 // `slot`; sd / so size the launches (the evaluation's own mask and source
 // grid, or the slot's capacity when the sequence is captured for replay).
@@ -327,7 +342,7 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             cudaMemsetAsync(&w.gs->not_spd_F, 0, sizeof(int), st);
             cudaMemcpyAsync(w.F, w.F0, bytes, cudaMemcpyDeviceToDevice, st);
             launch_regularization(so, w, Mc, regp, REG_F, st);
-            launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, w.linv, st);
+            launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, Mc, chol64_ctas(c), w.cholF, w.linv, st);
             launch_logdet(w.F, w.ldF, Mc, w, 0, st);
             launch_solve_fp64(w, Mc, st);
         }
@@ -375,6 +390,18 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
     } else {
         int r = ensure_fp64_mats(slot);
         if (r != QLP_OK) return r;
+        if (so.regularization) {
+            // R hangs on the active cells alone: its log det runs on the slot's
+            // second stream beside L', F and F's factor.  R couples a cell to
+            // cells at most two grid rows (2 snx active indices) away, so its
+            // factor stays within that band (dense it cost as much as F's).
+            cudaEventRecord(slot.side_fork, st);
+            cudaStreamWaitEvent(slot.side, slot.side_fork, 0);
+            launch_regularization(so, w, Mc, regp, REG_R, slot.side);
+            launch_cholesky_fp64(w.R, w.ldF, Mc, w.gs, 1, 2 * so.snx, 4, w.cholR, nullptr, slot.side);
+            launch_logdet(w.R, w.ldF, Mc, w, 1, slot.side);
+            cudaEventRecord(slot.side_join, slot.side);
+        }
         launch_psf(sd, so, w, Mc, st);
         launch_D(w, N_max, Mc, st);
         if (ev) cudaEventRecord(ev[3], st);
@@ -382,15 +409,15 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
         if (ev) cudaEventRecord(ev[4], st);
         if (part == PIPE_PRE)
             cudaMemcpyAsync(w.F0, w.F, sizeof(double) * (size_t)w.ldF * Mc, cudaMemcpyDeviceToDevice, st);
-        launch_regularization(so, w, Mc, regp, part == PIPE_PRE ? REG_R : (REG_F | REG_R), st);
-        if (so.regularization) {
-            launch_cholesky_fp64(w.R, w.ldF, Mc, w.gs, 1, w.linv, st);
-            launch_logdet(w.R, w.ldF, Mc, w, 1, st);
+        if (part == PIPE_PRE) {
+            if (so.regularization) cudaStreamWaitEvent(st, slot.side_join, 0);
+            return QLP_OK;
         }
-        if (part == PIPE_PRE) return QLP_OK;
-        launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, w.linv, st);
+        launch_regularization(so, w, Mc, regp, REG_F, st);
+        launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, Mc, chol64_ctas(c), w.cholF, w.linv, st);
         launch_logdet(w.F, w.ldF, Mc, w, 0, st);
         launch_solve_fp64(w, Mc, st);
+        if (so.regularization) cudaStreamWaitEvent(st, slot.side_join, 0);
     }
     if (ev) cudaEventRecord(ev[5], st);
     launch_model_chi2(sd, so, w, N_max, Mc, regp, st, mixed);
@@ -478,8 +505,8 @@ static int issue_eval(qlp_ctx* c, Slot& s, const StaticData& sd, const SrcOpts& 
         SrcOpts soc = so;
         soc.snx = s.snx_cap;
         soc.sny = s.sny_cap;
-        const int key[7] = {c->precision, s.N_cap, s.snx_cap, s.sny_cap, model_has_nfw(c) ? 1 : 0, c->nfw_mode,
-                            part};
+        const int key[7] = {c->precision | chol64_ctas(c) << 8, s.N_cap, s.snx_cap, s.sny_cap, model_has_nfw(c) ? 1 : 0,
+                            c->nfw_mode, part};
         const bool trial = (part == PIPE_TRIAL);
         const cudaGraphExec_t have = trial ? s.graph_trial : s.graph;
         const int* have_key = trial ? s.trial_key : s.graph_key;
@@ -610,6 +637,7 @@ int ctx_eval(qlp_ctx* c, const double* lens_params, double regparam, qlp_result*
     ep.regparam = (regparam > 0) ? regparam : c->opts.regparam;
     ep.shape = InstShape{c->sd.mpix, c->sd.n_mask, c->sd.n_sub, c->so.snx, c->so.sny};
     Slot& s = c->slots[0];
+    c->in_flight = 1;
     long long l0 = kernel_launch_counter();
     cudaStream_t st = c->stream;
     CK(cudaEventRecord(c->fork, st), "event");
@@ -718,6 +746,7 @@ int ctx_eval_batch(qlp_ctx* c, const double* params, const double* regparams, co
             break;
         }
     }
+    c->in_flight = S;
     int r = ensure_results(c, n);
     if (r != QLP_OK) return r;
     const bool timed = !c->use_graphs && !(c->regopt && c->so.regularization);  // stage events: direct launches

@@ -1,6 +1,5 @@
 // linalg.cu -- FP64 dense algebra of the inversion:
-//   D = L'^T C^-1 d, curvature R and F += lambda R (F = L'^T C^-1 L' itself: ozaki.cu),
-//   blocked Cholesky of F and R, log det, the two triangular solves, the
+//   D = L'^T C^-1 d, curvature R and F += lambda R, log det, the
 //   model image, chi^2, s^T R s and the final -2 log(evidence).
 // Reference: QLens::create_lensing_matrices_from_Lmatrix_dense
 // (pixelgrid.cpp:15590-15736), add_regularization_term_to_dense_Fmatrix
@@ -148,31 +147,11 @@ void launch_regularization(const SrcOpts& so, Work& w, int M_max, const double* 
     (void)M_max;
 }
 
-// ---- Cholesky, log det and solve: the templates of chol.cuh in FP64 ----
-// Attributes are per translation unit: each .cu has its own instance of a
-// kernel template, so mixed.cu sets those of its float instances itself.
-void linalg_init_attributes()
-{
-    solve_init_attributes<double>();
-}
-
-
-int launch_cholesky_fp64(double* A, int ld, int M_max, const GridState* gs, int which, double* linv, cudaStream_t st)
-{
-    return launch_cholesky_t<double>(A, ld, M_max, gs, which, st, linv);
-}
-
+// ---- log det of a factor (the factorisations and solves: cholfp64.cu) ----
 void launch_logdet(const double* A, int ld, int M_max, Work& w, int which, cudaStream_t st)
 {
     (void)M_max;
     k_logdet_t<double><<<1, 1024, 0, st>>>(A, ld, w.gs, w.out, which);
-    count_launches(1);
-}
-
-void launch_solve_fp64(Work& w, int M_max, cudaStream_t st)
-{
-    (void)M_max;
-    k_solve_t<double><<<1, 1024, solve_smem_bytes<double>(w.ldF), st>>>(w.F, w.ldF, w.linv, w.gs, w.D, w.s, w.ldF);
     count_launches(1);
 }
 

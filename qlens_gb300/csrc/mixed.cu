@@ -6,7 +6,7 @@
 //            per CTA, exact fixed-point sums), split into TF32 hi + lo  k_psf_x
 //   F32    = X X^T on tcgen05 (block-sparse over pixel blocks)   k_syrk_tc
 //   F32   += lambda R, R32 = R                                  k_reg32
-//   L_F L_F^T = F32, L_R L_R^T = R32 (FP32 blocked Cholesky)    chol.cuh
+//   L_F L_F^T = F32, L_R L_R^T = R32 (FP32 blocked Cholesky)    chol128.cuh
 //   log det F, log det R: 2 sum log diag, accumulated in FP64
 //   D = L^T P^T (C^-1 d)                     (FP64; L^T from L by source cell)
 //   s = F32^-1 D, then `refine` times: r = D - L^T P^T C^-1 P L s - lambda R s (FP64),

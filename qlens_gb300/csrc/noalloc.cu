@@ -11,7 +11,7 @@
 //
 // This is the dense inversion step of the likelihood (the FP64 Cholesky,
 // log det and triangular solves that qlp_eval runs on F, see linalg.cu and
-// chol.cuh) fused into one single-block kernel that works on a copy of F in
+// cholfp64.cu) fused into one single-block kernel that works on a copy of F in
 // the static scratch instead of an allocated workspace.
 #include <cuda_runtime.h>
 #include <mutex>

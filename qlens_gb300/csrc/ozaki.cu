@@ -11,6 +11,8 @@
 
 namespace qlpix {
 
+#define OZ_S 7                      // digits of L' (54 bits)
+
 // Digits of L' kept at a time: a larger L' goes in chunks of image pixels, the
 // integer sums of the chunks adding up.
 #define OZ_CHUNK_BYTES ((size_t)1 << 30)
@@ -120,7 +122,7 @@ __global__ void __launch_bounds__(256) k_oz_slice(const GridState* __restrict__ 
                 x = L[(size_t)r * ldL + cell];
                 if (use_noise_map && x != 0) x *= sqrt(cvec[r]);
             }
-            sq[c][k] = oz_bias(em > 0 && em < 2047 ? oz_fixed(x, em) : 0);
+            sq[c][k] = oz_bias<OZ_S>(em > 0 && em < 2047 ? oz_fixed54(x, em) : 0);
         }
     }
     __syncthreads();
@@ -131,12 +133,7 @@ __global__ void __launch_bounds__(256) k_oz_slice(const GridState* __restrict__ 
     __half* out = xs + (size_t)(cb * 64 + c) * Kc + (size_t)blockIdx.x * 32 + k0;
     #pragma unroll
     for (int d = 0; d < OZ_S; d++) {
-        uint4 v;
-        v.x = oz_digits(q[0], q[1], d);
-        v.y = oz_digits(q[2], q[3], d);
-        v.z = oz_digits(q[4], q[5], d);
-        v.w = oz_digits(q[6], q[7], d);
-        *reinterpret_cast<uint4*>(out + (size_t)d * M128 * Kc) = v;
+        *reinterpret_cast<uint4*>(out + (size_t)d * M128 * Kc) = oz_digits8<OZ_S>(q, d);
     }
 }
 
@@ -182,7 +179,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_syrk(const __grid_constant
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     oz_begin(pipe);
     long long hi[32];
-    int lo[32];
+    uint32_t lo[32];
     bool ok = true;
     if (warp == OZ_EPI) {
         // TMA: 32 stages' flags at a time, the live ones in order
@@ -197,7 +194,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_syrk(const __grid_constant
                 if (seen++ < s0) continue;
                 const int st = k0 + __ffs(live) - 1;
                 if (lane == 0) {
-                    good = good && oz_load_stage(pipe, smem, it, &map_a, &map_b, M128, (st - st0) * 32, I * OZ_TM,
+                    good = good && oz_load_stage<OZ_S>(pipe, smem, it, &map_a, &map_b, M128, (st - st0) * 32, I * OZ_TM,
                                                  j * OZ_TN);
                     if (good) pipe.n_issued = it + 1;
                 }
@@ -206,11 +203,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_syrk(const __grid_constant
             good = __shfl_sync(0xffffffffu, good, 0);
         }
     } else if (warp == OZ_EPI + 1) {
-        if (lane == 0) oz_mma_loop(pipe, smem, n);
+        if (lane == 0) {
+            oz_mma_loop<OZ_S>(pipe, smem, 0, 0, n);
+            mma_commit(&pipe.done);
+        }
     } else {
         #pragma unroll
         for (int c = 0; c < 32; c++) hi[c] = lo[c] = 0;
-        ok = oz_accumulate(pipe, n, hi, lo);
+        ok = oz_accumulate<OZ_S>(pipe, 0, n, hi, lo);
     }
     __syncwarp();
     oz_end(pipe);
@@ -282,13 +282,14 @@ int oz_alloc(OzWork** out, int N_cap, int M_cap)
     cudaError_t e = cudaSuccess;
     auto A = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes); };
     const size_t pbytes = (size_t)z->ntiles * 2 * OZ_TM * OZ_TN * sizeof(long long);
-    A((void**)&z->xs, (size_t)OZ_S * z->M128 * z->Kc * sizeof(__half));
+    // the factorisation of F keeps its digits (eight of M128 columns) in the same buffer
+    A((void**)&z->xs, sizeof(__half) * (size_t)z->M128 * std::max(OZ_S * z->Kc, 8 * z->M128));
     A((void**)&z->part, pbytes);
     A((void**)&z->emax, sizeof(int) * z->M128);
     A((void**)&z->nz, (size_t)(z->M128 / 64) * z->nst);
     if (e == cudaSuccess) e = cudaMemset(z->part, 0, pbytes);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_oz_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
+        e = cudaFuncSetAttribute(k_oz_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, oz_smem(OZ_S));
     int rc = QLP_OK;
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -303,6 +304,9 @@ int oz_alloc(OzWork** out, int N_cap, int M_cap)
     *out = z;
     return QLP_OK;
 }
+
+// The digits' buffer, free once F stands.
+void* oz_buffer(OzWork* z) { return z->xs; }
 
 void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st)
 {
@@ -327,7 +331,7 @@ void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaS
                                                 64}));
         k_oz_slice<<<dim3(cnt, ncb), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, w.cvec, sd.use_noise_map, z->emax, z->nz,
                                                    z->nst, s0, z->xs, z->M128, z->Kc);
-        k_oz_syrk<<<dim3(tiles, split), OZ_THREADS, OZ_SMEM, st>>>(z->map_a, z->map_b, w.gs, z->nz, z->nst, s0,
+        k_oz_syrk<<<dim3(tiles, split), OZ_THREADS, oz_smem(OZ_S), st>>>(z->map_a, z->map_b, w.gs, z->nz, z->nst, s0,
                                                                    s0 + cnt, z->M128, z->part);
         n += 2;
     }

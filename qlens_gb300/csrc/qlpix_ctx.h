@@ -98,6 +98,7 @@ struct qlp_ctx {
     std::vector<cudaEvent_t> ev_pool;     // (QLP_N_STAGES+1) per batched instance
     qlpix::EvalParams* h_ep = nullptr;    // pinned, one per batch instance
     int h_ep_cap = 0;
+    int in_flight = 1;                    // evaluations in flight in the current call
     int use_graphs = 1;                   // batched evaluation replays captured graphs
     int refine = 1;                       // FP64 refinement sweeps of the mixed path's amplitudes
     // regularisation-parameter optimisation (QLens 'optimize_regparam on'):

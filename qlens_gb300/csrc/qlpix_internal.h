@@ -159,6 +159,7 @@ __device__ __forceinline__ SrcOpts eval_grid(SrcOpts o, const StaticData& s)
 #endif
 
 struct OzWork;
+struct Chol64Work;
 
 // Per-evaluation device workspace (sized for the largest case at creation).
 struct Work {
@@ -177,6 +178,7 @@ struct Work {
     int* cidx;    double* cval; int* ccnt;   // compressed rows (duplicates summed), same capacity
     double* Lpsf;                      // N x ldL, FP64
     OzWork* oz;                        // plain path: workspace of the FP64 contraction (ozaki.cu)
+    Chol64Work* cholF;  Chol64Work* cholR;  // plain path: workspaces of the factorisations (cholfp64.cu)
     int ldL;                           // leading dimension of Lpsf (>= M_max)
     double* dvec; double* cvec;        // N: data and C^-1 per active row
     double* D;                         // M
@@ -188,7 +190,7 @@ struct Work {
     double* partial;                   // reduction scratch
     double* gpart;  int* gpart_cnt;    // source-grid bounds: per-block partials (1024 blocks at most)
     int* cpart;                        // compaction: per-block counts (3 x 1025)
-    double* linv;                      // 64x64 inverse of the current diagonal Cholesky block
+    double* linv;                      // per 64 columns: inverse of the diagonal block of F's factor
     GridState* gs;
     EvalOut* out;                      // this slot's result (copied to the host after each evaluation)
     EvalParams* ep;                    // this slot's per-evaluation parameters
@@ -222,12 +224,15 @@ void launch_D(Work& w, int N_max, int M_max, cudaStream_t st);
 void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st);
 int oz_alloc(OzWork** out, int N_cap, int M_cap);
 void oz_free(OzWork* z);
+void* oz_buffer(OzWork* z);
+int chol64_alloc(Chol64Work** out, int M_cap, void* shared);
+void chol64_free(Chol64Work* z);
 // parts: REG_F adds lambda R to F, REG_R writes R (both: the plain evaluation)
 #define REG_F 1
 #define REG_R 2
 void launch_regularization(const SrcOpts& so, Work& w, int M_max, const double* regp, int parts, cudaStream_t st);
-int  launch_cholesky_fp64(double* A, int ld, int M_max, const GridState* gs, int which, double* linv,
-                          cudaStream_t st);
+void launch_cholesky_fp64(double* A, int ld, int M_max, GridState* gs, int which, int half_width, int ctas,
+                          Chol64Work* z, double* linv, cudaStream_t st);
 void launch_logdet(const double* A, int ld, int M_max, Work& w, int which, cudaStream_t st);
 void launch_solve_fp64(Work& w, int M_max, cudaStream_t st);
 void launch_model_chi2(const StaticData& sd, const SrcOpts& so, Work& w, int N_max, int M_max,

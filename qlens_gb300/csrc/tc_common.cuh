@@ -2,7 +2,8 @@
 // tensor-core kernels (tc_syrk.cuh, chol128.cuh, surrogate.cu): bounded
 // mbarrier waits (~1 s of %globaltimer), 2D TMA loads, K-major 128-byte
 // swizzled shared-memory descriptors, the kind::tf32 instruction descriptor,
-// MMA issue / commit, 32-column TMEM loads and the swizzled-tile offset.
+// MMA issue / commit, 32-column TMEM loads, acquire / release flags and the
+// swizzled-tile offset.
 #pragma once
 #include <cuda.h>
 #include "qlpix_internal.h"
@@ -147,6 +148,18 @@ __device__ __forceinline__ void tmem_ld_32cols(uint32_t taddr, float* v)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+
+__device__ __forceinline__ int ld_acquire(const int* p)
+{
+    int v;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void st_release(int* p, int v)
+{
+    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 
 __device__ __forceinline__ uint32_t sw128_offset(int row, int k)
 {
