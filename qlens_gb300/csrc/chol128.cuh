@@ -1,31 +1,32 @@
-// chol128.cuh -- FP32 blocked Cholesky with 128-wide steps for the mixed path.
+// chol128.cuh -- FP32 Cholesky of the mixed path, 128-column blocks, one launch
+// per matrix.
 //
-// Right-looking, one 128-column block per step k:
-//   k_potrf128       one CTA factors the 128x128 diagonal block in shared
-//                    memory (four 32-column panels: a warp factors the 32x32
-//                    diagonal piece in registers, the rows below are solved
-//                    one per thread, the trailing piece is updated with 4x4
-//                    register blocks) and inverts the factor (diagonal 32x32
-//                    inverses by forward substitution, off-diagonal blocks by
-//                    V_ij = -V_ii sum_k L_ik V_kj);
-//   k_chol_tile128   mode 1 (panel solve): P_I <- P_I L_kk^-T for the 128-row
-//                    blocks below, as 128x128x128 products on the tensor cores
-//                    (tcgen05 kind::tf32, 3xTF32 split, accumulator in TMEM),
-//                    K in four quarters of 32; its epilogue also writes each
-//                    solved block once as F16 hi + lo, each row scaled by a
-//                    power of two (its largest entry near 2^14), into the
-//                    panel buffer;
-//   k_chol_upd16     the trailing update A_IJ -= P_I P_J^T for the
-//                    lower-triangle tiles: TMA loads of the split panel
-//                    blocks (128-byte swizzle), tcgen05 kind::f16 at twice
-//                    the TF32 rate, three products (hi*hi + hi*lo + lo*hi,
-//                    ~22 significant bits), the scales undone in the
-//                    epilogue.  (mode 0 of k_chol_tile128 computes the same
-//                    update from the FP32 panel, re-split per tile.)
-// `band` limits both to the tiles within that many 128-blocks of the
-// diagonal: the curvature matrix R couples a cell only to cells at most two
-// grid rows away, so its factor stays inside that band (dense F passes a
-// band larger than the matrix).
+// Left-looking: CTAs take 128x128 tiles, column by column, from a counter.  A
+// tile (i, j) subtracts L_ik L_jk^T over the finished columns k < j: TMA loads of
+// the split factor (F16 hi + lo, each row of a block scaled by a power of two
+// near 2^14; 64-column boxes, 128-byte swizzle), three products hi*hi + hi*lo +
+// lo*hi of tcgen05 kind::f16 (~22 significant bits), the accumulators in two TMEM
+// buffers, each column block's product subtracted in FP32 registers with its
+// scales undone exactly while the next one's MMAs run.  Then
+//   i = j   the block is factored and inverted in shared memory (potrf128: four
+//           32-column panels, a warp's register Cholesky for the 32x32 piece, the
+//           rows below one per thread, the trailing piece in 4x4 register blocks;
+//           the inverse's 32x32 blocks by distance) and the inverse is published
+//           split into TF32 hi + lo;
+//   i > j   L_ij = A_ij L_jj^-T by 3xTF32 products with that inverse, published as
+//           F16 hi + lo for the tiles to come and in FP32 for the solves.
+// A tile waits by flags on tiles with a smaller number only, which are finished
+// or held by running CTAs, so any grid size works; every wait is bounded (~1 s).
+// The operations and their order are those of the right-looking version that
+// this replaces (three launches per step, 188 an evaluation at a capacity of
+// 4,096 cells, most of them empty for a smaller grid; every trailing tile read
+// and written once per step), so the results are the same but
+// for a last digit now and then.  Bound by the
+// chain of pivot blocks: 66 us a column, 46 of them the block (11 its inverse) and
+// 20 from its end to the next diagonal tile's start; 4,096 cells with the solves
+// 2.6 -> 2.0 ms.
+// `band`: blocks below the diagonal that can be nonzero: the curvature matrix R
+// couples a cell only to cells at most two grid rows away.
 // QLens factors with Cholesky_dcmp_packed (pixelgrid.cpp:17071-17105): a
 // negative pivot is recorded and sqrt(|d|) used; the first such pivot is
 // reported through GridState::not_spd_F / not_spd_R.
@@ -36,9 +37,11 @@
 namespace qlpix {
 
 #define C2 128
-#define P128_SMEM (2 * C2 * (C2 + 1) * 4 + 32 * 33 * 4 + C2 * 4)         // S, V, T, 1/diag
-#define T128_SMEM (4 * TC_TILE_BYTES + 1024)                             // [A/B][hi/lo], one K quarter
-#define U16_SMEM (4 * TC_TILE_BYTES + 1024)                              // [A/B][hi/lo], one K half (64 F16)
+#define C2_STAGES 3
+#define C2_STAGE_BYTES (4 * TC_TILE_BYTES)                // [A/B][hi/lo] of 64 columns
+#define C2_SMEM (C2_STAGES * C2_STAGE_BYTES + 1024)
+#define C2_EPI 8                                          // epilogue warps
+#define C2_THREADS (32 * (C2_EPI + 2))                    // + TMA and MMA warps
 
 __device__ __forceinline__ int cpad128(int M) { return (M + C2 - 1) / C2 * C2; }
 
@@ -51,68 +54,125 @@ __device__ __forceinline__ void tri_ij(int t, int& i, int& j)
 }
 
 // One step of the register Cholesky of a 32x32 block held one row per lane
-// (lane l: a[c] = L[l][c]); unrolled at compile time so a[] stays in registers.
+// (lane l: a[c] = L[l][c], entries right of the diagonal are not kept);
+// unrolled at compile time so a[] stays in registers.  The finished column
+// goes round through shared memory (buf: 2 x 32 floats, alternating), 128-bit
+// broadcasts; only the next pivot's factor comes by a shuffle, so that the
+// chain from pivot to pivot is two shuffles and an rsqrt (all of them by
+// shuffles had the shuffle unit bound it).
 template <int J>
-__device__ __forceinline__ void warp_chol32(float (&a)[32], int lane, int* flag, int pivot0)
+__device__ __forceinline__ void warp_chol32(float (&a)[32], int lane, int& bad, float* buf)
 {
     if constexpr (J < 32) {
         const float d = __shfl_sync(0xffffffffu, a[J], J);
-        if (lane == 0 && d < 0.f && *flag == 0) *flag = pivot0 + J + 1;
+        bad = (d < 0.f && bad == 0) ? J + 1 : bad;      // the first negative pivot
         const float rs = rsqrtf(fabsf(d));      // FP32 path: 1/sqrt and a multiply, not sqrt and a divide
-        if (lane == J) a[J] = fabsf(d) * rs;
-        else if (lane > J) a[J] = a[J] * rs;
+        a[J] = (lane == J ? fabsf(d) : a[J]) * rs;
+        if constexpr (J < 30) buf[(J & 1) * 32 + lane] = a[J];
+        if constexpr (J < 31) a[J + 1] -= a[J] * __shfl_sync(0xffffffffu, a[J], J + 1);
+        __syncwarp();
+        const float4* col = reinterpret_cast<const float4*>(buf + (J & 1) * 32);
         #pragma unroll
-        for (int c = J + 1; c < 32; c++) {
-            const float vc = __shfl_sync(0xffffffffu, a[J], c);
-            if (lane >= c) a[c] -= a[J] * vc;
+        for (int q = (J + 2) / 4; q < 8; q++) {
+            const float4 v = col[q];
+            if (4 * q > J + 1) a[4 * q] -= a[J] * v.x;
+            if (4 * q + 1 > J + 1) a[4 * q + 1] -= a[J] * v.y;
+            if (4 * q + 2 > J + 1) a[4 * q + 2] -= a[J] * v.z;
+            if (4 * q + 3 > J + 1) a[4 * q + 3] -= a[J] * v.w;
         }
-        warp_chol32<J + 1>(a, lane, flag, pivot0);
+        warp_chol32<J + 1>(a, lane, bad, buf);
     }
 }
 
-__global__ void __launch_bounds__(256, 1) k_potrf128(float* __restrict__ A, int ld, int k, GridState* gs, int which,
-                                                  float* __restrict__ Linv)
+// barrier of the first 256 threads
+__device__ __forceinline__ void c2_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
+__device__ __forceinline__ float2 split_tf32(float x)
 {
-    extern __shared__ float p128_smem[];
+    uint32_t h, l;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(x - __uint_as_float(h)));
+    return make_float2(__uint_as_float(h), __uint_as_float(l));
+}
+
+// The B x B block (i0, j0) of the lower triangle less the panel's product: S -= P P^T
+// over the 32 columns from c0.
+template <int B>
+__device__ __forceinline__ void potrf_trail(float (*S)[C2 + 1], int i0, int j0, int c0)
+{
+    float acc[B][B];
+    #pragma unroll
+    for (int u = 0; u < B; u++)
+        #pragma unroll
+        for (int v = 0; v < B; v++) acc[u][v] = 0.f;
+    #pragma unroll 8
+    for (int m = 0; m < 32; m++) {
+        float ra[B], rb[B];
+        #pragma unroll
+        for (int u = 0; u < B; u++) { ra[u] = S[i0 + u][c0 + m]; rb[u] = S[j0 + u][c0 + m]; }
+        #pragma unroll
+        for (int u = 0; u < B; u++)
+            #pragma unroll
+            for (int v = 0; v < B; v++) acc[u][v] += ra[u] * rb[v];
+    }
+    #pragma unroll
+    for (int u = 0; u < B; u++)
+        #pragma unroll
+        for (int v = 0; v < B; v++)
+            if (j0 + v <= i0 + u) S[i0 + u][j0 + v] -= acc[u][v];
+}
+
+// Inverse of the 32x32 diagonal block at b0 by one warp, lane = column.
+__device__ __forceinline__ void potrf_inv32(float (*S)[C2 + 1], float (*V)[C2 + 1], const float* rdiag, int b0, int lane)
+{
+    float x[32];
+    #pragma unroll
+    for (int i = 0; i < 32; i++) {
+        float acc = (i == lane) ? 1.f : 0.f;
+        #pragma unroll
+        for (int m = 0; m < i; m++) acc -= S[b0 + i][b0 + m] * x[m];
+        x[i] = (i < lane) ? 0.f : acc * rdiag[b0 + i];
+    }
+    #pragma unroll
+    for (int i = 0; i < 32; i++) V[b0 + i][b0 + lane] = x[i];
+}
+
+// The 128x128 block at the head of p128_smem (rows of 129, upper part zero),
+// factored and inverted by the first 256 threads; the inverse split into TF32
+// hi + lo goes to ih, il.  o: the block's first pivot (for the flag).
+// What bounds it is one SM's chain of 128 pivots and its shared-memory reads: a
+// warp factors each 32x32 piece in registers while the other warps update the
+// rest of the trailing block (it updates the next piece itself first), the
+// pieces' inverses run beside the row solves, and the inverse's off-diagonal
+// blocks are formed in 4x4 register blocks (one product per read had made them a
+// third of the time).  Each entry's operations and their order are those of the
+// plain blocked algorithm.
+__device__ __forceinline__ void potrf128(float* p128_smem, int o, int* flag, float* __restrict__ ih,
+                                         float* __restrict__ il)
+{
     float (*S)[C2 + 1] = reinterpret_cast<float (*)[C2 + 1]>(p128_smem);
     float (*V)[C2 + 1] = reinterpret_cast<float (*)[C2 + 1]>(p128_smem + C2 * (C2 + 1));
-    float* rdiag = p128_smem + 2 * C2 * (C2 + 1) + 32 * 33;   // 1 / L_ii (after a 32 x 33 scratch)
-    const int Mp = cpad128(gs->M);
-    const int o = k * C2;
-    if (o >= Mp) return;
+    float* rdiag = p128_smem + 2 * C2 * (C2 + 1);         // 1 / L_ii
+    float* buf = rdiag + C2;                              // warp 0's column buffer
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    {   // all 16 float4 loads of a thread in flight at once
-        float4 v[16];
+    auto factor32 = [&](int c0) {
+        float a[32];
         #pragma unroll
-        for (int u = 0; u < 16; u++) {
-            const int idx = tid + u * 256, r = idx >> 5, c = (idx & 31) * 4;
-            v[u] = *reinterpret_cast<const float4*>(A + (size_t)(o + r) * ld + o + c);
-        }
+        for (int c = 0; c < 32; c++) a[c] = S[c0 + lane][c0 + c];
+        int bad = 0;
+        warp_chol32<0>(a, lane, bad, buf);
+        if (lane == 0 && bad != 0 && *flag == 0) *flag = o + c0 + bad;
         #pragma unroll
-        for (int u = 0; u < 16; u++) {
-            const int idx = tid + u * 256, r = idx >> 5, c = (idx & 31) * 4;
-            S[r][c] = (c <= r) ? v[u].x : 0.f;
-            S[r][c + 1] = (c + 1 <= r) ? v[u].y : 0.f;
-            S[r][c + 2] = (c + 2 <= r) ? v[u].z : 0.f;
-            S[r][c + 3] = (c + 3 <= r) ? v[u].w : 0.f;
+        for (int c = 0; c < 32; c++) {
+            S[c0 + lane][c0 + c] = (c <= lane) ? a[c] : 0.f;
+            if (c == lane) rdiag[c0 + lane] = 1.0f / a[c];
         }
-    }
-    __syncthreads();
-    for (int p = 0; p < 4; p++) {
-        const int c0 = p * 32;
-        if (warp == 0) {
-            float a[32];
-            #pragma unroll
-            for (int c = 0; c < 32; c++) a[c] = S[c0 + lane][c0 + c];
-            warp_chol32<0>(a, lane, which ? &gs->not_spd_R : &gs->not_spd_F, o + c0);
-            #pragma unroll
-            for (int c = 0; c < 32; c++) S[c0 + lane][c0 + c] = (c <= lane) ? a[c] : 0.f;
-        }
-        __syncthreads();
-        const int t0 = c0 + 32, below = C2 - t0;
-        if (tid < 32) rdiag[c0 + tid] = 1.0f / S[c0 + tid][c0 + tid];
-        if (below == 0) break;
-        __syncthreads();
+    };
+    if (warp == 0) factor32(0);
+    c2_sync();
+    #pragma unroll 1
+    for (int p = 0; p < 3; p++) {
+        const int c0 = p * 32, t0 = c0 + 32, below = C2 - t0;
         if (tid < below) {                       // rows below: x L_pp^T = a
             const int r = t0 + tid;
             float x[32];
@@ -131,23 +191,55 @@ __global__ void __launch_bounds__(256, 1) k_potrf128(float* __restrict__ A, int 
             }
             #pragma unroll
             for (int c = 0; c < 32; c++) S[r][c0 + c] = x[c];
+        } else if (warp == 7) {
+            potrf_inv32(S, V, rdiag, c0, lane);
         }
-        __syncthreads();
+        c2_sync();
+        // trailing lower triangle: the next 32x32 piece in 2x2 blocks by four
+        // warps, then its factorisation in warp 0 while the others do the rest in
+        // 4x4 blocks
         const int nb = below / 4, nblk = nb * (nb + 1) / 2;
-        for (int b = tid; b < nblk; b += blockDim.x) {   // trailing lower triangle, 4x4 blocks
-            int bi, bj;
-            tri_ij(b, bi, bj);
-            const int i0 = t0 + 4 * bi, j0 = t0 + 4 * bj;
-            float acc[4][4];
+        if (warp < 4) {
+            for (int b = tid; b < 136; b += 128) {
+                int bi, bj;
+                tri_ij(b, bi, bj);
+                potrf_trail<2>(S, t0 + 2 * bi, t0 + 2 * bj, c0);
+            }
+            asm volatile("bar.sync 3, 128;" ::: "memory");
+        }
+        if (warp == 0) {
+            factor32(t0);
+        } else {
+            for (int b = 36 + 255 - tid; b < nblk; b += 224) {
+                int bi, bj;
+                tri_ij(b, bi, bj);
+                potrf_trail<4>(S, t0 + 4 * bi, t0 + 4 * bj, c0);
+            }
+        }
+        c2_sync();
+    }
+    // ---- off-diagonal blocks of V = L^-1 by distance d: V_ij = -V_ii (sum_{k=j}^{i-1} L_ik V_kj) ----
+    // The blocks of one distance depend only on nearer ones, so all of them are
+    // formed together.  The products sum_k L_ik V_kj go into the upper triangle
+    // of V (block (j, i)), which nothing reads as V; those of distance 1 do not
+    // need the last diagonal block's inverse, which is formed beside them.
+    #pragma unroll 1
+    for (int d = 1; d < 4; d++) {
+        const int jb = tid >> 6, ib = jb + d, r = (tid >> 1) & 28, c = (tid & 7) * 4;
+        const bool mine = tid < (4 - d) * 64;
+        float acc[4][4];
+        if (d == 1 && warp == 7) potrf_inv32(S, V, rdiag, 96, lane);
+        if (mine) {
             #pragma unroll
             for (int u = 0; u < 4; u++)
                 #pragma unroll
                 for (int v = 0; v < 4; v++) acc[u][v] = 0.f;
+            const int m1 = ib * 32;
             #pragma unroll 8
-            for (int m = 0; m < 32; m++) {
+            for (int m = jb * 32; m < m1; m++) {
                 float ra[4], rb[4];
                 #pragma unroll
-                for (int u = 0; u < 4; u++) { ra[u] = S[i0 + u][c0 + m]; rb[u] = S[j0 + u][c0 + m]; }
+                for (int u = 0; u < 4; u++) { ra[u] = S[ib * 32 + r + u][m]; rb[u] = V[m][jb * 32 + c + u]; }
                 #pragma unroll
                 for (int u = 0; u < 4; u++)
                     #pragma unroll
@@ -156,59 +248,57 @@ __global__ void __launch_bounds__(256, 1) k_potrf128(float* __restrict__ A, int 
             #pragma unroll
             for (int u = 0; u < 4; u++)
                 #pragma unroll
-                for (int v = 0; v < 4; v++)
-                    if (j0 + v <= i0 + u) S[i0 + u][j0 + v] -= acc[u][v];
+                for (int v = 0; v < 4; v++) V[jb * 32 + r + u][ib * 32 + c + v] = acc[u][v];
         }
-        __syncthreads();
+        c2_sync();
+        if (mine) {
+            #pragma unroll
+            for (int u = 0; u < 4; u++)
+                #pragma unroll
+                for (int v = 0; v < 4; v++) acc[u][v] = 0.f;
+            #pragma unroll 4
+            for (int m = 0; m < r + 4; m++) {    // (V_ii is zero above its diagonal)
+                float ra[4], rb[4];
+                #pragma unroll
+                for (int u = 0; u < 4; u++) { ra[u] = V[ib * 32 + r + u][ib * 32 + m]; rb[u] = V[jb * 32 + m][ib * 32 + c + u]; }
+                #pragma unroll
+                for (int u = 0; u < 4; u++)
+                    #pragma unroll
+                    for (int v = 0; v < 4; v++) acc[u][v] += ra[u] * rb[v];
+            }
+            #pragma unroll
+            for (int u = 0; u < 4; u++)
+                #pragma unroll
+                for (int v = 0; v < 4; v++) V[ib * 32 + r + u][jb * 32 + c + v] = -acc[u][v];
+        }
+        c2_sync();
     }
-    __syncthreads();                 // the last panel's 1/L_ii
+    // the inverse's split (upper part zero), which the tiles below wait for
+    #pragma unroll 4
+    for (int u = 0; u < 16; u++) {
+        const int idx = tid + u * 256, r = idx >> 5, c = (idx & 31) * 4;
+        float2 v[4];
+        #pragma unroll
+        for (int e = 0; e < 4; e++) v[e] = split_tf32(c + e <= r ? V[r][c + e] : 0.f);
+        *reinterpret_cast<float4*>(ih + (size_t)r * C2 + c) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+        *reinterpret_cast<float4*>(il + (size_t)r * C2 + c) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+    }
+}
+
+// What nothing in the factorisation waits for: the factor's block to A, its
+// inverse (row-major, upper part zero) and the inverse's transpose to Linv.
+__device__ __forceinline__ void potrf128_store(float* p128_smem, float* __restrict__ A, int ld, float* __restrict__ Linv)
+{
+    float (*S)[C2 + 1] = reinterpret_cast<float (*)[C2 + 1]>(p128_smem);
+    float (*V)[C2 + 1] = reinterpret_cast<float (*)[C2 + 1]>(p128_smem + C2 * (C2 + 1));
+    const int tid = threadIdx.x;
     #pragma unroll 4
     for (int u = 0; u < 16; u++) {   // the factor (upper part of the block zero)
         const int idx = tid + u * 256, r = idx >> 5, c = (idx & 31) * 4;
-        *reinterpret_cast<float4*>(A + (size_t)(o + r) * ld + o + c) =
+        *reinterpret_cast<float4*>(A + (size_t)r * ld + c) =
             make_float4(S[r][c], S[r][c + 1], S[r][c + 2], S[r][c + 3]);
     }
-    // ---- V = L^-1: diagonal 32x32 blocks, one warp each, lane j = column j ----
-    if (warp < 4) {
-        const int b0 = warp * 32, j = lane;
-        float x[32];
-        #pragma unroll
-        for (int i = 0; i < 32; i++) {
-            float acc = (i == j) ? 1.f : 0.f;
-            #pragma unroll
-            for (int m = 0; m < i; m++) acc -= S[b0 + i][b0 + m] * x[m];
-            x[i] = (i < j) ? 0.f : acc * rdiag[b0 + i];
-        }
-        #pragma unroll
-        for (int i = 0; i < 32; i++) V[b0 + i][b0 + j] = x[i];
-    }
-    __syncthreads();
-    // ---- off-diagonal blocks by distance d: V_ij = -V_ii (sum_{k=j}^{i-1} L_ik V_kj) ----
-    // The blocks of one distance depend only on nearer ones, so all of them
-    // are formed together: two barriers per distance instead of two per
-    // block, each sum in its old order.  The products sum_k L_ik V_kj go into
-    // the upper triangle of V (block (j, i)), which nothing reads as V.
-    for (int d = 1; d < 4; d++) {
-        const int nbk = 4 - d;
-        for (int e = tid; e < nbk * 32 * 32; e += blockDim.x) {
-            const int jb = e >> 10, r = (e >> 5) & 31, c = e & 31, ib = jb + d;
-            float acc = 0.f;
-            for (int kb = jb; kb < ib; kb++)
-                #pragma unroll 8
-                for (int m = 0; m < 32; m++) acc += S[ib * 32 + r][kb * 32 + m] * V[kb * 32 + m][jb * 32 + c];
-            V[jb * 32 + r][ib * 32 + c] = acc;
-        }
-        __syncthreads();
-        for (int e = tid; e < nbk * 32 * 32; e += blockDim.x) {
-            const int jb = e >> 10, r = (e >> 5) & 31, c = e & 31, ib = jb + d;
-            float acc = 0.f;
-            #pragma unroll 8
-            for (int m = 0; m <= r; m++) acc += V[ib * 32 + r][ib * 32 + m] * V[jb * 32 + m][ib * 32 + c];
-            V[ib * 32 + r][jb * 32 + c] = -acc;
-        }
-        __syncthreads();
-    }
-    // Linv (row-major, upper part zero) and its transpose right after it
+    if (Linv == nullptr) return;
     #pragma unroll 4
     for (int u = 0; u < 16; u++) {
         const int idx = tid + u * 256, r = idx >> 5, c = (idx & 31) * 4;
@@ -221,324 +311,363 @@ __global__ void __launch_bounds__(256, 1) k_potrf128(float* __restrict__ A, int 
     }
 }
 
-// One K quarter (32 columns from col) of 128 rows from g0, eight float4 per
-// thread, into registers ...
-__device__ __forceinline__ void load_quarter(const float* __restrict__ src, size_t lds, int g0, int col,
-                                             float4 (&vv)[8])
+struct Flow128 {
+    uint64_t full[C2_STAGES], empty[C2_STAGES];
+    uint64_t acc_full[2], acc_empty[2], exp_full[2];      // per accumulator buffer; exp: the rows' scales
+    uint64_t b_full, sol[2], done;
+    uint32_t tmem;
+    int n_issued, n_used, n_exp;                          // stages loaded / consumed, scales loaded
+    volatile int abort;
+};
+
+// Untiled bulk copy to shared memory (16-byte aligned, a multiple of 16 bytes).
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar)
 {
-    #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        const int idx = threadIdx.x + u * 128;
-        const int row = idx >> 3, q = idx & 7;
-        vv[u] = *reinterpret_cast<const float4*>(src + (size_t)(g0 + row) * lds + col + q * 4);
-    }
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
 }
 
-// ... then split into TF32 hi + lo and stored in the SW128 layout of one K block.
-__device__ __forceinline__ void store_split_quarter(const float4 (&vv)[8], unsigned char* t_hi, unsigned char* t_lo)
+__device__ __forceinline__ void c2_arrive(uint64_t* bar)
 {
-    #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        const int idx = threadIdx.x + u * 128;
-        const int row = idx >> 3, kcol = (idx & 7) * 4;
-        float x[4] = {vv[u].x, vv[u].y, vv[u].z, vv[u].w};
-        float h[4], l[4];
-        #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            uint32_t uu;
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(uu) : "f"(x[e]));
-            h[e] = __uint_as_float(uu);
-            const float lo = x[e] - h[e];
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(uu) : "f"(lo));
-            l[e] = __uint_as_float(uu);
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ bool c2_wait_flag(const int* p, GridState* gs, volatile int* abort_flag)
+{
+    if (ld_acquire(p)) return true;
+    const uint64_t t0 = globaltimer();
+    while (!ld_acquire(p)) {
+        if (*abort_flag || *(volatile int*)&gs->status == QLP_ERR_TIMEOUT || globaltimer() - t0 > TC_WAIT_NS) {
+            *abort_flag = 1;
+            return false;
         }
-        const uint32_t off = sw128_offset(row, kcol);
-        *reinterpret_cast<float4*>(t_hi + off) = make_float4(h[0], h[1], h[2], h[3]);
-        *reinterpret_cast<float4*>(t_lo + off) = make_float4(l[0], l[1], l[2], l[3]);
+        __nanosleep(32);
     }
+    return true;
 }
 
-// mode 0: A_IJ -= P_I P_J^T (grid: lower-triangle tiles of the first `band`
-// block rows below step k); mode 1: P_I <- P_I Linv^T (grid: block rows).
-// K runs in four quarters of 32 columns (the same MMAs in the same order as
-// one pass over 128), so a CTA needs 65 KB of shared memory and three fit on
-// an SM: while one waits on its loads, the others' MMAs run.  Each quarter's
-// global loads are issued while the previous quarter's MMAs run.
-__global__ void __launch_bounds__(128, 3) k_chol_tile128(float* __restrict__ A, int ld, int k, GridState* gs, int mode,
-                                                         const float* __restrict__ Linv, int band,
-                                                         __half* __restrict__ P_hi, __half* __restrict__ P_lo,
-                                                         int* __restrict__ pexp)
+// The factorisation's arrays: the split factor Lh, Ll [rows][rows] with each
+// column block's row scales pexp[block][rows], the split inverses [rows][128]
+// and the flags: ready[column][row block], inverse[column], tile counter.
+struct Flow128Mem {
+    __half* Lh;
+    __half* Ll;
+    int* pexp;
+    float* ih;
+    float* il;
+    int* flags;
+    int rows;                                             // M_cap, a multiple of 128
+};
+
+__global__ void __launch_bounds__(C2_THREADS, 1) k_chol128(const __grid_constant__ CUtensorMap map_hi,
+                                                          const __grid_constant__ CUtensorMap map_lo,
+                                                          const __grid_constant__ CUtensorMap map_ih,
+                                                          const __grid_constant__ CUtensorMap map_il, float* A, int ld,
+                                                          GridState* gs, int which, int band, Flow128Mem mem,
+                                                          float* Linv)
 {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t done_bar;
-    __shared__ uint32_t tmem_slot;
-    __shared__ volatile int abort_flag;
-    const int Mp = cpad128(gs->M);
-    const int base = (k + 1) * C2;
-    if (base >= Mp) return;
-    const int nt = (Mp - base) / C2;
-    int I, J = 0;
-    if (mode == 0) tri_ij(blockIdx.x, I, J);
-    else I = blockIdx.x;
-    if (I >= nt || I >= band) return;
-    const int r0 = base + I * C2, c0 = base + J * C2;
-    const int o = k * C2;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ Flow128 f;
+    __shared__ __align__(16) int exps[2][2][C2];          // [buffer][rows, columns] scales
+    __shared__ float rmax[2][C2];
+    __shared__ int ticket;
+    const int nb = cpad128(gs->M) / C2, nbc = mem.rows / C2;
+    int* ready = mem.flags;
+    int* inv = ready + (size_t)nbc * nbc;
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    auto tile = [&](int op, int part) { return smem + (op * 2 + part) * TC_TILE_BYTES; };
-
-    if (threadIdx.x == 0) {
-        mbar_init(&done_bar, 1);
-        abort_flag = 0;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < C2_STAGES; s++) { mbar_init(&f.full[s], 1); mbar_init(&f.empty[s], 1); }
+        for (int b = 0; b < 2; b++) {
+            mbar_init(&f.acc_full[b], 1);
+            mbar_init(&f.acc_empty[b], C2_EPI);
+            mbar_init(&f.exp_full[b], 1);
+            mbar_init(&f.sol[b], 1);
+        }
+        mbar_init(&f.b_full, 1);
+        mbar_init(&f.done, 1);
+        f.n_issued = f.n_used = f.n_exp = 0;
+        f.abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(128)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    bool ok = true;
-    float4 ra[8], rb[8];
-    load_quarter(A, (size_t)ld, r0, o, ra);
-    if (mode == 0) load_quarter(A, (size_t)ld, c0, o, rb);
-    else load_quarter(Linv, (size_t)C2, 0, 0, rb);
-    for (int qt = 0; qt < 4 && ok; qt++) {
-        store_split_quarter(ra, tile(0, 0), tile(0, 1));
-        store_split_quarter(rb, tile(1, 0), tile(1, 1));
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        if (warp == 1 && lane == 0) {
-            const uint32_t tmem = tmem_slot;
-            const uint32_t idesc = idesc_tf32_128x128();
-            const uint64_t a_hi = sdesc_sw128(smem_u32(tile(0, 0)));
-            const uint64_t a_lo = sdesc_sw128(smem_u32(tile(0, 1)));
-            const uint64_t b_hi = sdesc_sw128(smem_u32(tile(1, 0)));
-            const uint64_t b_lo = sdesc_sw128(smem_u32(tile(1, 1)));
-            #pragma unroll
-            for (int kk = 0; kk < TC_KB / 8; kk++) {
-                const uint64_t off = (uint64_t)((kk * 32) >> 4);
-                mma_tf32(tmem, a_hi + off, b_hi + off, idesc, (qt > 0 || kk > 0) ? 1u : 0u);
-                mma_tf32(tmem, a_hi + off, b_lo + off, idesc, 1u);
-                mma_tf32(tmem, a_lo + off, b_hi + off, idesc, 1u);
-            }
-            mma_commit(&done_bar);
-        }
-        // the next quarter's loads fly while the MMAs run
-        if (qt + 1 < 4) {
-            load_quarter(A, (size_t)ld, r0, o + (qt + 1) * 32, ra);
-            if (mode == 0) load_quarter(A, (size_t)ld, c0, o + (qt + 1) * 32, rb);
-            else load_quarter(Linv, (size_t)C2, 0, (qt + 1) * 32, rb);
-        }
-        __syncthreads();
-        // the MMAs read shared memory asynchronously: wait before it is reused
-        ok = mbar_wait_bounded(&done_bar, (uint32_t)(qt & 1), &abort_flag, false);
-        tc_fence_after();
-        __syncthreads();
-    }
-    const uint32_t tmem = tmem_slot;
-    const int row = r0 + warp * 32 + lane;
-    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-    const bool good = __syncthreads_and(ok && !abort_flag) != 0;
-    if (good && mode == 0) {
-        #pragma unroll 1
-        for (int c = 0; c < TC_TILE; c += 32) {
-            float v[32];
-            tmem_ld_32cols(trow + (uint32_t)c, v);
-            float* dst = A + (size_t)row * ld + c0 + c;
-            #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-                float4 a = *reinterpret_cast<float4*>(dst + i);
-                a.x -= v[i]; a.y -= v[i + 1]; a.z -= v[i + 2]; a.w -= v[i + 3];
-                *reinterpret_cast<float4*>(dst + i) = a;
-            }
-        }
-    } else if (good) {
-        // the solved block: FP32 into A, and F16 hi + lo of 2^s x each row (s
-        // puts the row's largest entry just below 2^14) into rows 128 I.. of
-        // the panel buffer, with s in pexp, for k_chol_upd16
-        float mx = 0.f;
-        #pragma unroll 1
-        for (int c = 0; c < TC_TILE; c += 32) {
-            float v[32];
-            tmem_ld_32cols(trow + (uint32_t)c, v);
-            #pragma unroll
-            for (int i = 0; i < 32; i++) mx = fmaxf(mx, fabsf(v[i]));
-        }
-        int e = 0;
-        frexpf(mx, &e);                      // mx < 2^e
-        // kept within [-60, 60] so that 2^-(s_i + s_j) is a normal float
-        const int sc = (mx > 0.f) ? max(-60, min(60, 14 - e)) : 0;
-        pexp[I * C2 + warp * 32 + lane] = sc;
-        const float scf = __int_as_float((127 + sc) << 23);
-        const size_t prow = (size_t)(I * C2 + warp * 32 + lane) * C2;
-        #pragma unroll 1
-        for (int c = 0; c < TC_TILE; c += 32) {
-            float v[32];
-            tmem_ld_32cols(trow + (uint32_t)c, v);
-            float* dst = A + (size_t)row * ld + o + c;
-            #pragma unroll
-            for (int i = 0; i < 32; i += 4)
-                *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-            uint32_t hw[16], lw[16];
-            #pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const float a = v[2 * i] * scf, b = v[2 * i + 1] * scf;
-                const __half ah = __float2half_rn(a), bh = __float2half_rn(b);
-                const __half al = __float2half_rn(a - __half2float(ah)), bl = __float2half_rn(b - __half2float(bh));
-                hw[i] = (uint32_t)__half_as_ushort(ah) | ((uint32_t)__half_as_ushort(bh) << 16);
-                lw[i] = (uint32_t)__half_as_ushort(al) | ((uint32_t)__half_as_ushort(bl) << 16);
-            }
-            uint4* ph = reinterpret_cast<uint4*>(P_hi + prow + c);
-            uint4* pl = reinterpret_cast<uint4*>(P_lo + prow + c);
-            #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                ph[q] = make_uint4(hw[4 * q], hw[4 * q + 1], hw[4 * q + 2], hw[4 * q + 3]);
-                pl[q] = make_uint4(lw[4 * q], lw[4 * q + 1], lw[4 * q + 2], lw[4 * q + 3]);
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (!good && threadIdx.x == 0) atomicExch(&gs->status, QLP_ERR_TIMEOUT);
-    if (warp == 0) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128) : "memory");
-    }
-}
-
-// The trailing update of step k, A_IJ -= P_I P_J^T over the lower-triangle
-// tiles of the first `band` block rows below the step, from the split panel
-// that k_chol_tile128 (mode 1) wrote: map_hi / map_lo address its F16 parts
-// ([M_cap rows][128], 64 x 128 boxes, 128-byte swizzle), pexp[row] the
-// power-of-two scale of each of its rows.
-// K = 128 runs in two halves of 64 (12 MMAs each) through one 64 KB buffer,
-// so three CTAs share an SM and overlap each other's loads, MMAs and
-// epilogues.
-__global__ void __launch_bounds__(128, 3) k_chol_upd16(const __grid_constant__ CUtensorMap map_hi,
-                                                       const __grid_constant__ CUtensorMap map_lo,
-                                                       float* __restrict__ A, int ld, int k, GridState* gs,
-                                                       const int* __restrict__ pexp, int band)
-{
-    extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t full_bar, done_bar;
-    __shared__ uint32_t tmem_slot;
-    __shared__ volatile int abort_flag;
-    const int Mp = cpad128(gs->M);
-    const int base = (k + 1) * C2;
-    if (base >= Mp) return;
-    const int nt = (Mp - base) / C2;
-    int I, J;
-    tri_ij(blockIdx.x, I, J);
-    if (I >= nt || I >= band) return;
-    const int r0 = base + I * C2, c0 = base + J * C2;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    auto tile = [&](int op, int part) { return smem + (op * 2 + part) * TC_TILE_BYTES; };
-    if (threadIdx.x == 0) {
-        mbar_init(&full_bar, 1);
-        mbar_init(&done_bar, 1);
-        abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(128)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&f.tmem)),
+                     "r"(512)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
-    bool ok = true;
-    int issued = 0, landed = 0;      // K halves whose loads were issued / seen complete (thread 0)
-    float4 cpre[8];                  // the next 32 columns of this thread's row of the target tile
-    for (int h = 0; h < 2; h++) {
-        if (threadIdx.x == 0 && !abort_flag) {
-            mbar_expect_tx(&full_bar, 4 * TC_TILE_BYTES);
-            tma_load_2d(&map_hi, &full_bar, tile(0, 0), h * 64, I * C2);
-            tma_load_2d(&map_lo, &full_bar, tile(0, 1), h * 64, I * C2);
-            tma_load_2d(&map_hi, &full_bar, tile(1, 0), h * 64, J * C2);
-            tma_load_2d(&map_lo, &full_bar, tile(1, 1), h * 64, J * C2);
-            issued++;
-            if (mbar_wait_bounded(&full_bar, (uint32_t)(h & 1), &abort_flag, false)) {
-                landed++;
-                tc_fence_after();
-                const uint32_t idesc = idesc_f16_128x128();
-                const uint64_t a_hi = sdesc_sw128(smem_u32(tile(0, 0)));
-                const uint64_t a_lo = sdesc_sw128(smem_u32(tile(0, 1)));
-                const uint64_t b_hi = sdesc_sw128(smem_u32(tile(1, 0)));
-                const uint64_t b_lo = sdesc_sw128(smem_u32(tile(1, 1)));
-                #pragma unroll
-                for (int kk = 0; kk < 4; kk++) {
-                    const uint64_t off = (uint64_t)((kk * 32) >> 4);     // 16 F16 = 32 bytes along K
-                    mma_f16(tmem, a_hi + off, b_hi + off, idesc, (h > 0 || kk > 0) ? 1u : 0u);
-                    mma_f16(tmem, a_hi + off, b_lo + off, idesc, 1u);
-                    mma_f16(tmem, a_lo + off, b_hi + off, idesc, 1u);
+    const uint32_t tmem = f.tmem;
+
+    int it0 = 0, kc0 = 0, nsol = 0;              // stages, column blocks and panel solves so far
+    int j = 0, base = 0;                         // the ticket's column; the tickets before that column
+    while (true) {
+        if (tid == 0) ticket = atomicAdd(inv + nbc, 1);
+        __syncthreads();
+        const int tk = ticket;
+        while (j < nb && tk >= base + min(nb - j, band + 1)) { base += min(nb - j, band + 1); j++; }
+        if (j >= nb || f.abort) break;           // uniform: f.abort is raised between the barriers below only
+        const int i = j + tk - base;
+        const bool diag = i == j;
+        const int k0 = max(0, i - band), nk = j - k0;
+        const int r = 32 * (warp & 3) + lane, h = (warp >> 2) & 1;       // an epilogue thread's row and column half
+        const int row = i * C2 + r;
+        float acc[64];
+        if (warp == C2_EPI) {
+            if (lane == 0) {
+                bool ok = true;
+                for (int k = k0; k < j && ok; k++) {
+                    const int kc = kc0 + k - k0, b = kc & 1;
+                    const int* rk = ready + (size_t)k * nbc;
+                    ok = c2_wait_flag(rk + i, gs, &f.abort) && (diag || c2_wait_flag(rk + j, gs, &f.abort)) &&
+                         (kc < 2 || mbar_wait_bounded(&f.acc_empty[b], ((kc >> 1) & 1) ^ 1, &f.abort));
+                    if (!ok) break;
+                    asm volatile("fence.proxy.async;" ::: "memory");
+                    const int* pe = mem.pexp + (size_t)k * mem.rows;
+                    mbar_expect_tx(&f.exp_full[b], 2 * C2 * 4);
+                    bulk_load(exps[b][0], pe + i * C2, C2 * 4, &f.exp_full[b]);
+                    bulk_load(exps[b][1], pe + j * C2, C2 * 4, &f.exp_full[b]);
+                    f.n_exp = kc + 1;
+                    for (int half = 0; half < 2 && ok; half++) {
+                        const int it = it0 + 2 * (k - k0) + half, s = it % C2_STAGES, x = k * C2 + half * 64;
+                        if (it >= C2_STAGES)
+                            ok = mbar_wait_bounded(&f.empty[s], ((it / C2_STAGES) & 1) ^ 1, &f.abort);
+                        if (!ok) break;
+                        unsigned char* st = smem + s * C2_STAGE_BYTES;
+                        mbar_expect_tx(&f.full[s], diag ? 2 * TC_TILE_BYTES : 4 * TC_TILE_BYTES);
+                        tma_load_2d(&map_hi, &f.full[s], st, x, i * C2);
+                        tma_load_2d(&map_lo, &f.full[s], st + TC_TILE_BYTES, x, i * C2);
+                        if (!diag) {
+                            tma_load_2d(&map_hi, &f.full[s], st + 2 * TC_TILE_BYTES, x, j * C2);
+                            tma_load_2d(&map_lo, &f.full[s], st + 3 * TC_TILE_BYTES, x, j * C2);
+                        }
+                        f.n_issued = it + 1;
+                    }
                 }
             }
-            mma_commit(&done_bar);
-        }
-        __syncthreads();
-        // (before the last half's MMAs are waited for, each thread's first
-        // 32 columns of the target tile are loaded: their latency overlaps the MMAs)
-        if (h == 1) {
-            const float* src = A + (size_t)(r0 + warp * 32 + lane) * ld + c0;
+            __syncwarp();
+        } else if (warp == C2_EPI + 1) {
+            if (lane == 0) {
+                const uint32_t idesc = idesc_f16_128x128();
+                int n = 0;
+                bool ok = true;
+                for (int k = 0; k < nk && ok; k++) {
+                    const int kc = kc0 + k, b = kc & 1;
+                    ok = kc < 2 || mbar_wait_bounded(&f.acc_empty[b], ((kc >> 1) & 1) ^ 1, &f.abort);
+                    for (int half = 0; half < 2 && ok; half++) {
+                        const int it = it0 + 2 * k + half, s = it % C2_STAGES;
+                        ok = mbar_wait_bounded(&f.full[s], (it / C2_STAGES) & 1, &f.abort);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t st = smem_u32(smem + s * C2_STAGE_BYTES);
+                        const uint64_t a_hi = sdesc_sw128(st), a_lo = sdesc_sw128(st + TC_TILE_BYTES);
+                        const uint64_t b_hi = diag ? a_hi : sdesc_sw128(st + 2 * TC_TILE_BYTES);
+                        const uint64_t b_lo = diag ? a_lo : sdesc_sw128(st + 3 * TC_TILE_BYTES);
+                        #pragma unroll
+                        for (int kk = 0; kk < 4; kk++) {
+                            const uint64_t off = (uint64_t)((kk * 32) >> 4);     // 16 F16 = 32 bytes along K
+                            mma_f16(tmem + b * C2, a_hi + off, b_hi + off, idesc, (half > 0 || kk > 0) ? 1u : 0u);
+                            mma_f16(tmem + b * C2, a_hi + off, b_lo + off, idesc, 1u);
+                            mma_f16(tmem + b * C2, a_lo + off, b_hi + off, idesc, 1u);
+                        }
+                        mma_commit(&f.empty[s]);
+                        n = 2 * k + half + 1;
+                    }
+                    if (ok) mma_commit(&f.acc_full[b]);
+                }
+                f.n_used = it0 + n;
+            }
+            __syncwarp();
+        } else {
+            const float* src = A + (size_t)row * ld + j * C2 + 64 * h;
             #pragma unroll
-            for (int i = 0; i < 8; i++) cpre[i] = *reinterpret_cast<const float4*>(src + 4 * i);
-        }
-        // the MMAs read shared memory asynchronously: wait before the next half's loads reuse it
-        if (!mbar_wait_bounded(&done_bar, (uint32_t)(h & 1), &abort_flag, false)) ok = false;
-        tc_fence_after();
-        __syncthreads();
-    }
-    const bool good = __syncthreads_and(ok && !abort_flag) != 0;
-    if (good) {
-        const int row = r0 + warp * 32 + lane;
-        const int si = pexp[I * C2 + warp * 32 + lane];
-        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-        #pragma unroll 1
-        for (int c = 0; c < TC_TILE; c += 32) {
-            float v[32];
-            tmem_ld_32cols(trow + (uint32_t)c, v);
-            const int sj = pexp[J * C2 + c + lane];      // column c + lane's row scale, shared through the warp
-            float* dst = A + (size_t)row * ld + c0 + c;
-            float4 cur[8];
-            #pragma unroll
-            for (int i = 0; i < 8; i++) cur[i] = cpre[i];
-            if (c + 32 < TC_TILE) {                       // the next 32 columns' loads in flight meanwhile
+            for (int c = 0; c < 64; c += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(src + c);
+                acc[c] = v.x; acc[c + 1] = v.y; acc[c + 2] = v.z; acc[c + 3] = v.w;
+            }
+            const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(64 * h);
+            #pragma unroll 1
+            for (int k = 0; k < nk; k++) {
+                const int kc = kc0 + k, b = kc & 1;
+                if (!mbar_wait_bounded(&f.exp_full[b], (kc >> 1) & 1, &f.abort)) break;
+                if (!mbar_wait_bounded(&f.acc_full[b], (kc >> 1) & 1, &f.abort)) break;
+                tc_fence_after();
+                const int si = 127 - exps[b][0][r];
+                const int* sj = &exps[b][1][64 * h];
                 #pragma unroll
-                for (int i = 0; i < 8; i++) cpre[i] = *reinterpret_cast<const float4*>(dst + 32 + 4 * i);
-            }
-            #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-                float4 a = cur[i / 4];
-                // 2^-(s_i + s_j), exact (|s_i + s_j| <= 120)
-                a.x -= v[i] * __int_as_float((127 - si - __shfl_sync(0xffffffffu, sj, i)) << 23);
-                a.y -= v[i + 1] * __int_as_float((127 - si - __shfl_sync(0xffffffffu, sj, i + 1)) << 23);
-                a.z -= v[i + 2] * __int_as_float((127 - si - __shfl_sync(0xffffffffu, sj, i + 2)) << 23);
-                a.w -= v[i + 3] * __int_as_float((127 - si - __shfl_sync(0xffffffffu, sj, i + 3)) << 23);
-                *reinterpret_cast<float4*>(dst + i) = a;
+                for (int c = 0; c < 64; c += 32) {
+                    float v[32];
+                    tmem_ld_32cols(trow + (uint32_t)(b * C2 + c), v);
+                    #pragma unroll
+                    for (int q = 0; q < 32; q += 4) {
+                        // 2^-(s_i + s_j), exact (|s_i + s_j| <= 120)
+                        const int4 e = *reinterpret_cast<const int4*>(sj + c + q);
+                        acc[c + q] -= v[q] * __int_as_float((si - e.x) << 23);
+                        acc[c + q + 1] -= v[q + 1] * __int_as_float((si - e.y) << 23);
+                        acc[c + q + 2] -= v[q + 2] * __int_as_float((si - e.z) << 23);
+                        acc[c + q + 3] -= v[q + 3] * __int_as_float((si - e.w) << 23);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) c2_arrive(&f.acc_empty[b]);
             }
         }
+        it0 += 2 * nk;
+        kc0 += nk;
+        __syncthreads();                          // every MMA has read its stage: the buffers are free
+
+        if (diag) {
+            if (warp < C2_EPI) {
+                float* ps = reinterpret_cast<float*>(smem);
+                #pragma unroll
+                for (int c = 0; c < 64; c++) ps[r * (C2 + 1) + 64 * h + c] = (64 * h + c <= r) ? acc[c] : 0.f;
+                c2_sync();
+                float* Ajj = A + (size_t)j * C2 * ld + j * C2;
+                potrf128(ps, j * C2, which ? &gs->not_spd_R : &gs->not_spd_F,
+                         mem.ih + (size_t)j * C2 * C2, mem.il + (size_t)j * C2 * C2);
+                asm volatile("fence.proxy.async;" ::: "memory");
+                __threadfence();
+                c2_sync();
+                if (tid == 0) st_release(inv + j, 1);
+                potrf128_store(ps, Ajj, ld, Linv ? Linv + (size_t)j * 2 * C2 * C2 : nullptr);
+            }
+        } else {
+            // [quarter 0, 1][A hi, lo] | [quarter 2, 3][A hi, lo] | [two quarters][B hi, lo]
+            unsigned char* const at = smem;
+            unsigned char* const bt = smem + 8 * TC_TILE_BYTES;
+            if (warp == C2_EPI) {
+                if (lane == 0 && c2_wait_flag(inv + j, gs, &f.abort)) {
+                    asm volatile("fence.proxy.async;" ::: "memory");
+                    for (int rd = 0; rd < 2; rd++) {
+                        if (rd == 1 && !mbar_wait_bounded(&f.sol[0], nsol & 1, &f.abort)) break;
+                        mbar_expect_tx(&f.b_full, 4 * TC_TILE_BYTES);
+                        for (int u = 0; u < 2; u++) {
+                            tma_load_2d(&map_ih, &f.b_full, bt + (2 * u) * TC_TILE_BYTES, (2 * rd + u) * 32, j * C2);
+                            tma_load_2d(&map_il, &f.b_full, bt + (2 * u + 1) * TC_TILE_BYTES, (2 * rd + u) * 32, j * C2);
+                        }
+                        // landed before the buffers are used again, whatever the others do
+                        mbar_wait_bounded(&f.b_full, rd, &f.abort, false);
+                    }
+                }
+                __syncwarp();
+            } else if (warp == C2_EPI + 1) {
+                asm volatile("bar.sync 2, 288;" ::: "memory");
+                if (lane == 0) {
+                    const uint32_t idesc = idesc_tf32_128x128(), d = tmem + 2 * C2;
+                    for (int rd = 0; rd < 2; rd++) {
+                        if (!mbar_wait_bounded(&f.b_full, rd, &f.abort)) break;
+                        tc_fence_after();
+                        for (int u = 0; u < 2; u++) {
+                            const int qt = 2 * rd + u;
+                            const uint64_t a_hi = sdesc_sw128(smem_u32(at + (2 * qt) * TC_TILE_BYTES));
+                            const uint64_t a_lo = sdesc_sw128(smem_u32(at + (2 * qt + 1) * TC_TILE_BYTES));
+                            const uint64_t b_hi = sdesc_sw128(smem_u32(bt + (2 * u) * TC_TILE_BYTES));
+                            const uint64_t b_lo = sdesc_sw128(smem_u32(bt + (2 * u + 1) * TC_TILE_BYTES));
+                            #pragma unroll
+                            for (int kk = 0; kk < TC_KB / 8; kk++) {
+                                const uint64_t off = (uint64_t)((kk * 32) >> 4);
+                                mma_tf32(d, a_hi + off, b_hi + off, idesc, (qt > 0 || kk > 0) ? 1u : 0u);
+                                mma_tf32(d, a_hi + off, b_lo + off, idesc, 1u);
+                                mma_tf32(d, a_lo + off, b_hi + off, idesc, 1u);
+                            }
+                        }
+                        mma_commit(&f.sol[rd]);
+                    }
+                }
+                __syncwarp();
+            } else {
+                #pragma unroll
+                for (int c = 0; c < 64; c += 4) {
+                    float2 v[4];
+                    #pragma unroll
+                    for (int e = 0; e < 4; e++) v[e] = split_tf32(acc[c + e]);
+                    unsigned char* t = at + (2 * (2 * h + (c >> 5))) * TC_TILE_BYTES + sw128_offset(r, c & 31);
+                    *reinterpret_cast<float4*>(t) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+                    *reinterpret_cast<float4*>(t + TC_TILE_BYTES) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                tc_fence_before();
+                asm volatile("bar.sync 2, 288;" ::: "memory");
+                const bool ok = mbar_wait_bounded(&f.sol[1], nsol & 1, &f.abort);
+                tc_fence_after();
+                const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(2 * C2 + 64 * h);
+                float mx = 0.f;
+                if (ok) {
+                    #pragma unroll
+                    for (int c = 0; c < 64; c += 32) {
+                        float v[32];
+                        tmem_ld_32cols(trow + (uint32_t)c, v);
+                        #pragma unroll
+                        for (int q = 0; q < 32; q++) { acc[c + q] = v[q]; mx = fmaxf(mx, fabsf(v[q])); }
+                    }
+                    tc_fence_before();
+                }
+                rmax[h][r] = mx;
+                c2_sync();
+                mx = fmaxf(rmax[0][r], rmax[1][r]);
+                int e = 0;
+                frexpf(mx, &e);                      // mx < 2^e
+                // kept within [-60, 60] so that 2^-(s_i + s_j) is a normal float
+                const int sc = (mx > 0.f) ? max(-60, min(60, 14 - e)) : 0;
+                if (h == 0) mem.pexp[(size_t)j * mem.rows + row] = sc;
+                const float scf = __int_as_float((127 + sc) << 23);
+                const size_t at16 = (size_t)row * mem.rows + j * C2 + 64 * h;
+                #pragma unroll
+                for (int c = 0; c < 64; c += 8) {
+                    uint32_t hw[4], lw[4];
+                    #pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const float a = acc[c + 2 * q] * scf, b = acc[c + 2 * q + 1] * scf;
+                        const __half ah = __float2half_rn(a), bh = __float2half_rn(b);
+                        const __half al = __float2half_rn(a - __half2float(ah)), bl = __float2half_rn(b - __half2float(bh));
+                        hw[q] = (uint32_t)__half_as_ushort(ah) | ((uint32_t)__half_as_ushort(bh) << 16);
+                        lw[q] = (uint32_t)__half_as_ushort(al) | ((uint32_t)__half_as_ushort(bl) << 16);
+                    }
+                    *reinterpret_cast<uint4*>(mem.Lh + at16 + c) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+                    *reinterpret_cast<uint4*>(mem.Ll + at16 + c) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                }
+                asm volatile("fence.proxy.async;" ::: "memory");
+                __threadfence();
+                c2_sync();
+                if (tid == 0 && !f.abort) st_release(ready + (size_t)j * nbc + i, 1);
+                float* dst = A + (size_t)row * ld + j * C2 + 64 * h;
+                #pragma unroll
+                for (int c = 0; c < 64; c += 4)
+                    *reinterpret_cast<float4*>(dst + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
+            }
+            nsol++;
+        }
+        __syncthreads();
+        if (f.abort) break;
     }
-    if (threadIdx.x == 0 && issued > landed)       // copies issued but never seen complete: let them land
-        mbar_wait_bounded(&full_bar, (uint32_t)(landed & 1), &abort_flag, false);
+    if (tid == 32 * (C2_EPI + 1)) mma_commit(&f.done);
+    __syncwarp();
+    __syncthreads();
+    mbar_wait_bounded(&f.done, 0, &f.abort, false);
+    if (f.abort && tid == 0)                       // copies issued but never consumed land before the CTA ends
+        for (int it = f.n_used; it < f.n_issued; it++)
+            mbar_wait_bounded(&f.full[it % C2_STAGES], (it / C2_STAGES) & 1, &f.abort, false);
+    if (f.abort && tid == 0)
+        for (int kc = max(0, f.n_exp - 2); kc < f.n_exp; kc++)
+            mbar_wait_bounded(&f.exp_full[kc & 1], (kc >> 1) & 1, &f.abort, false);
+    tc_fence_after();
     tc_fence_before();
     __syncthreads();
-    if (!good && threadIdx.x == 0) atomicExch(&gs->status, QLP_ERR_TIMEOUT);
+    if (f.abort && tid == 0) atomicExch(&gs->status, QLP_ERR_TIMEOUT);
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
 }
 
 // ---------------------------------------------------------------------------
-// F z = r with the factor of k_potrf128 / k_chol_tile128 and the inverses of
+// F z = r with the factor of k_chol128 and the inverses of
 // its 128x128 diagonal blocks (Linv: per block the inverse and its transpose):
 //   forward  y_k = Linv_k (r_k - sum_{j<k} L_kj y_j)
 //   backward z_k = Linv_k^T (y_k - sum_{j>k} L_jk^T z_j)

@@ -767,6 +767,12 @@ int chol64_alloc(Chol64Work** out, int M_cap, void* shared)
     return QLP_OK;
 }
 
+// The flags of a factorisation and of one pair of solves.
+void chol64_clear(const Chol64Work* z, ClearList& l)
+{
+    l.add(z->flags, sizeof(int) * ((size_t)z->nbc * z->nbc + 3 * z->nbc + 1));
+}
+
 // which: 0 F, 1 R (the not-SPD flag).  half_width: how far below the diagonal
 // the matrix reaches (R: two grid rows), or past M.  ctas: the grid's size.
 void launch_cholesky_fp64(double* A, int ld, int M_max, GridState* gs, int which, int half_width, int ctas,
@@ -776,7 +782,6 @@ void launch_cholesky_fp64(double* A, int ld, int M_max, GridState* gs, int which
     // blocks that a band of half_width entries can reach, rounded up to even
     const int band = ((std::min(half_width, M_max) + C64 - 1) / C64 + 1) & ~1;
     const int tiles = nb * std::min((nb + 1) / 2, band / 2 + 1);
-    cudaMemsetAsync(z->flags, 0, sizeof(int) * ((size_t)z->nbc * z->nbc + z->nbc + 1), st);
     k_chol64_prep<<<(M_max + 255) / 256, 256, 0, st>>>(gs, A, ld, z->rexp);
     k_chol64<<<std::max(1, std::min(tiles, ctas)), OZ_THREADS, oz_smem(CS), st>>>(
         z->ls_a, z->ls_b, z->li_b, gs, A, ld, which, band, z->M128, z->nbc, z->ls, z->li, z->rexp, z->lexp, z->wexp,
@@ -789,7 +794,6 @@ void launch_solve_fp64(Work& w, int M_max, cudaStream_t st)
     Chol64Work* z = w.cholF;
     const int nb = (M_max + C64 - 1) / C64;
     int* flags = z->flags + (size_t)z->nbc * z->nbc + z->nbc + 1;
-    cudaMemsetAsync(flags, 0, sizeof(int) * 2 * z->nbc, st);
     k_trsv64_fwd<<<nb, 256, 0, st>>>(w.F, w.ldF, w.linv, w.gs, w.D, w.tmp, flags);
     k_trsv64_bwd<<<nb, 256, 0, st>>>(w.F, w.ldF, w.linv, w.gs, w.tmp, w.s, flags + z->nbc);
     count_launches(2);

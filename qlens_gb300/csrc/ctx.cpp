@@ -12,6 +12,7 @@
 namespace qlpix {
 
 void psf_init_attributes();
+void mapping_init_attributes();
 void sparseops_init_attributes();
 void sur_exact_init_attributes();
 
@@ -57,12 +58,11 @@ static void free_work(Work& w)
 
 static void drop_graph(Slot& s)
 {
-    if (s.graph) cudaGraphExecDestroy(s.graph);
-    s.graph = nullptr;
-    s.graph_gen = 0;
-    if (s.graph_trial) cudaGraphExecDestroy(s.graph_trial);
-    s.graph_trial = nullptr;
-    s.trial_gen = 0;
+    for (auto& part : s.graphs)
+        for (SlotGraph& g : part) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = SlotGraph{};
+        }
 }
 
 static void free_slot(Slot& s)
@@ -92,7 +92,7 @@ static int alloc_work(qlp_ctx* c, Slot& s, int n_mask, int nsub, int Mcells, int
     CK(dalloc(&w.cx, snx_max + 1), "alloc"); CK(dalloc(&w.cy, sny_max + 1), "alloc");
     CK(dalloc(&w.ccx, snx_max), "alloc"); CK(dalloc(&w.ccy, sny_max), "alloc");
     CK(dalloc(&w.cell3, 3 * n_sub), "alloc"); CK(dalloc(&w.w3, 3 * n_sub), "alloc");
-    CK(dalloc(&w.mapped, Mcells), "alloc"); CK(dalloc(&w.active_index, Mcells), "alloc");
+    CK(dalloc(&w.mapped, Mc), "alloc"); CK(dalloc(&w.active_index, Mc), "alloc");
     CK(dalloc(&w.pixmaps, n_mask), "alloc"); CK(dalloc(&w.rowidx, n_mask), "alloc");
     CK(dalloc(&w.pixindex, (size_t)c->nx * c->ny), "alloc");
     CK(dalloc(&w.rowpix, n_mask), "alloc");
@@ -113,7 +113,7 @@ static int alloc_work(qlp_ctx* c, Slot& s, int n_mask, int nsub, int Mcells, int
     CK(dalloc(&w.gs, 1), "alloc"); CK(dalloc(&w.out, 1), "alloc"); CK(dalloc(&w.ep, 1), "alloc");
     CK(dalloc(&w.fb_ray, n_sub), "alloc"); CK(dalloc(&w.fb_xy, 2 * n_sub), "alloc"); CK(dalloc(&w.fb_count, 1), "alloc");
     CK(dalloc(&w.sur_eps, n_sub), "alloc");
-    CK(dalloc(&w.xlist, n_sub), "alloc"); CK(dalloc(&w.xcount, 1), "alloc");
+    CK(dalloc(&w.xlist, n_sub), "alloc"); CK(dalloc(&w.xcount, 2), "alloc");
     CK(dalloc(&w.nfw_xy, 2 * n_sub), "alloc");
     s.M_cap = Mc;
     s.N_cap = n_mask;
@@ -162,6 +162,14 @@ static int ensure_slot(qlp_ctx* c, int k, int n_mask, int cells, int snx, int sn
     if (!s.side) CK(cudaStreamCreateWithFlags(&s.side, cudaStreamNonBlocking), "stream");
     if (!s.side_fork) CK(cudaEventCreateWithFlags(&s.side_fork, cudaEventDisableTiming), "event");
     if (!s.side_join) CK(cudaEventCreateWithFlags(&s.side_join, cudaEventDisableTiming), "event");
+    if (!c->jobs) {
+        CK(cudaMalloc((void**)&c->job_counts, sizeof(unsigned) * QLP_MAX_SLOTS), "jobs");
+        CK(cudaMemset(c->job_counts, 0, sizeof(unsigned) * QLP_MAX_SLOTS), "jobs");
+        CK(cudaStreamSynchronize(0), "jobs");
+        CK(cudaMallocHost((void**)&c->jobs, sizeof(Job) * QLP_JOB_RING * QLP_MAX_SLOTS), "jobs");
+    }
+    s.jobs = c->jobs + (size_t)k * QLP_JOB_RING;
+    s.job_count = c->job_counts + k;
     const int nsub = c->sd.nsub;
     if (s.N_cap >= n_mask && s.M_cap >= round64(std::max(cells, 64)) && s.snx_cap >= snx && s.sny_cap >= sny &&
         s.nsub_cap == nsub)
@@ -247,6 +255,7 @@ int ctx_init(qlp_ctx* c, const qlp_image* im, const qlp_psf* psf, const qlp_srcg
     so.regparam = opts->regparam;
 
     psf_init_attributes();
+    mapping_init_attributes();
     sparseops_init_attributes();
     sur_exact_init_attributes();
     int snx = std::max(so.snx, 2), sny = std::max(so.sny, 2);
@@ -265,11 +274,12 @@ void ctx_free(qlp_ctx* c)
     }
     c->slots.clear();
     void* ptrs[] = {c->d_xvals, c->d_yvals, c->d_data, c->d_covinv, c->d_psf, c->d_psf_int, c->d_mpix, c->d_inst_mpix,
-                    c->d_emask, c->d_inmask, c->d_epix, c->d_eoff};
+                    c->d_emask, c->d_inmask, c->d_epix, c->d_eoff, c->job_counts};
     for (void* p : ptrs) if (p) cudaFree(p);
     if (c->h_out) cudaFreeHost(c->h_out);
     if (c->h_ep) cudaFreeHost(c->h_ep);
     if (c->h_trial) cudaFreeHost(c->h_trial);
+    if (c->jobs) cudaFreeHost(c->jobs);
     for (int i = 0; i <= QLP_N_STAGES; i++) if (c->ev[i]) cudaEventDestroy(c->ev[i]);
     if (c->fork) cudaEventDestroy(c->fork);
     if (c->join) cudaEventDestroy(c->join);
@@ -306,12 +316,21 @@ static bool model_has_nfw(const qlp_ctx* c)
     return false;
 }
 
-// CTAs of one factorisation on the plain path: the whole GPU for an evaluation
-// alone, its share in a batch.  A CTA holds its SM while it waits, so the
-// factorisations in flight must fit side by side; at least 8 each, so that the
-// digit products (~25 SM ms at 3,000 cells) stay within the chain of pivot
-// blocks (~4 ms).
-static int chol64_ctas(const qlp_ctx* c) { return std::max(8, 148 / std::max(1, c->in_flight)); }
+// How full the GPU is: 0 one evaluation alone, 1 up to 8 in flight, 2 more.
+static int load_of(const qlp_ctx* c) { return c->in_flight <= 1 ? 0 : c->in_flight <= 8 ? 1 : 2; }
+
+// CTAs of a factorisation of nb block columns: the whole GPU for an evaluation
+// alone.  In a batch a CTA that waits keeps its SM from the other evaluations'
+// kernels, so only as many are taken as keep a column's tiles (~15 us each)
+// within its pivot block's time: a quarter of the block columns, and at least 16
+// while the SMs do for it.  (FP64, four optimising lambda: 35.7 ms with a
+// quarter, 32.6 with 12, 30.4 with 16, 31.1 with 37.  Mixed, 32 at 4,096 cells: 24.9 ms with 8,
+// 30.3 with 37.)
+int factor_ctas(const qlp_ctx* c, int nb)
+{
+    const int quarter = std::max(2, (nb + 3) / 4), load = load_of(c);
+    return load == 0 ? 148 : load == 1 ? std::max(16, quarter) : quarter;
+}
 
 // The launch sequence of one evaluation on stream st with the workspace of
 // `slot`; sd / so size the launches (the evaluation's own mask and source
@@ -338,11 +357,13 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             int r = run_inversion_mixed(c, slot, sd, so, regp, PIPE_TRIAL, st, nullptr);
             if (r != QLP_OK) return r;
         } else {
-            const size_t bytes = sizeof(double) * (size_t)w.ldF * Mc;
-            cudaMemsetAsync(&w.gs->not_spd_F, 0, sizeof(int), st);
-            cudaMemcpyAsync(w.F, w.F0, bytes, cudaMemcpyDeviceToDevice, st);
+            ClearList cl;
+            cl.add(&w.gs->not_spd_F, sizeof(int));
+            chol64_clear(w.cholF, cl);
+            launch_clear(cl, st);
+            launch_copy_square(w.F, w.F0, w.ldF, 8, 64, w.gs, Mc, st);
             launch_regularization(so, w, Mc, regp, REG_F, st);
-            launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, Mc, chol64_ctas(c), w.cholF, w.linv, st);
+            launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, Mc, factor_ctas(c, Mc / 64), w.cholF, w.linv, st);
             launch_logdet(w.F, w.ldF, Mc, w, 0, st);
             launch_solve_fp64(w, Mc, st);
         }
@@ -350,7 +371,25 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
         if (c->osb_on) launch_outside_sb(sd, so, c->osb, slot.osb, model_has_nfw(c), w, st);
         return QLP_OK;
     }
-    cudaMemsetAsync(w.out, 0, sizeof(EvalOut), st);
+    {
+        const int r = mixed ? mixed_init(slot) : ensure_fp64_mats(slot);
+        if (r != QLP_OK) return r;
+        ClearList cl;
+        cl.add(w.out, sizeof(EvalOut));
+        cl.add(w.mapped, sizeof(int) * Mc);
+        cl.add(w.pixmaps, sizeof(int) * std::max(sd.n_mask, 1));
+        cl.add(w.pixindex, sizeof(int) * sd.nx * sd.ny, 0xffffffffu);   // pixels outside the mask keep -1
+        cl.add(w.fb_count, sizeof(int));
+        cl.add(w.xcount, 2 * sizeof(int));
+        if (mixed) {
+            mixed_clear(slot, cl, false);
+        } else {
+            oz_clear(w.oz, cl);
+            chol64_clear(w.cholF, cl);
+            chol64_clear(w.cholR, cl);
+        }
+        launch_clear(cl, st);
+    }
     if (ev) cudaEventRecord(ev[0], st);
     if (c->nfw_mode == QLP_NFW_SURROGATE && model_has_nfw(c)) {
         // a single NFW lens on the last plane: its quadrature fallbacks can run
@@ -388,8 +427,6 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
         if (r != QLP_OK) return r;
         if (part == PIPE_PRE) return QLP_OK;
     } else {
-        int r = ensure_fp64_mats(slot);
-        if (r != QLP_OK) return r;
         if (so.regularization) {
             // R hangs on the active cells alone: its log det runs on the slot's
             // second stream beside L', F and F's factor.  R couples a cell to
@@ -397,6 +434,7 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             // factor stays within that band (dense it cost as much as F's).
             cudaEventRecord(slot.side_fork, st);
             cudaStreamWaitEvent(slot.side, slot.side_fork, 0);
+            launch_clear_band(w.R, w.ldF, 8, Mc, 64, (2 * so.snx + 63) / 64 + 2, w.gs, slot.side);
             launch_regularization(so, w, Mc, regp, REG_R, slot.side);
             launch_cholesky_fp64(w.R, w.ldF, Mc, w.gs, 1, 2 * so.snx, 4, w.cholR, nullptr, slot.side);
             launch_logdet(w.R, w.ldF, Mc, w, 1, slot.side);
@@ -408,13 +446,13 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
         launch_syrk_fp64(sd, w, N_max, Mc, st);
         if (ev) cudaEventRecord(ev[4], st);
         if (part == PIPE_PRE)
-            cudaMemcpyAsync(w.F0, w.F, sizeof(double) * (size_t)w.ldF * Mc, cudaMemcpyDeviceToDevice, st);
+            launch_copy_square(w.F0, w.F, w.ldF, 8, 64, w.gs, Mc, st);
         if (part == PIPE_PRE) {
             if (so.regularization) cudaStreamWaitEvent(st, slot.side_join, 0);
             return QLP_OK;
         }
         launch_regularization(so, w, Mc, regp, REG_F, st);
-        launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, Mc, chol64_ctas(c), w.cholF, w.linv, st);
+        launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, Mc, factor_ctas(c, Mc / 64), w.cholF, w.linv, st);
         launch_logdet(w.F, w.ldF, Mc, w, 0, st);
         launch_solve_fp64(w, Mc, st);
         if (so.regularization) cudaStreamWaitEvent(st, slot.side_join, 0);
@@ -459,71 +497,83 @@ static int prepare_slot(qlp_ctx* c, Slot& s)
 }
 
 // Capture the slot's launch sequence, sized for its capacity, as a graph.
-static int capture_graph(qlp_ctx* c, Slot& s, const StaticData& sd, const SrcOpts& so, const int key[7], int part)
+static int capture_graph(qlp_ctx* c, Slot& s, const StaticData& sd, const SrcOpts& so, const int key[7], int part,
+                         SlotGraph& sg)
 {
     const bool trial = (part == PIPE_TRIAL);
-    cudaGraphExec_t& slot_graph = trial ? s.graph_trial : s.graph;
-    if (slot_graph) cudaGraphExecDestroy(slot_graph);
-    slot_graph = nullptr;
+    if (sg.exec) cudaGraphExecDestroy(sg.exec);
+    sg = SlotGraph{};
     int r = prepare_slot(c, s);
     if (r != QLP_OK) return r;
     const long long l0 = kernel_launch_counter();
     CK(cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal), "capture");
+    launch_job_in(s.jobs, QLP_JOB_RING, s.job_count, s.w.ep, trial, s.stream);
     r = run_pipeline(c, s, sd, so, s.stream, nullptr, part);
+    launch_job_out(s.jobs, QLP_JOB_RING, s.job_count, s.w.out, s.stream);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s.stream, &g);
     const long long n = kernel_launch_counter() - l0;
     count_launches((int)-n);            // nothing ran yet: replays count them
     if (r != QLP_OK) { if (g) cudaGraphDestroy(g); return r; }
     if (e != cudaSuccess || !g) return cuda_fail(e, "stream capture");
-    e = cudaGraphInstantiate(&slot_graph, g, 0);
+    e = cudaGraphInstantiate(&sg.exec, g, 0);
     cudaGraphDestroy(g);
-    if (e != cudaSuccess) { slot_graph = nullptr; return cuda_fail(e, "graph instantiate"); }
-    for (int i = 0; i < 7; i++) (trial ? s.trial_key : s.graph_key)[i] = key[i];
-    (trial ? s.trial_gen : s.graph_gen) = c->graph_gen;
-    (trial ? s.trial_launches : s.graph_launches) = n;
+    if (e != cudaSuccess) { sg.exec = nullptr; return cuda_fail(e, "graph instantiate"); }
+    for (int i = 0; i < 7; i++) sg.key[i] = key[i];
+    sg.gen = c->graph_gen;
+    sg.launches = n;
     return QLP_OK;
 }
 
-// One evaluation on slot s: upload its parameters, run (replay or launch) the
-// sequence, copy its result to *h_dst -- all asynchronous on the slot stream.
+// One evaluation on slot s: its parameters in, the sequence (replayed or
+// launched), its result to *h_dst (pinned, like *h_ep) -- all asynchronous on
+// the slot stream.  A replayed graph fetches and delivers them itself, from the
+// slot's ring of jobs, and holds no memset node: behind either of these a stream
+// waits in one of the few hardware queues that all streams share and holds up the
+// streams behind it there.  With both, no more than 8 of 32 evaluations ran at a
+// time (the default queue count, which a process that made its CUDA context
+// before this library keeps): 32 at 576 cells, mixed, 4.72 ms, now 2.49.
 static int issue_eval(qlp_ctx* c, Slot& s, const StaticData& sd, const SrcOpts& so, const EvalParams* h_ep,
                       EvalOut* h_dst, cudaEvent_t* ev, int part = PIPE_ALL)
 {
-    if (part == PIPE_TRIAL)      // a lambda trial changes lambda only
-        CK(cudaMemcpyAsync(&s.w.ep->regparam, &h_ep->regparam, sizeof(double), cudaMemcpyHostToDevice, s.stream),
-           "h2d");
-    else
-        CK(cudaMemcpyAsync(s.w.ep, h_ep, sizeof(EvalParams), cudaMemcpyHostToDevice, s.stream), "h2d");
     if (c->use_graphs && ev == nullptr) {
         // one graph per slot for every mask and source grid that fits its
         // capacity: the launches are sized for the capacity, the kernels read
-        // the actual sizes from the EvalParams just uploaded
+        // the actual sizes from the EvalParams
         StaticData sdc = sd;
         sdc.n_mask = s.N_cap;
         sdc.n_sub = s.N_cap * sd.nsub;
         SrcOpts soc = so;
         soc.snx = s.snx_cap;
         soc.sny = s.sny_cap;
-        const int key[7] = {c->precision | chol64_ctas(c) << 8, s.N_cap, s.snx_cap, s.sny_cap, model_has_nfw(c) ? 1 : 0,
-                            c->nfw_mode, part};
-        const bool trial = (part == PIPE_TRIAL);
-        const cudaGraphExec_t have = trial ? s.graph_trial : s.graph;
-        const int* have_key = trial ? s.trial_key : s.graph_key;
-        bool ok = have && (trial ? s.trial_gen : s.graph_gen) == c->graph_gen;
-        for (int i = 0; ok && i < 7; i++) ok = (have_key[i] == key[i]);
+        const int key[7] = {c->precision, s.N_cap, s.snx_cap, s.sny_cap, model_has_nfw(c) ? 1 : 0, c->nfw_mode, part};
+        SlotGraph& sg = s.graphs[part == PIPE_TRIAL ? 1 : 0][load_of(c)];
+        bool ok = sg.exec && sg.gen == c->graph_gen;
+        for (int i = 0; ok && i < 7; i++) ok = (sg.key[i] == key[i]);
         if (!ok) {
-            int r = capture_graph(c, s, sdc, soc, key, part);
+            int r = capture_graph(c, s, sdc, soc, key, part, sg);
             if (r != QLP_OK) return r;
         }
-        CK(cudaGraphLaunch(trial ? s.graph_trial : s.graph, s.stream), "graph launch");
-        count_launches((int)(trial ? s.trial_launches : s.graph_launches));
-    } else {
-        int r = prepare_slot(c, s);
-        if (r != QLP_OK) return r;
-        r = run_pipeline(c, s, sd, so, s.stream, ev, part);
-        if (r != QLP_OK) return r;
+        // the ring's entries of the launches still in the stream stay as they are
+        if (s.job_no - s.job_synced >= QLP_JOB_RING) {
+            CK(cudaStreamSynchronize(s.stream), "jobs");
+            s.job_synced = s.job_no;
+        }
+        s.jobs[s.job_no % QLP_JOB_RING] = Job{h_ep, h_dst};
+        CK(cudaGraphLaunch(sg.exec, s.stream), "graph launch");
+        s.job_no++;
+        count_launches((int)sg.launches);
+        return QLP_OK;
     }
+    if (part == PIPE_TRIAL)      // a lambda trial changes lambda only
+        CK(cudaMemcpyAsync(&s.w.ep->regparam, &h_ep->regparam, sizeof(double), cudaMemcpyHostToDevice, s.stream),
+           "h2d");
+    else
+        CK(cudaMemcpyAsync(s.w.ep, h_ep, sizeof(EvalParams), cudaMemcpyHostToDevice, s.stream), "h2d");
+    int r = prepare_slot(c, s);
+    if (r != QLP_OK) return r;
+    r = run_pipeline(c, s, sd, so, s.stream, ev, part);
+    if (r != QLP_OK) return r;
     if (part != PIPE_PRE)
         CK(cudaMemcpyAsync(h_dst, s.w.out, sizeof(EvalOut), cudaMemcpyDeviceToHost, s.stream), "d2h");
     return QLP_OK;

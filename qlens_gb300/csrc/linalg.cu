@@ -24,6 +24,103 @@ namespace qlpix {
 
 __device__ __forceinline__ int mpad64(int M) { return (M + 63) & ~63; }
 
+// ---- a graph replay's parameters and result, from and to pinned host memory ----
+__global__ void k_job_in(const Job* jobs, unsigned ring, const unsigned* count, EvalParams* ep, int trial)
+{
+    const EvalParams* src = jobs[*count & (ring - 1)].ep;
+    if (trial) {
+        if (threadIdx.x == 0) ep->regparam = src->regparam;
+        return;
+    }
+    const unsigned long long* s = reinterpret_cast<const unsigned long long*>(src);
+    unsigned long long* d = reinterpret_cast<unsigned long long*>(ep);
+    for (int i = threadIdx.x; i < (int)(sizeof(EvalParams) / 8); i += blockDim.x) d[i] = s[i];
+}
+
+__global__ void k_job_out(const Job* jobs, unsigned ring, unsigned* count, const EvalOut* out)
+{
+    static_assert(sizeof(EvalParams) % 8 == 0 && sizeof(EvalOut) % 8 == 0, "copied as 8-byte words");
+    const unsigned q = *count;
+    EvalOut* dst = jobs[q & (ring - 1)].out;
+    if (dst)
+        for (int i = threadIdx.x; i < (int)(sizeof(EvalOut) / 8); i += blockDim.x)
+            reinterpret_cast<unsigned long long*>(dst)[i] = reinterpret_cast<const unsigned long long*>(out)[i];
+    __syncthreads();
+    if (threadIdx.x == 0) *count = q + 1;
+}
+
+void launch_job_in(const Job* jobs, unsigned ring, unsigned* count, EvalParams* ep, bool trial, cudaStream_t st)
+{
+    k_job_in<<<1, 256, 0, st>>>(jobs, ring, count, ep, trial ? 1 : 0);
+    count_launches(1);
+}
+
+void launch_job_out(const Job* jobs, unsigned ring, unsigned* count, const EvalOut* out, cudaStream_t st)
+{
+    k_job_out<<<1, 32, 0, st>>>(jobs, ring, count, out);
+    count_launches(1);
+}
+
+// ---- clearing and copying ----
+__global__ void __launch_bounds__(256) k_clear(ClearList l)
+{
+    for (int k = 0; k < l.n; k++) {
+        const ClearItem it = l.item[k];
+        const uint4 v = make_uint4(it.value, it.value, it.value, it.value);
+        uint4* p4 = reinterpret_cast<uint4*>(it.p);
+        const unsigned n4 = ((size_t)it.p & 15) == 0 ? it.words / 4 : 0;
+        for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) p4[i] = v;
+        unsigned* p = reinterpret_cast<unsigned*>(it.p);
+        for (unsigned i = 4 * n4 + blockIdx.x * blockDim.x + threadIdx.x; i < it.words; i += gridDim.x * blockDim.x)
+            p[i] = it.value;
+    }
+}
+
+void launch_clear(const ClearList& l, cudaStream_t st)
+{
+    size_t words = 0;
+    for (int k = 0; k < l.n; k++) words += l.item[k].words;
+    const int blocks = (int)((words / 4 + 1023) / 1024);
+    k_clear<<<blocks < 1 ? 1 : (blocks > 152 * 2 ? 152 * 2 : blocks), 256, 0, st>>>(l);
+    count_launches(1);
+}
+
+__global__ void __launch_bounds__(256) k_clear_band(char* __restrict__ A, size_t ld_bytes, int esize, int blk, int back,
+                                                    const GridState* __restrict__ gs)
+{
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), i = row / blk;
+    if (row >= (gs->M + blk - 1) / blk * blk) return;
+    const int c0 = blk * max(0, i - back), c1 = blk * (i + 1);
+    uint4* p = reinterpret_cast<uint4*>(A + row * ld_bytes + (size_t)c0 * esize);
+    for (int k = threadIdx.x & 31; k < (c1 - c0) * esize / 16; k += 32) p[k] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+void launch_clear_band(void* A, int ld, int esize, int rows, int blk, int back, const GridState* gs, cudaStream_t st)
+{
+    k_clear_band<<<(rows + 7) / 8, 256, 0, st>>>((char*)A, (size_t)ld * esize, esize, blk, back, gs);
+    count_launches(1);
+}
+
+__global__ void __launch_bounds__(256) k_copy_square(char* __restrict__ dst, const char* __restrict__ src,
+                                                     size_t ld_bytes, int esize, int blk,
+                                                     const GridState* __restrict__ gs)
+{
+    const int Mp = (gs->M + blk - 1) / blk * blk, row = blockIdx.x;
+    if (row >= Mp) return;
+    const uint4* s = reinterpret_cast<const uint4*>(src + row * ld_bytes);
+    uint4* d = reinterpret_cast<uint4*>(dst + row * ld_bytes);
+    // the lower triangle, in whole blocks
+    const int n = blk * (row / blk + 1) * esize / 16;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) d[k] = s[k];
+}
+
+void launch_copy_square(void* dst, const void* src, int ld, int esize, int blk, const GridState* gs, int rows,
+                        cudaStream_t st)
+{
+    k_copy_square<<<rows, 256, 0, st>>>((char*)dst, (const char*)src, (size_t)ld * esize, esize, blk, gs);
+    count_launches(1);
+}
+
 // ---- data and inverse-variance per active row ----
 __global__ void k_dvec(StaticData sd, const GridState* __restrict__ gs, const int* __restrict__ rowpix,
                        double* __restrict__ dvec, double* __restrict__ cvec)
@@ -139,7 +236,6 @@ __global__ void k_reg(const GridState* __restrict__ gs, const int* __restrict__ 
 void launch_regularization(const SrcOpts& so, Work& w, int M_max, const double* regp, int parts, cudaStream_t st)
 {
     const int ncell = so.snx * so.sny;
-    if (so.regularization && (parts & REG_R)) cudaMemsetAsync(w.R, 0, sizeof(double) * (size_t)w.ldF * w.ldF, st);
     int total = ncell + 64;
     k_reg<<<(total + 255) / 256, 256, 0, st>>>(w.gs, w.active_index, regp, w.F, w.R, w.ldF, so.regularization,
                                                parts);

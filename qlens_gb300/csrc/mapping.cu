@@ -204,8 +204,6 @@ __global__ void __launch_bounds__(256) k_locate(StaticData sd_, SrcOpts so_, con
 
 void launch_locate(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream_t st)
 {
-    cudaMemsetAsync(w.mapped, 0, sizeof(int) * so.snx * so.sny, st);
-    cudaMemsetAsync(w.pixmaps, 0, sizeof(int) * (sd.n_mask > 0 ? sd.n_mask : 1), st);
     if (sd.n_sub == 0) return;
     size_t smem = sizeof(double) * (2 * (so.snx + so.sny) + 2);
     int blocks = (sd.n_sub + 255) / 256;
@@ -377,8 +375,6 @@ __global__ void __launch_bounds__(256) k_compact_write(StaticData sd_, SrcOpts s
 
 void launch_compact(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream_t st)
 {
-    // pixels outside the mask keep -1 in pixindex
-    cudaMemsetAsync(w.pixindex, 0xff, sizeof(int) * sd.nx * sd.ny, st);
     const int nshare = std::max(1, std::min(1024, std::max((sd.n_mask + 255) / 256, (so.snx * so.sny + 255) / 256)));
     k_compact_count<<<nshare, 256, 0, st>>>(sd, so, w.mapped, w.cell3, w.pixmaps, w.cpart);
     k_compact_scan<<<1, 1024, 0, st>>>(nshare, w.cpart, w.rowptr, w.gs);
@@ -394,25 +390,28 @@ void launch_compact(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream
 // i.e. exactly the row of convert_Lmatrix_to_dense, pixelgrid.cpp:13734-13739),
 // which the PSF kernel gathers from.
 // ---------------------------------------------------------------------------
-#define BUILD_L_MAXD 192      // entries of one row merged in local arrays (3 per sub-pixel, up to 8x8 split)
+#define BUILD_L_MAXD 192      // entries of one row merged in shared memory (3 per sub-pixel, up to 8x8 split)
+#define BUILD_L_THREADS 32
 
-__global__ void __launch_bounds__(128) k_build_L(StaticData sd_, const int* __restrict__ rowidx,
+__global__ void __launch_bounds__(BUILD_L_THREADS) k_build_L(StaticData sd_, const int* __restrict__ rowidx,
                                                  const int* __restrict__ rowptr, const int* __restrict__ cell3,
                                                  const double* __restrict__ w3, const int* __restrict__ active_index,
                                                  int* __restrict__ Lidx, double* __restrict__ Lval,
                                                  int* __restrict__ cidx, double* __restrict__ cval,
                                                  int* __restrict__ ccnt)
 {
+    extern __shared__ __align__(16) unsigned char build_smem[];
     const StaticData sd = eval_shape(sd_);
     const int nsub = sd.nsub;
     if (3 * nsub <= BUILD_L_MAXD) {
         // one pass: each entry is written to the CSR row and merged at once
-        // into the row's distinct cells, kept in this thread's local arrays
-        // (a search over the distinct cells so far, not over all entries);
-        // a cell's sum starts from 0.0 and adds its entries in CSR order, and
-        // the distinct cells keep their first-occurrence order
-        int di[BUILD_L_MAXD];
-        double dv[BUILD_L_MAXD];
+        // into the row's distinct cells (a search over the distinct cells so
+        // far, not over all entries); a cell's sum starts from 0.0 and adds its
+        // entries in CSR order, and the distinct cells keep their
+        // first-occurrence order.  A thread's distinct cells sit in shared
+        // memory, entry-major (as local arrays they took 2.3 KB of stack a thread).
+        double* dv = reinterpret_cast<double*>(build_smem) + threadIdx.x;
+        int* di = reinterpret_cast<int*>(build_smem + sizeof(double) * 3 * nsub * BUILD_L_THREADS) + threadIdx.x;
         for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < sd.n_mask; m += gridDim.x * blockDim.x) {
             const int r = rowidx[m];
             if (r < 0) continue;
@@ -430,14 +429,19 @@ __global__ void __launch_bounds__(128) k_build_L(StaticData sd_, const int* __re
                     Lval[e] = val;
                     e++;
                     int j = 0;
-                    while (j < nc && di[j] != idx) j++;
-                    if (j == nc) { di[nc] = idx; dv[nc] = 0.0 + val; nc++; }
-                    else dv[j] += val;
+                    while (j < nc && di[j * BUILD_L_THREADS] != idx) j++;
+                    if (j == nc) {
+                        di[nc * BUILD_L_THREADS] = idx;
+                        dv[nc * BUILD_L_THREADS] = 0.0 + val;
+                        nc++;
+                    } else {
+                        dv[j * BUILD_L_THREADS] += val;
+                    }
                 }
             }
             for (int j = 0; j < nc; j++) {
-                cidx[e0 + j] = di[j];
-                cval[e0 + j] = dv[j];
+                cidx[e0 + j] = di[j * BUILD_L_THREADS];
+                cval[e0 + j] = dv[j * BUILD_L_THREADS];
             }
             ccnt[r] = nc;
         }
@@ -480,10 +484,18 @@ void launch_build_L(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream
     if (sd.n_mask == 0) return;
     // a thread per masked pixel, each a long serial merge: 32-thread CTAs spread
     // the few warps over all SMs
-    int blocks = (sd.n_mask + 31) / 32;
-    k_build_L<<<blocks, 32, 0, st>>>(sd, w.rowidx, w.rowptr, w.cell3, w.w3, w.active_index, w.Lidx, w.Lval, w.cidx,
-                                      w.cval, w.ccnt);
+    const int blocks = (sd.n_mask + BUILD_L_THREADS - 1) / BUILD_L_THREADS;
+    const size_t smem = 3 * sd.nsub <= BUILD_L_MAXD ? (sizeof(double) + sizeof(int)) * 3 * sd.nsub * BUILD_L_THREADS : 0;
+    k_build_L<<<blocks, BUILD_L_THREADS, smem, st>>>(sd, w.rowidx, w.rowptr, w.cell3, w.w3, w.active_index, w.Lidx,
+                                                     w.Lval, w.cidx, w.cval, w.ccnt);
     count_launches(1);
+}
+
+// (the 8x8 split's distinct cells need more than 48 KB)
+void mapping_init_attributes()
+{
+    cudaFuncSetAttribute(k_build_L, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(double) + sizeof(int)) * BUILD_L_MAXD * BUILD_L_THREADS);
 }
 
 }  // namespace qlpix

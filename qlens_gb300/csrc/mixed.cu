@@ -27,6 +27,8 @@
 
 namespace qlpix {
 
+#define MIXED_SOLVES 5    // solves of one evaluation: one and up to four refinement sweeps
+
 struct MixedWork {
     double* t = nullptr;     // N (image-plane scratch)
     // L by source cell (CSC of the merged pre-PSF rows), for k_psf_x
@@ -60,18 +62,14 @@ struct MixedWork {
     double* y = nullptr;     // M (solve scratch)
     double* img = nullptr;   // npix_pad: dense padded image for the FP64 convolutions
     float* linvF = nullptr;  // per 128-block of F: inverse of its diagonal factor, then its transpose
-    float* linv128 = nullptr; // the same for R's current diagonal block
     float* yf = nullptr;     // M_cap: forward-solve result
     float* zf = nullptr;     // M_cap: backward-solve result (FP32 copy read by other CTAs)
-    int* flags = nullptr;    // 2 x nb: per-block "published" flags of the two sweeps
+    int* flags = nullptr;    // per solve 2 x nb: per-block "published" flags of the two sweeps
     int nb = 0;              // 128-blocks of M_cap
     CUtensorMap map_hi, map_lo;
-    // the Cholesky's current panel, split for its trailing update (k_chol_upd16):
-    // F16 hi + lo [M_cap][128] and the scale exponent of each row;
-    // one set for F, one for R (factored concurrently on the side stream)
-    __half* Pf_hi = nullptr; __half* Pf_lo = nullptr; int* Pf_exp = nullptr;
-    __half* Pr_hi = nullptr; __half* Pr_lo = nullptr; int* Pr_exp = nullptr;
-    CUtensorMap map_pf_hi, map_pf_lo, map_pr_hi, map_pr_lo;
+    // the factorisations of F and R (k_chol128; concurrent, R on the side stream)
+    Flow128Mem cf{}, cr{};
+    CUtensorMap cf_maps[4], cr_maps[4];   // the split factor hi, lo and the split inverses hi, lo
     bool ready = false;
 };
 
@@ -875,9 +873,10 @@ void mixed_free(Slot& c)
     MixedWork* m = mw_of(c);
     if (!m) return;
     void* ptrs[] = {m->t, m->X_hi, m->X_lo, m->nz, m->F32, m->R32, m->u, m->v, m->r, m->z, m->y, m->img,
-                    m->linvF, m->linv128, m->yf, m->zf, m->flags, m->colcnt, m->cursor, m->colrow, m->colval,
-                    m->sqc, m->col_u, m->src_u, m->colval64, m->pixT, m->F0, m->Pf_hi, m->Pf_lo, m->Pf_exp,
-                    m->Pr_hi, m->Pr_lo, m->Pr_exp, m->psfx_meta};
+                    m->linvF, m->yf, m->zf, m->flags, m->colcnt, m->cursor, m->colrow, m->colval,
+                    m->sqc, m->col_u, m->src_u, m->colval64, m->pixT, m->F0, m->psfx_meta,
+                    m->cf.Lh, m->cf.Ll, m->cf.pexp, m->cf.ih, m->cf.il, m->cf.flags,
+                    m->cr.Lh, m->cr.Ll, m->cr.pexp, m->cr.ih, m->cr.il, m->cr.flags};
     for (void* p : ptrs) if (p) cudaFree(p);
     delete m;
     c.mixed = nullptr;
@@ -899,6 +898,18 @@ static void psfx_band_geom(int nx, int ny, int pnx, int pny, int split, int& H, 
     smem = sizeof(long long) * (size_t)H * W + tap_bytes;
 }
 
+static size_t flow128_flags(int nb) { return (size_t)nb * nb + nb + 1; }
+
+static int flow_maps(const Flow128Mem& f, CUtensorMap* maps)
+{
+    for (int k = 0; k < 2; k++) {
+        int r = make_map(&maps[k], k ? f.Ll : f.Lh, f.rows, f.rows, true);
+        if (r == QLP_OK) r = make_map(&maps[2 + k], k ? f.il : f.ih, f.rows, C2, false);
+        if (r != QLP_OK) return r;
+    }
+    return QLP_OK;
+}
+
 int mixed_init(Slot& c)
 {
     MixedWork* m = mw_of(c);
@@ -917,7 +928,7 @@ int mixed_init(Slot& c)
     const size_t xbytes = (m->half ? 2 : 4) * (size_t)M_cap * K_cap;
     A((void**)&m->X_hi, xbytes);
     A((void**)&m->X_lo, xbytes);
-    A((void**)&m->nz, (size_t)(M_cap / TC_TILE) * m->nkb_cap);
+    A((void**)&m->nz, (size_t)(M_cap / TC_TILE) * m->nkb_cap + 3);
     {
         int H = 1;
         size_t sm = 0;
@@ -945,16 +956,18 @@ int mixed_init(Slot& c)
     A((void**)&m->y, sizeof(double) * M_cap);
     m->nb = M_cap / C2;
     A((void**)&m->linvF, sizeof(float) * (size_t)m->nb * 2 * C2 * C2);
-    A((void**)&m->linv128, sizeof(float) * 2 * C2 * C2);
     A((void**)&m->yf, sizeof(float) * (size_t)M_cap);
     A((void**)&m->zf, sizeof(float) * (size_t)M_cap);
-    A((void**)&m->flags, sizeof(int) * (size_t)2 * m->nb);
-    A((void**)&m->Pf_hi, sizeof(__half) * (size_t)M_cap * C2);
-    A((void**)&m->Pf_lo, sizeof(__half) * (size_t)M_cap * C2);
-    A((void**)&m->Pr_hi, sizeof(__half) * (size_t)M_cap * C2);
-    A((void**)&m->Pr_lo, sizeof(__half) * (size_t)M_cap * C2);
-    A((void**)&m->Pf_exp, sizeof(int) * (size_t)M_cap);
-    A((void**)&m->Pr_exp, sizeof(int) * (size_t)M_cap);
+    A((void**)&m->flags, sizeof(int) * (size_t)2 * m->nb * MIXED_SOLVES);
+    for (Flow128Mem* f : {&m->cf, &m->cr}) {
+        f->rows = M_cap;
+        A((void**)&f->Lh, sizeof(__half) * (size_t)M_cap * M_cap);
+        A((void**)&f->Ll, sizeof(__half) * (size_t)M_cap * M_cap);
+        A((void**)&f->pexp, sizeof(int) * (size_t)m->nb * M_cap);
+        A((void**)&f->ih, sizeof(float) * (size_t)M_cap * C2);
+        A((void**)&f->il, sizeof(float) * (size_t)M_cap * C2);
+        A((void**)&f->flags, sizeof(int) * flow128_flags(m->nb));
+    }
     if (e != cudaSuccess) {
         set_error("%s (%d)", "mixed-precision workspace allocation failed", (int)e);
         return QLP_ERR_NOMEM;
@@ -963,10 +976,7 @@ int mixed_init(Slot& c)
     cudaMemset(m->X_lo, 0, xbytes);
     if (make_map(&m->map_hi, m->X_hi, M_cap, K_cap, m->half) != QLP_OK ||
         make_map(&m->map_lo, m->X_lo, M_cap, K_cap, m->half) != QLP_OK ||
-        make_map(&m->map_pf_hi, m->Pf_hi, M_cap, C2, true) != QLP_OK ||
-        make_map(&m->map_pf_lo, m->Pf_lo, M_cap, C2, true) != QLP_OK ||
-        make_map(&m->map_pr_hi, m->Pr_hi, M_cap, C2, true) != QLP_OK ||
-        make_map(&m->map_pr_lo, m->Pr_lo, M_cap, C2, true) != QLP_OK) {
+        flow_maps(m->cf, m->cf_maps) != QLP_OK || flow_maps(m->cr, m->cr_maps) != QLP_OK) {
         set_error("%s (%d)", "cuTensorMapEncodeTiled unavailable or failed", 0);
         return QLP_ERR_CUDA;
     }
@@ -982,9 +992,7 @@ int mixed_init(Slot& c)
         opt((const void*)k_psf_x_rows, 227 * 1024);
         opt((const void*)k_psf_x_band<true>, 227 * 1024);
         opt((const void*)k_psf_x_band<false>, 227 * 1024);
-        opt((const void*)k_potrf128, P128_SMEM);
-        opt((const void*)k_chol_tile128, T128_SMEM);
-        opt((const void*)k_chol_upd16, U16_SMEM);
+        opt((const void*)k_chol128, C2_SMEM);
         opt((const void*)k_syrk_tc<false>, TC_SMEM);
         opt((const void*)k_syrk_tc<true>, TC_SMEM);
         if (ea != cudaSuccess) {
@@ -996,32 +1004,18 @@ int mixed_init(Slot& c)
     return QLP_OK;
 }
 
-// FP32 blocked Cholesky for the mixed path (chol128.cuh): per 128-column step
-// the diagonal factor and its inverse in one CTA, the panel solve on the
-// tensor cores (which also leaves the panel split into F16 hi + lo in
-// P_hi / P_lo, addressed by map_hi / map_lo), and the trailing update from
-// that split panel on the tensor cores.  band: 128-blocks below the diagonal
-// that can be nonzero (the whole matrix for F).  The inverse of diagonal
-// block k goes to linv + k * linv_stride (stride 0: one scratch block).
-static int cholesky_mixed(float* A, int ld, int M_cap128, GridState* gs, int which, int band, float* linv,
-                          size_t linv_stride, __half* P_hi, __half* P_lo, int* pexp, const CUtensorMap& map_hi,
-                          const CUtensorMap& map_lo, cudaStream_t st)
+// FP32 Cholesky of the mixed path (k_chol128).  band: 128-blocks below the
+// diagonal that can be nonzero (the whole matrix for F); linv: per diagonal
+// block its inverse and the inverse's transpose for the solves, or null; ctas:
+// the grid's size.
+static void cholesky_mixed(float* A, int ld, GridState* gs, int which, int band, float* linv, const Flow128Mem& f,
+                           const CUtensorMap* maps, int ctas, cudaStream_t st)
 {
-    const int nb = M_cap128 / C2;
-    int n = 0;
-    for (int k = 0; k < nb; k++) {
-        float* lk = linv + (size_t)k * linv_stride;
-        k_potrf128<<<1, 256, P128_SMEM, st>>>(A, ld, k, gs, which, lk);
-        n++;
-        const int rem = nb - k - 1;
-        if (rem == 0) break;
-        const int bt = std::min(rem, band);
-        k_chol_tile128<<<bt, 128, T128_SMEM, st>>>(A, ld, k, gs, 1, lk, band, P_hi, P_lo, pexp);
-        k_chol_upd16<<<bt * (bt + 1) / 2, 128, U16_SMEM, st>>>(map_hi, map_lo, A, ld, k, gs, pexp, band);
-        n += 2;
-    }
-    count_launches(n);
-    return n;
+    const int nb = f.rows / C2;
+    const int tiles = nb * std::min(nb, band + 1);
+    ctas = std::min(tiles, ctas);
+    k_chol128<<<ctas, C2_THREADS, C2_SMEM, st>>>(maps[0], maps[1], maps[2], maps[3], A,
+                                                                             ld, gs, which, band, f, linv);
 }
 
 // The lambda optimisation's F0 = X X^T (before lambda R): allocated outside
@@ -1040,6 +1034,20 @@ int mixed_ensure_f0(Slot& slot)
     return QLP_OK;
 }
 
+// What an evaluation (or one lambda trial) starts from cleared.
+void mixed_clear(Slot& slot, ClearList& l, bool trial)
+{
+    MixedWork* m = mw_of(slot);
+    l.add(m->cf.flags, sizeof(int) * flow128_flags(m->nb));
+    l.add(m->flags, sizeof(int) * (size_t)2 * m->nb * MIXED_SOLVES);
+    if (trial) return;
+    l.add(m->cr.flags, sizeof(int) * flow128_flags(m->nb));
+    l.add(m->nz, (size_t)(m->M_cap / TC_TILE) * m->nkb_cap);
+    l.add(m->colcnt, sizeof(int) * (size_t)(m->M_cap + 1));
+    l.add(m->pixT, sizeof(int2) * (size_t)slot.npix_pad, 0xffffffffu);
+    l.add(m->img, sizeof(double) * (size_t)slot.npix_pad);
+}
+
 // part: PIPE_ALL the whole inversion at the slot's lambda; PIPE_PRE everything
 // that does not depend on lambda (D, X, F0 = X X^T kept aside, R and its log
 // det); PIPE_TRIAL one lambda of the optimisation (F = F0 + lambda R, its
@@ -1054,7 +1062,6 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
     Work& w = slot.w;
     const int N_cap = sd.n_mask;
     const int Mc = slot.M_cap;
-    const size_t f_bytes = sizeof(float) * (size_t)m->ld32 * m->M_cap;
     const int ltw_blocks = (m->M_cap + 7) / 8;
     int n = 0;
     if (part != PIPE_ALL && !m->F0) {
@@ -1062,19 +1069,35 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
         return QLP_ERR_ARG;
     }
     if (part == PIPE_TRIAL) {
-        cudaMemsetAsync(&w.gs->not_spd_F, 0, sizeof(int), st);
-        cudaMemcpyAsync(m->F32, m->F0, f_bytes, cudaMemcpyDeviceToDevice, st);
+        ClearList cl;
+        cl.add(&w.gs->not_spd_F, sizeof(int));
+        mixed_clear(slot, cl, true);
+        launch_clear(cl, st);
+        launch_copy_square(m->F32, m->F0, m->ld32, 4, C2, w.gs, m->M_cap, st);
         k_reg32<<<(so.snx * so.sny + 128 + 255) / 256, 256, 0, st>>>(w.gs, w.active_index, regp, m->F32, m->R32,
                                                                     m->ld32, so.regularization, REG_F);
         n++;
     } else {
 
+    if (so.regularization) {
+        // R hangs on the active cells alone: its factorisation (log det R only)
+        // runs on the slot's second stream beside everything up to the evidence.
+        // R couples a cell to cells at most two grid rows (2 snx active indices)
+        // away, so its factor stays within that band.
+        const int band_R = (2 * so.snx - 1) / C2 + 1;
+        cudaEventRecord(slot.side_fork, st);
+        cudaStreamWaitEvent(slot.side, slot.side_fork, 0);
+        launch_clear_band(m->R32, m->ld32, 4, m->M_cap, C2, band_R, w.gs, slot.side);
+        k_reg32<<<(so.snx * so.sny + 128 + 255) / 256, 256, 0, slot.side>>>(w.gs, w.active_index, regp, m->F32, m->R32,
+                                                                           m->ld32, so.regularization, REG_R);
+        cholesky_mixed(m->R32, m->ld32, w.gs, 1, band_R, nullptr, m->cr, m->cr_maps, 2, slot.side);
+        k_logdet_t<float><<<1, 1024, 0, slot.side>>>(m->R32, m->ld32, w.gs, w.out, 1);
+        n += 3;
+        cudaEventRecord(slot.side_join, slot.side);
+    }
     // L by source cell (CSC, rows ascending within a column)
-    cudaMemsetAsync(m->nz, 0, (size_t)(m->M_cap / TC_TILE) * m->nkb_cap, st);
-    cudaMemsetAsync(m->colcnt, 0, sizeof(int) * (size_t)(m->M_cap + 1), st);
     {
         const int rb = std::min((N_cap + 255) / 256, 152 * 8);
-        cudaMemsetAsync(m->pixT, 0xff, sizeof(int2) * (size_t)slot.npix_pad, st);
         k_csc_count<<<std::max(rb, 1), 256, 0, st>>>(sd, w.gs, w.rowptr, w.cidx, w.ccnt, w.cvec, w.rowpix, m->colcnt,
                                                      m->sqc, m->pixT);
         k_csc_scan<<<1, 1024, 0, st>>>(w.gs, m->colcnt, m->cursor);
@@ -1152,33 +1175,18 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
         n++;
     }
     if (ev) cudaEventRecord(ev[4], st);
-    if (part == PIPE_PRE) cudaMemcpyAsync(m->F0, m->F32, f_bytes, cudaMemcpyDeviceToDevice, st);
-    if (so.regularization) cudaMemsetAsync(m->R32, 0, sizeof(float) * (size_t)m->ld32 * m->ld32, st);
-    k_reg32<<<(so.snx * so.sny + 128 + 255) / 256, 256, 0, st>>>(w.gs, w.active_index, regp, m->F32, m->R32,
-                                                                m->ld32, so.regularization,
-                                                                part == PIPE_PRE ? REG_R : (REG_F | REG_R));
-    n++;
-    if (so.regularization) {
-        // R's factorisation (log det R only) runs on the slot's second stream,
-        // beside F's.  R couples a cell to cells at most two grid rows
-        // (2 snx active indices) away, so its factor stays within that band.
-        cudaEventRecord(slot.side_fork, st);
-        cudaStreamWaitEvent(slot.side, slot.side_fork, 0);
-        const int band_R = (2 * so.snx - 1) / C2 + 1;
-        n += cholesky_mixed(m->R32, m->ld32, m->M_cap, w.gs, 1, band_R, m->linv128, 0, m->Pr_hi, m->Pr_lo,
-                            m->Pr_exp, m->map_pr_hi, m->map_pr_lo, slot.side);
-        k_logdet_t<float><<<1, 1024, 0, slot.side>>>(m->R32, m->ld32, w.gs, w.out, 1);
-        n++;
-        cudaEventRecord(slot.side_join, slot.side);
-    }
+    if (part == PIPE_PRE) launch_copy_square(m->F0, m->F32, m->ld32, 4, C2, w.gs, m->M_cap, st);
     if (part == PIPE_PRE) {
         if (so.regularization) cudaStreamWaitEvent(st, slot.side_join, 0);
         count_launches(n);
         return QLP_OK;
     }
+    k_reg32<<<(so.snx * so.sny + 128 + 255) / 256, 256, 0, st>>>(w.gs, w.active_index, regp, m->F32, m->R32,
+                                                                m->ld32, so.regularization, REG_F);
+    n++;
     }   // part != PIPE_TRIAL
-    n += cholesky_mixed(m->F32, m->ld32, m->M_cap, w.gs, 0, 1 << 20, m->linvF, (size_t)2 * C2 * C2, m->Pf_hi,
-                        m->Pf_lo, m->Pf_exp, m->map_pf_hi, m->map_pf_lo, st);
+    cholesky_mixed(m->F32, m->ld32, w.gs, 0, 1 << 20, m->linvF, m->cf, m->cf_maps, factor_ctas(c, m->nb), st);
+    n++;
     k_logdet_t<float><<<1, 1024, 0, st>>>(m->F32, m->ld32, w.gs, w.out, 0);
     n++;
     if (so.regularization && part == PIPE_ALL) cudaStreamWaitEvent(st, slot.side_join, 0);
@@ -1186,10 +1194,10 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
     k_copy_init<<<(Mc + 255) / 256, 256, 0, st>>>(w.gs, w.D, m->r, w.s);
     n++;
     for (int it = 0; it <= refine; it++) {
-        cudaMemsetAsync(m->flags, 0, sizeof(int) * (size_t)2 * m->nb, st);
-        k_trsv128_fwd<<<m->nb, 256, 0, st>>>(m->F32, m->ld32, m->linvF, w.gs, m->r, m->yf, m->flags);
+        int* const tf = m->flags + (size_t)it * 2 * m->nb;
+        k_trsv128_fwd<<<m->nb, 256, 0, st>>>(m->F32, m->ld32, m->linvF, w.gs, m->r, m->yf, tf);
         k_trsv128_bwd<<<m->nb, 256, 0, st>>>(m->F32, m->ld32, m->linvF, w.gs, m->yf, m->zf, m->z,
-                                              m->flags + m->nb);
+                                              tf + m->nb);
         k_axpy<<<(Mc + 255) / 256, 256, 0, st>>>(w.gs, m->z, w.s);
         n += 3;
         if (it == refine) break;

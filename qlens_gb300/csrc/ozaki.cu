@@ -305,6 +305,8 @@ int oz_alloc(OzWork** out, int N_cap, int M_cap)
     return QLP_OK;
 }
 
+void oz_clear(const OzWork* z, ClearList& l) { l.add(z->emax, sizeof(int) * z->M128); }
+
 // The digits' buffer, free once F stands.
 void* oz_buffer(OzWork* z) { return z->xs; }
 
@@ -313,7 +315,6 @@ void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaS
     OzWork* z = w.oz;
     const int nI = (M_max + OZ_TM - 1) / OZ_TM, tiles = nI * (nI + 1), ncb = 2 * nI;
     int n = 0;
-    cudaMemsetAsync(z->emax, 0, sizeof(int) * z->M128, st);
     if (N_max > 0) {
         k_oz_scan<<<dim3((N_max + 127) / 128, ncb), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, z->emax, z->nz, z->nst);
         n++;

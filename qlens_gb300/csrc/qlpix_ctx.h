@@ -7,8 +7,22 @@
 
 #define QLP_N_STAGES 6
 #define QLP_MAX_SLOTS 64
+#define QLP_LOADS 3                 // alone, a few evaluations in flight, many (load_of)
+#define QLP_JOB_RING 1024           // graph replays queued per slot (a power of two: the device's count wraps)
 
 namespace qlpix {
+
+// The launch sequence captured as a CUDA graph, sized for the slot's capacity
+// (any mask and source grid that fit), valid for one (precision, capacity, NFW,
+// NFW mode, lambda optimisation) combination and graph generation; with the
+// lambda optimisation on there is one for the lambda-independent part and one
+// for a lambda trial.
+struct SlotGraph {
+    cudaGraphExec_t exec = nullptr;
+    int key[7] = {0, 0, 0, 0, 0, 0, 0};
+    long long gen = 0;
+    long long launches = 0;         // kernels per replay
+};
 
 // One evaluation lane: a stream and the full per-evaluation workspace.  A
 // batch spreads its instances over several slots so that the sequential
@@ -30,19 +44,13 @@ struct Slot {
     // second stream of the slot: R's factorisation runs beside F's
     cudaStream_t side = nullptr;
     cudaEvent_t side_fork = nullptr, side_join = nullptr;
-    // the launch sequence captured as a CUDA graph, sized for the slot's
-    // capacity (any mask and source grid that fit), valid for one
-    // (precision, capacity, NFW, NFW mode, lambda optimisation) combination and
-    // graph generation; with the lambda optimisation on, `graph` holds the
-    // lambda-independent part and `graph_trial` one lambda trial
-    cudaGraphExec_t graph = nullptr;
-    int graph_key[7] = {0, 0, 0, 0, 0, 0, 0};
-    long long graph_gen = 0;
-    long long graph_launches = 0;   // kernels per replay
-    cudaGraphExec_t graph_trial = nullptr;
-    int trial_key[7] = {0, 0, 0, 0, 0, 0, 0};
-    long long trial_gen = 0;
-    long long trial_launches = 0;
+    SlotGraph graphs[2][QLP_LOADS];     // [a lambda trial's][load_of]
+    // what the graph's replays work on: replay number q takes entry q % QLP_JOB_RING
+    // of the ring (pinned); the device counts the replays that are done
+    Job* jobs = nullptr;
+    unsigned* job_count = nullptr;
+    unsigned long long job_no = 0;      // replays launched
+    unsigned long long job_synced = 0;  // ... at the stream's last synchronisation for the ring
     OsbWork osb{};                  // outside-surface-brightness pass (allocated when the prior is on)
     int osb_nsub = 0;               // its capacity in sub-pixels
 };
@@ -91,6 +99,8 @@ struct qlp_ctx {
     qlpix::EvalOut* h_out = nullptr;      // pinned, one per batch instance
     int h_out_cap = 0;
     qlpix::EvalOut* h_trial = nullptr;    // pinned, one per slot: results of lambda trials
+    qlpix::Job* jobs = nullptr;           // pinned: the slots' rings of jobs
+    unsigned* job_counts = nullptr;       // device: replays run, one per slot
     std::vector<double> regopt_lam;       // per batch instance: the lambda of its result
     std::vector<int> regopt_evals;        // per batch instance: lambda trials run
     cudaEvent_t ev[QLP_N_STAGES + 1] = {};
@@ -135,6 +145,7 @@ int ctx_eval_batch(qlp_ctx* c, const double* params, const double* regparams, co
 int ctx_dump(qlp_ctx* c, double* srcpt_xy, int* L_rowptr, int* L_index, double* L_value, int* active_index,
              double* D, double* s, double* model);
 int ctx_dump_Lpsf(qlp_ctx* c, int rows, double* out);
+int factor_ctas(const qlp_ctx* c, int nb);
 int make_lens_rec(LensRec& L, const qlp_lens& d, const double* p);
 int fit_set(qlp_ctx* c, const qlp_fit_param* fp, int n);
 int fit_loglike_batch(qlp_ctx* c, const double* x, int n, double* loglike, qlp_result* out);
@@ -152,6 +163,7 @@ void mixed_free(Slot& slot);
 #define PIPE_PRE 1
 #define PIPE_TRIAL 2
 int mixed_ensure_f0(Slot& slot);
+void mixed_clear(Slot& slot, ClearList& l, bool trial);
 int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, const SrcOpts& so, const double* regp,
                         int part, cudaStream_t st,
                         cudaEvent_t* ev);

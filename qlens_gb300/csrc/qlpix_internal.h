@@ -76,6 +76,13 @@ struct EvalOut {
     double osb_penalty;                // the outside-surface-brightness prior's penalty (0 when off)
 };
 
+// One graph replay: where its parameters come from and its result goes (pinned
+// host memory; out null: nowhere).
+struct Job {
+    const EvalParams* ep;
+    EvalOut* out;
+};
+
 // The outside-surface-brightness prior (QLens 'outside_sb_prior'): static
 // tables of the extended mask, uploaded once per setting.
 struct OsbStatic {
@@ -198,7 +205,7 @@ struct Work {
     int* fb_ray;  double* fb_xy;  int* fb_count;
     double* nfw_xy;                    // 2 n_sub: rays' positions on the NFW lens's plane (k_ray_pre)
     float* sur_eps;                    // n_sub: bound on each ray's source-point error on the surrogate path
-    int* xlist;  int* xcount;          // n_sub, 1: rays the surrogate path traces again exactly
+    int* xlist;  int* xcount;          // n_sub, 2 (per step): rays the surrogate path traces again exactly
     double* F0;                        // plain path, lambda optimisation: L'^T C^-1 L' before lambda R
 };
 
@@ -219,14 +226,34 @@ void launch_psf(const StaticData& sd, const SrcOpts& so, Work& w, int M_max, cud
 void op_Ls(Work& w, int N_cap, const double* s, double* t, cudaStream_t st);
 void op_conv(const StaticData& sd, Work& w, int N_cap, bool transpose, const double* in, const double* scale_in,
              double* out, double* img, const int2* pixT, cudaStream_t st);
+// Buffers that an evaluation starts from cleared, in one kernel (not memset
+// nodes: see issue_eval).
+struct ClearItem { void* p; unsigned words, value; };
+struct ClearList {
+    ClearItem item[16];
+    int n = 0;
+    void add(void* p, size_t bytes, unsigned value = 0) { item[n++] = ClearItem{p, (unsigned)((bytes + 3) / 4), value}; }
+};
+void launch_clear(const ClearList& l, cudaStream_t st);
+// columns [blk max(0, i - back), blk (i + 1)) of every row of block row i = row / blk, rows below the padded M
+void launch_clear_band(void* A, int ld, int esize, int rows, int blk, int back, const GridState* gs, cudaStream_t st);
+// the lower triangle of the padded M, in whole blk x blk blocks, from src to dst
+void launch_copy_square(void* dst, const void* src, int ld, int esize, int blk, const GridState* gs, int rows,
+                        cudaStream_t st);
+// a graph's first and last kernel: the parameters of its job into ep (trial:
+// lambda only), its result to the job's place
+void launch_job_in(const Job* jobs, unsigned ring, unsigned* count, EvalParams* ep, bool trial, cudaStream_t st);
+void launch_job_out(const Job* jobs, unsigned ring, unsigned* count, const EvalOut* out, cudaStream_t st);
 void launch_dvec(const StaticData& sd, Work& w, int N_max, cudaStream_t st);
 void launch_D(Work& w, int N_max, int M_max, cudaStream_t st);
 void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st);
 int oz_alloc(OzWork** out, int N_cap, int M_cap);
 void oz_free(OzWork* z);
+void oz_clear(const OzWork* z, ClearList& l);
 void* oz_buffer(OzWork* z);
 int chol64_alloc(Chol64Work** out, int M_cap, void* shared);
 void chol64_free(Chol64Work* z);
+void chol64_clear(const Chol64Work* z, ClearList& l);
 // parts: REG_F adds lambda R to F, REG_R writes R (both: the plain evaluation)
 #define REG_F 1
 #define REG_R 2

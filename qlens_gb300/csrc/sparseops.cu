@@ -197,13 +197,12 @@ void op_Ls(Work& w, int N_cap, const double* s, double* t, cudaStream_t st)
 }
 
 // out = P in, or P^T (scale .* in) when transpose; img: scratch of
-// (nx + 2 (pnx/2)) (ny + 2 (pny/2)) doubles; pixT: the active row of every
+// (nx + 2 (pnx/2)) (ny + 2 (pny/2)) doubles, cleared at the start of the
+// evaluation (every scatter writes the same active pixels); pixT: the active row of every
 // padded-image pixel (-1 elsewhere)
 void op_conv(const StaticData& sd, Work& w, int N_cap, bool transpose, const double* in, const double* scale_in,
              double* out, double* img, const int2* pixT, cudaStream_t st)
 {
-    const size_t npad = (size_t)(sd.nx + 2 * (sd.pnx / 2)) * (sd.ny + 2 * (sd.pny / 2));
-    cudaMemsetAsync(img, 0, sizeof(double) * npad, st);
     const size_t smem_df = conv_df_smem(sd.pnx, sd.pny);
     if (smem_df <= 160 * 1024) {
         float2* img2 = reinterpret_cast<float2*>(img);

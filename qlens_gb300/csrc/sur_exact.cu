@@ -233,21 +233,21 @@ int launch_surrogate_exact(const StaticData& sd, const SrcOpts& so, Work& w, dou
 {
     if (sd.n_sub == 0) return QLP_OK;
     if (step == 0 && !so.auto_grid) return QLP_OK;
-    cudaMemsetAsync(w.xcount, 0, sizeof(int), st);
+    int* const xcount = w.xcount + (step != 0);
     if (step == 0) {
         const int blocks = std::max(1, std::min((sd.n_mask + 255) / 256, 152 * 8));
         k_sur_exact_extremes<<<blocks, 256, 0, st>>>(sd, so, w.spx, w.spy, w.sur_eps, w.gs, eps_g,
-                                                      &w.out->n_exact, w.xlist, w.xcount);
+                                                      &w.out->n_exact, w.xlist, xcount);
     } else {
         const size_t smem = (sizeof(double) + sizeof(float)) * (2 * (so.snx + so.sny) + 2);
         const int blocks = std::max(1, std::min((sd.n_sub + 255) / 256, 152 * 8));
         k_sur_exact_cells<<<blocks, 256, smem, st>>>(sd, so, w.spx, w.spy, w.sur_eps, w.cx, w.cy, w.ccx, w.ccy,
-                                                     &w.out->n_exact, w.xlist, w.xcount);
+                                                     &w.out->n_exact, w.xlist, xcount);
     }
     // the listed rays: 2 CTAs per SM of 8 warps, a warp per ray
     const size_t wb = sizeof(double) * (SUR_EXACT_THREADS / 32) * SUR_EXACT_WBUF;
     k_sur_exact_trace<<<152 * 2, SUR_EXACT_THREADS, wb, st>>>(sd, w.ep, w.spx, w.spy, w.sur_eps, w.xlist,
-                                                              w.xcount);
+                                                              xcount);
     count_launches(2);
     return QLP_OK;
 }

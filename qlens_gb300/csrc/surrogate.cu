@@ -1560,7 +1560,6 @@ int launch_raytrace_sur(const StaticData& sd, Work& w, double thresh, int defer_
         return QLP_ERR_ARG;
     }
     SurState& S = g_sur[dev];
-    cudaMemsetAsync(w.fb_count, 0, sizeof(int), st);
     const SurRayOut q{w.fb_count, w.fb_ray, w.fb_xy};
     int n = 1;
     if (defer_lens >= 0) {
