@@ -98,10 +98,11 @@ namespace qlpix {
 
 // LensProfile::deflection (profile.cpp:1782-1805); Shear::deflection (models.cpp:2266-2272).
 // NFW = false compiles the kernel without the quadrature (no NFW lens in the model).
-// wbuf: see nfw_deflection (null: one ray per thread).
+// wbuf, tab: see nfw_deflection (null: one ray per thread; no table).
 template <bool NFW>
 __device__ __forceinline__ void lens_deflection(const LensRec& L, double x, double y, double& dx, double& dy,
-                                                const double* rho_tab = nullptr, double* wbuf = nullptr)
+                                                const double* rho_tab = nullptr, double* wbuf = nullptr,
+                                                const NfwTab* tab = nullptr)
 {
     if (L.type == QLP_LENS_SHEAR) {
         x -= L.xc; y -= L.yc;
@@ -119,7 +120,7 @@ __device__ __forceinline__ void lens_deflection(const LensRec& L, double x, doub
     }
     double ax, ay;
     if (!NFW || L.type == QLP_LENS_SPLE) sple_deflection(L, x, y, ax, ay, rho_tab);
-    else nfw_deflection(L, x, y, ax, ay, wbuf);
+    else nfw_deflection(L, x, y, ax, ay, wbuf, tab);
     if (rot) {
         double xp = ax * L.costheta - ay * L.sintheta;
         ay = ax * L.sintheta + ay * L.costheta;
@@ -160,10 +161,11 @@ __device__ __forceinline__ void subpix_centre(const StaticData& sd, int ns, int 
 
 // QLens::deflection + QLens::find_sourcept (lenscalc.cpp:81-113, 325-330).
 // rho_tab: SPLE_RHO_TAB series coefficients per lens (lens k at k *
-// SPLE_RHO_TAB), or null.
+// SPLE_RHO_TAB), or null; nfw_tab: a table per lens (nfw_tables), or null.
 template <bool NFW>
 __device__ __forceinline__ void find_sourcept(const LensModel& lm, double x, double y, double& bx, double& by,
-                                              const double* rho_tab = nullptr, double* wbuf = nullptr)
+                                              const double* rho_tab = nullptr, double* wbuf = nullptr,
+                                                const NfwTab* nfw_tab = nullptr)
 {
     double defx = 0, defy = 0;
     double dsx[QLP_MAX_PLANES], dsy[QLP_MAX_PLANES];
@@ -182,7 +184,7 @@ __device__ __forceinline__ void find_sourcept(const LensModel& lm, double x, dou
                 if (lm.lens[k].plane != i) continue;
                 double ax, ay;
                 lens_deflection<NFW>(lm.lens[k], xi, yi, ax, ay, rho_tab ? rho_tab + k * SPLE_RHO_TAB : nullptr,
-                                     wbuf);
+                                     wbuf, NFW && nfw_tab ? nfw_tab + k : nullptr);
                 dsx[i] += ax; dsy[i] += ay;
             }
             dsx[i] *= lm.zfac[i];

@@ -61,6 +61,8 @@ __global__ void __launch_bounds__(256) k_osb_rays(StaticData sd, const EvalParam
         const LensRec& L = lm.lens[e / SPLE_RHO_TAB];
         rho_tab[e] = (L.type == QLP_LENS_SPLE && L.kind == 2) ? sple_rho(L, e % SPLE_RHO_TAB + 1) : 0.0;
     }
+    __shared__ NfwTab nfw_tab[NFW ? QLP_MAX_LENSES : 1];
+    if (NFW) nfw_tables(lm, nfw_tab);
     __syncthreads();
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < os.nsub_e; t += gridDim.x * blockDim.x) {
         const int e = owner(os.eoff, os.ne, t);
@@ -74,7 +76,7 @@ __global__ void __launch_bounds__(256) k_osb_rays(StaticData sd, const EvalParam
         const double px = (1 - u0) * sd.xvals[i] + u0 * sd.xvals[i + 1];
         const double py = (1 - w0) * sd.yvals[j] + w0 * sd.yvals[j + 1];
         double bx, by;
-        find_sourcept<NFW>(lm, px, py, bx, by, rho_tab);
+        find_sourcept<NFW>(lm, px, py, bx, by, rho_tab, nullptr, NFW ? nfw_tab : nullptr);
         sp[2 * t] = bx;
         sp[2 * t + 1] = by;
     }

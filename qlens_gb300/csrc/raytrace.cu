@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256) k_raytrace(StaticData sd_, const EvalPara
     // the sub-pixel fractions u0 = (1 + 2 ii) / (2 ns) and 1 - u0, formed once
     // per CTA by the same expressions (the same bits): no FP64 divide per ray
     __shared__ double frac_u[SUBPIX_TAB], frac_1mu[SUBPIX_TAB];
+    __shared__ NfwTab nfw_tab[NFW ? QLP_MAX_LENSES : 1];
     {
         const double* src = reinterpret_cast<const double*>(&ep->lm);
         double* dst = reinterpret_cast<double*>(&lm);
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(256) k_raytrace(StaticData sd_, const EvalPara
     }
     const int ns = sd.nsplit, nsub = sd.nsub;
     subpix_table(ns, frac_u, frac_1mu);
+    if (NFW) nfw_tables(lm, nfw_tab);
     __syncthreads();
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < sd.n_sub; t += gridDim.x * blockDim.x) {
         int m = t / nsub, k = t - m * nsub;
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(256) k_raytrace(StaticData sd_, const EvalPara
         double px, py;
         subpix_centre(sd, ns, ii, jj, i, j, frac_u, frac_1mu, px, py);
         double bx, by;
-        find_sourcept<NFW>(lm, px, py, bx, by, rho_tab);
+        find_sourcept<NFW>(lm, px, py, bx, by, rho_tab, nullptr, NFW ? nfw_tab : nullptr);
         spx[t] = bx;
         spy[t] = by;
     }

@@ -1108,9 +1108,13 @@ __global__ void k_nfw_fallback(const EvalParams* __restrict__ ep, int lens, cons
     const int n = *fb_count;
     const LensRec& L = ep->lm.lens[lens];
     const double z = ep->lm.zfac[L.plane];
+    if ((int)(blockIdx.x * blockDim.x) >= n) return;
+    __shared__ NfwTab tab;
+    for (int i = threadIdx.x; i < NFW_KEEP; i += blockDim.x) nfw_node_lens(L, 8 * i + 7, tab.uq[i], tab.rq[i], tab.c0[i]);
+    __syncthreads();
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         double bx, by;
-        nfw_deflection(L, fb_xy[2 * (size_t)e], fb_xy[2 * (size_t)e + 1], bx, by);
+        nfw_deflection(L, fb_xy[2 * (size_t)e], fb_xy[2 * (size_t)e + 1], bx, by, nullptr, &tab);
         if (L.sintheta != 0) {
             const double xp = bx * L.costheta - by * L.sintheta;
             by = bx * L.sintheta + by * L.costheta;
