@@ -260,95 +260,6 @@ __global__ void k_sur_affine(int n, float* __restrict__ T, float mu0, float mu1,
     }
 }
 
-// ---------------------------------------------------------------------------
-// training: FP32 SIMT GEMM C[M][N] = op(A)[M][K] op(B)[K][N] with generic
-// strides, 64x64 tiles, 256 threads, 4x4 outputs per thread, and epilogues
-//   EPI_STORE      C = acc
-//   EPI_TANH       C = tanh(acc + bias)       hidden layer, forward
-//   EPI_BIAS       C = acc + bias             output layer, forward
-//   EPI_DTANH      C = acc * (1 - Aux^2)      backward through tanh
-// gridDim.z > 1 splits K: split z writes C + z * M * N.
-// ---------------------------------------------------------------------------
-#define EPI_STORE 0
-#define EPI_TANH 1
-#define EPI_BIAS 2
-#define EPI_DTANH 3
-
-template <int EPI>
-__global__ void __launch_bounds__(256) k_sur_gemm(int M, int N, int K, const float* __restrict__ A, int a_rs, int a_cs,
-                                                  const float* __restrict__ B, int b_rs, int b_cs,
-                                                  float* __restrict__ C, const float* __restrict__ bias,
-                                                  const float* __restrict__ aux)
-{
-    __shared__ float As[16][64 + 4];
-    __shared__ float Bs[16][64 + 4];
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    const int ksplit = (K + gridDim.z - 1) / gridDim.z;
-    const int kbeg = blockIdx.z * ksplit, kend = min(K, kbeg + ksplit);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    for (int k0 = kbeg; k0 < kend; k0 += 16) {
-        for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-            const int kk = e >> 6, mm = e & 63;
-            const int gm = m0 + mm, gk = k0 + kk;
-            As[kk][mm] = (gm < M && gk < kend) ? A[(size_t)gm * a_rs + (size_t)gk * a_cs] : 0.f;
-            const int gn = n0 + mm;
-            Bs[kk][mm] = (gn < N && gk < kend) ? B[(size_t)gk * b_rs + (size_t)gn * b_cs] : 0.f;
-        }
-        __syncthreads();
-        #pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            float a[4], b[4];
-            #pragma unroll
-            for (int u = 0; u < 4; u++) { a[u] = As[kk][ty * 4 + u]; b[u] = Bs[kk][tx * 4 + u]; }
-            #pragma unroll
-            for (int u = 0; u < 4; u++)
-                #pragma unroll
-                for (int v = 0; v < 4; v++) acc[u][v] = __fmaf_rn(a[u], b[v], acc[u][v]);
-        }
-        __syncthreads();
-    }
-    float* Cz = C + (size_t)blockIdx.z * M * N;
-    #pragma unroll
-    for (int u = 0; u < 4; u++)
-        #pragma unroll
-        for (int v = 0; v < 4; v++) {
-            const int gm = m0 + ty * 4 + u, gn = n0 + tx * 4 + v;
-            if (gm >= M || gn >= N) continue;
-            float x = acc[u][v];
-            if (EPI == EPI_TANH) x = sur_tanh(x + bias[gn]);
-            else if (EPI == EPI_BIAS) x = x + bias[gn];
-            else if (EPI == EPI_DTANH) { const float a = aux[(size_t)gm * N + gn]; x = x * (1.f - a * a); }
-            Cz[(size_t)gm * N + gn] = x;
-        }
-}
-
-// out[i] = sum_z part[z][i] in order (deterministic split-K reduction)
-__global__ void k_sur_reduce(int n, int nz, const float* __restrict__ part, float* __restrict__ out)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int z = 0; z < nz; z++) s += part[(size_t)z * n + i];
-        out[i] = s;
-    }
-}
-
-// bias gradients: column sums of D [rows][n], one block per column, fixed order
-__global__ void __launch_bounds__(256) k_sur_colsum(int rows, int n, const float* __restrict__ D, float* __restrict__ out)
-{
-    __shared__ float red[256];
-    const int c = blockIdx.x;
-    float s = 0.f;
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) s += D[(size_t)r * n + c];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[c] = red[0];
-}
-
 // output-layer gradient dL/dy = 2 w (y - t) / batch (w = 1 without weights);
 // per-block partial sums of w (y - t)^2
 __global__ void __launch_bounds__(256) k_sur_mse(int batch, const float* __restrict__ Y, const float* __restrict__ T,
@@ -372,18 +283,9 @@ __global__ void __launch_bounds__(256) k_sur_mse(int batch, const float* __restr
     if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-__global__ void k_sur_adam(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m1,
-                           float* __restrict__ m2, float lr, float b1, float b2, float c1, float c2)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float a = b1 * m1[i] + (1.f - b1) * gi;
-        const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
-        m1[i] = a;
-        m2[i] = b;
-        p[i] -= lr * (a * c1) / (sqrtf(b * c2) + 1e-8f);
-    }
-}
+}  // namespace qlpix
+#include "sur_train.cuh"
+namespace qlpix {
 
 // ---------------------------------------------------------------------------
 // inference on the tensor cores
@@ -1204,8 +1106,7 @@ __global__ void k_sur_bound(int nbins, const float* __restrict__ Tnet, const dou
     }
 }
 
-// Persistent MLP kernels: one CTA per SM at most, two 128-point groups per CTA at a time.
-static int sur_grid(int n)
+static int sur_sms()
 {
     static int sms = 0;
     if (!sms) {
@@ -1214,8 +1115,14 @@ static int sur_grid(int n)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (sms <= 0) sms = 152;
     }
+    return sms;
+}
+
+// Persistent MLP kernels: one CTA per SM at most, two 128-point groups per CTA at a time.
+static int sur_grid(int n)
+{
     const int pairs = (n + 255) / 256;
-    return std::max(1, std::min(pairs, sms));
+    return std::max(1, std::min(pairs, sur_sms()));
 }
 
 #define SCK(x)                                                                    \
@@ -1241,46 +1148,6 @@ static void sur_offsets(size_t* off, size_t* boff)
     }
 }
 
-// One forward + backward pass of the training kernels: activations in act
-// (6 x bs x 128), gradient into grad.  W (per-sample loss weights) may be null.
-static void sur_fwd_bwd(cudaStream_t s, const float* P, const float* xb, const float* tb, const float* W, int bs,
-                        float* act, float* dz, float* dz2, float* gpart, int KS, float* grad, double* lpart,
-                        int mse_blocks)
-{
-    size_t off[5], boff[5];
-    sur_offsets(off, boff);
-    float* a[6];
-    for (int l = 0; l < 6; l++) a[l] = act + (size_t)l * bs * SUR_H;
-    const float* in = xb;
-    for (int l = 0; l < 5; l++) {
-        dim3 g((g_dims[l + 1] + 63) / 64, (bs + 63) / 64, 1);
-        if (l < 4)
-            k_sur_gemm<EPI_TANH><<<g, 256, 0, s>>>(bs, g_dims[l + 1], g_dims[l], in, g_dims[l], 1, P + off[l],
-                                                   g_dims[l + 1], 1, a[l + 1], P + boff[l], nullptr);
-        else
-            k_sur_gemm<EPI_BIAS><<<g, 256, 0, s>>>(bs, 2, SUR_H, in, SUR_H, 1, P + off[l], 2, 1, a[5], P + boff[l],
-                                                   nullptr);
-        in = a[l + 1];
-    }
-    k_sur_mse<<<mse_blocks, 256, 0, s>>>(bs, a[5], tb, W, dz, lpart);
-    // backward: dcur = dL/dz of layer l; weight gradient a[l]^T dcur, bias gradient colsum(dcur)
-    float* dcur = dz;
-    float* dnext = dz2;
-    for (int l = 4; l >= 0; l--) {
-        const float* al = (l == 0) ? xb : a[l];
-        const int ni = g_dims[l], no = g_dims[l + 1];
-        dim3 gw((no + 63) / 64, (ni + 63) / 64, KS);
-        k_sur_gemm<EPI_STORE><<<gw, 256, 0, s>>>(ni, no, bs, al, 1, ni, dcur, no, 1, gpart, nullptr, nullptr);
-        k_sur_reduce<<<(ni * no + 255) / 256, 256, 0, s>>>(ni * no, KS, gpart, grad + off[l]);
-        k_sur_colsum<<<no, 256, 0, s>>>(bs, no, dcur, grad + boff[l]);
-        if (l == 0) break;
-        // dz_prev = (dcur W_l^T) * (1 - a[l]^2)
-        dim3 gb((ni + 63) / 64, (bs + 63) / 64, 1);
-        k_sur_gemm<EPI_DTANH><<<gb, 256, 0, s>>>(bs, ni, no, dcur, no, 1, P + off[l], 1, no, dnext, nullptr, a[l]);
-        std::swap(dcur, dnext);
-    }
-}
-
 int surrogate_train(int device, const qlp_surrogate_opts* o, qlp_surrogate_report* rep)
 {
     std::lock_guard<std::mutex> lock(g_sur_mu);
@@ -1294,7 +1161,7 @@ int surrogate_train(int device, const qlp_surrogate_opts* o, qlp_surrogate_repor
     const int mse_blocks = 64;
     cudaStream_t s = nullptr;
     float *X = nullptr, *T = nullptr, *Wtr = nullptr, *Xv = nullptr, *Tv = nullptr, *Tnet = nullptr, *act = nullptr;
-    float *dz = nullptr, *dz2 = nullptr, *grad = nullptr, *gpart = nullptr, *m1 = nullptr, *m2 = nullptr;
+    float *dz = nullptr, *grad = nullptr, *gpart = nullptr, *cpart = nullptr, *PT = nullptr, *m1 = nullptr, *m2 = nullptr;
     double *Gv = nullptr, *Bv = nullptr, *Qv = nullptr, *lpart = nullptr, *stats = nullptr;
     int* dstatus = nullptr;
     int rc = QLP_OK;
@@ -1321,10 +1188,11 @@ int surrogate_train(int device, const qlp_surrogate_opts* o, qlp_surrogate_repor
     SCK(cudaMalloc(&Bv, sizeof(double) * (size_t)nval));
     SCK(cudaMalloc(&Qv, sizeof(double) * (size_t)nval));
     SCK(cudaMalloc(&act, sizeof(float) * 6 * (size_t)bs * SUR_H));
-    SCK(cudaMalloc(&dz, sizeof(float) * (size_t)bs * SUR_H));
-    SCK(cudaMalloc(&dz2, sizeof(float) * (size_t)bs * SUR_H));
+    SCK(cudaMalloc(&dz, sizeof(float) * (size_t)bs * (4 * SUR_H + 2)));
     SCK(cudaMalloc(&grad, sizeof(float) * SUR_NP));
-    SCK(cudaMalloc(&gpart, sizeof(float) * (size_t)KS * SUR_H * SUR_H));
+    SCK(cudaMalloc(&gpart, sizeof(float) * st_gpart_floats(KS)));
+    SCK(cudaMalloc(&cpart, sizeof(float) * ST_CPART_FLOATS));
+    SCK(cudaMalloc(&PT, sizeof(float) * 3 * ST_HH));
     SCK(cudaMalloc(&m1, sizeof(float) * SUR_NP));
     SCK(cudaMalloc(&m2, sizeof(float) * SUR_NP));
     SCK(cudaMalloc(&lpart, sizeof(double) * mse_blocks));
@@ -1372,18 +1240,22 @@ int surrogate_train(int device, const qlp_surrogate_opts* o, qlp_surrogate_repor
     {
         const float b1 = 0.9f, b2 = 0.999f;
         double p1 = 1, p2 = 1;
+        SurTrain tr{bs, KS, (bs + KS - 1) / KS, X, T, Wtr, st.params, PT, m1, m2, grad, act, dz, gpart, cpart, lpart};
+        k_sur_transpose<<<(3 * ST_HH + 255) / 256, 256, 0, s>>>(st.params, PT);
         for (int it = 0; it < steps; it++) {
             const size_t base = ((size_t)it * bs) % (size_t)(ntr - bs + 1);
-            sur_fwd_bwd(s, st.params, X + 3 * base, T + 2 * base, Wtr + base, bs, act, dz, dz2, gpart, KS, grad,
-                        lpart, mse_blocks);
+            tr.x = X + 3 * base;
+            tr.t = T + 2 * base;
+            tr.w = Wtr + base;
+            tr.lpart = it == steps - 1 ? lpart : nullptr;
+            SCK(st_fwd_bwd(tr, sur_sms(), mse_blocks, s));
             // Adam: linear warm-up over the first 2 % of the steps, then a
             // cosine decay of the learning rate to 0.1 % of o->lr
             p1 *= b1; p2 *= b2;
             const double frac = (double)it / steps;
             const double warm = std::min(1.0, (it + 1) / (0.02 * steps + 1));
             const float lr = (float)(o->lr * warm * (0.001 + 0.999 * 0.5 * (1 + cos(M_PI * frac))));
-            k_sur_adam<<<(SUR_NP + 255) / 256, 256, 0, s>>>(SUR_NP, st.params, grad, m1, m2, lr, b1, b2,
-                                                            (float)(1.0 / (1 - p1)), (float)(1.0 / (1 - p2)));
+            st_update(tr, true, lr, b1, b2, (float)(1.0 / (1 - p1)), (float)(1.0 / (1 - p2)), s);
         }
         double hp[64];
         SCK(cudaMemcpyAsync(hp, lpart, sizeof(double) * mse_blocks, cudaMemcpyDeviceToHost, s));
@@ -1442,7 +1314,7 @@ int surrogate_train(int device, const qlp_surrogate_opts* o, qlp_surrogate_repor
         if (rep) *rep = st.rep;
     }
 done:
-    void* bufs[] = {X, T, Wtr, Xv, Tv, Tnet, Gv, Bv, Qv, act, dz, dz2, grad, gpart, m1, m2, lpart, stats, dstatus};
+    void* bufs[] = {X, T, Wtr, Xv, Tv, Tnet, Gv, Bv, Qv, act, dz, grad, gpart, cpart, PT, m1, m2, lpart, stats, dstatus};
     for (void* b : bufs)
         if (b) cudaFree(b);
     if (s) cudaStreamDestroy(s);
@@ -1458,8 +1330,8 @@ int surrogate_grad_check(int device, const float* params, const float* x, const 
 {
     if (cudaSetDevice(device) != cudaSuccess) return QLP_ERR_NO_DEVICE;
     const int bs = batch, KS = std::max(1, bs / 256), mse_blocks = 64;
-    float *P = nullptr, *X = nullptr, *T = nullptr, *act = nullptr, *dz = nullptr, *dz2 = nullptr, *grad = nullptr,
-          *gpart = nullptr;
+    float *P = nullptr, *X = nullptr, *T = nullptr, *act = nullptr, *dz = nullptr, *grad = nullptr, *gpart = nullptr,
+          *cpart = nullptr, *PT = nullptr;
     double* lpart = nullptr;
     int rc = QLP_OK;
     double hp[64];
@@ -1469,15 +1341,22 @@ int surrogate_grad_check(int device, const float* params, const float* x, const 
     SCK(cudaMalloc(&X, sizeof(float) * 3 * (size_t)bs));
     SCK(cudaMalloc(&T, sizeof(float) * 2 * (size_t)bs));
     SCK(cudaMalloc(&act, sizeof(float) * 6 * (size_t)bs * SUR_H));
-    SCK(cudaMalloc(&dz, sizeof(float) * (size_t)bs * SUR_H));
-    SCK(cudaMalloc(&dz2, sizeof(float) * (size_t)bs * SUR_H));
+    SCK(cudaMalloc(&dz, sizeof(float) * (size_t)bs * (4 * SUR_H + 2)));
     SCK(cudaMalloc(&grad, sizeof(float) * SUR_NP));
-    SCK(cudaMalloc(&gpart, sizeof(float) * (size_t)KS * SUR_H * SUR_H));
+    SCK(cudaMalloc(&gpart, sizeof(float) * st_gpart_floats(KS)));
+    SCK(cudaMalloc(&cpart, sizeof(float) * ST_CPART_FLOATS));
+    SCK(cudaMalloc(&PT, sizeof(float) * 3 * ST_HH));
     SCK(cudaMalloc(&lpart, sizeof(double) * mse_blocks));
     SCK(cudaMemcpyAsync(P, params, sizeof(float) * SUR_NP, cudaMemcpyHostToDevice, s));
     SCK(cudaMemcpyAsync(X, x, sizeof(float) * 3 * (size_t)bs, cudaMemcpyHostToDevice, s));
     SCK(cudaMemcpyAsync(T, t, sizeof(float) * 2 * (size_t)bs, cudaMemcpyHostToDevice, s));
-    sur_fwd_bwd(s, P, X, T, nullptr, bs, act, dz, dz2, gpart, KS, grad, lpart, mse_blocks);
+    {
+        const SurTrain tr{bs, KS, (bs + KS - 1) / KS, X, T, nullptr, P, PT, nullptr, nullptr, grad, act, dz, gpart, cpart,
+                          lpart};
+        k_sur_transpose<<<(3 * ST_HH + 255) / 256, 256, 0, s>>>(P, PT);
+        SCK(st_fwd_bwd(tr, sur_sms(), mse_blocks, s));
+        st_update(tr, false, 0.f, 0.f, 0.f, 0.f, 0.f, s);
+    }
     SCK(cudaGetLastError());
     SCK(cudaMemcpyAsync(hp, lpart, sizeof(double) * mse_blocks, cudaMemcpyDeviceToHost, s));
     SCK(cudaMemcpyAsync(grad_out, grad, sizeof(float) * SUR_NP, cudaMemcpyDeviceToHost, s));
@@ -1488,7 +1367,7 @@ int surrogate_grad_check(int device, const float* params, const float* x, const 
         *loss = l / bs;
     }
 done:
-    void* bufs[] = {P, X, T, act, dz, dz2, grad, gpart, lpart};
+    void* bufs[] = {P, X, T, act, dz, grad, gpart, cpart, PT, lpart};
     for (void* b : bufs)
         if (b) cudaFree(b);
     if (s) cudaStreamDestroy(s);
