@@ -215,9 +215,6 @@ int ctx_init(qlp_ctx* c, const qlp_image* im, const qlp_psf* psf, const qlp_srcg
     sd.nsub = opts->nsplit * opts->nsplit;
     sd.n_sub = sd.n_mask * sd.nsub;
     sd.pnx = psf->nx; sd.pny = psf->ny;
-    // default PSF-to-X schedule: the dense window of image rows pays off once
-    // the footprint work dominates (measured: 31x31 PSFs gain, 21x21 lose on
-    // an annular mask); the autotuner can override it
     if (c->psfx_mode < 0) c->psfx_mode = (psf->nx * psf->ny >= 500) ? 1 : 0;
     sd.use_noise_map = noise_map ? 1 : 0;
     sd.cov_inverse = cov_inverse;

@@ -35,8 +35,7 @@ struct MixedWork {
     int* colcnt = nullptr;   // M_cap + 1 counts, then the column pointers
     int* cursor = nullptr;   // M_cap
     int* colrow = nullptr;   // nnz_cap
-    float* colval = nullptr; // nnz_cap
-    float* sqc = nullptr;    // N_cap: sqrt(C^-1) per active row
+    int2* ent = nullptr;     // nnz_cap: (image column << 16 | image row, L on the grid 2^-PSFX_LEXP)
     int nnz_cap = 0;
     int2* pixT = nullptr;    // image pixels, x fastest: (active row or -1, sqrt(C^-1))
     float* F0 = nullptr;     // lambda optimisation: X X^T before lambda R (allocated on first use)
@@ -50,8 +49,9 @@ struct MixedWork {
     int M_cap = 0;           // rows of X, multiple of 128
     unsigned char* nz = nullptr;
     int nkb_cap = 0;
-    int4* psfx_meta = nullptr; // band schedule: 2 int4 per (cell, band) item (k_psfx_meta)
-    int psfx_bands = 0;        // bands it has room for
+    uint2* tiles = nullptr;    // (cell, image tile) items of the PSF-to-X build
+    unsigned* tile_active = nullptr; // bitmap of the image's tiles with active pixels, then the items' count
+    int psfx_words = 0;        // words of the bitmap
     float* F32 = nullptr;
     float* R32 = nullptr;
     int ld32 = 0;
@@ -83,15 +83,14 @@ static int make_map(CUtensorMap* map, void* base, int rows, int cols, bool half)
 
 // ---------------------------------------------------------------------------
 // X = (P L sqrt(C^-1))^T as TF32 hi + lo, and the nonzero flags of its
-// 128-cell x 32-pixel blocks, built one source cell (one row of X) at a time.
+// 128-cell x 32-pixel blocks.
 //
 // Row s of X is the PSF-convolved image of source cell s: every pixel q that
 // sees s (column s of the pre-PSF L) spreads L[q][s] over its PSF neighbours
 // p with weight psf[k][l] (the transpose of QLens's gather,
 // pixelgrid.cpp:14126-14168); the sum at p is then scaled by sqrt(C^-1) of p.
-// The sums are accumulated as 64-bit fixed point in shared memory, so they
-// are exact and independent of the order the atomics land in (the result is
-// the same bits every run): each product is the exact product of two 32-bit
+// The sums are 64-bit fixed point, so they are exact and independent of the
+// order of the entries: each product is the exact product of two 32-bit
 // integers, the tap on its grid (StaticData::psf_int) and the L entry on the
 // grid 2^-PSFX_LEXP (2^-28: 4e-9 absolute, far below FP32 resolution of the
 // entries) -- one wide multiply per tap.  No dense L' is stored.
@@ -123,7 +122,7 @@ __device__ __forceinline__ bool store_x(void* Xh, void* Xl, size_t idx, float v,
     return h != 0.0f || l != 0.0f;
 }
 
-// column counts of the merged pre-PSF L, sqrt(C^-1) per active row, and the
+// column counts of the merged pre-PSF L, the image tiles with active pixels, and the
 // image pixel -> (active row, sqrt(C^-1)) table that k_psf_x reads: x fastest,
 // with a border of half a PSF on every side so that no tap needs a bounds
 // check (pixT[(j + pny/2) * (nx + 2 (pnx/2)) + i + pnx/2]; the rows of
@@ -131,18 +130,20 @@ __device__ __forceinline__ bool store_x(void* Xh, void* Xl, size_t idx, float v,
 __global__ void k_csc_count(StaticData sd, const GridState* __restrict__ gs, const int* __restrict__ rowptr,
                             const int* __restrict__ cidx, const int* __restrict__ ccnt,
                             const double* __restrict__ cvec, const int* __restrict__ rowpix,
-                            int* __restrict__ colcnt, float* __restrict__ sqc, int2* __restrict__ pixT)
+                            int* __restrict__ colcnt, int2* __restrict__ pixT, int ntx,
+                            unsigned* __restrict__ active)
 {
     const int N = gs->N;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
         const int b = rowptr[r], n = ccnt[r];
         for (int e = 0; e < n; e++) atomicAdd(&colcnt[cidx[b + e]], 1);
         const float sq = sqrtf((float)cvec[r]);
-        sqc[r] = sq;
         const int pix = rowpix[r];
         const int i = pix / sd.ny, j = pix - i * sd.ny;
         const int nxp = sd.nx + 2 * (sd.pnx / 2);
         pixT[(size_t)(j + sd.pny / 2) * nxp + i + sd.pnx / 2] = make_int2(r, __float_as_int(sq));
+        const int tile = j / 8 * ntx + i / 32;                  // PSFX_R rows
+        if (!(active[tile >> 5] >> (tile & 31) & 1u)) atomicOr(&active[tile >> 5], 1u << (tile & 31));
     }
 }
 
@@ -189,6 +190,13 @@ __global__ void k_csc_fill(const GridState* __restrict__ gs, const int* __restri
     }
 }
 
+// An entry of a column as the PSF-to-X build reads it: its pixel and L on its grid.
+__device__ __forceinline__ int2 psfx_entry(int row, double v, const int* __restrict__ rowpix, int ny)
+{
+    const int pix = rowpix[row], iq = pix / ny;
+    return make_int2((iq << 16) | (pix - iq * ny), __float2int_rn((float)v * ldexpf(1.0f, PSFX_LEXP)));
+}
+
 // Each column's entries in increasing row order, so that every sum over a
 // column runs in a fixed order (k_csc_fill places them in atomic order).
 // Rows are distinct within a column of the merged L, so the order is a
@@ -201,7 +209,8 @@ __global__ void k_csc_fill(const GridState* __restrict__ gs, const int* __restri
 __global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ gs, const int* __restrict__ colptr,
                                                   const int* __restrict__ col_u, const int* __restrict__ src_u,
                                                   const double* __restrict__ cval, int* __restrict__ colrow,
-                                                  float* __restrict__ colval, double* __restrict__ colval64)
+                                                  int2* __restrict__ ent, double* __restrict__ colval64,
+                                                  const int* __restrict__ rowpix, int ny)
 {
     __shared__ int key[CSC_SORT_MAX];
     __shared__ int pos[CSC_SORT_MAX];
@@ -236,7 +245,7 @@ __global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ 
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
             const double v = cval[pos[i]];
             colrow[b + i] = key[i];
-            colval[b + i] = (float)v;
+            ent[b + i] = psfx_entry(key[i], v, rowpix, ny);
             colval64[b + i] = v;
         }
         return;
@@ -247,7 +256,7 @@ __global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ 
         for (int j = 0; j < n; j++) rank += (col_u[b + j] < ri) ? 1 : 0;
         const double v = cval[src_u[b + i]];
         colrow[b + rank] = ri;
-        colval[b + rank] = (float)v;
+        ent[b + rank] = psfx_entry(ri, v, rowpix, ny);
         colval64[b + rank] = v;
     }
 }
@@ -269,8 +278,8 @@ __device__ __forceinline__ void csc_bitonic_step(int& key, int& pos, int e, int 
 template <int R>
 __device__ __forceinline__ void csc_sort_warp(const int* __restrict__ col_u, const int* __restrict__ src_u,
                                               const double* __restrict__ cval, int b, int n, int lane,
-                                              int* __restrict__ colrow, float* __restrict__ colval,
-                                              double* __restrict__ colval64)
+                                              int* __restrict__ colrow, int2* __restrict__ ent,
+                                              double* __restrict__ colval64, const int* __restrict__ rowpix, int ny)
 {
     int key[R], pos[R];
     #pragma unroll
@@ -307,7 +316,7 @@ __device__ __forceinline__ void csc_sort_warp(const int* __restrict__ col_u, con
         if (e < n) {
             const double v = cval[pos[h]];
             colrow[b + e] = key[h];
-            colval[b + e] = (float)v;
+            ent[b + e] = psfx_entry(key[h], v, rowpix, ny);
             colval64[b + e] = v;
         }
     }
@@ -317,14 +326,15 @@ __global__ void __launch_bounds__(256, 4) k_csc_sort_w(const GridState* __restri
                                                        const int* __restrict__ colptr,
                                                        const int* __restrict__ col_u, const int* __restrict__ src_u,
                                                        const double* __restrict__ cval, int* __restrict__ colrow,
-                                                       float* __restrict__ colval, double* __restrict__ colval64)
+                                                       int2* __restrict__ ent, double* __restrict__ colval64,
+                                                  const int* __restrict__ rowpix, int ny)
 {
     const int lane = threadIdx.x & 31;
     const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= gs->M) return;                                // whole warps
     const int b = colptr[s], n = colptr[s + 1] - b;
-    if (n <= 32) csc_sort_warp<1>(col_u, src_u, cval, b, n, lane, colrow, colval, colval64);
-    else if (n <= CSC_SORT_WARP) csc_sort_warp<2>(col_u, src_u, cval, b, n, lane, colrow, colval, colval64);
+    if (n <= 32) csc_sort_warp<1>(col_u, src_u, cval, b, n, lane, colrow, ent, colval64, rowpix, ny);
+    else if (n <= CSC_SORT_WARP) csc_sort_warp<2>(col_u, src_u, cval, b, n, lane, colrow, ent, colval64, rowpix, ny);
 }
 
 // out[s] = sum over column s of L of value * w[row]: one warp per column, lane
@@ -346,66 +356,6 @@ __global__ void __launch_bounds__(256) k_LTw_csc(const GridState* __restrict__ g
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (lane == 0) out[s] = acc;
     }
-}
-
-// Schedule "bands": grid (M_cap cells, image-row bands).  Each CTA accumulates, for source cell
-// s, the PSF-convolved image of column s of L on the image rows [j0, j1) of
-// its band, in 64-bit fixed point on a dense shared-memory window that spans
-// the bounding box of the footprints reaching the band (at most H rows x
-// (nx + pnx - 1) columns), then writes X[s][r] = sqrt(C^-1)_r times that sum
-// for every active pixel r of the band (zero outside the box).  The column's
-// entries are sorted by active row, i.e. by image row j (j-outer order), so
-// the entries that reach the band are one contiguous range, and so are the
-// band's active rows; for each entry only the PSF rows that land in the band
-// are visited, lanes along x (consecutive accumulators: the 64-bit shared
-// atomics of one instruction do not collide).
-__device__ __forceinline__ int lower_bound_row(const int* __restrict__ rowpix, const int* __restrict__ idx, int n,
-                                               int ny, int jmin)
-{
-    // first position p in [0, n) whose pixel (rowpix[idx ? idx[p] : p]) has y index >= jmin
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const int pix = rowpix[idx ? idx[mid] : mid];
-        if (pix - (pix / ny) * ny < jmin) lo = mid + 1; else hi = mid;
-    }
-    return lo;
-}
-
-// The same search by a whole warp (all lanes, converged): 32 probes per
-// round narrow the range 32-fold, so a few rounds of dependent loads instead
-// of log2(n).
-__device__ __forceinline__ int warp_lower_bound_row(const int* __restrict__ rowpix, const int* __restrict__ idx,
-                                                    int n, int ny, int jmin)
-{
-    const int lane = threadIdx.x & 31;
-    int lo = 0, hi = n;                       // the answer lies in [lo, hi]
-    while (hi - lo > 32) {
-        const int step = (hi - lo + 31) / 32;
-        const int p = lo + lane * step;
-        bool ge = true;
-        if (p < hi) {
-            const int pix = rowpix[idx ? idx[p] : p];
-            ge = pix - (pix / ny) * ny >= jmin;
-        }
-        const unsigned b = __ballot_sync(0xffffffffu, ge);
-        if (b == 0) {
-            lo = lo + 31 * step + 1;
-        } else {
-            const int f = __ffs(b) - 1;
-            const int pf = lo + f * step;
-            if (f > 0) lo = lo + (f - 1) * step + 1;
-            hi = min(hi, pf);
-        }
-    }
-    const int p = lo + lane;
-    bool ge = true;
-    if (p < hi) {
-        const int pix = rowpix[idx ? idx[p] : p];
-        ge = pix - (pix / ny) * ny >= jmin;
-    }
-    const unsigned b = __ballot_sync(0xffffffffu, ge);
-    return b ? lo + __ffs(b) - 1 : hi;
 }
 
 // int64 -> float, rounded to nearest even, in integer arithmetic (the same
@@ -431,337 +381,194 @@ __device__ __forceinline__ float ll2f_rn_int(long long v)
     return __uint_as_float(sign | ((unsigned)(e + 127) << 23) | (m & 0x7fffffu));
 }
 
-// Eight consecutive entries of X (idx a multiple of 8): the F16 hi + lo
-// parts as 16-byte stores (or the TF32 parts as 32-byte pairs).  Returns
-// whether any part is nonzero.
-__device__ __forceinline__ bool store_x8(void* Xh, void* Xl, size_t idx, const float* v, float xs, bool half)
-{
-    bool any = false;
-    if (half) {
-        __align__(16) __half h[8], l[8];
-        #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const float vs = v[u] * xs;
-            h[u] = __float2half_rn(vs);
-            l[u] = __float2half_rn(vs - __half2float(h[u]));
-            any |= __half2float(h[u]) != 0.0f || __half2float(l[u]) != 0.0f;
-        }
-        *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(Xh) + idx) = *reinterpret_cast<const uint4*>(h);
-        *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(Xl) + idx) = *reinterpret_cast<const uint4*>(l);
-        return any;
-    }
-    __align__(16) float h[8], l[8];
-    #pragma unroll
-    for (int u = 0; u < 8; u++) {
-        h[u] = to_tf32(v[u]);
-        l[u] = to_tf32(v[u] - h[u]);
-        any |= h[u] != 0.0f || l[u] != 0.0f;
-    }
-    float4* ph = reinterpret_cast<float4*>(reinterpret_cast<float*>(Xh) + idx);
-    float4* pl = reinterpret_cast<float4*>(reinterpret_cast<float*>(Xl) + idx);
-    ph[0] = *reinterpret_cast<const float4*>(h);
-    ph[1] = *reinterpret_cast<const float4*>(h + 4);
-    pl[0] = *reinterpret_cast<const float4*>(l);
-    pl[1] = *reinterpret_cast<const float4*>(l + 4);
-    return any;
-}
-
-// Entries of a column staged in shared memory at a time by the band kernel
-#define PSFX_ECHUNK 512
-
-// The band schedule's per-item set-up, one warp per (source cell s, band):
-// the range [e0, e1) of s's entries whose footprints reach the band's image
-// rows [j0, j1), their bounding box and the window's image rows [wr0, wr1).
-// meta[2 i] = (e0, e1, imin, imax), meta[2 i + 1] = (wr0, wr1, -, -) for
-// item i = s * nband + band; an item without entries gets e0 = e1.
-__global__ void __launch_bounds__(256) k_psfx_meta(StaticData sd, const GridState* __restrict__ gs,
-                                                   const int* __restrict__ colptr, const int* __restrict__ colrow,
-                                                   const int* __restrict__ rowpix, int H, int nband,
-                                                   int4* __restrict__ meta)
+// The first of n entries sorted by image row (low half of x) whose row is at
+// least jmin, by a whole warp: 32 probes a round.
+__device__ __forceinline__ int warp_lower_bound_row(const int2* __restrict__ ent, int n, int jmin)
 {
     const int lane = threadIdx.x & 31;
-    const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int M = gs->M;
-    const int Mp = (M + TC_TILE - 1) / TC_TILE * TC_TILE;
-    const int s = item / nband, band = item - s * nband;
-    if (s >= Mp) return;
-    const int nyh = sd.pny / 2;
-    const int j0 = band * H, j1 = min(j0 + H, sd.ny);
-    const int b = (s < M) ? colptr[s] : 0, n = (s < M) ? colptr[s + 1] - b : 0;
-    const int e0 = warp_lower_bound_row(rowpix, colrow + b, n, sd.ny, j0 - nyh);
-    const int e1 = warp_lower_bound_row(rowpix, colrow + b, n, sd.ny, j1 + nyh);
-    int4 m0 = make_int4(e0, e0, 0, 0), m1 = make_int4(j0, j0, 0, 0);
-    if (e1 > e0) {
-        int imn = INT_MAX, imx = INT_MIN, jmn = INT_MAX, jmx = INT_MIN;
-        for (int e = e0 + lane; e < e1; e += 32) {
-            const int pix = rowpix[colrow[b + e]];
-            const int iq = pix / sd.ny, jq = pix - iq * sd.ny;
-            imn = min(imn, iq); imx = max(imx, iq); jmn = min(jmn, jq); jmx = max(jmx, jq);
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            imn = min(imn, __shfl_xor_sync(0xffffffffu, imn, o));
-            imx = max(imx, __shfl_xor_sync(0xffffffffu, imx, o));
-            jmn = min(jmn, __shfl_xor_sync(0xffffffffu, jmn, o));
-            jmx = max(jmx, __shfl_xor_sync(0xffffffffu, jmx, o));
-        }
-        const int wr0 = max(j0, jmn - nyh), wr1 = min(j1, jmx - nyh + sd.pny);
-        m0 = make_int4(e0, e1, imn, imx);
-        m1 = make_int4(wr0, wr1, 0, 0);
-    }
-    if (lane == 0) {
-        meta[2 * (size_t)item] = m0;
-        meta[2 * (size_t)item + 1] = m1;
-    }
-}
-
-// X's first Mp rows (cells) cleared by 16-byte stores, every column of X
-// (K_cap, a multiple of 64): after the SYRK of the "rows" schedule, which
-// writes every entry of its rows, so that X is all zero again for a band
-// evaluation (whose own writes k_x_clean undoes).
-__global__ void k_zero_x(const GridState* __restrict__ gs, uint4* __restrict__ Xh, uint4* __restrict__ Xl,
-                         size_t row_vec)
-{
-    const int M = gs->M;
-    const size_t n = (size_t)((M + TC_TILE - 1) / TC_TILE * TC_TILE) * row_vec;
-    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        Xh[i] = z;
-        Xl[i] = z;
-    }
-}
-
-// After the SYRK has read X: the entries the band kernel wrote (the active
-// pixels of each item's window) set back to zero, so that X is all zero when
-// the next evaluation's band kernel starts -- instead of clearing all of it
-// (k_zero_x: ~480 MB per cfg5 evaluation) before.  The "rows" schedule
-// writes every entry of its rows and clears X with k_zero_x after the SYRK.
-__global__ void __launch_bounds__(256) k_x_clean(StaticData sd, const GridState* __restrict__ gs,
-                                                 const int2* __restrict__ pixT, int nband,
-                                                 const int4* __restrict__ meta, void* __restrict__ Xh,
-                                                 void* __restrict__ Xl, int half, int K_cap)
-{
-    const int M = gs->M;
-    const int Mp = (M + TC_TILE - 1) / TC_TILE * TC_TILE;
-    const int s = blockIdx.x;
-    if (s >= Mp) return;
-    const size_t item = (size_t)s * nband + blockIdx.y;
-    const int4 m0 = meta[2 * item], m1 = meta[2 * item + 1];
-    if (m0.y <= m0.x) return;
-    const int nxh = sd.pnx / 2, nyh = sd.pny / 2, nxp = sd.nx + 2 * nxh;
-    const int imin = m0.z, Wb = m0.w - imin + sd.pnx, wr0 = m1.x, area = (m1.y - m1.x) * Wb;
-    for (int e = threadIdx.x; e < area; e += blockDim.x) {
-        const int jr = e / Wb, wc = e - jr * Wb;
-        const int i = imin - nxh + wc, j = wr0 + jr;
-        if (i < 0 || i >= sd.nx) continue;
-        const int r = pixT[(size_t)(j + nyh) * nxp + i + nxh].x;
-        if (r < 0) continue;
-        const size_t idx = (size_t)s * K_cap + r;
-        if (half) {
-            reinterpret_cast<__half*>(Xh)[idx] = __float2half_rn(0.0f);
-            reinterpret_cast<__half*>(Xl)[idx] = __float2half_rn(0.0f);
+    int lo = 0, hi = n;                       // the answer lies in [lo, hi]
+    while (hi - lo > 32) {
+        const int step = (hi - lo + 31) / 32;
+        const int p = lo + lane * step;
+        const unsigned b = __ballot_sync(0xffffffffu, p >= hi || (ent[p].x & 0xffff) >= jmin);
+        if (b == 0) {
+            lo = lo + 31 * step + 1;
         } else {
-            reinterpret_cast<float*>(Xh)[idx] = 0.0f;
-            reinterpret_cast<float*>(Xl)[idx] = 0.0f;
+            const int f = __ffs(b) - 1;
+            const int pf = lo + f * step;
+            if (f > 0) lo = lo + (f - 1) * step + 1;
+            hi = min(hi, pf);
         }
+    }
+    const int p = lo + lane;
+    const unsigned b = __ballot_sync(0xffffffffu, p >= hi || (ent[p].x & 0xffff) >= jmin);
+    return b ? min(lo + __ffs(b) - 1, hi) : hi;
+}
+
+// X by image tiles of 32 pixels along x and PSFX_R rows.  k_psfx_tiles lists the
+// tiles with active pixels that some footprint of a cell reaches, a warp a cell;
+// k_psf_x gives each listed tile to a warp, lane x keeping its column's sums in
+// registers and adding tap x L for every entry whose footprint meets the tile
+// (found by the entries' sorted rows and a ballot over their columns; the taps
+// carry a border of zeros, so that none is tested).  Every entry of X outside the
+// listed tiles is zero: X is all zero between evaluations, k_x_clean takes the
+// tiles back.
+// Scattering a footprint tap by tap into shared memory took a 64-bit shared atomic
+// a tap, which bounded it.  Now a tap is a 32-bit load from shared memory, which
+// bounds it, and a wide multiply-add, 2 to 3 of them a useful one (tiles that a
+// footprint fills in part; 16 rows were 10-40 % slower).  A warp's tiles come from
+// all cells: with a CTA a cell, cells of many entries were left over at the end.
+// us, before -> now: a 21 x 21 PSF and 3,500 cells on 11,800 pixels 263 -> 68, on
+// 36,000 pixels 970 -> 118; a 31 x 31 PSF on 42,000 pixels 383 -> 180.
+// PAD = false (PSFs whose bordered taps pass PSFX_PAD_BYTES): taps by their
+// bounds from global memory.
+#define PSFX_R 8
+#define PSFX_PAD_BYTES (96 * 1024)
+__host__ __device__ __forceinline__ int psfx_pitch(int pny) { return (pny + 2 * PSFX_R - 2) | 1; }
+static inline size_t psfx_tap_bytes(int pnx, int pny) { return sizeof(int) * (size_t)(pnx + 62) * psfx_pitch(pny); }
+
+// a warp per cell, its bitmap of the image's tiles in shared memory
+__global__ void k_psfx_tiles(StaticData sd, const GridState* __restrict__ gs, const int* __restrict__ colptr,
+                             const int2* __restrict__ ent_g, int ntx, int nwords, const unsigned* __restrict__ active,
+                             int* __restrict__ count, uint2* __restrict__ list)
+{
+    extern __shared__ unsigned mark_all[];
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, s = blockIdx.x * nw + (threadIdx.x >> 5);
+    if (s >= gs->M) return;                                       // whole warps
+    unsigned* mark = mark_all + (threadIdx.x >> 5) * nwords;
+    const int pnx = sd.pnx, pny = sd.pny, nxh = pnx / 2, nyh = pny / 2;
+    const int n = colptr[s + 1] - colptr[s];
+    const int2* ent = ent_g + colptr[s];
+    for (int i = lane; i < nwords; i += 32) mark[i] = 0;
+    __syncwarp();
+    for (int e = lane; e < n; e += 32) {
+        const int en = ent[e].x, i0 = (en >> 16) - nxh, j0 = (en & 0xffff) - nyh;
+        const int c0 = max(i0, 0) >> 5, c1 = (min(i0 + pnx, sd.nx) - 1) >> 5;
+        const int t0 = max(j0, 0) / PSFX_R, t1 = (min(j0 + pny, sd.ny) - 1) / PSFX_R;
+        for (int t = t0; t <= t1; t++)
+            for (int c = c0; c <= c1; c++) {
+                const int k = t * ntx + c;
+                if (!(mark[k >> 5] >> (k & 31) & 1u)) atomicOr(&mark[k >> 5], 1u << (k & 31));
+            }
+    }
+    __syncwarp();
+    for (int w0 = 0; w0 < nwords; w0 += 32) {
+        const int wd = w0 + lane;
+        unsigned bits = wd < nwords ? mark[wd] & active[wd] : 0u;
+        int at = __popc(bits);
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += v;
+        }
+        const int total = __shfl_sync(0xffffffffu, at, 31);
+        if (total == 0) continue;
+        int base = 0;
+        if (lane == 0) base = atomicAdd(count, total);
+        at += __shfl_sync(0xffffffffu, base, 0) - __popc(bits);
+        for (; bits; bits &= bits - 1) list[at++] = make_uint2(s, 32 * wd + __ffs(bits) - 1);
     }
 }
 
-// REGPSF (PSFs of at most 32 x 32 taps): lane pk holds PSF column pk in
-// registers and an entry's footprint is visited row by row, fully unrolled
-// -- no shared-memory loads of taps or offsets per tap, independent atomics
-// back to back.  The integer sums are the same either way.
-template <bool REGPSF>
-__global__ void __launch_bounds__(512) k_psf_x_band(StaticData sd, const GridState* __restrict__ gs,
-                                               const int* __restrict__ colptr, const int* __restrict__ colrow,
-                                               const float* __restrict__ colval, const int* __restrict__ rowpix,
-                                               const int2* __restrict__ pixT, int nband,
-                                               const int4* __restrict__ meta, void* __restrict__ Xh,
-                                               void* __restrict__ Xl, float xs, int half, int K_cap,
-                                               unsigned char* __restrict__ nz, int nkb_cap)
+template <bool PAD>
+__global__ void __launch_bounds__(512) k_psf_x(StaticData sd, const int* __restrict__ colptr,
+                                               const int2* __restrict__ ent_g, const int2* __restrict__ pixT, int ntx,
+                                               const int* __restrict__ count, const uint2* __restrict__ list,
+                                               void* __restrict__ Xh, void* __restrict__ Xl, float xs, int half,
+                                               int K_cap, unsigned char* __restrict__ nz, int nkb_cap)
 {
-    extern __shared__ __align__(16) unsigned char psfx_smem[];
-    const int pnx = sd.pnx, pny = sd.pny, nxh = pnx / 2, nyh = pny / 2;
-    const int nT = pnx * pny;
-    const int M = gs->M;
-    const int Mp = (M + TC_TILE - 1) / TC_TILE * TC_TILE;
-    const int s = blockIdx.x;
-    if (s >= Mp) return;
-    const size_t item = (size_t)s * nband + blockIdx.y;
-    const int4 m0 = meta[2 * item], m1 = meta[2 * item + 1];
-    const int e0 = m0.x, e1 = m0.y, imin = m0.z;
-    if (e1 <= e0) return;                                // nothing reaches the band: X stays zero
-    const int wr0 = m1.x, wr1 = m1.y;
-    const int Wb = m0.w - imin + pnx;                    // window columns imin - nxh .. imin - nxh + Wb - 1
-    long long* acc = reinterpret_cast<long long*>(psfx_smem);
-    int* tpsf = reinterpret_cast<int*>(acc + (size_t)(wr1 - wr0) * Wb);
-    int* toff = tpsf + nT;
-    int2* ent = reinterpret_cast<int2*>(toff + nT);      // staged entries (iq << 16 | jq, L): 8 nT bytes on, aligned
+    extern __shared__ __align__(16) int taps[];  // [pnx + 62][pitch]: column pk + 31, row pl + R - 1
+    constexpr int R = PSFX_R;
+    const int pnx = sd.pnx, pny = sd.pny, nxh = pnx / 2, nyh = pny / 2, nxp = sd.nx + 2 * nxh;
+    const int pitch = psfx_pitch(pny);
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, items = *count;
+    if ((int)blockIdx.x * nw >= items) return;
+    if (PAD) {
+        for (int t = threadIdx.x; t < (pnx + 62) * pitch; t += blockDim.x) {
+            const int pk = t / pitch - 31, pl = t % pitch - (R - 1);
+            taps[t] = (pk >= 0 && pk < pnx && pl >= 0 && pl < pny) ? sd.psf_int[pl * pnx + pk] : 0;
+        }
+        __syncthreads();
+    }
     const float inv = ldexpf(1.0f, -sd.fix_exp_x);
-    const float lscale = ldexpf(1.0f, PSFX_LEXP);
-    const int b = colptr[s];
-    for (int i = threadIdx.x; i < (wr1 - wr0) * Wb; i += blockDim.x) acc[i] = 0;
-    // taps in x-fastest order: tpsf[pl * pnx + pk] = psf[pk][pl] on its grid,
-    // and the tap's offset in the window from the footprint's corner (the
-    // register path reads the taps directly)
-    if (!REGPSF) {
-        for (int t = threadIdx.x; t < nT; t += blockDim.x) {
-            const int pl = t / pnx, pk = t - pl * pnx;
-            tpsf[t] = sd.psf_int[t];
-            toff[t] = pl * Wb + pk;
+    for (int it = blockIdx.x * nw + (threadIdx.x >> 5); it < items; it += gridDim.x * nw) {
+        const uint2 item = list[it];
+        const int s = item.x, y0 = (int)item.y / ntx * R, x0 = ((int)item.y % ntx) * 32, x = x0 + lane;
+        const int n = colptr[s + 1] - colptr[s];
+        const int2* ent = ent_g + colptr[s];
+        int lo = 0, hi = n;
+        if (n > 64) {
+            lo = warp_lower_bound_row(ent, n, y0 + nyh - pny + 1);
+            hi = warp_lower_bound_row(ent, n, y0 + R + nyh);
         }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int col[32];
-    if (REGPSF) {
+        long long acc[R];
         #pragma unroll
-        for (int pl = 0; pl < 32; pl++) col[pl] = (lane < pnx && pl < pny) ? sd.psf_int[pl * pnx + lane] : 0;
-    }
-    // the entries, PSFX_ECHUNK at a time: their pixel and L value staged in
-    // shared memory by all threads (independent loads), then spread
-    for (int c0 = e0; c0 < e1; c0 += PSFX_ECHUNK) {
-        const int cn = min(PSFX_ECHUNK, e1 - c0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < cn; e += blockDim.x) {
-            const int pix = rowpix[colrow[b + c0 + e]];
-            const int iq = pix / sd.ny, jq = pix - iq * sd.ny;
-            ent[e] = make_int2((iq << 16) | jq, __float2int_rn(colval[b + c0 + e] * lscale));
-        }
-        __syncthreads();
-        for (int e = warp; e < cn; e += nw) {
-            const int2 en = ent[e];
-            const int iq = en.x >> 16, jq = en.x & 0xffff;
-            const int v = en.y;
-            // PSF rows pl land on image row jq - nyh + pl; keep those in [wr0, wr1)
-            const int pl0 = max(0, wr0 - (jq - nyh)), pl1 = min(pny, wr1 - (jq - nyh));
-            if (REGPSF) {
-                unsigned long long* cl = reinterpret_cast<unsigned long long*>(acc) + (jq - nyh - wr0) * Wb +
-                                         (iq - imin) + lane;
-                if (lane < pnx) {
+        for (int r = 0; r < R; r++) acc[r] = 0;
+        for (int e0 = lo; e0 < hi; e0 += 32) {
+            int dx = -32, dy = 0, v = 0;
+            if (e0 + lane < hi) {
+                const int2 en = ent[e0 + lane];
+                dx = x0 - ((en.x >> 16) - nxh);          // column of lane 0's tap
+                dy = y0 - ((en.x & 0xffff) - nyh);       // row of the first row's tap
+                v = en.y;
+            }
+            unsigned hit = __ballot_sync(0xffffffffu, dx > -32 && dx < pnx && dy > -R && dy < pny);
+            for (; hit; hit &= hit - 1) {
+                const int f = __ffs(hit) - 1;
+                const int ox = __shfl_sync(0xffffffffu, dx, f) + lane, oy = __shfl_sync(0xffffffffu, dy, f);
+                const long long ve = __shfl_sync(0xffffffffu, v, f);
+                if (PAD) {
+                    const int* tp = taps + (ox + 31) * pitch + oy + R - 1;
                     #pragma unroll
-                    for (int pl = 0; pl < 32; pl++)
-                        if (pl >= pl0 && pl < pl1)
-                            atomicAdd(cl + pl * Wb, (unsigned long long)((long long)col[pl] * (long long)v));
+                    for (int r = 0; r < R; r++) acc[r] += (long long)tp[r] * ve;
+                } else if (ox >= 0 && ox < pnx) {
+                    #pragma unroll
+                    for (int r = 0; r < R; r++)
+                        if (oy + r >= 0 && oy + r < pny) acc[r] += (long long)sd.psf_int[(oy + r) * pnx + ox] * ve;
                 }
-            } else {
-                // the footprint's corner (iq - nxh, jq - nyh) in window coordinates
-                unsigned long long* corner =
-                    reinterpret_cast<unsigned long long*>(acc) + (jq - nyh - wr0) * Wb + (iq - imin);
-                const int t1 = pl1 * pnx;
-                for (int t = pl0 * pnx + lane; t < t1; t += 32)
-                    atomicAdd(corner + toff[t], (unsigned long long)((long long)tpsf[t] * (long long)v));
             }
         }
-    }
-    __syncthreads();
-    // X[s][r] for the active pixels r of the window: v = sqrt(C^-1)_r * sum,
-    // split into hi + lo; the window's pixels are visited x fastest through
-    // the padded image's (active row, sqrt(C^-1)) table.  Every other entry
-    // of X's row s is zero (X is all zero between evaluations: k_x_clean).
-    {
-        const int nxp = sd.nx + 2 * nxh;
-        const int area = (wr1 - wr0) * Wb;
-        for (int e = threadIdx.x; e < area; e += blockDim.x) {
-            const int jr = e / Wb, wc = e - jr * Wb;
-            const int i = imin - nxh + wc, j = wr0 + jr;
-            if (i < 0 || i >= sd.nx) continue;
-            const int2 pt = pixT[(size_t)(j + nyh) * nxp + i + nxh];
-            if (pt.x < 0) continue;
-            const float v = (ll2f_rn_int(acc[e]) * inv) * __int_as_float(pt.y);
+        // X[s][row] for the tile's active pixels: sqrt(C^-1) times the sum, split into hi + lo
+        if (x >= sd.nx) continue;
+        #pragma unroll
+        for (int r = 0; r < R; r++) {
+            if (y0 + r >= sd.ny) break;
+            const int2 pt = pixT[(size_t)(y0 + r + nyh) * nxp + x + nxh];
+            if (pt.x < 0 || acc[r] == 0) continue;
+            const float v = (ll2f_rn_int(acc[r]) * inv) * __int_as_float(pt.y);
             if (store_x(Xh, Xl, (size_t)s * K_cap + pt.x, v, xs, half))
                 nz[(size_t)(s / TC_TILE) * nkb_cap + pt.x / TC_KB] = 1;
         }
     }
 }
 
-// Schedule "rows": grid (M_cap cells, chunks of active rows); one CTA holds
-// the 64-bit accumulators of a chunk of active rows and scatters each entry
-// of column s over its PSF footprint through the active-row table of the
-// padded image (pixT).  Each product psf x L is the same exact integer
-// product and sqrt(C^-1) is applied to the sum as in the "bands" schedule, so
-// both give the same bits.
-__global__ void __launch_bounds__(512) k_psf_x_rows(StaticData sd, const GridState* __restrict__ gs,
-                                               const int* __restrict__ colptr, const int* __restrict__ colrow,
-                                               const float* __restrict__ colval, const int* __restrict__ rowpix,
-                                               const int2* __restrict__ pixT, const float* __restrict__ sqc,
-                                               int chunk, void* __restrict__ Xh, void* __restrict__ Xl, float xs,
-                                               int half, int K_cap, unsigned char* __restrict__ nz,
-                                               int nkb_cap)
+// After the SYRK has read X: the listed tiles' pixels back to zero (clearing all of
+// X moved ~480 MB at 4,096 cells x 58,000 pixels).
+__global__ void __launch_bounds__(256) k_x_clean(StaticData sd, const int2* __restrict__ pixT, int ntx,
+                                                 const int* __restrict__ count, const uint2* __restrict__ list,
+                                                 void* __restrict__ Xh, void* __restrict__ Xl, int half, int K_cap)
 {
-    extern __shared__ __align__(16) unsigned char psfx_smem[];
-    long long* acc = reinterpret_cast<long long*>(psfx_smem);
-    int* tpsf = reinterpret_cast<int*>(acc + chunk);
-    const int N = gs->N, M = gs->M;
-    const int Mp = (M + TC_TILE - 1) / TC_TILE * TC_TILE;
-    const int Np = (N + 63) & ~63;                           // whole 64-pixel stages for the F16 SYRK
-    const int s = blockIdx.x;
-    const int r0 = blockIdx.y * chunk, r1 = min(r0 + chunk, Np);
-    if (s >= Mp || r0 >= Np) return;
-    const int nT = sd.pnx * sd.pny;
-    const float inv = ldexpf(1.0f, -sd.fix_exp_x);
-    const int pnx = sd.pnx;
-    const int nxp = sd.nx + 2 * (pnx / 2);                    // padded width of pixT
-    int* toff = reinterpret_cast<int*>(tpsf + nT);
-    for (int i = threadIdx.x; i < r1 - r0; i += blockDim.x) acc[i] = 0;
-    // taps in x-fastest order: tpsf[pl * pnx + pk] = psf[pk][pl] on its grid
-    // (StaticData::psf_int), and the tap's offset in pixT from the
-    // footprint's corner
-    for (int t = threadIdx.x; t < nT; t += blockDim.x) {
-        const int pl = t / pnx, pk = t - pl * pnx;
-        tpsf[t] = sd.psf_int[t];
-        toff[t] = pl * nxp + pk;
-    }
-    const float lscale = ldexpf(1.0f, PSFX_LEXP);
-    __syncthreads();
-    if (s < M) {
-        const int b = colptr[s], n = colptr[s + 1] - b;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        for (int e = warp; e < n; e += nw) {
-            const int q = colrow[b + e];
-            const long long v = __float2int_rn(colval[b + e] * lscale);     // L on its grid
-            const int pix = rowpix[q];
-            const int iq = pix / sd.ny, jq = pix - iq * sd.ny;
-            // the footprint's corner (iq - pnx/2, jq - pny/2) sits at (iq, jq) of
-            // the padded table; lanes run along x, so the targets of one
-            // instruction are consecutive active rows and its 64-bit shared
-            // atomics do not collide
-            const int2* corner = pixT + (size_t)jq * nxp + iq;
-            // four taps per lane in flight: their table loads are independent
-            for (int t0 = lane; t0 < nT; t0 += 128) {
-                int2 P[4];
-                int w[4];
-                #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int t = t0 + 32 * u;
-                    P[u] = make_int2(-1, 0);
-                    w[u] = 0;
-                    if (t < nT) {
-                        P[u] = corner[toff[t]];
-                        w[u] = tpsf[t];
-                    }
-                }
-                #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    if (P[u].x >= r0 && P[u].x < r1)                // inactive (-1) or another chunk
-                        atomicAdd(reinterpret_cast<unsigned long long*>(&acc[P[u].x - r0]),
-                                  (unsigned long long)((long long)w[u] * v));
-                }
+    const int lane = threadIdx.x & 31, items = *count;
+    const int nxh = sd.pnx / 2, nyh = sd.pny / 2, nxp = sd.nx + 2 * nxh;
+    for (int it = blockIdx.x * 8 + (threadIdx.x >> 5); it < items; it += gridDim.x * 8) {
+        const uint2 item = list[it];
+        const int y0 = (int)item.y / ntx * PSFX_R, x = ((int)item.y % ntx) * 32 + lane;
+        if (x >= sd.nx) continue;
+        int row[PSFX_R];
+        #pragma unroll
+        for (int r = 0; r < PSFX_R; r++)
+            row[r] = y0 + r < sd.ny ? pixT[(size_t)(y0 + r + nyh) * nxp + x + nxh].x : -1;
+        #pragma unroll
+        for (int r = 0; r < PSFX_R; r++) {
+            if (row[r] < 0) continue;
+            const size_t idx = (size_t)item.x * K_cap + row[r];
+            if (half) {
+                reinterpret_cast<__half*>(Xh)[idx] = __float2half_rn(0.0f);
+                reinterpret_cast<__half*>(Xl)[idx] = __float2half_rn(0.0f);
+            } else {
+                reinterpret_cast<float*>(Xh)[idx] = 0.0f;
+                reinterpret_cast<float*>(Xl)[idx] = 0.0f;
             }
         }
-    }
-    __syncthreads();
-    // write row s of X for pixels [r0, r1): v = sqrt(C^-1)_r * sum split into
-    // hi + lo (zero beyond the N active rows); one warp covers one 32-pixel block
-    const int span = r1 - r0;
-    for (int i0 = 0; i0 < span; i0 += blockDim.x) {
-        const int i = i0 + threadIdx.x;
-        bool nonzero = false;
-        if (i < span) {
-            const float v = (r0 + i < N) ? (ll2f_rn_int(acc[i]) * inv) * sqc[r0 + i] : 0.0f;
-            nonzero = store_x(Xh, Xl, (size_t)s * K_cap + r0 + i, v, xs, half);
-        }
-        const unsigned any = __ballot_sync(0xffffffffu, nonzero);
-        if ((threadIdx.x & 31) == 0 && any && i < span)
-            nz[(size_t)(s / TC_TILE) * nkb_cap + (r0 + i) / TC_KB] = 1;
     }
 }
 
@@ -873,29 +680,13 @@ void mixed_free(Slot& c)
     MixedWork* m = mw_of(c);
     if (!m) return;
     void* ptrs[] = {m->t, m->X_hi, m->X_lo, m->nz, m->F32, m->R32, m->u, m->v, m->r, m->z, m->y, m->img,
-                    m->linvF, m->yf, m->zf, m->flags, m->colcnt, m->cursor, m->colrow, m->colval,
-                    m->sqc, m->col_u, m->src_u, m->colval64, m->pixT, m->F0, m->psfx_meta,
+                    m->linvF, m->yf, m->zf, m->flags, m->colcnt, m->cursor, m->colrow, m->ent,
+                    m->col_u, m->src_u, m->colval64, m->pixT, m->F0, m->tiles, m->tile_active,
                     m->cf.Lh, m->cf.Ll, m->cf.pexp, m->cf.ih, m->cf.il, m->cf.flags,
                     m->cr.Lh, m->cr.Ll, m->cr.pexp, m->cr.ih, m->cr.il, m->cr.flags};
     for (void* p : ptrs) if (p) cudaFree(p);
     delete m;
     c.mixed = nullptr;
-}
-
-// The band schedule's geometry: image rows per band H -- as many as fit
-// beside the PSF tables in about half an SM's shared memory (two CTAs per
-// SM), divided by `split` -- the number of bands and the dynamic shared
-// memory of a CTA.
-static void psfx_band_geom(int nx, int ny, int pnx, int pny, int split, int& H, int& nband, size_t& smem)
-{
-    const int nT = pnx * pny;
-    const int W = nx + pnx - 1;
-    const size_t tap_bytes = 2 * sizeof(int) * (size_t)nT + 8 * sizeof(int) + 2 * sizeof(int) * PSFX_ECHUNK;
-    const size_t avail = (110 * 1024 > tap_bytes) ? 110 * 1024 - tap_bytes : 0;
-    const int fit = std::max(1, (int)(avail / (sizeof(long long) * W)));
-    H = std::max(1, std::min(ny, fit) / split);
-    nband = (ny + H - 1) / H;
-    smem = sizeof(long long) * (size_t)H * W + tap_bytes;
 }
 
 static size_t flow128_flags(int nb) { return (size_t)nb * nb + nb + 1; }
@@ -930,10 +721,10 @@ int mixed_init(Slot& c)
     A((void**)&m->X_lo, xbytes);
     A((void**)&m->nz, (size_t)(M_cap / TC_TILE) * m->nkb_cap + 3);
     {
-        int H = 1;
-        size_t sm = 0;
-        psfx_band_geom(c.img_nx, c.img_ny, c.psf_nx, c.psf_ny, 4, H, m->psfx_bands, sm);   // the finest split
-        A((void**)&m->psfx_meta, sizeof(int4) * 2 * (size_t)M_cap * m->psfx_bands);
+        const int ntile = (c.img_nx + 31) / 32 * ((c.img_ny + PSFX_R - 1) / PSFX_R);
+        m->psfx_words = (ntile + 31) / 32;
+        A((void**)&m->tiles, sizeof(uint2) * (size_t)M_cap * std::min(ntile, c.N_cap));
+        A((void**)&m->tile_active, sizeof(unsigned) * (m->psfx_words + 1));
     }
     A((void**)&m->F32, sizeof(float) * (size_t)M_cap * M_cap);
     A((void**)&m->R32, sizeof(float) * (size_t)M_cap * M_cap);
@@ -941,13 +732,12 @@ int mixed_init(Slot& c)
     A((void**)&m->colcnt, sizeof(int) * (size_t)(M_cap + 1));
     A((void**)&m->cursor, sizeof(int) * (size_t)M_cap);
     A((void**)&m->colrow, sizeof(int) * (size_t)m->nnz_cap);
-    A((void**)&m->colval, sizeof(float) * (size_t)m->nnz_cap);
+    A((void**)&m->ent, sizeof(int2) * (size_t)m->nnz_cap);
     A((void**)&m->col_u, sizeof(int) * (size_t)m->nnz_cap);
     A((void**)&m->pixT, sizeof(int2) * (size_t)c.npix_pad);
     A((void**)&m->img, sizeof(double) * (size_t)c.npix_pad);
     A((void**)&m->src_u, sizeof(int) * (size_t)m->nnz_cap);
     A((void**)&m->colval64, sizeof(double) * (size_t)m->nnz_cap);
-    A((void**)&m->sqc, sizeof(float) * (size_t)(c.N_cap + 64));
     A((void**)&m->t, sizeof(double) * (size_t)(c.N_cap + 64));
     A((void**)&m->u, sizeof(double) * (size_t)(c.N_cap + 64));
     A((void**)&m->v, sizeof(double) * M_cap);
@@ -989,9 +779,8 @@ int mixed_init(Slot& c)
             const cudaError_t r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
             if (ea == cudaSuccess) ea = r;
         };
-        opt((const void*)k_psf_x_rows, 227 * 1024);
-        opt((const void*)k_psf_x_band<true>, 227 * 1024);
-        opt((const void*)k_psf_x_band<false>, 227 * 1024);
+        opt((const void*)k_psf_x<true>, 227 * 1024);
+        opt((const void*)k_psf_x<false>, 227 * 1024);
         opt((const void*)k_chol128, C2_SMEM);
         opt((const void*)k_syrk_tc<false>, TC_SMEM);
         opt((const void*)k_syrk_tc<true>, TC_SMEM);
@@ -1044,6 +833,7 @@ void mixed_clear(Slot& slot, ClearList& l, bool trial)
     l.add(m->cr.flags, sizeof(int) * flow128_flags(m->nb));
     l.add(m->nz, (size_t)(m->M_cap / TC_TILE) * m->nkb_cap);
     l.add(m->colcnt, sizeof(int) * (size_t)(m->M_cap + 1));
+    l.add(m->tile_active, sizeof(unsigned) * (m->psfx_words + 1));
     l.add(m->pixT, sizeof(int2) * (size_t)slot.npix_pad, 0xffffffffu);
     l.add(m->img, sizeof(double) * (size_t)slot.npix_pad);
 }
@@ -1099,13 +889,13 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
     {
         const int rb = std::min((N_cap + 255) / 256, 152 * 8);
         k_csc_count<<<std::max(rb, 1), 256, 0, st>>>(sd, w.gs, w.rowptr, w.cidx, w.ccnt, w.cvec, w.rowpix, m->colcnt,
-                                                     m->sqc, m->pixT);
+                                                     m->pixT, (sd.nx + 31) / 32, m->tile_active);
         k_csc_scan<<<1, 1024, 0, st>>>(w.gs, m->colcnt, m->cursor);
         k_csc_fill<<<std::max(rb, 1), 256, 0, st>>>(w.gs, w.rowptr, w.cidx, w.ccnt, m->cursor, m->col_u, m->src_u);
         k_csc_sort_w<<<(m->M_cap + 7) / 8, 256, 0, st>>>(w.gs, m->colcnt, m->col_u, m->src_u, w.cval, m->colrow,
-                                                        m->colval, m->colval64);
-        k_csc_sort<<<m->M_cap, 256, 0, st>>>(w.gs, m->colcnt, m->col_u, m->src_u, w.cval, m->colrow, m->colval,
-                                            m->colval64);
+                                                        m->ent, m->colval64, w.rowpix, sd.ny);
+        k_csc_sort<<<m->M_cap, 256, 0, st>>>(w.gs, m->colcnt, m->col_u, m->src_u, w.cval, m->colrow, m->ent,
+                                            m->colval64, w.rowpix, sd.ny);
         n += 5;
     }
     // D = L^T P^T (C^-1 d), FP64
@@ -1114,44 +904,20 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
     n++;
     // X = (P L sqrt(C^-1))^T and its block flags, from L by source cell
     const float xs = m->half ? ldexpf(1.0f, sd.x_exp) : 1.0f;     // F16 scale of X
-    int band_nband = 0;                                               // bands of the band schedule (0: rows)
+    const int ntx = (sd.nx + 31) / 32;
+    const int* ntiles = reinterpret_cast<const int*>(m->tile_active + m->psfx_words);
     {
-        const int nT = sd.pnx * sd.pny;
-        const int split = std::max(1, std::min(c->psfx_split, 4));
+        const size_t wmark = sizeof(unsigned) * m->psfx_words;
+        const int tw = (int)std::max<size_t>(1, std::min<size_t>(8, 48 * 1024 / wmark));      // cells a CTA
+        k_psfx_tiles<<<(m->M_cap + tw - 1) / tw, 32 * tw, wmark * tw, st>>>(
+            sd, w.gs, m->colcnt, m->ent, ntx, m->psfx_words, m->tile_active, const_cast<int*>(ntiles), m->tiles);
         const int pt = (c->psfx_threads == 128 || c->psfx_threads == 512) ? c->psfx_threads : 256;
-        if (c->psfx_mode == 1) {
-            int H = 1, nband = 1;
-            size_t smem = 0;
-            psfx_band_geom(sd.nx, sd.ny, sd.pnx, sd.pny, split, H, nband, smem);
-            // each item's set-up, then the windows (X is all zero here: the
-            // previous evaluation cleaned it after its SYRK, see below)
-            band_nband = nband;
-            k_psfx_meta<<<(m->M_cap * nband + 7) / 8, 256, 0, st>>>(sd, w.gs, m->colcnt, m->colrow, w.rowpix, H,
-                                                                  nband, m->psfx_meta);
-            if (sd.pnx <= 32 && sd.pny <= 32)
-                k_psf_x_band<true><<<dim3(m->M_cap, nband), pt, smem, st>>>(
-                    sd, w.gs, m->colcnt, m->colrow, m->colval, w.rowpix, m->pixT, nband, m->psfx_meta, m->X_hi,
-                    m->X_lo, xs, m->half ? 1 : 0, m->K_cap, m->nz, m->nkb_cap);
-            else
-                k_psf_x_band<false><<<dim3(m->M_cap, nband), pt, smem, st>>>(
-                    sd, w.gs, m->colcnt, m->colrow, m->colval, w.rowpix, m->pixT, nband, m->psfx_meta, m->X_hi,
-                    m->X_lo, xs, m->half ? 1 : 0, m->K_cap, m->nz, m->nkb_cap);
-            n += 1;
-        } else {
-            // accumulator rows per CTA: the active rows split into psfx_split
-            // chunks (or more, if a chunk does not fit beside the PSF in 227 KB)
-            const int fit = (int)(((227 * 1024 - (sizeof(float) + sizeof(int)) * (size_t)nT) / sizeof(long long)) &
-                                  ~(size_t)31);
-            const int want = ((m->K_cap + split - 1) / split + 31) & ~31;
-            const int chunk = std::max(32, std::min(want, fit));
-            const int nchunk = (m->K_cap + chunk - 1) / chunk;
-            const size_t smem = sizeof(long long) * (size_t)chunk + (sizeof(float) + sizeof(int)) * (size_t)nT;
-            k_psf_x_rows<<<dim3(m->M_cap, nchunk), pt, smem, st>>>(sd, w.gs, m->colcnt, m->colrow, m->colval,
-                                                                    w.rowpix, m->pixT, m->sqc, chunk, m->X_hi,
-                                                                    m->X_lo, xs, m->half ? 1 : 0, m->K_cap, m->nz,
-                                                                    m->nkb_cap);
-        }
-        n++;
+        const size_t taps = psfx_tap_bytes(sd.pnx, sd.pny);
+        const bool pad = taps <= PSFX_PAD_BYTES;
+        auto k = pad ? k_psf_x<true> : k_psf_x<false>;
+        k<<<152 * 1024 / pt, pt, pad ? taps : 0, st>>>(sd, m->colcnt, m->ent, m->pixT, ntx, ntiles, m->tiles, m->X_hi,
+                                                       m->X_lo, xs, m->half ? 1 : 0, m->K_cap, m->nz, m->nkb_cap);
+        n += 2;
     }
     if (ev) cudaEventRecord(ev[3], st);
     {
@@ -1164,14 +930,8 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
                                                                        m->nkb_cap, m->F32, m->ld32, 1.0f);
         n++;
         // X back to all zero for the next evaluation
-        if (band_nband > 0) {
-            k_x_clean<<<dim3(m->M_cap, band_nband), 256, 0, st>>>(sd, w.gs, m->pixT, band_nband, m->psfx_meta,
-                                                                  m->X_hi, m->X_lo, m->half ? 1 : 0, m->K_cap);
-        } else {
-            const size_t row_vec = (size_t)m->K_cap * (m->half ? 2 : 4) / 16;
-            k_zero_x<<<152 * 8, 256, 0, st>>>(w.gs, reinterpret_cast<uint4*>(m->X_hi),
-                                              reinterpret_cast<uint4*>(m->X_lo), row_vec);
-        }
+        k_x_clean<<<152 * 8, 256, 0, st>>>(sd, m->pixT, ntx, ntiles, m->tiles, m->X_hi, m->X_lo, m->half ? 1 : 0,
+                                           m->K_cap);
         n++;
     }
     if (ev) cudaEventRecord(ev[4], st);
