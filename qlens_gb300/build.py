@@ -26,7 +26,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=o
 UNITS = [
     ("raytrace.cu", ["--fmad=false"]),
     ("mapping.cu", ["--fmad=false"]),
-    ("psf.cu", ["--fmad=false"]),
+    ("psf.cu", []),
     ("linalg.cu", []),
     ("ozaki.cu", []),
     ("cholfp64.cu", []),
@@ -44,7 +44,7 @@ UNITS = [
     ("qlpix_api.cpp", []),
 ]
 HEADERS = ["qlpix_internal.h", "qlpix_ctx.h", "lens_device.cuh", "nfw_device.cuh", "patterson_rule.h", "nfw_kappa_table.h", "sur_train.cuh", "chol.cuh", "chol128.cuh", "tc_common.cuh", "tc_syrk.cuh",
-           "ozaki.cuh", "tma_map.h", "brent.h"]
+           "ozaki.cuh", "tma_map.h", "psf_tiles.cuh", "brent.h"]
 
 
 def _newer(src, obj, deps):

@@ -47,9 +47,10 @@ static void free_work(Work& w)
 {
     void* ptrs[] = {w.spx, w.spy, w.cx, w.cy, w.ccx, w.ccy, w.cell3, w.w3, w.mapped, w.active_index, w.pixmaps,
                     w.rowidx, w.pixindex, w.rowpix, w.rowptr, w.Lidx, w.Lval, w.cidx, w.cval, w.ccnt, w.Lpsf,
-                    w.dvec, w.cvec, w.D, w.F, w.R, w.s, w.tmp, w.model, w.partial, w.linv, w.gs, w.out, w.ep,
+                    w.dvec, w.cvec, w.D, w.F, w.R, w.s, w.tmp, w.model, w.linv, w.gs, w.out, w.ep,
                     w.fb_ray, w.fb_xy, w.fb_count, w.F0, w.gpart, w.gpart_cnt, w.cpart, w.sur_eps, w.xlist, w.xcount, w.nfw_xy};
     for (void* p : ptrs) if (p) cudaFree(p);
+    csc_free(w.csc);
     chol64_free(w.cholF);
     chol64_free(w.cholR);
     oz_free(w.oz);
@@ -99,14 +100,12 @@ static int alloc_work(qlp_ctx* c, Slot& s, int n_mask, int nsub, int Mcells, int
     CK(dalloc(&w.rowptr, n_mask + 1), "alloc");
     CK(dalloc(&w.Lidx, nnz), "alloc"); CK(dalloc(&w.Lval, nnz), "alloc");
     CK(dalloc(&w.cidx, nnz), "alloc"); CK(dalloc(&w.cval, nnz), "alloc"); CK(dalloc(&w.ccnt, n_mask), "alloc");
-    w.ldL = Mc;
+    w.ldL = (n_mask + 31) / 32 * 32;
     CK(dalloc(&w.dvec, n_mask), "alloc"); CK(dalloc(&w.cvec, n_mask), "alloc");
     w.ldF = Mc;
     CK(dalloc(&w.D, Mc), "alloc");
     CK(dalloc(&w.s, Mc), "alloc"); CK(dalloc(&w.tmp, Mc), "alloc");
     CK(dalloc(&w.model, n_mask), "alloc");
-    const size_t part = std::max((size_t)((n_mask + 255) / 256 + 1) * Mc, (size_t)Mc * 4);
-    CK(dalloc(&w.partial, part), "alloc");
     CK(dalloc(&w.gpart, 4 * 1024), "alloc"); CK(dalloc(&w.gpart_cnt, 1024), "alloc");
     CK(dalloc(&w.cpart, 3 * 1025), "alloc");
     CK(dalloc(&w.linv, (size_t)Mc * 64), "alloc");
@@ -130,9 +129,11 @@ static int alloc_work(qlp_ctx* c, Slot& s, int n_mask, int nsub, int Mcells, int
 static int ensure_fp64_mats(Slot& s)
 {
     if (s.fp64_mats) return QLP_OK;
-    if (!s.w.Lpsf) {
-        CK(dalloc(&s.w.Lpsf, (size_t)s.N_cap * s.M_cap), "alloc L'");
-        CK(cudaMemset(s.w.Lpsf, 0, sizeof(double) * (size_t)s.N_cap * s.M_cap), "memset");
+    if (!s.w.Lpsf) CK(dalloc(&s.w.Lpsf, (size_t)s.w.ldL * s.M_cap), "alloc L'");
+    if (!s.w.csc.colcnt) {
+        const cudaError_t e = csc_alloc(s.w.csc, s, s.M_cap, true);
+        if (e != cudaSuccess) csc_free(s.w.csc);
+        CK(e, "alloc L by source cell");
     }
     if (!s.w.oz) {
         const int r = oz_alloc(&s.w.oz, s.N_cap, s.M_cap);
@@ -239,6 +240,34 @@ int ctx_init(qlp_ctx* c, const qlp_image* im, const qlp_psf* psf, const qlp_srcg
         CK(dalloc(&c->d_psf_int, pi.size()), "alloc");
         CK(cudaMemcpy(c->d_psf_int, pi.data(), sizeof(int) * pi.size(), cudaMemcpyHostToDevice), "h2d");
         sd.psf_int = c->d_psf_int;
+        // ... and the plain path's, in two parts
+        double tmax = 0;
+        int taps = 0, emax = 0, esum = 0;
+        for (int t = 0; t < pnx * pny; t++) {
+            tmax = std::max(tmax, fabs(psf->matrix[t]));
+            taps += psf->matrix[t] != 0;
+        }
+        std::vector<int2> pf((size_t)pnx * pny, make_int2(0, 0));
+        sd.psf_fixed = 0;
+        if (std::isfinite(psum) && psum > 0) {
+            frexp(tmax, &emax);
+            frexp(psum, &esum);
+            sd.psf_t = std::min(30 - emax, 33 - esum);
+            sd.psf_w = std::max(4, std::min(30, (int)floor(34.85 - log2((double)taps))));
+            // half a unit within 2^-51 of the largest tap: the sum of a few such
+            // errors stays within an FP64 sum's rounding
+            sd.psf_fixed = log2(tmax) + sd.psf_t + sd.psf_w + 1 >= 51;
+            for (int pl = 0; pl < pny && sd.psf_fixed; pl++)
+                for (int pk = 0; pk < pnx; pk++) {
+                    const long long q = llrint(ldexp(psf->matrix[(size_t)pk * pny + pl], sd.psf_t + sd.psf_w));
+                    int2& f = pf[(size_t)pl * pnx + pk];
+                    f.x = (int)((q + (1ll << (sd.psf_w - 1))) >> sd.psf_w);
+                    f.y = (int)(q - ((long long)f.x << sd.psf_w));
+                }
+        }
+        CK(dalloc(&c->d_psf_fine, pf.size()), "alloc");
+        CK(cudaMemcpy(c->d_psf_fine, pf.data(), sizeof(int2) * pf.size(), cudaMemcpyHostToDevice), "h2d");
+        sd.psf_fine = c->d_psf_fine;
     }
 
     SrcOpts& so = c->so;
@@ -270,7 +299,7 @@ void ctx_free(qlp_ctx* c)
         if (s.side_join) cudaEventDestroy(s.side_join);
     }
     c->slots.clear();
-    void* ptrs[] = {c->d_xvals, c->d_yvals, c->d_data, c->d_covinv, c->d_psf, c->d_psf_int, c->d_mpix, c->d_inst_mpix,
+    void* ptrs[] = {c->d_xvals, c->d_yvals, c->d_data, c->d_covinv, c->d_psf, c->d_psf_int, c->d_psf_fine, c->d_mpix, c->d_inst_mpix,
                     c->d_emask, c->d_inmask, c->d_epix, c->d_eoff, c->job_counts};
     for (void* p : ptrs) if (p) cudaFree(p);
     if (c->h_out) cudaFreeHost(c->h_out);
@@ -382,6 +411,7 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             mixed_clear(slot, cl, false);
         } else {
             oz_clear(w.oz, cl);
+            csc_clear(w.csc, cl);
             chol64_clear(w.cholF, cl);
             chol64_clear(w.cholR, cl);
         }
@@ -418,7 +448,6 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
     launch_build_L(sd, so, w, st);
     launch_rowpix(sd, w, st);
     if (ev) cudaEventRecord(ev[2], st);
-    launch_dvec(sd, w, N_max, st);
     if (mixed) {
         int r = run_inversion_mixed(c, slot, sd, so, regp, part, st, ev);
         if (r != QLP_OK) return r;
@@ -437,8 +466,9 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             launch_logdet(w.R, w.ldF, Mc, w, 1, slot.side);
             cudaEventRecord(slot.side_join, slot.side);
         }
-        launch_psf(sd, so, w, Mc, st);
-        launch_D(w, N_max, Mc, st);
+        const int rp = launch_psf(sd, w, N_max, Mc, st);
+        if (rp != QLP_OK) return rp;
+        launch_D(w, Mc, st);
         if (ev) cudaEventRecord(ev[3], st);
         launch_syrk_fp64(sd, w, N_max, Mc, st);
         if (ev) cudaEventRecord(ev[4], st);
@@ -975,8 +1005,11 @@ int ctx_dump_Lpsf(qlp_ctx* c, int rows, double* out)
     CK(cudaMemcpy(&gs, w.gs, sizeof(gs), cudaMemcpyDeviceToHost), "d2h");
     if (rows > gs.N) rows = gs.N;
     if (rows <= 0 || gs.M <= 0 || !w.Lpsf) return QLP_OK;
-    CK(cudaMemcpy2D(out, sizeof(double) * gs.M, w.Lpsf, sizeof(double) * w.ldL, sizeof(double) * gs.M, rows,
+    std::vector<double> t((size_t)gs.M * rows);               // by source cell
+    CK(cudaMemcpy2D(t.data(), sizeof(double) * rows, w.Lpsf, sizeof(double) * w.ldL, sizeof(double) * rows, gs.M,
                     cudaMemcpyDeviceToHost), "d2h");
+    for (int r = 0; r < rows; r++)
+        for (int s = 0; s < gs.M; s++) out[(size_t)r * gs.M + s] = t[(size_t)s * rows + r];
     return QLP_OK;
 }
 

@@ -121,61 +121,56 @@ void launch_copy_square(void* dst, const void* src, int ld, int esize, int blk, 
     count_launches(1);
 }
 
-// ---- data and inverse-variance per active row ----
-__global__ void k_dvec(StaticData sd, const GridState* __restrict__ gs, const int* __restrict__ rowpix,
-                       double* __restrict__ dvec, double* __restrict__ cvec)
+// ---- D = L'^T (C^-1 d) ----
+// Eight cells a CTA over the live 32-pixel stages of their 64-cell block: a warp
+// takes every eighth stage, its lanes the stage's pixels, all eight cells beside
+// each other (C^-1 d is formed once for them); then a shuffle tree and the warps in
+// order.  The FP64 pipe bounds it (one multiply-add a live entry; skipping the zeros
+// among them by a test cost more than they).  Two multiplies and an add for every
+// entry of a row-wise L' before: 2,934 cells x 11,772 pixels 194 -> 72 us, and the
+// model image likewise 76 -> 54 us.
+#define D_CELLS 8
+__global__ void __launch_bounds__(256) k_D(const GridState* __restrict__ gs, const double* __restrict__ L, int ldL,
+                                           const unsigned char* __restrict__ nz, int nst,
+                                           const double* __restrict__ dvec, const double* __restrict__ cvec,
+                                           double* __restrict__ D)
 {
-    const int N = gs->N;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
-        int pix = rowpix[r];
-        dvec[r] = sd.data[pix];
-        cvec[r] = sd.use_noise_map ? sd.covinv[pix] : sd.cov_inverse;
+    __shared__ double part[8][D_CELLS];
+    const int N = gs->N, M = gs->M;
+    const int c0 = blockIdx.x * D_CELLS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (c0 >= mpad64(M)) return;
+    double acc[D_CELLS];
+    #pragma unroll
+    for (int k = 0; k < D_CELLS; k++) acc[k] = 0;
+    if (c0 < M) {
+        const unsigned char* live = nz + (size_t)(c0 / 64) * nst;
+        for (int st = warp; st * 32 < N; st += 8) {
+            const int r = st * 32 + lane;
+            if (!live[st] || r >= N) continue;
+            const double w = dvec[r] * cvec[r];
+            #pragma unroll
+            for (int k = 0; k < D_CELLS; k++)
+                if (c0 + k < M) acc[k] = fma(L[(size_t)(c0 + k) * ldL + r], w, acc[k]);
+        }
+    }
+    #pragma unroll
+    for (int k = 0; k < D_CELLS; k++) {
+        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+        if (lane == 0) part[warp][k] = acc[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < D_CELLS) {
+        double a = 0;
+        for (int k = 0; k < 8; k++) a += part[k][threadIdx.x];
+        D[c0 + threadIdx.x] = a;
     }
 }
 
-void launch_dvec(const StaticData& sd, Work& w, int N_max, cudaStream_t st)
+void launch_D(Work& w, int M_max, cudaStream_t st)
 {
-    if (N_max == 0) return;
-    k_dvec<<<(N_max + 255) / 256, 256, 0, st>>>(sd, w.gs, w.rowpix, w.dvec, w.cvec);
+    k_D<<<(M_max + 63) / 64 * (64 / D_CELLS), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, oz_nz(w.oz), oz_nst(w.oz),
+                                                                 w.dvec, w.cvec, w.D);
     count_launches(1);
-}
-
-// ---- D = L'^T (C^-1 d): column sums over row chunks, then a fixed-order sum ----
-#define D_CHUNK 256
-__global__ void k_D_partial(const GridState* __restrict__ gs, const double* __restrict__ L, int ldL,
-                            const double* __restrict__ dvec, const double* __restrict__ cvec,
-                            double* __restrict__ part, int M_max)
-{
-    const int N = gs->N, M = gs->M;
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r0 = blockIdx.y * D_CHUNK;
-    if (col >= M || r0 >= N) return;
-    const int r1 = min(r0 + D_CHUNK, N);
-    double acc = 0;
-    for (int r = r0; r < r1; r++) acc += L[(size_t)r * ldL + col] * dvec[r] * cvec[r];
-    part[(size_t)blockIdx.y * M_max + col] = acc;
-}
-
-__global__ void k_D_final(const GridState* __restrict__ gs, const double* __restrict__ part, double* __restrict__ D,
-                          int M_max)
-{
-    const int N = gs->N, M = gs->M;
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= mpad64(M)) return;
-    double acc = 0;
-    if (col < M) {
-        const int nch = (N + D_CHUNK - 1) / D_CHUNK;
-        for (int c = 0; c < nch; c++) acc += part[(size_t)c * M_max + col];
-    }
-    D[col] = acc;
-}
-
-void launch_D(Work& w, int N_max, int M_max, cudaStream_t st)
-{
-    dim3 g((M_max + 127) / 128, (N_max + D_CHUNK - 1) / D_CHUNK);
-    k_D_partial<<<g, 128, 0, st>>>(w.gs, w.Lpsf, w.ldL, w.dvec, w.cvec, w.partial, M_max);
-    k_D_final<<<(w.ldF + 127) / 128, 128, 0, st>>>(w.gs, w.partial, w.D, M_max);
-    count_launches(2);
 }
 
 // ---- curvature R (dense lower) and F += lambda R ----
@@ -252,17 +247,34 @@ void launch_logdet(const double* A, int ld, int M_max, Work& w, int which, cudaS
 }
 
 // ---- model image, chi^2, s^T R s and the evidence ----
+// 32 pixels a CTA, a lane each; a warp takes eight cells of every live 64-cell
+// block, then the warps' sums in order.
 __global__ void __launch_bounds__(256) k_model(const GridState* __restrict__ gs, const double* __restrict__ L,
-                                               int ldL, const double* __restrict__ s, double* __restrict__ model)
+                                               int ldL, const unsigned char* __restrict__ nz, int nst,
+                                               const double* __restrict__ s, double* __restrict__ model)
 {
+    __shared__ double part[8][32];
     const int N = gs->N, M = gs->M;
-    const int lane = threadIdx.x & 31;
-    for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < N; r += gridDim.x * (blockDim.x >> 5)) {
-        const double* row = L + (size_t)r * ldL;
-        double acc = 0;
-        for (int c = lane; c < M; c += 32) acc += row[c] * s[c];
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) model[r] = acc;
+    const int st = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = st * 32 + lane;
+    if (st * 32 >= N) return;
+    double acc = 0;
+    for (int cb = 0; cb * 64 < M; cb++) {
+        if (!nz[(size_t)cb * nst + st]) continue;
+        const int c0 = cb * 64 + warp * 8;
+        const double* p = L + (size_t)c0 * ldL + r;
+        double v[8];
+        #pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = (c0 + k < M && r < N) ? p[(size_t)k * ldL] : 0.0;
+        #pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (c0 + k < M) acc = fma(v[k], s[c0 + k], acc);
+    }
+    part[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && r < N) {
+        double a = 0;
+        for (int k = 0; k < 8; k++) a += part[k][lane];
+        model[r] = a;
     }
 }
 
@@ -360,9 +372,7 @@ void launch_model_chi2(const StaticData& sd, const SrcOpts& so, Work& w, int N_m
 {
     (void)M_max;
     if (N_max > 0 && !model_ready) {
-        int blocks = (N_max + 7) / 8;
-        if (blocks > 152 * 16) blocks = 152 * 16;
-        k_model<<<blocks, 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, w.s, w.model);
+        k_model<<<(N_max + 31) / 32, 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, oz_nz(w.oz), oz_nst(w.oz), w.s, w.model);
     }
     k_final<<<1, 1024, 0, st>>>(sd, so, w.gs, w.rowidx, w.model, w.s, w.active_index, regp, w.out);
     count_launches(2);

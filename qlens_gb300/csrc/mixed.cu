@@ -23,6 +23,7 @@
 #include "chol.cuh"
 #include "tc_syrk.cuh"
 #include "tma_map.h"
+#include "psf_tiles.cuh"
 #include "chol128.cuh"
 
 namespace qlpix {
@@ -31,17 +32,8 @@ namespace qlpix {
 
 struct MixedWork {
     double* t = nullptr;     // N (image-plane scratch)
-    // L by source cell (CSC of the merged pre-PSF rows), for k_psf_x
-    int* colcnt = nullptr;   // M_cap + 1 counts, then the column pointers
-    int* cursor = nullptr;   // M_cap
-    int* colrow = nullptr;   // nnz_cap
-    int2* ent = nullptr;     // nnz_cap: (image column << 16 | image row, L on the grid 2^-PSFX_LEXP)
-    int nnz_cap = 0;
-    int2* pixT = nullptr;    // image pixels, x fastest: (active row or -1, sqrt(C^-1))
+    Csc csc{};               // L by source cell, for k_psf_x and L^T
     float* F0 = nullptr;     // lambda optimisation: X X^T before lambda R (allocated on first use)
-    int* col_u = nullptr;    // nnz_cap: rows of each column in atomic (fill) order
-    int* src_u = nullptr;    // nnz_cap: their positions in the merged CSR rows
-    double* colval64 = nullptr; // nnz_cap: FP64 values, rows ascending within a column
     void* X_hi = nullptr;    // F16 (or TF32 in FP32 storage) parts of X
     void* X_lo = nullptr;
     bool half = true;        // X in F16 for the kind::f16 SYRK
@@ -49,9 +41,6 @@ struct MixedWork {
     int M_cap = 0;           // rows of X, multiple of 128
     unsigned char* nz = nullptr;
     int nkb_cap = 0;
-    uint2* tiles = nullptr;    // (cell, image tile) items of the PSF-to-X build
-    unsigned* tile_active = nullptr; // bitmap of the image's tiles with active pixels, then the items' count
-    int psfx_words = 0;        // words of the bitmap
     float* F32 = nullptr;
     float* R32 = nullptr;
     int ld32 = 0;
@@ -142,7 +131,7 @@ __global__ void k_csc_count(StaticData sd, const GridState* __restrict__ gs, con
         const int i = pix / sd.ny, j = pix - i * sd.ny;
         const int nxp = sd.nx + 2 * (sd.pnx / 2);
         pixT[(size_t)(j + sd.pny / 2) * nxp + i + sd.pnx / 2] = make_int2(r, __float_as_int(sq));
-        const int tile = j / 8 * ntx + i / 32;                  // PSFX_R rows
+        const int tile = j / PSFX_R * ntx + i / 32;
         if (!(active[tile >> 5] >> (tile & 31) & 1u)) atomicOr(&active[tile >> 5], 1u << (tile & 31));
     }
 }
@@ -190,11 +179,19 @@ __global__ void k_csc_fill(const GridState* __restrict__ gs, const int* __restri
     }
 }
 
-// An entry of a column as the PSF-to-X build reads it: its pixel and L on its grid.
-__device__ __forceinline__ int2 psfx_entry(int row, double v, const int* __restrict__ rowpix, int ny)
+// Entry k of the sorted columns: as the PSF-to-X build reads it (its pixel and L
+// on its grid) with its row and FP64 value, or (fine) as the plain path's build
+// of L' does.
+__device__ __forceinline__ void csc_store(const Csc& o, int k, int row, double v, const int* __restrict__ rowpix, int ny)
 {
-    const int pix = rowpix[row], iq = pix / ny;
-    return make_int2((iq << 16) | (pix - iq * ny), __float2int_rn((float)v * ldexpf(1.0f, PSFX_LEXP)));
+    const int pix = rowpix[row], i = pix / ny, j = pix - i * ny;
+    if (o.fine) {
+        o.fine[k] = psf64_entry(i, j, v);
+        return;
+    }
+    o.colrow[k] = row;
+    o.ent[k] = make_int2((i << 16) | j, __float2int_rn((float)v * ldexpf(1.0f, PSFX_LEXP)));
+    o.colval64[k] = v;
 }
 
 // Each column's entries in increasing row order, so that every sum over a
@@ -206,61 +203,6 @@ __device__ __forceinline__ int2 psfx_entry(int row, double v, const int* __restr
 // CSC_SORT_MAX entries, and past that each entry's rank counted directly.
 #define CSC_SORT_MAX 4096
 #define CSC_SORT_WARP 64    // columns sorted a warp each (k_csc_sort_w)
-__global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ gs, const int* __restrict__ colptr,
-                                                  const int* __restrict__ col_u, const int* __restrict__ src_u,
-                                                  const double* __restrict__ cval, int* __restrict__ colrow,
-                                                  int2* __restrict__ ent, double* __restrict__ colval64,
-                                                  const int* __restrict__ rowpix, int ny)
-{
-    __shared__ int key[CSC_SORT_MAX];
-    __shared__ int pos[CSC_SORT_MAX];
-    const int s = blockIdx.x;
-    if (s >= gs->M) return;
-    const int b = colptr[s], n = colptr[s + 1] - b;
-    if (n <= CSC_SORT_WARP) return;                       // k_csc_sort_w's
-    if (n <= CSC_SORT_MAX) {
-        int p2 = 1;
-        while (p2 < n) p2 <<= 1;
-        for (int i = threadIdx.x; i < p2; i += blockDim.x) {
-            key[i] = (i < n) ? col_u[b + i] : INT_MAX;
-            pos[i] = (i < n) ? src_u[b + i] : 0;
-        }
-        __syncthreads();
-        for (int k = 2; k <= p2; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = threadIdx.x; i < p2; i += blockDim.x) {
-                    const int l = i ^ j;
-                    if (l > i) {
-                        const bool up = (i & k) == 0;
-                        const int ki = key[i], kl = key[l];
-                        if ((ki > kl) == up) {
-                            key[i] = kl; key[l] = ki;
-                            const int t = pos[i]; pos[i] = pos[l]; pos[l] = t;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const double v = cval[pos[i]];
-            colrow[b + i] = key[i];
-            ent[b + i] = psfx_entry(key[i], v, rowpix, ny);
-            colval64[b + i] = v;
-        }
-        return;
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int ri = col_u[b + i];
-        int rank = 0;
-        for (int j = 0; j < n; j++) rank += (col_u[b + j] < ri) ? 1 : 0;
-        const double v = cval[src_u[b + i]];
-        colrow[b + rank] = ri;
-        ent[b + rank] = psfx_entry(ri, v, rowpix, ny);
-        colval64[b + rank] = v;
-    }
-}
-
 // Columns of up to CSC_SORT_WARP entries, a warp each: the same permutation
 // by a bitonic network in registers (R = 1 or 2 entries a lane, entry
 // lane + 32 h in register h; partners 32 apart within the lane, the others
@@ -278,8 +220,7 @@ __device__ __forceinline__ void csc_bitonic_step(int& key, int& pos, int e, int 
 template <int R>
 __device__ __forceinline__ void csc_sort_warp(const int* __restrict__ col_u, const int* __restrict__ src_u,
                                               const double* __restrict__ cval, int b, int n, int lane,
-                                              int* __restrict__ colrow, int2* __restrict__ ent,
-                                              double* __restrict__ colval64, const int* __restrict__ rowpix, int ny)
+                                              const Csc& out, const int* __restrict__ rowpix, int ny)
 {
     int key[R], pos[R];
     #pragma unroll
@@ -313,28 +254,81 @@ __device__ __forceinline__ void csc_sort_warp(const int* __restrict__ col_u, con
     #pragma unroll
     for (int h = 0; h < R; h++) {
         const int e = lane + 32 * h;
-        if (e < n) {
-            const double v = cval[pos[h]];
-            colrow[b + e] = key[h];
-            ent[b + e] = psfx_entry(key[h], v, rowpix, ny);
-            colval64[b + e] = v;
+        if (e < n) csc_store(out, b + e, key[h], cval[pos[h]], rowpix, ny);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ gs, const int* __restrict__ colptr,
+                                                  const int* __restrict__ col_u, const int* __restrict__ src_u,
+                                                  const double* __restrict__ cval, Csc out,
+                                                  const int* __restrict__ rowpix, int ny, double* __restrict__ clear,
+                                                  int ld)
+{
+    __shared__ int key[CSC_SORT_MAX];
+    __shared__ int pos[CSC_SORT_MAX];
+    const int s = blockIdx.x;
+    if (s >= gs->M) return;
+    const int b = colptr[s], n = colptr[s + 1] - b;
+    if (clear) {
+        double2* row = reinterpret_cast<double2*>(clear + (size_t)s * ld);
+        for (int i = threadIdx.x; i < (gs->N + 1) / 2; i += blockDim.x) row[i] = make_double2(0.0, 0.0);
+    }
+    if (n <= CSC_SORT_WARP) {
+        if (clear && threadIdx.x < 32) {
+            if (n <= 32) csc_sort_warp<1>(col_u, src_u, cval, b, n, threadIdx.x, out, rowpix, ny);
+            else csc_sort_warp<2>(col_u, src_u, cval, b, n, threadIdx.x, out, rowpix, ny);
         }
+        return;                                           // else k_csc_sort_w's
+    }
+    if (n <= CSC_SORT_MAX) {
+        int p2 = 1;
+        while (p2 < n) p2 <<= 1;
+        for (int i = threadIdx.x; i < p2; i += blockDim.x) {
+            key[i] = (i < n) ? col_u[b + i] : INT_MAX;
+            pos[i] = (i < n) ? src_u[b + i] : 0;
+        }
+        __syncthreads();
+        for (int k = 2; k <= p2; k <<= 1) {
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                for (int i = threadIdx.x; i < p2; i += blockDim.x) {
+                    const int l = i ^ j;
+                    if (l > i) {
+                        const bool up = (i & k) == 0;
+                        const int ki = key[i], kl = key[l];
+                        if ((ki > kl) == up) {
+                            key[i] = kl; key[l] = ki;
+                            const int t = pos[i]; pos[i] = pos[l]; pos[l] = t;
+                        }
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            csc_store(out, b + i, key[i], cval[pos[i]], rowpix, ny);
+        }
+        return;
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int ri = col_u[b + i];
+        int rank = 0;
+        for (int j = 0; j < n; j++) rank += (col_u[b + j] < ri) ? 1 : 0;
+        csc_store(out, b + rank, ri, cval[src_u[b + i]], rowpix, ny);
     }
 }
 
 __global__ void __launch_bounds__(256, 4) k_csc_sort_w(const GridState* __restrict__ gs,
                                                        const int* __restrict__ colptr,
                                                        const int* __restrict__ col_u, const int* __restrict__ src_u,
-                                                       const double* __restrict__ cval, int* __restrict__ colrow,
-                                                       int2* __restrict__ ent, double* __restrict__ colval64,
-                                                  const int* __restrict__ rowpix, int ny)
+                                                       const double* __restrict__ cval, Csc out,
+                                                       const int* __restrict__ rowpix, int ny)
 {
     const int lane = threadIdx.x & 31;
     const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= gs->M) return;                                // whole warps
     const int b = colptr[s], n = colptr[s + 1] - b;
-    if (n <= 32) csc_sort_warp<1>(col_u, src_u, cval, b, n, lane, colrow, ent, colval64, rowpix, ny);
-    else if (n <= CSC_SORT_WARP) csc_sort_warp<2>(col_u, src_u, cval, b, n, lane, colrow, ent, colval64, rowpix, ny);
+    if (n <= 32) csc_sort_warp<1>(col_u, src_u, cval, b, n, lane, out, rowpix, ny);
+    else if (n <= CSC_SORT_WARP) csc_sort_warp<2>(col_u, src_u, cval, b, n, lane, out, rowpix, ny);
 }
 
 // out[s] = sum over column s of L of value * w[row]: one warp per column, lane
@@ -381,30 +375,6 @@ __device__ __forceinline__ float ll2f_rn_int(long long v)
     return __uint_as_float(sign | ((unsigned)(e + 127) << 23) | (m & 0x7fffffu));
 }
 
-// The first of n entries sorted by image row (low half of x) whose row is at
-// least jmin, by a whole warp: 32 probes a round.
-__device__ __forceinline__ int warp_lower_bound_row(const int2* __restrict__ ent, int n, int jmin)
-{
-    const int lane = threadIdx.x & 31;
-    int lo = 0, hi = n;                       // the answer lies in [lo, hi]
-    while (hi - lo > 32) {
-        const int step = (hi - lo + 31) / 32;
-        const int p = lo + lane * step;
-        const unsigned b = __ballot_sync(0xffffffffu, p >= hi || (ent[p].x & 0xffff) >= jmin);
-        if (b == 0) {
-            lo = lo + 31 * step + 1;
-        } else {
-            const int f = __ffs(b) - 1;
-            const int pf = lo + f * step;
-            if (f > 0) lo = lo + (f - 1) * step + 1;
-            hi = min(hi, pf);
-        }
-    }
-    const int p = lo + lane;
-    const unsigned b = __ballot_sync(0xffffffffu, p >= hi || (ent[p].x & 0xffff) >= jmin);
-    return b ? min(lo + __ffs(b) - 1, hi) : hi;
-}
-
 // X by image tiles of 32 pixels along x and PSFX_R rows.  k_psfx_tiles lists the
 // tiles with active pixels that some footprint of a cell reaches, a warp a cell;
 // k_psf_x gives each listed tile to a warp, lane x keeping its column's sums in
@@ -422,53 +392,6 @@ __device__ __forceinline__ int warp_lower_bound_row(const int2* __restrict__ ent
 // 36,000 pixels 970 -> 118; a 31 x 31 PSF on 42,000 pixels 383 -> 180.
 // PAD = false (PSFs whose bordered taps pass PSFX_PAD_BYTES): taps by their
 // bounds from global memory.
-#define PSFX_R 8
-#define PSFX_PAD_BYTES (96 * 1024)
-__host__ __device__ __forceinline__ int psfx_pitch(int pny) { return (pny + 2 * PSFX_R - 2) | 1; }
-static inline size_t psfx_tap_bytes(int pnx, int pny) { return sizeof(int) * (size_t)(pnx + 62) * psfx_pitch(pny); }
-
-// a warp per cell, its bitmap of the image's tiles in shared memory
-__global__ void k_psfx_tiles(StaticData sd, const GridState* __restrict__ gs, const int* __restrict__ colptr,
-                             const int2* __restrict__ ent_g, int ntx, int nwords, const unsigned* __restrict__ active,
-                             int* __restrict__ count, uint2* __restrict__ list)
-{
-    extern __shared__ unsigned mark_all[];
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, s = blockIdx.x * nw + (threadIdx.x >> 5);
-    if (s >= gs->M) return;                                       // whole warps
-    unsigned* mark = mark_all + (threadIdx.x >> 5) * nwords;
-    const int pnx = sd.pnx, pny = sd.pny, nxh = pnx / 2, nyh = pny / 2;
-    const int n = colptr[s + 1] - colptr[s];
-    const int2* ent = ent_g + colptr[s];
-    for (int i = lane; i < nwords; i += 32) mark[i] = 0;
-    __syncwarp();
-    for (int e = lane; e < n; e += 32) {
-        const int en = ent[e].x, i0 = (en >> 16) - nxh, j0 = (en & 0xffff) - nyh;
-        const int c0 = max(i0, 0) >> 5, c1 = (min(i0 + pnx, sd.nx) - 1) >> 5;
-        const int t0 = max(j0, 0) / PSFX_R, t1 = (min(j0 + pny, sd.ny) - 1) / PSFX_R;
-        for (int t = t0; t <= t1; t++)
-            for (int c = c0; c <= c1; c++) {
-                const int k = t * ntx + c;
-                if (!(mark[k >> 5] >> (k & 31) & 1u)) atomicOr(&mark[k >> 5], 1u << (k & 31));
-            }
-    }
-    __syncwarp();
-    for (int w0 = 0; w0 < nwords; w0 += 32) {
-        const int wd = w0 + lane;
-        unsigned bits = wd < nwords ? mark[wd] & active[wd] : 0u;
-        int at = __popc(bits);
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, at, o);
-            if (lane >= o) at += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, at, 31);
-        if (total == 0) continue;
-        int base = 0;
-        if (lane == 0) base = atomicAdd(count, total);
-        at += __shfl_sync(0xffffffffu, base, 0) - __popc(bits);
-        for (; bits; bits &= bits - 1) list[at++] = make_uint2(s, 32 * wd + __ffs(bits) - 1);
-    }
-}
-
 template <bool PAD>
 __global__ void __launch_bounds__(512) k_psf_x(StaticData sd, const int* __restrict__ colptr,
                                                const int2* __restrict__ ent_g, const int2* __restrict__ pixT, int ntx,
@@ -680,13 +603,80 @@ void mixed_free(Slot& c)
     MixedWork* m = mw_of(c);
     if (!m) return;
     void* ptrs[] = {m->t, m->X_hi, m->X_lo, m->nz, m->F32, m->R32, m->u, m->v, m->r, m->z, m->y, m->img,
-                    m->linvF, m->yf, m->zf, m->flags, m->colcnt, m->cursor, m->colrow, m->ent,
-                    m->col_u, m->src_u, m->colval64, m->pixT, m->F0, m->tiles, m->tile_active,
+                    m->linvF, m->yf, m->zf, m->flags, m->F0,
                     m->cf.Lh, m->cf.Ll, m->cf.pexp, m->cf.ih, m->cf.il, m->cf.flags,
                     m->cr.Lh, m->cr.Ll, m->cr.pexp, m->cr.ih, m->cr.il, m->cr.flags};
     for (void* p : ptrs) if (p) cudaFree(p);
+    csc_free(m->csc);
     delete m;
     c.mixed = nullptr;
+}
+
+void csc_free(Csc& o)
+{
+    void* ptrs[] = {o.colcnt, o.cursor, o.colrow, o.ent, o.fine, o.col_u, o.src_u, o.colval64, o.pixT, o.tiles,
+                    o.tile_active};
+    for (void* p : ptrs) if (p) cudaFree(p);
+    o = Csc{};
+}
+
+// Workspace of L by source cell for M_cap cells of a slot; fine: the plain path's.
+cudaError_t csc_alloc(Csc& o, const Slot& c, int M_cap, bool fine)
+{
+    cudaError_t e = cudaSuccess;
+    auto A = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes > 0 ? bytes : 16); };
+    const int ntile = (c.img_nx + 31) / 32 * ((c.img_ny + PSFX_R - 1) / PSFX_R);
+    const size_t nnz = (size_t)3 * c.N_cap * c.nsub_cap;
+    o.words = (ntile + 31) / 32;
+    o.M_cap = M_cap;
+    o.npix_pad = c.npix_pad;
+    A((void**)&o.tiles, sizeof(uint2) * (size_t)M_cap * std::min(ntile, c.N_cap));
+    A((void**)&o.tile_active, sizeof(unsigned) * (o.words + 1));
+    A((void**)&o.colcnt, sizeof(int) * (size_t)(M_cap + 1));
+    A((void**)&o.cursor, sizeof(int) * (size_t)M_cap);
+    A((void**)&o.col_u, sizeof(int) * nnz);
+    A((void**)&o.src_u, sizeof(int) * nnz);
+    A((void**)&o.pixT, sizeof(int2) * (size_t)c.npix_pad);
+    if (fine) {
+        A((void**)&o.fine, sizeof(int4) * nnz);
+    } else {
+        A((void**)&o.colrow, sizeof(int) * nnz);
+        A((void**)&o.ent, sizeof(int2) * nnz);
+        A((void**)&o.colval64, sizeof(double) * nnz);
+    }
+    return e;
+}
+
+void csc_clear(const Csc& o, ClearList& l)
+{
+    l.add(o.colcnt, sizeof(int) * (size_t)(o.M_cap + 1));
+    l.add(o.tile_active, sizeof(unsigned) * (o.words + 1));
+    l.add(o.pixT, sizeof(int2) * (size_t)o.npix_pad, 0xffffffffu);
+}
+
+// L by source cell (CSC, rows ascending within a column) and the list of the
+// (cell, tile) pairs that its footprints reach.  clear: M rows of N of the plain
+// path's L', set to zero on the way.
+void launch_csc(const StaticData& sd, const Work& w, const Csc& o, int N_cap, double* clear, int ld, cudaStream_t st)
+{
+    const int rb = std::max(1, std::min((N_cap + 255) / 256, 152 * 8)), ntx = (sd.nx + 31) / 32;
+    k_csc_count<<<rb, 256, 0, st>>>(sd, w.gs, w.rowptr, w.cidx, w.ccnt, w.cvec, w.rowpix, o.colcnt, o.pixT, ntx,
+                                    o.tile_active);
+    k_csc_scan<<<1, 1024, 0, st>>>(w.gs, o.colcnt, o.cursor);
+    k_csc_fill<<<rb, 256, 0, st>>>(w.gs, w.rowptr, w.cidx, w.ccnt, o.cursor, o.col_u, o.src_u);
+    // the plain path's CTAs are there for the clearing anyway and take the short columns too
+    if (!clear)
+        k_csc_sort_w<<<(o.M_cap + 7) / 8, 256, 0, st>>>(w.gs, o.colcnt, o.col_u, o.src_u, w.cval, o, w.rowpix, sd.ny);
+    k_csc_sort<<<o.M_cap, 256, 0, st>>>(w.gs, o.colcnt, o.col_u, o.src_u, w.cval, o, w.rowpix, sd.ny, clear, ld);
+    const size_t wmark = sizeof(unsigned) * o.words;
+    const int tw = (int)std::max<size_t>(1, std::min<size_t>(8, 48 * 1024 / wmark));      // cells a CTA
+    if (o.fine)
+        k_psfx_tiles<<<(o.M_cap + tw - 1) / tw, 32 * tw, wmark * tw, st>>>(sd, w.gs, o.colcnt, o.fine, ntx, o.words,
+                                                                          o.tile_active, o.ntiles(), o.tiles);
+    else
+        k_psfx_tiles<<<(o.M_cap + tw - 1) / tw, 32 * tw, wmark * tw, st>>>(sd, w.gs, o.colcnt, o.ent, ntx, o.words,
+                                                                          o.tile_active, o.ntiles(), o.tiles);
+    count_launches(clear ? 5 : 6);
 }
 
 static size_t flow128_flags(int nb) { return (size_t)nb * nb + nb + 1; }
@@ -720,24 +710,10 @@ int mixed_init(Slot& c)
     A((void**)&m->X_hi, xbytes);
     A((void**)&m->X_lo, xbytes);
     A((void**)&m->nz, (size_t)(M_cap / TC_TILE) * m->nkb_cap + 3);
-    {
-        const int ntile = (c.img_nx + 31) / 32 * ((c.img_ny + PSFX_R - 1) / PSFX_R);
-        m->psfx_words = (ntile + 31) / 32;
-        A((void**)&m->tiles, sizeof(uint2) * (size_t)M_cap * std::min(ntile, c.N_cap));
-        A((void**)&m->tile_active, sizeof(unsigned) * (m->psfx_words + 1));
-    }
     A((void**)&m->F32, sizeof(float) * (size_t)M_cap * M_cap);
     A((void**)&m->R32, sizeof(float) * (size_t)M_cap * M_cap);
-    m->nnz_cap = 3 * c.N_cap * c.nsub_cap;
-    A((void**)&m->colcnt, sizeof(int) * (size_t)(M_cap + 1));
-    A((void**)&m->cursor, sizeof(int) * (size_t)M_cap);
-    A((void**)&m->colrow, sizeof(int) * (size_t)m->nnz_cap);
-    A((void**)&m->ent, sizeof(int2) * (size_t)m->nnz_cap);
-    A((void**)&m->col_u, sizeof(int) * (size_t)m->nnz_cap);
-    A((void**)&m->pixT, sizeof(int2) * (size_t)c.npix_pad);
     A((void**)&m->img, sizeof(double) * (size_t)c.npix_pad);
-    A((void**)&m->src_u, sizeof(int) * (size_t)m->nnz_cap);
-    A((void**)&m->colval64, sizeof(double) * (size_t)m->nnz_cap);
+    if (e == cudaSuccess) e = csc_alloc(m->csc, c, M_cap, false);
     A((void**)&m->t, sizeof(double) * (size_t)(c.N_cap + 64));
     A((void**)&m->u, sizeof(double) * (size_t)(c.N_cap + 64));
     A((void**)&m->v, sizeof(double) * M_cap);
@@ -832,9 +808,7 @@ void mixed_clear(Slot& slot, ClearList& l, bool trial)
     if (trial) return;
     l.add(m->cr.flags, sizeof(int) * flow128_flags(m->nb));
     l.add(m->nz, (size_t)(m->M_cap / TC_TILE) * m->nkb_cap);
-    l.add(m->colcnt, sizeof(int) * (size_t)(m->M_cap + 1));
-    l.add(m->tile_active, sizeof(unsigned) * (m->psfx_words + 1));
-    l.add(m->pixT, sizeof(int2) * (size_t)slot.npix_pad, 0xffffffffu);
+    csc_clear(m->csc, l);
     l.add(m->img, sizeof(double) * (size_t)slot.npix_pad);
 }
 
@@ -885,39 +859,23 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
         n += 3;
         cudaEventRecord(slot.side_join, slot.side);
     }
-    // L by source cell (CSC, rows ascending within a column)
-    {
-        const int rb = std::min((N_cap + 255) / 256, 152 * 8);
-        k_csc_count<<<std::max(rb, 1), 256, 0, st>>>(sd, w.gs, w.rowptr, w.cidx, w.ccnt, w.cvec, w.rowpix, m->colcnt,
-                                                     m->pixT, (sd.nx + 31) / 32, m->tile_active);
-        k_csc_scan<<<1, 1024, 0, st>>>(w.gs, m->colcnt, m->cursor);
-        k_csc_fill<<<std::max(rb, 1), 256, 0, st>>>(w.gs, w.rowptr, w.cidx, w.ccnt, m->cursor, m->col_u, m->src_u);
-        k_csc_sort_w<<<(m->M_cap + 7) / 8, 256, 0, st>>>(w.gs, m->colcnt, m->col_u, m->src_u, w.cval, m->colrow,
-                                                        m->ent, m->colval64, w.rowpix, sd.ny);
-        k_csc_sort<<<m->M_cap, 256, 0, st>>>(w.gs, m->colcnt, m->col_u, m->src_u, w.cval, m->colrow, m->ent,
-                                            m->colval64, w.rowpix, sd.ny);
-        n += 5;
-    }
+    launch_csc(sd, w, m->csc, N_cap, nullptr, 0, st);
     // D = L^T P^T (C^-1 d), FP64
-    op_conv(sd, w, N_cap, true, w.dvec, w.cvec, m->t, m->img, m->pixT, st);
-    k_LTw_csc<<<ltw_blocks, 256, 0, st>>>(w.gs, m->colcnt, m->colrow, m->colval64, m->t, w.D);
+    op_conv(sd, w, N_cap, true, w.dvec, w.cvec, m->t, m->img, m->csc.pixT, st);
+    k_LTw_csc<<<ltw_blocks, 256, 0, st>>>(w.gs, m->csc.colcnt, m->csc.colrow, m->csc.colval64, m->t, w.D);
     n++;
     // X = (P L sqrt(C^-1))^T and its block flags, from L by source cell
     const float xs = m->half ? ldexpf(1.0f, sd.x_exp) : 1.0f;     // F16 scale of X
     const int ntx = (sd.nx + 31) / 32;
-    const int* ntiles = reinterpret_cast<const int*>(m->tile_active + m->psfx_words);
+    const int* ntiles = m->csc.ntiles();
     {
-        const size_t wmark = sizeof(unsigned) * m->psfx_words;
-        const int tw = (int)std::max<size_t>(1, std::min<size_t>(8, 48 * 1024 / wmark));      // cells a CTA
-        k_psfx_tiles<<<(m->M_cap + tw - 1) / tw, 32 * tw, wmark * tw, st>>>(
-            sd, w.gs, m->colcnt, m->ent, ntx, m->psfx_words, m->tile_active, const_cast<int*>(ntiles), m->tiles);
         const int pt = (c->psfx_threads == 128 || c->psfx_threads == 512) ? c->psfx_threads : 256;
-        const size_t taps = psfx_tap_bytes(sd.pnx, sd.pny);
+        const size_t taps = sizeof(int) * psfx_taps(sd.pnx, sd.pny);
         const bool pad = taps <= PSFX_PAD_BYTES;
         auto k = pad ? k_psf_x<true> : k_psf_x<false>;
-        k<<<152 * 1024 / pt, pt, pad ? taps : 0, st>>>(sd, m->colcnt, m->ent, m->pixT, ntx, ntiles, m->tiles, m->X_hi,
+        k<<<152 * 1024 / pt, pt, pad ? taps : 0, st>>>(sd, m->csc.colcnt, m->csc.ent, m->csc.pixT, ntx, ntiles, m->csc.tiles, m->X_hi,
                                                        m->X_lo, xs, m->half ? 1 : 0, m->K_cap, m->nz, m->nkb_cap);
-        n += 2;
+        n++;
     }
     if (ev) cudaEventRecord(ev[3], st);
     {
@@ -930,7 +888,7 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
                                                                        m->nkb_cap, m->F32, m->ld32, 1.0f);
         n++;
         // X back to all zero for the next evaluation
-        k_x_clean<<<152 * 8, 256, 0, st>>>(sd, m->pixT, ntx, ntiles, m->tiles, m->X_hi, m->X_lo, m->half ? 1 : 0,
+        k_x_clean<<<152 * 8, 256, 0, st>>>(sd, m->csc.pixT, ntx, ntiles, m->csc.tiles, m->X_hi, m->X_lo, m->half ? 1 : 0,
                                            m->K_cap);
         n++;
     }
@@ -962,9 +920,9 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
         n += 3;
         if (it == refine) break;
         op_Ls(w, N_cap, w.s, m->t, st);
-        op_conv(sd, w, N_cap, false, m->t, nullptr, m->u, m->img, m->pixT, st);
-        op_conv(sd, w, N_cap, true, m->u, w.cvec, m->t, m->img, m->pixT, st);
-        k_LTw_csc<<<ltw_blocks, 256, 0, st>>>(w.gs, m->colcnt, m->colrow, m->colval64, m->t, m->v);
+        op_conv(sd, w, N_cap, false, m->t, nullptr, m->u, m->img, m->csc.pixT, st);
+        op_conv(sd, w, N_cap, true, m->u, w.cvec, m->t, m->img, m->csc.pixT, st);
+        k_LTw_csc<<<ltw_blocks, 256, 0, st>>>(w.gs, m->csc.colcnt, m->csc.colrow, m->csc.colval64, m->t, m->v);
         n++;
         k_residual<<<(so.snx * so.sny + 255) / 256, 256, 0, st>>>(w.gs, w.D, m->v, w.active_index, regp,
                                                                   so.regularization, w.s, m->r);
@@ -972,7 +930,7 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
     }
     // model image P L s in FP64 for chi^2
     op_Ls(w, N_cap, w.s, m->t, st);
-    op_conv(sd, w, N_cap, false, m->t, nullptr, w.model, m->img, m->pixT, st);
+    op_conv(sd, w, N_cap, false, m->t, nullptr, w.model, m->img, m->csc.pixT, st);
     count_launches(n);
     return QLP_OK;
 }

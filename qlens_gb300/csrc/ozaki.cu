@@ -1,5 +1,5 @@
 // ozaki.cu -- the plain path's FP64 contraction F = L'^T C^-1 L' on the tensor
-// cores: L' cut into digits (k_oz_scan, k_oz_slice), the digit products
+// cores: L' cut into digits (k_oz_slice), the digit products
 // (k_oz_syrk, ozaki.cuh) and the integers turned into F (k_oz_finish).
 // Reference: QLens::create_lensing_matrices_from_Lmatrix_dense
 // (pixelgrid.cpp:15590-15736).
@@ -39,41 +39,6 @@ __device__ __forceinline__ void oz_tile(int t, int& I, int& j)
     j = t - i * (i + 1);
 }
 
-// Each source cell's largest biased exponent and the 32-pixel stages of each
-// 64 cells that hold a nonzero.  Reads the dense L' once (memory bound); the
-// tests are on the bits, FP64 compares would bound it instead.  A CTA takes
-// 64 cells x 128 pixels.
-__global__ void __launch_bounds__(256) k_oz_scan(const GridState* __restrict__ gs, const double* __restrict__ L,
-                                                 int ldL, int* __restrict__ emax, unsigned char* __restrict__ nz,
-                                                 int nst)
-{
-    __shared__ int se[4][64];
-    __shared__ int any[4];
-    const int N = gs->N, M = gs->M;
-    const int cb = blockIdx.y, p0 = blockIdx.x * 128;
-    if (cb * 64 >= M || p0 >= N) return;
-    const int c = threadIdx.x & 63, q = threadIdx.x >> 6;      // pixels [32 q, 32 q + 32) of the chunk: one stage
-    const int cell = cb * 64 + c;
-    if (threadIdx.x < 4) any[threadIdx.x] = 0;
-    int e = 0;
-    if (cell < M) {
-        const int r0 = p0 + 32 * q, r1 = min(r0 + 32, N);
-        const double* col = L + cell;
-        #pragma unroll 8
-        for (int r = r0; r < r1; r++) e = max(e, oz_exponent(col[(size_t)r * ldL]));
-    }
-    __syncthreads();
-    se[q][c] = e;
-    if (__any_sync(0xffffffffu, e != 0) && (threadIdx.x & 31) == 0) any[q] = 1;
-    __syncthreads();
-    if (threadIdx.x < 64) {
-        const int m = max(max(se[0][c], se[1][c]), max(se[2][c], se[3][c]));
-        if (m > 0) atomicMax(&emax[cell], m);
-    }
-    if (threadIdx.x < 4 && p0 + 32 * (int)threadIdx.x < N)
-        nz[(size_t)cb * nst + (p0 >> 5) + threadIdx.x] = any[threadIdx.x] ? 1 : 0;
-}
-
 // With a noise map the operand is L' sqrt(C^-1): the exponent of the largest
 // sqrt(C^-1) is added to every cell's bound (an upper bound of the product's).
 __global__ void __launch_bounds__(1024) k_oz_noise_exp(const GridState* __restrict__ gs,
@@ -93,44 +58,40 @@ __global__ void __launch_bounds__(1024) k_oz_noise_exp(const GridState* __restri
     }
 }
 
-// The digits of 64 cells x 32 pixels of L'^T (sqrt(C^-1)): L' is read along the
-// cells (512-byte rows), transposed through shared memory as integers and
-// written along the pixels, 16 bytes a thread and digit.  Stages without a
-// nonzero in the cells' 128-row block are never loaded by the products, so they
-// are skipped.  14 bytes written per 8 read: memory bound.
+// The digits of 64 cells x 32 pixels of L'^T (sqrt(C^-1)), eight pixels a thread.
+// Stages without a nonzero in the cells' 128-row block are never loaded by the
+// products, so they are skipped.  14 bytes written per 8 read: memory bound.
 __global__ void __launch_bounds__(256) k_oz_slice(const GridState* __restrict__ gs, const double* __restrict__ L,
                                                   int ldL, const double* __restrict__ cvec, int use_noise_map,
                                                   const int* __restrict__ emax, const unsigned char* __restrict__ nz,
                                                   int nst, int st0, __half* __restrict__ xs, int M128, int Kc)
 {
-    __shared__ unsigned long long sq[64][33];
     const int N = gs->N, M = gs->M;
-    const int cb = blockIdx.y, st = st0 + blockIdx.x, p0 = st * 32;
+    const int cb = blockIdx.y, st = st0 + blockIdx.x;
     const int ncb = (M + 63) / 64;
-    if (cb >= ((ncb + 1) & ~1) || p0 >= N) return;
+    if (cb >= ((ncb + 1) & ~1) || st * 32 >= N) return;
     const int other = cb ^ 1;
-    if (!((cb < ncb && nz[(size_t)cb * nst + st]) || (other < ncb && nz[(size_t)other * nst + st]))) return;
-    {
-        const int c = threadIdx.x & 63, q = threadIdx.x >> 6;
-        const int cell = cb * 64 + c;
-        const int em = (cell < M) ? emax[cell] : 0;
-        #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int k = q + 4 * u, r = p0 + k;
-            double x = 0;
-            if (cell < M && r < N) {
-                x = L[(size_t)r * ldL + cell];
-                if (use_noise_map && x != 0) x *= sqrt(cvec[r]);
-            }
-            sq[c][k] = oz_bias<OZ_S>(em > 0 && em < 2047 ? oz_fixed54(x, em) : 0);
-        }
-    }
-    __syncthreads();
-    const int c = threadIdx.x >> 2, k0 = (threadIdx.x & 3) * 8;
+    const bool live = cb < ncb && nz[(size_t)cb * nst + st];
+    if (!(live || (other < ncb && nz[(size_t)other * nst + st]))) return;
+    const int c = threadIdx.x >> 2, k0 = (threadIdx.x & 3) * 8, cell = cb * 64 + c, r0 = st * 32 + k0;
     unsigned long long q[8];
     #pragma unroll
-    for (int u = 0; u < 8; u++) q[u] = sq[c][k0 + u];
-    __half* out = xs + (size_t)(cb * 64 + c) * Kc + (size_t)blockIdx.x * 32 + k0;
+    for (int u = 0; u < 8; u++) q[u] = oz_bias<OZ_S>(0);
+    const int em = (cell < M) ? emax[cell] : 0;
+    if (live && em > 0 && em < 2047) {
+        #pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+            const double2 v = *reinterpret_cast<const double2*>(L + (size_t)cell * ldL + r0 + u);
+            #pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int r = r0 + u + k;
+                double x = r < N ? (k ? v.y : v.x) : 0.0;
+                if (use_noise_map && x != 0) x *= sqrt(cvec[r]);
+                q[u + k] = oz_bias<OZ_S>(oz_fixed54(x, em));
+            }
+        }
+    }
+    __half* out = xs + (size_t)cell * Kc + (size_t)blockIdx.x * 32 + k0;
     #pragma unroll
     for (int d = 0; d < OZ_S; d++) {
         *reinterpret_cast<uint4*>(out + (size_t)d * M128 * Kc) = oz_digits8<OZ_S>(q, d);
@@ -286,7 +247,7 @@ int oz_alloc(OzWork** out, int N_cap, int M_cap)
     A((void**)&z->xs, sizeof(__half) * (size_t)z->M128 * std::max(OZ_S * z->Kc, 8 * z->M128));
     A((void**)&z->part, pbytes);
     A((void**)&z->emax, sizeof(int) * z->M128);
-    A((void**)&z->nz, (size_t)(z->M128 / 64) * z->nst);
+    A((void**)&z->nz, (size_t)(z->M128 / 64) * z->nst + 3);
     if (e == cudaSuccess) e = cudaMemset(z->part, 0, pbytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_oz_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, oz_smem(OZ_S));
@@ -305,7 +266,17 @@ int oz_alloc(OzWork** out, int N_cap, int M_cap)
     return QLP_OK;
 }
 
-void oz_clear(const OzWork* z, ClearList& l) { l.add(z->emax, sizeof(int) * z->M128); }
+void oz_clear(const OzWork* z, ClearList& l)
+{
+    l.add(z->emax, sizeof(int) * z->M128);
+    l.add(z->nz, (size_t)(z->M128 / 64) * z->nst);
+}
+
+// What the build of L' (k_psf64) fills in: each cell's largest exponent and the
+// live 32-pixel stages of each 64 cells.
+int* oz_emax(OzWork* z) { return z->emax; }
+unsigned char* oz_nz(OzWork* z) { return z->nz; }
+int oz_nst(const OzWork* z) { return z->nst; }
 
 // The digits' buffer, free once F stands.
 void* oz_buffer(OzWork* z) { return z->xs; }
@@ -315,13 +286,9 @@ void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaS
     OzWork* z = w.oz;
     const int nI = (M_max + OZ_TM - 1) / OZ_TM, tiles = nI * (nI + 1), ncb = 2 * nI;
     int n = 0;
-    if (N_max > 0) {
-        k_oz_scan<<<dim3((N_max + 127) / 128, ncb), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, z->emax, z->nz, z->nst);
+    if (N_max > 0 && sd.use_noise_map) {
+        k_oz_noise_exp<<<1, 1024, 0, st>>>(w.gs, w.cvec, z->emax);
         n++;
-        if (sd.use_noise_map) {
-            k_oz_noise_exp<<<1, 1024, 0, st>>>(w.gs, w.cvec, z->emax);
-            n++;
-        }
     }
     const int nst = (N_max + 31) / 32, per = z->Kc / 32;
     for (int s0 = 0; s0 < nst; s0 += per) {

@@ -1,148 +1,210 @@
-// psf.cu -- PSF convolution of the lensing matrix into the dense L'.
+// psf.cu -- PSF convolution of the lensing matrix into the plain path's dense L',
+// kept by source cell.
 //
 // QLens::PSF_convolution_Lmatrix_dense, direct path (pixelgrid.cpp:14092-14176):
 //   L'[p][s] = sum over PSF taps (k-major, then l) of psf[k][l] * Ldense[q][s],
 //   q = the active pixel at (i_p + nx/2 - k, j_p + ny/2 - l).
-// The reference multiplies every dense row; this kernel gathers only the
-// merged nonzeros of each tapped row (about 3*nsub of M entries), adding them
-// in the same tap order, so in FP64 every L' entry is the same sum of the same
-// products in the same order (zero terms dropped).  One warp per output row
-// accumulates in shared memory; taps are separated by __syncwarp so the
-// per-entry order is the reference's.  Built with --fmad=false.
-//
-// The accumulator type is a template parameter; the plain path instantiates
-// double (bit-exact rows).  The mixed path builds its TF32 operand column by
-// column instead (k_psf_x, mixed.cu).
-#include "qlpix_internal.h"
+// The sums are exact in 64-bit fixed point (psf_tiles.cuh, StaticData::psf_fine):
+// L on the grid 2^-57, the taps to 2^-51 or better of the largest (2^-57 for a
+// Gaussian of 21 x 21), by halves; of a product (th 2^w + tl) (vh 2^29 + vl) only
+// tl vl is left out, below 2^-59 of the largest tap where that is an eighth of their
+// sum.  An FP64 sum rounds at 2^-53 of each product and partial sum.  Other PSFs are
+// summed in FP64.
+#include "qlpix_ctx.h"
+#include "psf_tiles.cuh"
 
 namespace qlpix {
 
-#define PSF_G 8          // taps whose entries are loaded before they are applied
+// outside the normal numbers; out of line, for eight of them inlined cost more to fetch
+// than a small problem's sums
+__device__ __noinline__ double fixed_scaled(long long s, int k) { return scalbn((double)s, -k); }
 
-template <typename T>
-__global__ void k_psf(StaticData sd, const GridState* __restrict__ gs, const int* __restrict__ rowpix,
-                      const int* __restrict__ pixindex, const int* __restrict__ rowptr,
-                      const int* __restrict__ cidx, const double* __restrict__ cval, const int* __restrict__ ccnt,
-                      T* __restrict__ Lpsf, int ldL, int M_max)
+// s 2^-k, |s| < 2^63, rounded to nearest even; integer arithmetic (FP64 conversions
+// go to the FP64 pipe) but for results outside the normal numbers.
+__device__ __forceinline__ double fixed_to_double(long long s, int k)
 {
-    extern __shared__ __align__(16) unsigned char psf_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const int nT = sd.pnx * sd.pny;
-    const int Tpad = (nT + PSF_G - 1) / PSF_G * PSF_G;
-    // per warp: M_max accumulators (T), Tpad psf values (T), Tpad (base, count)
-    unsigned char* mine = psf_smem + (size_t)warp * (sizeof(T) * (M_max + Tpad) + sizeof(int2) * Tpad);
-    T* acc = reinterpret_cast<T*>(mine);
-    T* tpsf = acc + M_max;
-    int2* tmeta = reinterpret_cast<int2*>(tpsf + Tpad);
-    const int N = gs->N, M = gs->M;
-    const int Mpad = (M + 63) & ~63;
-    const int nxh = sd.pnx / 2, nyh = sd.pny / 2;
-    for (int r = blockIdx.x * wpb + warp; r < N; r += gridDim.x * wpb) {
-        for (int s = lane; s < Mpad; s += 32) acc[s] = T(0);
-        const int pix = rowpix[r];
-        const int k = pix / sd.ny, l = pix - k * sd.ny;
-        // tap metadata, all loads independent
-        for (int t = lane; t < Tpad; t += 32) {
-            int base = 0, cnt = 0;
-            T pv = 0;
-            if (t < nT) {
-                const int pk = t / sd.pny, pl = t - pk * sd.pny;
-                const int ii = k + nxh - pk, jj = l + nyh - pl;
-                if (ii >= 0 && ii < sd.nx && jj >= 0 && jj < sd.ny) {
-                    const int q = pixindex[ii * sd.ny + jj];
-                    if (q >= 0) { base = rowptr[q]; cnt = ccnt[q]; pv = (T)sd.psf[t]; }
-                }
-            }
-            tmeta[t] = make_int2(base, cnt);
-            tpsf[t] = pv;
+    if (s == 0) return 0.0;
+    unsigned long long a = s < 0 ? 0ull - (unsigned long long)s : (unsigned long long)s;
+    int e = 63 - __clzll((long long)a);
+    if (e + 1022 - k < 1 || e + 1024 - k > 2046) return fixed_scaled(s, k);
+    if (e <= 52) {
+        a <<= 52 - e;
+    } else {
+        const int sh = e - 52;
+        const unsigned long long rem = a & ((1ull << sh) - 1), half = 1ull << (sh - 1);
+        a >>= sh;
+        if (rem > half || (rem == half && (a & 1))) a++;           // a carry to 2^53 moves the exponent below
+    }
+    const unsigned long long b = a + ((unsigned long long)(e + 1022 - k) << 52);
+    return __longlong_as_double((long long)(b | (s < 0 ? 1ull << 63 : 0)));
+}
+
+__device__ __forceinline__ int exponent_of(double x)
+{
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x) << 1;
+    return u == 0 ? 0 : max(1, (int)(u >> 53));
+}
+
+// L' by image tiles, as k_psf_x builds X: a warp takes a listed (cell, 32 x 8
+// pixels) pair, lane x keeps its column's sums and adds tap x L for every entry
+// whose footprint meets the tile, three wide multiply-adds and a 64-bit load from
+// shared memory a tap.  With the values go each cell's largest biased exponent and
+// the live 32-pixel stages of each 64 cells, for the digits.
+// The multiplies bound it.  A warp per image row that scattered tapped rows into
+// shared memory in FP64, a tap after the other, waited on those.  2,934 cells x
+// 11,772 pixels, 441 taps: 1,940 -> 146 us (and 46 us for the entries by cell and
+// the clearing of L'); 738 x 6,220, 49 taps: 101 -> 38 us; 16 uneven evaluations at
+// up to 4,096 cells, 121 taps: 14.2 -> 10.4 ms.  In FP64 these sums alone would take
+// the pipe 250 us.
+// FIXED = false (StaticData::psf_fixed, or bordered taps past PSF64_PAD_BYTES): FP64
+// sums, taps by their bounds from global memory.
+#define PSF64_PAD_BYTES (200 * 1024)
+template <bool FIXED>
+__global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* __restrict__ gs,
+                                               const int* __restrict__ colptr, const int4* __restrict__ ent_g,
+                                               const int2* __restrict__ pixT, int ntx, const int* __restrict__ count,
+                                               const uint2* __restrict__ list, double* __restrict__ L, int ldL,
+                                               int* __restrict__ emax, unsigned char* __restrict__ nz, int nst)
+{
+    extern __shared__ __align__(16) int2 taps64[];  // [pnx + 62][pitch]: column pk + 31, row pl + R - 1
+    constexpr int R = PSFX_R;
+    const int pnx = sd.pnx, pny = sd.pny, nxh = pnx / 2, nyh = pny / 2, nxp = sd.nx + 2 * nxh;
+    const int pitch = psfx_pitch(pny);
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, items = *count;
+    if ((int)blockIdx.x * nw >= items) return;
+    if (FIXED) {
+        for (int t = threadIdx.x; t < (pnx + 62) * pitch; t += blockDim.x) {
+            const int pk = t / pitch - 31, pl = t % pitch - (R - 1);
+            taps64[t] = (pk >= 0 && pk < pnx && pl >= 0 && pl < pny) ? sd.psf_fine[pl * pnx + pk] : make_int2(0, 0);
         }
-        __syncwarp();
-        for (int t0 = 0; t0 < Tpad; t0 += PSF_G) {
-            int si[PSF_G][2];
-            T sv[PSF_G][2];
-            #pragma unroll
-            for (int g = 0; g < PSF_G; g++) {
-                const int2 md = tmeta[t0 + g];
-                const T pv = tpsf[t0 + g];
-                #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const int e = lane + 32 * j;
-                    si[g][j] = -1;
-                    sv[g][j] = 0;
-                    if (e < md.y) { si[g][j] = cidx[md.x + e]; sv[g][j] = pv * (T)cval[md.x + e]; }
-                }
+        __syncthreads();
+    }
+    for (int it = blockIdx.x * nw + (threadIdx.x >> 5); it < items; it += gridDim.x * nw) {
+        const uint2 item = list[it];
+        const int s = item.x, y0 = (int)item.y / ntx * R, x0 = ((int)item.y % ntx) * 32, x = x0 + lane;
+        const int n = colptr[s + 1] - colptr[s];
+        const int4* ent = ent_g + colptr[s];
+        int lo = 0, hi = n;
+        if (n > 64) {
+            lo = warp_lower_bound_row(ent, n, y0 + nyh - pny + 1);
+            hi = warp_lower_bound_row(ent, n, y0 + R + nyh);
+        }
+        // th vh, th vl and tl vh: at most 2^62, 2^62 and 2^63 (StaticData::psf_w)
+        long long hh[R], hl[R], lh[R];
+        double acc[R];
+        #pragma unroll
+        for (int r = 0; r < R; r++) hh[r] = hl[r] = lh[r] = 0;
+        #pragma unroll
+        for (int r = 0; r < R; r++) acc[r] = 0;
+        unsigned bad = 0;
+        for (int e0 = lo; e0 < hi; e0 += 32) {
+            int dx = -32, dy = 0, vh = 0, vl = 0;
+            if (e0 + lane < hi) {
+                const int4 en = ent[e0 + lane];
+                dx = x0 - (ent_col(en) - nxh);           // column of lane 0's tap
+                dy = y0 - (ent_row(en) - nyh);           // row of the first row's tap
+                vh = en.y;
+                vl = en.z;
             }
-            #pragma unroll
-            for (int g = 0; g < PSF_G; g++) {
-                #pragma unroll
-                for (int j = 0; j < 2; j++)
-                    if (si[g][j] >= 0) acc[si[g][j]] = acc[si[g][j]] + sv[g][j];
-                const int2 md = tmeta[t0 + g];
-                if (md.y > 64) {   // rows with more than 64 merged entries: the rest in order
-                    const T pv = tpsf[t0 + g];
-                    for (int e = 64 + lane; e < md.y; e += 32) {
-                        const int s = cidx[md.x + e];
-                        acc[s] = acc[s] + pv * (T)cval[md.x + e];
+            unsigned hit = __ballot_sync(0xffffffffu, dx > -32 && dx < pnx && dy > -R && dy < pny);
+            const unsigned nan = __ballot_sync(0xffffffffu, vh == PSF64_BAD);
+            for (; hit; hit &= hit - 1) {
+                const int f = __ffs(hit) - 1;
+                const int ox = __shfl_sync(0xffffffffu, dx, f) + lane, oy = __shfl_sync(0xffffffffu, dy, f);
+                const int eh = __shfl_sync(0xffffffffu, vh, f), el = __shfl_sync(0xffffffffu, vl, f);
+                if (nan >> f & 1) {
+                    if (ox >= 0 && ox < pnx)
+                        for (int r = 0; r < R; r++) bad |= (oy + r >= 0 && oy + r < pny) ? 1u << r : 0u;
+                } else if (FIXED) {
+                    const int2* tp = taps64 + (ox + 31) * pitch + oy + R - 1;
+                    #pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        const int2 t = tp[r];
+                        hh[r] += (long long)t.x * eh;
+                        hl[r] += (long long)t.x * el;
+                        lh[r] += (long long)t.y * eh;
                     }
+                } else if (ox >= 0 && ox < pnx) {
+                    const double v = ((double)eh * 0x1p29 + (double)el) * 0x1p-57;
+                    #pragma unroll
+                    for (int r = 0; r < R; r++)
+                        if (oy + r >= 0 && oy + r < pny) acc[r] = fma(sd.psf[ox * pny + oy + r], v, acc[r]);
                 }
-                __syncwarp();
             }
         }
-        T* out = Lpsf + (size_t)r * ldL;
-        for (int s = lane; s < Mpad; s += 32) out[s] = acc[s];
-        __syncwarp();
+        int top = 0;
+        if (x < sd.nx) {
+            #pragma unroll
+            for (int r = 0; r < R; r++) {
+                if (y0 + r >= sd.ny) break;
+                const int row = pixT[(size_t)(y0 + r + nyh) * nxp + x + nxh].x;
+                if (row < 0) continue;
+                double v = acc[r];
+                if (FIXED) {
+                    // as many of the lower halves' bits as there is room for
+                    const int sh = max(0, min(20, __clzll(hh[r] < 0 ? -hh[r] : hh[r]) - 3));
+                    v = fixed_to_double((hh[r] << sh) + (hl[r] >> (29 - sh)) + (lh[r] >> (sd.psf_w - sh)),
+                                        sd.psf_t + 28 + sh);
+                }
+                if (bad >> r & 1) v = __longlong_as_double(0x7ff8000000000000ll);
+                const int e = exponent_of(v);
+                if (e == 0) continue;
+                L[(size_t)s * ldL + row] = v;
+                nz[(size_t)(s / 64) * nst + row / 32] = 1;
+                top = max(top, e);
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+        if (lane == 0 && top > 0) atomicMax(&emax[s], top);
     }
 }
 
-// Active row -> image pixel, the inverse of the compaction's pixindex.
-__global__ void k_rowpix(StaticData sd_, const int* __restrict__ rowidx, int* __restrict__ rowpix)
+// Active row -> image pixel, the inverse of the compaction's pixindex, and the
+// row's data and C^-1.
+__global__ void k_rowpix(StaticData sd_, const int* __restrict__ rowidx, int* __restrict__ rowpix,
+                         double* __restrict__ dvec, double* __restrict__ cvec)
 {
     const StaticData sd = eval_shape(sd_);
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < sd.n_mask; m += gridDim.x * blockDim.x) {
-        int r = rowidx[m];
-        if (r >= 0) rowpix[r] = sd.mpix[m];
+        const int r = rowidx[m];
+        if (r < 0) continue;
+        const int pix = sd.mpix[m];
+        rowpix[r] = pix;
+        dvec[r] = sd.data[pix];
+        cvec[r] = sd.use_noise_map ? sd.covinv[pix] : sd.cov_inverse;
     }
 }
 
 void psf_init_attributes()
 {
-    cudaFuncSetAttribute(k_psf<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-}
-
-template <typename T>
-static size_t psf_bytes_per_warp(int M_max, int nT)
-{
-    const int Tpad = (nT + PSF_G - 1) / PSF_G * PSF_G;
-    return sizeof(T) * ((size_t)M_max + Tpad) + sizeof(int2) * Tpad;
-}
-
-template <typename T>
-static void launch_psf_t(const StaticData& sd, Work& w, T* out, int ld, int M_max, cudaStream_t st)
-{
-    if (sd.n_mask == 0) return;
-    const int nT = sd.pnx * sd.pny;
-    const size_t per_warp = psf_bytes_per_warp<T>(M_max, nT);
-    int wpb = (int)((200 * 1024) / per_warp);
-    if (wpb > 8) wpb = 8;
-    if (wpb < 1) wpb = 1;
-    int blocks = (sd.n_mask + wpb - 1) / wpb;
-    if (blocks > 152 * 32) blocks = 152 * 32;
-    k_psf<T><<<blocks, 32 * wpb, per_warp * wpb, st>>>(sd, w.gs, w.rowpix, w.pixindex, w.rowptr, w.cidx, w.cval,
-                                                       w.ccnt, out, ld, M_max);
+    cudaFuncSetAttribute(k_psf64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PSF64_PAD_BYTES);
 }
 
 void launch_rowpix(const StaticData& sd, Work& w, cudaStream_t st)
 {
     if (sd.n_mask == 0) return;
-    k_rowpix<<<(sd.n_mask + 255) / 256, 256, 0, st>>>(sd, w.rowidx, w.rowpix);
+    k_rowpix<<<(sd.n_mask + 255) / 256, 256, 0, st>>>(sd, w.rowidx, w.rowpix, w.dvec, w.cvec);
     count_launches(1);
 }
 
-void launch_psf(const StaticData& sd, const SrcOpts& so, Work& w, int M_max, cudaStream_t st)
+int launch_psf(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st)
 {
-    (void)so;
-    launch_psf_t<double>(sd, w, w.Lpsf, w.ldL, M_max, st);
+    if (N_max == 0) return QLP_OK;
+    // the plain path's stated range of PSFs and source grids
+    const size_t nT = ((size_t)sd.pnx * sd.pny + 7) / 8 * 8;
+    if (8 * (M_max + nT) + 8 * nT > 227 * 1024) {
+        set_error("%s (%d)", "PSF and source grid too large for the plain path", (int)nT);
+        return QLP_ERR_CUDA;
+    }
+    launch_csc(sd, w, w.csc, N_max, w.Lpsf, w.ldL, st);
+    const size_t taps = sizeof(int2) * psfx_taps(sd.pnx, sd.pny);
+    const bool fixed = sd.psf_fixed && taps <= PSF64_PAD_BYTES;
+    auto k = fixed ? k_psf64<true> : k_psf64<false>;
+    k<<<152 * 3, 256, fixed ? taps : 0, st>>>(sd, w.gs, w.csc.colcnt, w.csc.fine, w.csc.pixT, (sd.nx + 31) / 32,
+                                            w.csc.ntiles(), w.csc.tiles, w.Lpsf, w.ldL, oz_emax(w.oz), oz_nz(w.oz),
+                                            oz_nst(w.oz));
     count_launches(1);
+    return QLP_OK;
 }
 
 }  // namespace qlpix

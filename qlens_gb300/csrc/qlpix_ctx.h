@@ -84,6 +84,7 @@ struct qlp_ctx {
     double* d_data = nullptr;
     double* d_covinv = nullptr;
     double* d_psf = nullptr;
+    int2* d_psf_fine = nullptr;    // the plain path's (StaticData::psf_fine)
     int* d_psf_int = nullptr;      // the PSF on the PSF-to-X fixed-point grid (StaticData::psf_int)
     int* d_mpix = nullptr;
 
@@ -155,6 +156,7 @@ void set_error(const char* fmt, const char* a, int code);
 // mixed.cu
 int mixed_init(Slot& slot);
 void mixed_free(Slot& slot);
+cudaError_t csc_alloc(Csc& o, const Slot& c, int M_cap, bool fine);
 // launch sequences of one evaluation: the whole of it, or, for the
 // regularisation-parameter optimisation, its lambda-independent part and one
 // lambda trial

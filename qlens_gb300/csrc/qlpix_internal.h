@@ -126,6 +126,12 @@ struct StaticData {            // per-context, uploaded once
     // the PSF on its grid, x fastest: psf_int[pl * pnx + pk] =
     // round(psf[pk * pny + pl] * 2^(fix_exp_x - PSFX_LEXP))
     const int* psf_int;
+    // the plain path's fixed-point PSF (k_psf64): tap = (hi 2^psf_w + lo) 2^-(psf_t + psf_w),
+    // |hi| <= 2^30, sum |hi| <= 2^33, |lo| <= 2^(psf_w - 1), x fastest; psf_w is the
+    // widest for which a sum of lo times |L| <= 2 (2^29 on its grid) stays within 64 bits
+    const int2* psf_fine;
+    int psf_t, psf_w;
+    int psf_fixed;             // 0: the taps are summed in FP64 instead (not finite, or below 2^-51 of the largest)
     // F16 operands of the mixed path's SYRK: X scaled by 2^x_exp puts its
     // largest possible entry (4 sum|psf| max sqrt(C^-1)) at or below 2^14
     int x_exp;
@@ -168,6 +174,25 @@ __device__ __forceinline__ SrcOpts eval_grid(SrcOpts o, const StaticData& s)
 struct OzWork;
 struct Chol64Work;
 
+// L by source cell (CSC of the merged pre-PSF rows), for the PSF builds by image
+// tiles (psf_tiles.cuh).
+struct Csc {
+    int* colcnt;               // M_cap + 1 counts, then the column pointers
+    int* cursor;               // M_cap
+    int* colrow;               // rows, ascending within a column
+    int2* ent;                 // (image column << 16 | image row, L on the grid 2^-PSFX_LEXP)
+    int4* fine;                // the plain path's entries (psf64_entry), in place of colrow, ent and colval64
+    double* colval64;          // FP64 values
+    int* col_u;                // rows of each column in atomic (fill) order
+    int* src_u;                // their positions in the merged CSR rows
+    int2* pixT;                // image pixels, x fastest: (active row or -1, sqrt(C^-1))
+    uint2* tiles;              // (cell, image tile) items
+    unsigned* tile_active;     // bitmap of the image's tiles with active pixels, then the items' count
+    int words;                 // words of the bitmap
+    int M_cap, npix_pad;
+    int* ntiles() const { return reinterpret_cast<int*>(tile_active + words); }
+};
+
 // Per-evaluation device workspace (sized for the largest case at creation).
 struct Work {
     double* spx;  double* spy;         // n_sub source points
@@ -183,10 +208,11 @@ struct Work {
     int* rowptr;                       // N+1
     int* Lidx;    double* Lval;        // pre-PSF L, CSR
     int* cidx;    double* cval; int* ccnt;   // compressed rows (duplicates summed), same capacity
-    double* Lpsf;                      // N x ldL, FP64
+    double* Lpsf;                      // M x ldL, FP64: L' by source cell (plain path)
+    Csc csc;                           // plain path: L by source cell
     OzWork* oz;                        // plain path: workspace of the FP64 contraction (ozaki.cu)
     Chol64Work* cholF;  Chol64Work* cholR;  // plain path: workspaces of the factorisations (cholfp64.cu)
-    int ldL;                           // leading dimension of Lpsf (>= M_max)
+    int ldL;                           // leading dimension of Lpsf (>= N_max, a multiple of 32)
     double* dvec; double* cvec;        // N: data and C^-1 per active row
     double* D;                         // M
     double* F;                         // M x ldF (lower triangle)
@@ -194,7 +220,6 @@ struct Work {
     int ldF;
     double* s;   double* tmp;          // M
     double* model;                     // N
-    double* partial;                   // reduction scratch
     double* gpart;  int* gpart_cnt;    // source-grid bounds: per-block partials (1024 blocks at most)
     int* cpart;                        // compaction: per-block counts (3 x 1025)
     double* linv;                      // per 64 columns: inverse of the diagonal block of F's factor
@@ -222,7 +247,7 @@ void launch_locate(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream_
 void launch_compact(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream_t st);
 void launch_build_L(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream_t st);
 void launch_rowpix(const StaticData& sd, Work& w, cudaStream_t st);
-void launch_psf(const StaticData& sd, const SrcOpts& so, Work& w, int M_max, cudaStream_t st);
+int launch_psf(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st);
 void op_Ls(Work& w, int N_cap, const double* s, double* t, cudaStream_t st);
 void op_conv(const StaticData& sd, Work& w, int N_cap, bool transpose, const double* in, const double* scale_in,
              double* out, double* img, const int2* pixT, cudaStream_t st);
@@ -244,13 +269,18 @@ void launch_copy_square(void* dst, const void* src, int ld, int esize, int blk, 
 // lambda only), its result to the job's place
 void launch_job_in(const Job* jobs, unsigned ring, unsigned* count, EvalParams* ep, bool trial, cudaStream_t st);
 void launch_job_out(const Job* jobs, unsigned ring, unsigned* count, const EvalOut* out, cudaStream_t st);
-void launch_dvec(const StaticData& sd, Work& w, int N_max, cudaStream_t st);
-void launch_D(Work& w, int N_max, int M_max, cudaStream_t st);
+void launch_D(Work& w, int M_max, cudaStream_t st);
 void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st);
 int oz_alloc(OzWork** out, int N_cap, int M_cap);
 void oz_free(OzWork* z);
 void oz_clear(const OzWork* z, ClearList& l);
 void* oz_buffer(OzWork* z);
+int* oz_emax(OzWork* z);
+unsigned char* oz_nz(OzWork* z);
+int oz_nst(const OzWork* z);
+void csc_free(Csc& o);
+void csc_clear(const Csc& o, ClearList& l);
+void launch_csc(const StaticData& sd, const Work& w, const Csc& o, int N_cap, double* clear, int ld, cudaStream_t st);
 int chol64_alloc(Chol64Work** out, int M_cap, void* shared);
 void chol64_free(Chol64Work* z);
 void chol64_clear(const Chol64Work* z, ClearList& l);
