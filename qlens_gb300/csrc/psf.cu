@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* _
                 double v = acc[r];
                 if (FIXED) {
                     // as many of the lower halves' bits as there is room for
-                    const int sh = max(0, min(20, __clzll(hh[r] < 0 ? -hh[r] : hh[r]) - 3));
+                    const int sh = max(0, min(min(20, sd.psf_w), __clzll(hh[r] < 0 ? -hh[r] : hh[r]) - 3));
                     v = fixed_to_double((hh[r] << sh) + (hl[r] >> (29 - sh)) + (lh[r] >> (sd.psf_w - sh)),
                                         sd.psf_t + 28 + sh);
                 }
