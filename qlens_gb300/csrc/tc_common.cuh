@@ -106,11 +106,12 @@ __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64
         : "memory");
 }
 
-// Instruction descriptor: kind::f16 with F16 A and B, D=F32, both K-major, M=128, N=128.
-__device__ __forceinline__ uint32_t idesc_f16_128x128()
+// Instruction descriptor: kind::f16 with F16 A and B, D=F32, both K-major, M x N.
+__device__ __forceinline__ uint32_t idesc_f16(int m, int n)
 {
-    return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
+__device__ __forceinline__ uint32_t idesc_f16_128x128() { return idesc_f16(128, 128); }
 
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc)
 {

@@ -12,14 +12,23 @@
 //   warp 0 / lane 0  TMA producer: 128-row boxes of 128 B (128 B swizzle) of
 //                    X_hi, X_lo for the tile's row block and column block
 //                    into a 3-stage shared-memory ring;
-//   warp 1 / lane 0  MMA issuer: 3 products x 4 k-steps of
-//                    tcgen05.mma.cta_group::1 (M=128, N=128) per stage into a
-//                    128x128 FP32 accumulator in TMEM;
-//   all 4 warps      epilogue: tcgen05.ld 32x32b.x32, FP32 stores to F.
+//   warp 1 / lane 0  MMA issuer, 4 k-steps of tcgen05.mma.cta_group::1 per stage
+//                    into FP32 accumulators in TMEM: F16 hi*(hi, lo) as one
+//                    N = 256 product (lo's rows follow hi's in shared memory) and
+//                    lo*hi into the second half, TF32 three N = 128 products;
+//   all 4 warps      epilogue: tcgen05.ld 32x32b.x32, the halves added, FP32
+//                    stores to F.
 // Block sparsity: a stage is processed only if both the row block and the
 // column block of X have a nonzero among its pixels (flags per 32 pixels from
 // the PSF-to-X build), so the work follows the overlap of the two source-cell
 // blocks' footprints in the image instead of the full pixel count.
+// All threads list the live stages before the first is loaded.
+// What bounds it: shared memory (an N = 128 product of F16 reads its 128 bytes a
+// clock, the N = 256 one less) and L2, which feeds a CTA 64 KB per 768 clocks of
+// products; the tensor pipe ran at 40 %.  Two single threads that tested every
+// stage as they came to it lost the time of the dead ones.  us, three products and
+// tests as they came -> now: 2,934 cells x 11,772 pixels 130 -> 95, 3,700 x 42,700
+// 262 -> 186, 2,304 x 40,000 292 -> 241, 738 x 6,220 51 -> 40.
 // Every mbarrier wait is bounded by ~1 s of %globaltimer; on expiry the
 // kernel raises QLP_ERR_TIMEOUT in the GridState, stops issuing work, frees
 // its TMEM and returns.
@@ -27,6 +36,8 @@
 #include "tc_common.cuh"
 
 namespace qlpix {
+
+#define TC_LIST 4096              // stages looked through at a time
 
 // grid: one CTA per lower-triangle 128x128 tile of the M_cap x M_cap output.
 // nzflags[rb * nkb_cap + kb] != 0 when rows [128 rb, 128 rb + 128) of X have a
@@ -47,6 +58,8 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
     __shared__ uint32_t tmem_slot;
     __shared__ int n_active;
     __shared__ int n_issued;
+    __shared__ int wsum[4];
+    __shared__ unsigned short live_kb[TC_LIST];
     __shared__ volatile int abort_flag;
 
     int bi, bj;
@@ -80,7 +93,7 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
     __syncwarp();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(128)
+                     "r"(HALF ? 256 : 128)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -97,58 +110,77 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
         return fi[kb] && fj[kb];
     };
 
-    if (warp == 0 && lane == 0) {
-        // ---- TMA producer ----
-        int it = 0;
-        for (int kb = 0; kb < nkb; kb++) {
-            if (!live(kb)) continue;
-            const int s = it % TC_STAGES;
-            if (it >= TC_STAGES) {
-                if (!mbar_wait_bounded(&empty_bar[s], ((it / TC_STAGES) & 1) ^ 1, &abort_flag)) break;
+    int it_p = 0, it_m = 0;                            // stages loaded (warp 0), multiplied (warp 1)
+    for (int k0 = 0; k0 < nkb; k0 += TC_LIST) {
+        // ---- the live stages of this stretch, in order, by all threads ----
+        const int k1 = min(k0 + TC_LIST, nkb);
+        int n = 0;
+        for (int c = k0; c < k1; c += 128) {
+            const int kb = c + threadIdx.x;
+            const bool on = kb < k1 && live(kb);
+            const unsigned bits = __ballot_sync(0xffffffffu, on);
+            if (lane == 0) wsum[warp] = __popc(bits);
+            __syncthreads();
+            int at = n + __popc(bits & ((1u << lane) - 1));
+            for (int w = 0; w < 4; w++) {
+                if (w < warp) at += wsum[w];
+                n += wsum[w];
             }
-            unsigned char* st = smem + s * TC_STAGE_BYTES;
-            mbar_expect_tx(&full_bar[s], TC_STAGE_BYTES);
-            tma_load_2d(&map_hi, &full_bar[s], st, kb * KPS, bi * TC_TILE);
-            tma_load_2d(&map_lo, &full_bar[s], st + TC_TILE_BYTES, kb * KPS, bi * TC_TILE);
-            tma_load_2d(&map_hi, &full_bar[s], st + 2 * TC_TILE_BYTES, kb * KPS, bj * TC_TILE);
-            tma_load_2d(&map_lo, &full_bar[s], st + 3 * TC_TILE_BYTES, kb * KPS, bj * TC_TILE);
-            it++;
+            if (on) live_kb[at] = (unsigned short)(kb - k0);
+            __syncthreads();
         }
-        n_issued = it;
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer ----
-        const uint32_t idesc = HALF ? idesc_f16_128x128() : idesc_tf32_128x128();
-        int it = 0;
-        for (int kb = 0; kb < nkb; kb++) {
-            if (!live(kb)) continue;
-            const int s = it % TC_STAGES;
-            if (!mbar_wait_bounded(&full_bar[s], (it / TC_STAGES) & 1, &abort_flag)) break;
-            tc_fence_after();
-            unsigned char* st = smem + s * TC_STAGE_BYTES;
-            const uint64_t a_hi = sdesc_sw128(smem_u32(st));
-            const uint64_t a_lo = sdesc_sw128(smem_u32(st + TC_TILE_BYTES));
-            const uint64_t b_hi = sdesc_sw128(smem_u32(st + 2 * TC_TILE_BYTES));
-            const uint64_t b_lo = sdesc_sw128(smem_u32(st + 3 * TC_TILE_BYTES));
-            #pragma unroll
-            for (int kk = 0; kk < 4; kk++) {
-                // one MMA takes 32 bytes along K: 8 TF32 or 16 F16 values
-                const uint64_t off = (uint64_t)((kk * 32) >> 4);
-                if (HALF) {
-                    mma_f16(tmem, a_hi + off, b_hi + off, idesc, (it > 0 || kk > 0) ? 1u : 0u);
-                    mma_f16(tmem, a_hi + off, b_lo + off, idesc, 1u);
-                    mma_f16(tmem, a_lo + off, b_hi + off, idesc, 1u);
-                } else {
-                    mma_tf32(tmem, a_hi + off, b_hi + off, idesc, (it > 0 || kk > 0) ? 1u : 0u);
-                    mma_tf32(tmem, a_hi + off, b_lo + off, idesc, 1u);
-                    mma_tf32(tmem, a_lo + off, b_hi + off, idesc, 1u);
+        if (warp == 0 && lane == 0) {
+            // ---- TMA producer ----
+            for (int u = 0; u < n; u++, it_p++) {
+                const int x = (k0 + live_kb[u]) * KPS, s = it_p % TC_STAGES;
+                if (it_p >= TC_STAGES) {
+                    if (!mbar_wait_bounded(&empty_bar[s], ((it_p / TC_STAGES) & 1) ^ 1, &abort_flag)) break;
                 }
+                unsigned char* st = smem + s * TC_STAGE_BYTES;
+                mbar_expect_tx(&full_bar[s], TC_STAGE_BYTES);
+                tma_load_2d(&map_hi, &full_bar[s], st, x, bi * TC_TILE);
+                tma_load_2d(&map_lo, &full_bar[s], st + TC_TILE_BYTES, x, bi * TC_TILE);
+                tma_load_2d(&map_hi, &full_bar[s], st + 2 * TC_TILE_BYTES, x, bj * TC_TILE);
+                tma_load_2d(&map_lo, &full_bar[s], st + 3 * TC_TILE_BYTES, x, bj * TC_TILE);
             }
-            mma_commit(&empty_bar[s]);
-            it++;
+            n_issued = it_p;
+        } else if (warp == 1 && lane == 0) {
+            // ---- MMA issuer ----
+            const uint32_t idesc = HALF ? idesc_f16_128x128() : idesc_tf32_128x128();
+            const uint32_t idesc2 = idesc_f16(128, 256);
+            for (int u = 0; u < n; u++, it_m++) {
+                const int s = it_m % TC_STAGES;
+                if (!mbar_wait_bounded(&full_bar[s], (it_m / TC_STAGES) & 1, &abort_flag)) break;
+                tc_fence_after();
+                unsigned char* st = smem + s * TC_STAGE_BYTES;
+                const uint64_t a_hi = sdesc_sw128(smem_u32(st));
+                const uint64_t a_lo = sdesc_sw128(smem_u32(st + TC_TILE_BYTES));
+                const uint64_t b_hi = sdesc_sw128(smem_u32(st + 2 * TC_TILE_BYTES));
+                const uint64_t b_lo = sdesc_sw128(smem_u32(st + 3 * TC_TILE_BYTES));
+                #pragma unroll
+                for (int kk = 0; kk < 4; kk++) {
+                    // one MMA takes 32 bytes along K: 8 TF32 or 16 F16 values
+                    const uint64_t off = (uint64_t)((kk * 32) >> 4);
+                    const uint32_t acc = (it_m > 0 || kk > 0) ? 1u : 0u;
+                    if (HALF) {
+                        // b_lo's rows follow b_hi's: hi*hi and hi*lo are one N = 256
+                        // product, side by side in TMEM; lo*hi joins hi*lo
+                        mma_f16(tmem, a_hi + off, b_hi + off, idesc2, acc);
+                        mma_f16(tmem + TC_TILE, a_lo + off, b_hi + off, idesc, 1u);
+                    } else {
+                        mma_tf32(tmem, a_hi + off, b_hi + off, idesc, acc);
+                        mma_tf32(tmem, a_hi + off, b_lo + off, idesc, 1u);
+                        mma_tf32(tmem, a_lo + off, b_hi + off, idesc, 1u);
+                    }
+                }
+                mma_commit(&empty_bar[s]);
+            }
+            n_active = it_m;
         }
-        n_active = it;
-        mma_commit(&done_bar);
+        __syncthreads();
+        if (abort_flag) break;                         // uniform: raised between the barriers only
     }
+    if (warp == 1 && lane == 0) mma_commit(&done_bar);
     __syncthreads();
     // ---- epilogue ----
     // Wait for the committed MMAs even after an abort: TMEM is freed below.
@@ -167,6 +199,12 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
             float v[32];
             const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c;
             tmem_ld_32cols(taddr, v);
+            if (HALF) {
+                float lo[32];
+                tmem_ld_32cols(taddr + TC_TILE, lo);
+                #pragma unroll
+                for (int i = 0; i < 32; i++) v[i] += lo[i];
+            }
             #pragma unroll
             for (int i = 0; i < 32; i += 4)
                 *reinterpret_cast<float4*>(out + c + i) =
@@ -180,7 +218,7 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
     if (abort_flag && threadIdx.x == 0) atomicExch(&gs->status, QLP_ERR_TIMEOUT);
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(HALF ? 256 : 128) : "memory");
     }
 }
 

@@ -62,3 +62,22 @@ def test_taps_past_shared_memory():
     wide[35:96, 41:86] = kernel
     a, b = (_evaluate(k, (15, 17), abi.QLP_MIXED) for k in (kernel, wide))
     assert a["logdet_F"] == b["logdet_F"] and a["L_nnz"] == b["L_nnz"]
+
+
+def test_more_pixels_than_the_contraction_lists_at_once():
+    # 4,096 stages of 64 pixels a stretch: 262,144 pixels, and a second stretch past them
+    from qlens_gb300 import PixelLikelihood, abi
+    n, pixel = 530, 0.004
+    rng = np.random.default_rng(9)
+    xv = (np.arange(n + 1) - n / 2) * pixel
+    data = 0.05 * rng.normal(size=(n, n))
+    out = []
+    for precision in (abi.QLP_FP64, abi.QLP_MIXED):
+        pl = PixelLikelihood(xv, xv, data, np.ones((n, n), np.uint8), _kernel((3, 3)), covinv=None, bg_noise=0.05,
+                             nsplit=1, src_npixels=(9, 16), regparam=5.0, precision=precision)
+        pl.set_lens_model([{"type": "sple", "params": [0.6, 1.0, 0.0, 0.75, 30.0, 0.02, -0.01]}])
+        out.append(pl.invert_image_surface_brightness_map())
+        pl.close()
+    p, m = out
+    assert p["n_active_pixels"] > 4096 * 64 and all(p[k] == m[k] for k in ("n_active_src", "L_nnz", "n_active_pixels"))
+    assert abs(p["logdet_F"] - m["logdet_F"]) <= p["n_active_src"] * 2.0 ** -22 * 1e3
