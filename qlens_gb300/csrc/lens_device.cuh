@@ -32,12 +32,35 @@ __device__ __forceinline__ bool sple_series_continues(double orr, double oi, dou
     return a * a > 1e-16 * (c * c);
 }
 
+// |x| in FP32 by the bits, low by less than 2^-20 of itself (0 below 2^-126): a
+// conversion instruction would go to the FP64 pipe.
+__device__ __forceinline__ float fp32_below(double x)
+{
+    const int h = (__double2hiint(x) & 0x7fffffff) - ((1023 - 127) << 20);
+    return h < (1 << 20) ? 0.0f : __int_as_float(min(h, 254 << 20) << 3);
+}
+
+// |rho_1|^2, |rho_1 rho_2|^2, ... in FP32 (to 48 roundings, 3e-6): |o_i|^2 but for a few
+// FP64 ulp, for the stopping test.  mod holds the FP32 coefficients; one thread a lens.
+__device__ __forceinline__ void sple_moduli(float* mod)
+{
+    float m = 1.0f;
+    for (int i = 0; i < SPLE_RHO_TAB; i++) {
+        m *= mod[i] * mod[i];
+        mod[i] = m;
+    }
+}
+
 // SPLE_Lens::deflection_angular_factor (models.cpp:336-351): the Tessore et
 // al. (2015) series for the core-free elliptical power law, complex products
 // written out as (ac - bd, ad + bc).  rho_tab: rho_1 .. rho_SPLE_RHO_TAB for
-// this lens (sple_rho), or null.
+// this lens (sple_rho), or null; mod: sple_moduli of them, or null.
+// The FP64 pipe bounds it, and the stopping test took 11 of its 21 operations a term.
+// |o_i| hangs on the lens alone, so FP32 decides it unless the two sides are within
+// 1e-4 of each other (FP32 and fp32_below are good to 1e-5): the same number of terms,
+// the same bits.  188,000 rays 160 -> 133 us.
 __device__ __forceinline__ void sple_angular_factor(const LensRec& L, double phi, double& fr, double& fi,
-                                                    const double* rho_tab)
+                                                    const double* rho_tab, const float* mod)
 {
     double s1, c1;
     sincos(phi, &s1, &c1);
@@ -46,6 +69,7 @@ __device__ __forceinline__ void sple_angular_factor(const LensRec& L, double phi
     double s2, c2;
     sincos(2 * phi, &s2, &c2);
     int i = 1;
+    bool more;
     do {
         const double rho = (rho_tab && i <= SPLE_RHO_TAB) ? rho_tab[i - 1] : sple_rho(L, i);
         double pr = -(rho * c2), pi = -(rho * s2);
@@ -53,12 +77,17 @@ __device__ __forceinline__ void sple_angular_factor(const LensRec& L, double phi
         double ni = pr * oi + pi * orr;
         orr = nr; oi = ni;
         fr += orr; fi += oi;
+        const float A = (mod && i <= SPLE_RHO_TAB) ? mod[i - 1] : 0.0f;
+        const float a = fp32_below(fr), c = fp32_below(fi), t = 1e-16f * (a * a + c * c);
+        if (A > 1e-30f && t > 1e-30f && A > t * 1.0001f) more = true;
+        else if (A > 1e-30f && t > 1e-30f && A < t * 0.9999f) more = false;
+        else more = sple_series_continues(orr, oi, fr, fi);
         i++;
-    } while (sple_series_continues(orr, oi, fr, fi) && i < 1000);
+    } while (more && i < 1000);
 }
 
 __device__ __forceinline__ void sple_deflection(const LensRec& L, double x, double y, double& dx, double& dy,
-                                                const double* rho_tab = nullptr)
+                                                const double* rho_tab = nullptr, const float* mod = nullptr)
 {
     if (L.kind == 1) {
         // SPLE_Lens::deflection_elliptical_iso (models.cpp:208-216)
@@ -78,7 +107,7 @@ __device__ __forceinline__ void sple_deflection(const LensRec& L, double x, doub
             phi = -phi;
         }
         double fr, fi;
-        sple_angular_factor(L, phi, fr, fi, rho_tab);
+        sple_angular_factor(L, phi, fr, fi, rho_tab, mod);
         double scal = 2 * L.bprime * L.q / (1 + L.q) * pow(L.bprime / R, L.alpha - 1);
         dx = scal * fr;
         dy = scal * fi;
@@ -102,7 +131,7 @@ namespace qlpix {
 template <bool NFW>
 __device__ __forceinline__ void lens_deflection(const LensRec& L, double x, double y, double& dx, double& dy,
                                                 const double* rho_tab = nullptr, double* wbuf = nullptr,
-                                                const NfwTab* tab = nullptr)
+                                                const NfwTab* tab = nullptr, const float* mod = nullptr)
 {
     if (L.type == QLP_LENS_SHEAR) {
         x -= L.xc; y -= L.yc;
@@ -119,7 +148,7 @@ __device__ __forceinline__ void lens_deflection(const LensRec& L, double x, doub
         x = xp;
     }
     double ax, ay;
-    if (!NFW || L.type == QLP_LENS_SPLE) sple_deflection(L, x, y, ax, ay, rho_tab);
+    if (!NFW || L.type == QLP_LENS_SPLE) sple_deflection(L, x, y, ax, ay, rho_tab, mod);
     else nfw_deflection(L, x, y, ax, ay, wbuf, tab);
     if (rot) {
         double xp = ax * L.costheta - ay * L.sintheta;
@@ -161,11 +190,12 @@ __device__ __forceinline__ void subpix_centre(const StaticData& sd, int ns, int 
 
 // QLens::deflection + QLens::find_sourcept (lenscalc.cpp:81-113, 325-330).
 // rho_tab: SPLE_RHO_TAB series coefficients per lens (lens k at k *
-// SPLE_RHO_TAB), or null; nfw_tab: a table per lens (nfw_tables), or null.
+// SPLE_RHO_TAB), or null; nfw_tab: a table per lens (nfw_tables), or null; mod_tab:
+// the coefficients' moduli (sple_moduli), or null.
 template <bool NFW>
 __device__ __forceinline__ void find_sourcept(const LensModel& lm, double x, double y, double& bx, double& by,
                                               const double* rho_tab = nullptr, double* wbuf = nullptr,
-                                                const NfwTab* nfw_tab = nullptr)
+                                                const NfwTab* nfw_tab = nullptr, const float* mod_tab = nullptr)
 {
     double defx = 0, defy = 0;
     double dsx[QLP_MAX_PLANES], dsy[QLP_MAX_PLANES];
@@ -184,7 +214,8 @@ __device__ __forceinline__ void find_sourcept(const LensModel& lm, double x, dou
                 if (lm.lens[k].plane != i) continue;
                 double ax, ay;
                 lens_deflection<NFW>(lm.lens[k], xi, yi, ax, ay, rho_tab ? rho_tab + k * SPLE_RHO_TAB : nullptr,
-                                     wbuf, NFW && nfw_tab ? nfw_tab + k : nullptr);
+                                     wbuf, NFW && nfw_tab ? nfw_tab + k : nullptr,
+                                     mod_tab ? mod_tab + k * SPLE_RHO_TAB : nullptr);
                 dsx[i] += ax; dsy[i] += ay;
             }
             dsx[i] *= lm.zfac[i];

@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(256) k_raytrace(StaticData sd_, const EvalPara
     // loop would compute; used only by core-free power laws)
     __shared__ __align__(16) LensModel lm;
     __shared__ double rho_tab[QLP_MAX_LENSES * SPLE_RHO_TAB];
+    __shared__ float mod_tab[QLP_MAX_LENSES * SPLE_RHO_TAB];
     // the sub-pixel fractions u0 = (1 + 2 ii) / (2 ns) and 1 - u0, formed once
     // per CTA by the same expressions (the same bits): no FP64 divide per ray
     __shared__ double frac_u[SUBPIX_TAB], frac_1mu[SUBPIX_TAB];
@@ -36,10 +37,13 @@ __global__ void __launch_bounds__(256) k_raytrace(StaticData sd_, const EvalPara
     for (int e = threadIdx.x; e < lm.nlens * SPLE_RHO_TAB; e += blockDim.x) {
         const LensRec& L = lm.lens[e / SPLE_RHO_TAB];
         rho_tab[e] = (L.type == QLP_LENS_SPLE && L.kind == 2) ? sple_rho(L, e % SPLE_RHO_TAB + 1) : 0.0;
+        mod_tab[e] = (float)rho_tab[e];
     }
     const int ns = sd.nsplit, nsub = sd.nsub;
     subpix_table(ns, frac_u, frac_1mu);
     if (NFW) nfw_tables(lm, nfw_tab);
+    __syncthreads();
+    if (threadIdx.x < lm.nlens) sple_moduli(mod_tab + threadIdx.x * SPLE_RHO_TAB);
     __syncthreads();
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < sd.n_sub; t += gridDim.x * blockDim.x) {
         int m = t / nsub, k = t - m * nsub;
@@ -49,7 +53,8 @@ __global__ void __launch_bounds__(256) k_raytrace(StaticData sd_, const EvalPara
         double px, py;
         subpix_centre(sd, ns, ii, jj, i, j, frac_u, frac_1mu, px, py);
         double bx, by;
-        find_sourcept<NFW>(lm, px, py, bx, by, rho_tab, nullptr, NFW ? nfw_tab : nullptr);
+        find_sourcept<NFW>(lm, px, py, bx, by, rho_tab, nullptr, NFW ? nfw_tab : nullptr,
+                         mod_tab);
         spx[t] = bx;
         spy[t] = by;
     }
