@@ -43,7 +43,7 @@ UNITS = [
     ("fitparam.cpp", []),
     ("qlpix_api.cpp", []),
 ]
-HEADERS = ["qlpix_internal.h", "qlpix_ctx.h", "lens_device.cuh", "nfw_device.cuh", "patterson_rule.h", "nfw_kappa_table.h", "sur_train.cuh", "chol.cuh", "chol128.cuh", "tc_common.cuh", "tc_syrk.cuh",
+HEADERS = ["qlpix_internal.h", "qlpix_ctx.h", "lens_device.cuh", "nfw_device.cuh", "patterson_rule.h", "nfw_kappa_table.h", "sie_arc_table.h", "sur_train.cuh", "chol.cuh", "chol128.cuh", "tc_common.cuh", "tc_syrk.cuh",
            "ozaki.cuh", "tma_map.h", "psf_tiles.cuh", "brent.h"]
 
 

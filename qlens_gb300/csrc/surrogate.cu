@@ -47,6 +47,7 @@
 #include <vector>
 #include "qlpix_ctx.h"
 #include "lens_device.cuh"
+#include "sie_arc_table.h"
 #include "tc_common.cuh"
 
 namespace qlpix {
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__(SUR_THREADS, 1) k_sur_infer(int n, const float
 // sub-pixel fractions.  Any threads fill them; a barrier precedes their use.
 struct SurTabs {
     double inv_rs[QLP_MAX_LENSES], inv_q[QLP_MAX_LENSES];
-    double sie_u[QLP_MAX_LENSES], sie_pre[QLP_MAX_LENSES];
+    double sie_u[QLP_MAX_LENSES], sie_uq[QLP_MAX_LENSES], sie_pre[QLP_MAX_LENSES];
     double frac_u[SUBPIX_TAB], frac_1mu[SUBPIX_TAB];
     // an NFW lens's constants in FP32 for the surrogate's per-ray arithmetic:
     // 1/rs, q, 1/q, ks, cos and sin of its angle, and the network's q feature
@@ -649,6 +650,7 @@ __device__ __forceinline__ void sur_tabs_fill(const EvalParams* __restrict__ ep,
         // SIE without core (sple_deflection kind 1, s = 0)
         const bool sie0 = L.type == QLP_LENS_SPLE && L.kind == 1 && L.sprime == 0.0 && L.ssq == 0.0;
         T.sie_u[threadIdx.x] = sie0 ? sqrt(1 - L.qsq) : 0.0;
+        T.sie_uq[threadIdx.x] = sie0 ? sqrt(1 - L.qsq) / L.q : 0.0;
         T.sie_pre[threadIdx.x] = sie0 ? L.bprime * L.q / sqrt(1 - L.qsq) : 0.0;
         const bool nfw = L.type == QLP_LENS_NFW;
         T.f_inv_rs[threadIdx.x] = nfw ? (float)(1.0 / L.rs) : 0.f;
@@ -680,8 +682,64 @@ __device__ __forceinline__ void sur_ray_pos(const StaticData& sd, const SurTabs&
     subpix_centre(sd, ns, ii, jj, i, j, T.frac_u, T.frac_1mu, px, py);
 }
 
-// SPLE_Lens::deflection_elliptical_iso with s = 0 (T.sie_u[k] != 0): both
-// components share the reciprocal u / psi
+// atan(sqrt s) / sqrt s (G = 0) and asinh(sqrt s) / sqrt s (G = 1): below 2^-20 by
+// their series, to 2^12 (axis ratios down to 1/64) by the table, else closed.
+static __device__ const __align__(16) double c_sie[2 * QLP_SIE_N * 6] = QLP_SIE_C_INIT;
+static __device__ const __align__(16) float c_sie32[2 * QLP_SIE_N * 4] = QLP_SIE_F_INIT;
+
+template <int G>
+static __device__ __noinline__ double sie_arc_closed(double s)
+{
+    if (s < 1e-6) return G == 0 ? 1.0 - s * (1.0 / 3.0 - s * 0.2) : 1.0 - s * (1.0 / 6.0 - s * 0.075);
+    const double z = sqrt(s);
+    return (G == 0 ? atan(z) : asinh(z)) / z;
+}
+
+template <int G>
+__device__ __forceinline__ double sie_arc(double s)
+{
+    const int hi = __double2hiint(s);
+    const unsigned lo = (unsigned)__double2loint(s);
+    unsigned k = (unsigned)(hi - ((1023 + QLP_SIE_E0) << 20)) >> 16;
+    if (k >= QLP_SIE_N) return sie_arc_closed<G>(s);
+    k += G * QLP_SIE_N;
+    // interval and offset from the bits of s, as for the NFW convergence (nfw_kappa)
+    const double t = __hiloint2double(0x3ff00000 | ((hi << 4) & 0xfffff) | (int)(lo >> 28), (int)(lo << 4)) - 1.5;
+    const float tf = (float)(int)((((unsigned)hi << 16) | (lo >> 16)) ^ 0x80000000u) * 2.3283064365386963e-10f;
+    const float4 f = __ldg(reinterpret_cast<const float4*>(c_sie32) + k);
+    const double2* c = reinterpret_cast<const double2*>(c_sie) + 3 * k;
+    const double2 c45 = __ldg(c + 2), c23 = __ldg(c + 1), c01 = __ldg(c);
+    const int r = __float_as_int(__fmaf_rn(__fmaf_rn(f.z, tf, f.y), tf, f.x));
+    double v = __hiloint2double((r & 0x80000000) | (((r & 0x7fffffff) >> 3) + (896 << 20)), r << 29);
+    v = __fma_rn(v, t, c45.y);
+    v = __fma_rn(v, t, c45.x);
+    v = __fma_rn(v, t, c23.y);
+    v = __fma_rn(v, t, c23.x);
+    v = __fma_rn(v, t, c01.y);
+    return __fma_rn(v, t, c01.x);
+}
+
+// 1 / sqrt(w): the FP32 estimate from w's bits (2^-20) and one step of third order
+// (below 2^-60), five FP64 operations; outside FP32's range as ever.
+__device__ __forceinline__ double fast_rsqrt(double w)
+{
+    const float a = fp32_below(w);
+    if (!(a > 1e-30f && a < 1e30f)) return 1.0 / sqrt(w);
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+    const int r = __float_as_int(y);
+    const double d = __hiloint2double((r >> 3) + (896 << 20), r << 29);
+    const double e = __fma_rn(-(w * d), d, 1.0);
+    return __fma_rn(d * e, __fma_rn(e, 0.375, 0.5), d);
+}
+
+// SPLE_Lens::deflection_elliptical_iso with s = 0 (T.sie_u[k] != 0).  With psi^2 =
+// q^2 x^2 + y^2 and rho^2 = x^2 + y^2, psi^2 - u^2 y^2 = q^2 rho^2, so atanh(u y / psi) =
+// asinh(u y / (q rho)), which is smooth where atanh is not.
+// The FP64 pipe bounds k_ray_pre: a square root, a division, atan and atanh were
+// ~110 operations a ray and lens, now two reciprocal roots and two polynomials
+// (sie_arc_table.h: six FP64 terms, the rest below 1e-9 of the value in FP32; within
+// 3e-16 of the exact values), ~40: 679,000 rays 183 -> 130 us.
 __device__ __forceinline__ void sur_sie0(const LensRec& L, const SurTabs& T, int k, double xi, double yi,
                                          double& ax, double& ay)
 {
@@ -692,8 +750,9 @@ __device__ __forceinline__ void sur_sie0(const LensRec& L, const SurTabs& T, int
         y = -x * L.sintheta + y * L.costheta;
         x = xp;
     }
-    const double r = T.sie_u[k] / sqrt(L.qsq * x * x + y * y);
-    double bx = T.sie_pre[k] * atan(x * r), by = T.sie_pre[k] * atanh(y * r);
+    const double xx = x * x, yy = y * y;
+    const double zx = T.sie_u[k] * x * fast_rsqrt(fma(L.qsq, xx, yy)), zy = T.sie_uq[k] * y * fast_rsqrt(xx + yy);
+    double bx = T.sie_pre[k] * (zx * sie_arc<0>(zx * zx)), by = T.sie_pre[k] * (zy * sie_arc<1>(zy * zy));
     if (rot) {
         const double xp = bx * L.costheta - by * L.sintheta;
         by = bx * L.sintheta + by * L.costheta;
