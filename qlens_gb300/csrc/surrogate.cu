@@ -1506,7 +1506,10 @@ int launch_raytrace_sur(const StaticData& sd, Work& w, double thresh, int defer_
     int n = 1;
     if (defer_lens >= 0) {
         // one NFW lens, on the last plane: the other lenses first, at full occupancy
-        k_ray_pre<<<(sd.n_sub + 255) / 256, 256, 0, st>>>(sd, w.ep, defer_lens, w.spx, w.spy, w.nfw_xy);
+        // one wave of three CTAs an SM, the rays shared out evenly: the tables' FP64
+        // divisions, per CTA, were a tenth of the time at a CTA per 256 rays
+        const int blocks = (sd.n_sub + 255) / 256, per = (blocks + 3 * 152 - 1) / (3 * 152);
+        k_ray_pre<<<(blocks + per - 1) / per, 256, 0, st>>>(sd, w.ep, defer_lens, w.spx, w.spy, w.nfw_xy);
         k_raytrace_sur<true><<<sur_grid(sd.n_sub), SUR_THREADS, SUR_SMEM, st>>>(
             sd, w.ep, w.spx, w.spy, w.nfw_xy, S.wimg, S.small, S.bound, thresh, defer_lens, q, w.sur_eps, w.gs,
             w.out);
