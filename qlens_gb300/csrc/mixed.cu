@@ -197,17 +197,15 @@ __device__ __forceinline__ void csc_store(const Csc& o, int k, int row, double v
 // Each column's entries in increasing row order, so that every sum over a
 // column runs in a fixed order (k_csc_fill places them in atomic order).
 // Rows are distinct within a column of the merged L, so the order is a
-// permutation: a bitonic sort of the (row, source position) pairs, a warp
-// per column in registers for columns of up to CSC_SORT_WARP entries
-// (k_csc_sort_w), else one CTA per column in shared memory for up to
-// CSC_SORT_MAX entries, and past that each entry's rank counted directly.
-#define CSC_SORT_MAX 4096
+// permutation: columns of up to CSC_SORT_WARP entries are sorted by a warp in
+// registers (k_csc_sort_w), longer ones by a CTA that marks their rows in a bitmap
+// and takes each entry's rank from the marks below it.
 #define CSC_SORT_WARP 64    // columns sorted a warp each (k_csc_sort_w)
+#define CSC_WORDS 4096      // bitmap words a pass: 131,072 rows
 // Columns of up to CSC_SORT_WARP entries, a warp each: the same permutation
 // by a bitonic network in registers (R = 1 or 2 entries a lane, entry
 // lane + 32 h in register h; partners 32 apart within the lane, the others
-// through lane shuffles; no barriers); k_csc_sort takes the longer columns
-// (with more entries a lane the network's cost passed the block sort's).
+// through lane shuffles; no barriers); k_csc_sort takes the longer columns.
 // The rows are distinct, so any sort gives the same order.
 __device__ __forceinline__ void csc_bitonic_step(int& key, int& pos, int e, int j, int k)
 {
@@ -258,20 +256,23 @@ __device__ __forceinline__ void csc_sort_warp(const int* __restrict__ col_u, con
     }
 }
 
+// Five barriers a pass, where a bitonic network took 28 to 45 (us, 3,700 columns of 60 to
+// 300 entries 69 -> 11; 2,304 columns 37 -> 10).
 __global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ gs, const int* __restrict__ colptr,
                                                   const int* __restrict__ col_u, const int* __restrict__ src_u,
                                                   const double* __restrict__ cval, Csc out,
                                                   const int* __restrict__ rowpix, int ny, double* __restrict__ clear,
                                                   int ld)
 {
-    __shared__ int key[CSC_SORT_MAX];
-    __shared__ int pos[CSC_SORT_MAX];
+    __shared__ unsigned bits[CSC_WORDS];
+    __shared__ int below[CSC_WORDS];
+    __shared__ int wsum[8];
     const int s = blockIdx.x;
     if (s >= gs->M) return;
-    const int b = colptr[s], n = colptr[s + 1] - b;
+    const int N = gs->N, b = colptr[s], n = colptr[s + 1] - b;
     if (clear) {
         double2* row = reinterpret_cast<double2*>(clear + (size_t)s * ld);
-        for (int i = threadIdx.x; i < (gs->N + 1) / 2; i += blockDim.x) row[i] = make_double2(0.0, 0.0);
+        for (int i = threadIdx.x; i < (N + 1) / 2; i += blockDim.x) row[i] = make_double2(0.0, 0.0);
     }
     if (n <= CSC_SORT_WARP) {
         if (clear && threadIdx.x < 32) {
@@ -280,40 +281,50 @@ __global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ 
         }
         return;                                           // else k_csc_sort_w's
     }
-    if (n <= CSC_SORT_MAX) {
-        int p2 = 1;
-        while (p2 < n) p2 <<= 1;
-        for (int i = threadIdx.x; i < p2; i += blockDim.x) {
-            key[i] = (i < n) ? col_u[b + i] : INT_MAX;
-            pos[i] = (i < n) ? src_u[b + i] : 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int placed = 0;                                       // entries of the passes before
+    for (int r0 = 0; r0 < N; r0 += 32 * CSC_WORDS) {
+        const int words = min(CSC_WORDS, (N - r0 + 31) / 32);
+        for (int w = threadIdx.x; w < words; w += 256) bits[w] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += 256) {
+            const unsigned r = (unsigned)(col_u[b + i] - r0);
+            if (r < 32u * words) atomicOr(&bits[r >> 5], 1u << (r & 31));
         }
         __syncthreads();
-        for (int k = 2; k <= p2; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = threadIdx.x; i < p2; i += blockDim.x) {
-                    const int l = i ^ j;
-                    if (l > i) {
-                        const bool up = (i & k) == 0;
-                        const int ki = key[i], kl = key[l];
-                        if ((ki > kl) == up) {
-                            key[i] = kl; key[l] = ki;
-                            const int t = pos[i]; pos[i] = pos[l]; pos[l] = t;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
+        // the marks below each word: a thread a run of words, then a scan of the runs
+        const int per = (words + 255) / 256, w0 = threadIdx.x * per, w1 = min(w0 + per, words);
+        int sum = 0;
+        for (int w = w0; w < w1; w++) sum += __popc(bits[w]);
+        int at = sum;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += v;
         }
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            csc_store(out, b + i, key[i], cval[pos[i]], rowpix, ny);
+        if (lane == 31) wsum[warp] = at;
+        __syncthreads();
+        int total = 0;
+        #pragma unroll
+        for (int w = 0; w < 8; w++) {
+            if (w < warp) at += wsum[w];
+            total += wsum[w];
         }
-        return;
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int ri = col_u[b + i];
-        int rank = 0;
-        for (int j = 0; j < n; j++) rank += (col_u[b + j] < ri) ? 1 : 0;
-        csc_store(out, b + rank, ri, cval[src_u[b + i]], rowpix, ny);
+        at += placed - sum;
+        for (int w = w0; w < w1; w++) {
+            below[w] = at;
+            at += __popc(bits[w]);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += 256) {
+            const int row = col_u[b + i];
+            const unsigned r = (unsigned)(row - r0);
+            if (r < 32u * words)
+                csc_store(out, b + below[r >> 5] + __popc(bits[r >> 5] & ((1u << (r & 31)) - 1)), row,
+                          cval[src_u[b + i]], rowpix, ny);
+        }
+        placed += total;
+        __syncthreads();
     }
 }
 

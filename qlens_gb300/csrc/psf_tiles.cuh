@@ -73,16 +73,24 @@ __global__ void k_psfx_tiles(StaticData sd, const GridState* __restrict__ gs, co
     const E* ent = ent_g + colptr[s];
     for (int i = lane; i < nwords; i += 32) mark[i] = 0;
     __syncwarp();
-    for (int e = lane; e < n; e += 32) {
-        const E en = ent[e];
+    for (int e0 = 0; e0 < n; e0 += 32) {
+        const E en = ent[min(e0 + lane, n - 1)];
         const int i0 = ent_col(en) - nxh, j0 = ent_row(en) - nyh;
         const int c0 = max(i0, 0) >> 5, c1 = (min(i0 + pnx, sd.nx) - 1) >> 5;
         const int t0 = max(j0, 0) / PSFX_R, t1 = (min(j0 + pny, sd.ny) - 1) / PSFX_R;
-        for (int t = t0; t <= t1; t++)
-            for (int c = c0; c <= c1; c++) {
-                const int k = t * ntx + c;
-                if (!(mark[k >> 5] >> (k & 31) & 1u)) atomicOr(&mark[k >> 5], 1u << (k & 31));
+        // neighbours along a row mostly reach the same tiles: only the first marks them
+        const int cc = c0 << 16 | c1, tt = t0 << 16 | t1;
+        const int pc = __shfl_up_sync(0xffffffffu, cc, 1), pt = __shfl_up_sync(0xffffffffu, tt, 1);
+        if (lane > 0 && pc == cc && pt == tt) continue;
+        for (int t = t0; t <= t1; t++) {
+            const int k0 = t * ntx + c0, k1 = t * ntx + c1;
+            for (int w = k0 >> 5; w <= k1 >> 5; w++) {
+                unsigned m = 0xffffffffu;
+                if (w == k0 >> 5) m &= 0xffffffffu << (k0 & 31);
+                if (w == k1 >> 5) m &= 0xffffffffu >> (31 - (k1 & 31));
+                if ((mark[w] & m) != m) atomicOr(&mark[w], m);
             }
+        }
     }
     __syncwarp();
     for (int w0 = 0; w0 < nwords; w0 += 32) {
