@@ -415,7 +415,11 @@ struct SurWG {
 // The 256 threads of a ray group call this together, two per ray (row
 // threadIdx.x % 128), each with its ray's inputs; both return the network's
 // two outputs.  ok is cleared if a bounded wait ran out.
-__device__ void sur_mlp_wg(SurWG& S, float f0, float f1, float f2, float& t0, float& t1, bool& ok)
+// side(l): what a thread does while layer l's products run, the second half's in
+// layer 1 and the first half's in layer 2.
+template <typename Side>
+__device__ __forceinline__ void sur_mlp_wg(SurWG& S, float f0, float f1, float f2, float& t0, float& t1, bool& ok,
+                                           Side&& side)
 {
     const int tid = threadIdx.x & 127, warp = tid >> 5;
     const uint32_t row = S.tmem + (((uint32_t)(warp * 32)) << 16);   // this warp's 32 lanes
@@ -450,7 +454,8 @@ __device__ void sur_mlp_wg(SurWG& S, float f0, float f1, float f2, float& t0, fl
         tc_fence_before();
         wg_sync(S.wg);
         tc_fence_after();
-        if ((threadIdx.x & (SUR_RG - 1)) == 0) {
+        // issuing takes a warp the products' time: of the half that has nothing beside them
+        if ((threadIdx.x & (SUR_RG - 1)) == (l == 2 ? SUR_RG / 2 : 0)) {
             const uint32_t idesc = idesc_f16_128x128();
             const unsigned char* wl = S.w + (size_t)(l - 1) * 2 * SUR_OPB;
             #pragma unroll
@@ -470,6 +475,7 @@ __device__ void sur_mlp_wg(SurWG& S, float f0, float f1, float f2, float& t0, fl
             mma_commit(S.mma_bar);
         }
         __syncwarp();
+        side(l);
         const bool done = mbar_wait_bounded(S.mma_bar, S.phase & 1, S.abort, false);
         tc_fence_after();
         S.phase++;
@@ -596,7 +602,7 @@ __global__ void __launch_bounds__(SUR_THREADS, 1) k_sur_infer(int n, const float
         float f0 = 0.f, f1 = 0.f, f2 = 0.f;
         if (i < n) { f0 = X[3 * (size_t)i]; f1 = X[3 * (size_t)i + 1]; f2 = X[3 * (size_t)i + 2]; }
         float t0, t1;
-        sur_mlp_wg(S, f0, f1, f2, t0, t1, ok);
+        sur_mlp_wg(S, f0, f1, f2, t0, t1, ok, [](int) {});
         if (i < n && S.half == 0) { T[2 * (size_t)i] = t0; T[2 * (size_t)i + 1] = t1; }
     }
     if (!ok && tid == 0) atomicExch(status, QLP_ERR_TIMEOUT);
@@ -777,6 +783,79 @@ struct SurRayOut {
 // 1e-6), added to every surrogate ray's bound
 #define SUR_F32_REL 2e-6f
 
+// A ray's position in NFW lens L's frame.
+__device__ __forceinline__ void sur_lens_frame(const LensRec& L, double xi, double yi, double& x, double& y)
+{
+    x = xi - L.xc; y = yi - L.yc;
+    if (L.sintheta != 0) {
+        const double xp = x * L.costheta + y * L.sintheta;
+        y = -x * L.sintheta + y * L.costheta;
+        x = xp;
+    }
+}
+
+// What the network takes of a ray (f0, f1; the third input is the lens's) and what
+// its output is applied with: the baseline B and the bound on the relative error, -1
+// where the ray lies outside the trained cells or at the centre.
+struct SurRayIn {
+    float f0, f1, B, bnd;
+};
+
+__device__ __forceinline__ SurRayIn sur_inputs(const LensRec& L, int k, const SurTabs& T, const float* __restrict__ bound,
+                                            double x, double y)
+{
+    SurRayIn r;
+    const float xf = (float)x, yf = (float)y;
+    const bool centre = (fabsf(xf) < 1e-14f) && (fabsf(yf) < 1e-14f);
+    // the network's inputs (log R, polar angle, q), its error cell, and
+    // the baseline B at xi^2 = q X^2 + Y^2 / q
+    const float Xa = fabsf(xf * T.f_inv_rs[k]), Ya = fabsf(yf * T.f_inv_rs[k]);
+    const float rho = 0.5f * __logf(__fmaf_rn(Xa, Xa, Ya * Ya));
+    const float phi = atan2f(Ya, Xa);
+    const float hr = (float)(0.5 * (SUR_RHO_HI - SUR_RHO_LO)), mr = (float)(0.5 * (SUR_RHO_HI + SUR_RHO_LO));
+    r.f0 = fminf(fmaxf((rho - mr) / hr, -2.0f), 2.0f);
+    r.f1 = phi * (float)(4.0 / M_PI) - 1.0f;
+    const int bin = sur_cell_f(rho, phi, T.qbin[k]);
+    const float xi2 = T.f_q[k] * Xa * Xa + Ya * Ya * T.f_inv_q[k];
+    float brel = 0.f;
+    if (xi2 >= (float)SUR_B32_MIN) {
+        r.B = sur_B32(xi2);
+        brel = (float)SUR_B32_REL;
+    } else {                                   // small radius: the FP64 form (its series cancels)
+        const double Xd = x * T.inv_rs[k], Yd = y * T.inv_rs[k];
+        r.B = (float)nfw_kapavg_spherical_rsq(1.0, 1.0, L.q * Xd * Xd + Yd * Yd * T.inv_q[k]);
+    }
+    // the cell's bound on the relative error of G, plus B's and the FP32 arithmetic's
+    r.bnd = bin >= 0 && !centre ? bound[bin] + brel + SUR_F32_REL : -1.0f;
+    return r;
+}
+
+// Before the network: |alpha| ~ ks B |(x, y)| (G is within a few tens of percent of
+// B), so a group none of whose rays can pass the gate skips the network and sends
+// every ray to the quadrature (squares compared).
+__device__ __forceinline__ bool sur_maybe(const SurTabs& T, int k, const SurRayIn& in, float xf, float yf, float thr)
+{
+    const float gb = T.f_ks[k] * in.B * in.bnd;
+    return in.bnd >= 0.f && gb * gb * (xf * xf + yf * yf) <= 2.25f * thr * thr;
+}
+
+// The deflection in the lens's frame from the network's outputs, the gate, and the
+// ray's error bound.
+__device__ __forceinline__ bool sur_apply(const SurTabs& T, int k, const SurRayIn& in, float xf, float yf, float t0,
+                                          float t1, bool ok, float thr, double zabs, float& bxf, float& byf,
+                                          double& eps)
+{
+    const float oq = 1.0f - T.f_q[k];
+    const float kb = T.f_ks[k] * in.B;
+    bxf = xf * (kb * expf(oq * t0));
+    byf = yf * (kb * expf(oq * t1));
+    const float m2 = bxf * bxf + byf * byf;
+    const bool use = ok && in.bnd >= 0.f && m2 * in.bnd * in.bnd <= thr * thr;
+    // |alpha| rounded up by far more than its error
+    if (use) eps += 2.0 * zabs * (double)(sqrtf(m2) * 1.000001f * in.bnd);
+    return use;
+}
+
 __device__ __forceinline__ void sur_nfw(SurWG& S, bool& ok, const LensRec& L, int k, const SurTabs& T,
                                         const float* __restrict__ bound, double thresh, double zabs, bool valid,
                                         int t, int defer_lens, const SurRayOut& q, int& fb, double& eps,
@@ -790,68 +869,31 @@ __device__ __forceinline__ void sur_nfw(SurWG& S, bool& ok, const LensRec& L, in
     // SUR_F32_REL covers it in the bound.
     const int tid = threadIdx.x & 127;
     const bool first = S.half == 0;
+    const bool rot = first && L.sintheta != 0;
     double x = 0, y = 0;
-    float xf = 0.f, yf = 0.f, bnd = 0.f, B = 0.f;
-    bool rot = false, centre = false, inb = false, maybe = false;
-    float f0 = 0.f, f1 = 0.f, f2 = 0.f;
+    SurRayIn in{0.f, 0.f, 0.f, -1.f};
+    bool maybe = false;
+    const float f2 = T.f_feat_q[k];
+    float f0 = 0.f, f1 = 0.f;
     const float thr = (float)thresh;
     if (first) {
-        x = xi - L.xc; y = yi - L.yc;
-        rot = (L.sintheta != 0);
-        if (rot) {
-            const double xp = x * L.costheta + y * L.sintheta;
-            y = -x * L.sintheta + y * L.costheta;
-            x = xp;
-        }
-        xf = (float)x; yf = (float)y;
-        centre = (fabsf(xf) < 1e-14f) && (fabsf(yf) < 1e-14f);
-        // the network's inputs (log R, polar angle, q), its error cell, and
-        // the baseline B at xi^2 = q X^2 + Y^2 / q
-        const float Xa = fabsf(xf * T.f_inv_rs[k]), Ya = fabsf(yf * T.f_inv_rs[k]);
-        const float rho = 0.5f * __logf(__fmaf_rn(Xa, Xa, Ya * Ya));
-        const float phi = atan2f(Ya, Xa);
-        const float hr = (float)(0.5 * (SUR_RHO_HI - SUR_RHO_LO)), mr = (float)(0.5 * (SUR_RHO_HI + SUR_RHO_LO));
-        f0 = fminf(fmaxf((rho - mr) / hr, -2.0f), 2.0f);
-        f1 = phi * (float)(4.0 / M_PI) - 1.0f;
-        f2 = T.f_feat_q[k];
-        const int bin = sur_cell_f(rho, phi, T.qbin[k]);
-        inb = bin >= 0;
-        const float xi2 = T.f_q[k] * Xa * Xa + Ya * Ya * T.f_inv_q[k];
-        float brel = 0.f;
-        if (xi2 >= (float)SUR_B32_MIN) {
-            B = sur_B32(xi2);
-            brel = (float)SUR_B32_REL;
-        } else {                                   // small radius: the FP64 form (its series cancels)
-            const double Xd = x * T.inv_rs[k], Yd = y * T.inv_rs[k];
-            B = (float)nfw_kapavg_spherical_rsq(1.0, 1.0, L.q * Xd * Xd + Yd * Yd * T.inv_q[k]);
-        }
-        // the cell's bound on the relative error of G, plus B's and the FP32 arithmetic's
-        bnd = inb ? bound[bin] + brel + SUR_F32_REL : 0.f;
-        // before the network: |alpha| ~ ks B |(x, y)| (G is within a few tens of
-        // percent of B), so a group none of whose rays can pass the gate skips
-        // the network and sends every ray to the quadrature (squares compared)
-        const float gb = T.f_ks[k] * B * bnd;
-        maybe = valid && !centre && inb && gb * gb * (xf * xf + yf * yf) <= 2.25f * thr * thr;
-        S.xin[tid] = make_float4(f0, f1, f2, 0.f);
+        sur_lens_frame(L, xi, yi, x, y);
+        in = sur_inputs(L, k, T, bound, x, y);
+        maybe = valid && sur_maybe(T, k, in, (float)x, (float)y, thr);
+        f0 = in.f0; f1 = in.f1;
+        S.xin[tid] = make_float4(f0, f1, 0.f, 0.f);
     }
     float bxf = 0.f, byf = 0.f;
     bool use = false;
     if (wg_any(S.wg, maybe)) {
         if (!first) {
             const float4 v = S.xin[tid];
-            f0 = v.x; f1 = v.y; f2 = v.z;
+            f0 = v.x; f1 = v.y;
         }
         float t0, t1;
-        sur_mlp_wg(S, f0, f1, f2, t0, t1, ok);
+        sur_mlp_wg(S, f0, f1, f2, t0, t1, ok, [](int) {});
         if (first) {
-            const float oq = 1.0f - T.f_q[k];
-            const float kb = T.f_ks[k] * B;
-            bxf = xf * (kb * expf(oq * t0));
-            byf = yf * (kb * expf(oq * t1));
-            const float m2 = bxf * bxf + byf * byf;
-            use = ok && !centre && inb && m2 * bnd * bnd <= thr * thr;
-            // |alpha| rounded up by far more than its error
-            if (use) eps += 2.0 * zabs * (double)(sqrtf(m2) * 1.000001f * bnd);
+            use = sur_apply(T, k, in, (float)x, (float)y, t0, t1, ok, thr, zabs, bxf, byf, eps);
         }
     }
     if (!first) { ax = 0; ay = 0; return; }
@@ -921,7 +963,79 @@ __global__ void __launch_bounds__(SUR_THREADS, 1) k_raytrace_sur(StaticData sd_,
     bool ok = sur_cta_begin(S, smem_raw, wimg, small_g, &w_bar, mma_bar, &tmem_slot, &abort_flag, xo);
     const int tid = threadIdx.x & 127;
     int fb = 0;
-    for (int grp = blockIdx.x * 2 + S.wg; grp * 128 < sd.n_sub; grp += gridDim.x * 2) {
+    if (PRE) {
+        // One group's network runs while the group before it is finished (first
+        // half) and the next one's inputs are formed (second half), beside the
+        // products of layers 2 and 1: three sets of inputs are live.  One after the other
+        // these took a fifth of a group's time with the tensor cores idle: 679,000 rays
+        // 293 -> 260 us.
+        __shared__ float4 stash[2][3][128];
+        const LensRec& L = lm.lens[defer_lens];
+        const double z = lm.zfac[L.plane];
+        const float thr = (float)thresh, f2 = T.f_feat_q[defer_lens];
+        const int step = gridDim.x * 2;
+        auto inputs = [&](int grp, int slot) -> bool {               // the second half's
+            const int t = grp * 128 + tid;
+            if (S.half == 0 || t >= sd.n_sub) return false;
+            double x, y;
+            sur_lens_frame(L, nfw_xy[2 * (size_t)t], nfw_xy[2 * (size_t)t + 1], x, y);
+            const SurRayIn in = sur_inputs(L, defer_lens, T, bound, x, y);
+            stash[S.wg][slot][tid] = make_float4(in.f0, in.f1, in.B, in.bnd);
+            return sur_maybe(T, defer_lens, in, (float)x, (float)y, thr);
+        };
+        auto finish = [&](int grp, int slot, bool net, float t0, float t1) {     // the first half's
+            const int t = grp * 128 + tid;
+            if (S.half != 0 || t >= sd.n_sub) return;
+            const float4 v = stash[S.wg][slot][tid];
+            const SurRayIn in{v.x, v.y, v.z, v.w};
+            const double sx = spx[t], sy = spy[t];
+            double x, y, eps = 1e-12;
+            sur_lens_frame(L, nfw_xy[2 * (size_t)t], nfw_xy[2 * (size_t)t + 1], x, y);
+            float bxf = 0.f, byf = 0.f;
+            if (net && sur_apply(T, defer_lens, in, (float)x, (float)y, t0, t1, ok, thr, fabs(z), bxf, byf, eps)) {
+                if (L.sintheta != 0) {
+                    const float xp = bxf * T.f_cos[defer_lens] - byf * T.f_sin[defer_lens];
+                    byf = bxf * T.f_sin[defer_lens] + byf * T.f_cos[defer_lens];
+                    bxf = xp;
+                }
+                spx[t] = sx - z * (double)bxf;
+                spy[t] = sy - z * (double)byf;
+            } else {                                                 // to k_nfw_fallback
+                fb++;
+                const int e = atomicAdd(q.fb_count, 1);
+                q.fb_ray[e] = t;
+                q.fb_xy[2 * (size_t)e] = x;
+                q.fb_xy[2 * (size_t)e + 1] = y;
+            }
+            sur_eps[t] = (float)eps;
+        };
+        int grp = blockIdx.x * 2 + S.wg, slot = 0, before = -1;
+        bool maybe = inputs(grp, 0), net_before = false;
+        float t0 = 0.f, t1 = 0.f;
+        for (; grp * 128 < sd.n_sub; grp += step) {
+            if (wg_any(S.wg, !ok || abort_flag)) { ok = false; break; }
+            const bool net = wg_any(S.wg, maybe);                    // (orders the stash, too)
+            const int next = slot == 2 ? 0 : slot + 1, last = slot == 0 ? 2 : slot - 1;
+            auto side = [&](int l) {
+                if (l == 1) maybe = inputs(grp + step, next);
+                if (l == 2 && before >= 0) finish(before, last, net_before, t0, t1);
+            };
+            if (net) {
+                const float4 v = stash[S.wg][slot][tid];
+                float n0, n1;
+                sur_mlp_wg(S, v.x, v.y, f2, n0, n1, ok, side);
+                t0 = n0; t1 = n1;
+            } else {
+                side(1);
+                side(2);
+            }
+            before = grp;
+            net_before = net;
+            slot = next;
+        }
+        if (before >= 0) finish(before, slot == 0 ? 2 : slot - 1, net_before, t0, t1);
+    }
+    for (int grp = blockIdx.x * 2 + S.wg; !PRE && grp * 128 < sd.n_sub; grp += gridDim.x * 2) {
         if (wg_any(S.wg, !ok || abort_flag)) { ok = false; break; }
         const int t = grp * 128 + tid;
         // both threads of a ray trace it; the first half stores it, queues
@@ -932,26 +1046,6 @@ __global__ void __launch_bounds__(SUR_THREADS, 1) k_raytrace_sur(StaticData sd_,
         // summed in another order) plus, per surrogate deflection, twice its
         // plane factor times its bound
         double eps = 1e-12;
-        if (PRE) {
-            const LensRec& L = lm.lens[defer_lens];
-            const double z = lm.zfac[L.plane];
-            double xi = 0, yi = 0, sx = 0, sy = 0;
-            if (valid) {
-                xi = nfw_xy[2 * (size_t)t];
-                yi = nfw_xy[2 * (size_t)t + 1];
-                sx = spx[t];
-                sy = spy[t];
-            }
-            double ax, ay;
-            sur_nfw(S, ok, L, defer_lens, T, bound, thresh, fabs(z), valid, t, defer_lens, q, fb, eps, xi, yi,
-                    ax, ay);
-            if (valid) {
-                spx[t] = sx - z * ax;
-                spy[t] = sy - z * ay;
-                sur_eps[t] = (float)eps;
-            }
-            continue;
-        }
         double px = 0, py = 0;
         if (valid) sur_ray_pos(sd, T, t, px, py);
         double defx = 0, defy = 0;

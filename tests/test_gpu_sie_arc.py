@@ -36,3 +36,23 @@ def test_source_points_match_oracle(trained, q, theta):
     got, ref = pl.dump(g.n_sub, r)["srcpt"], O.get("srcpt")
     pl.close()
     assert np.abs(got - ref).max() <= (1e-14 + 2e-15 / q ** 2) * (np.abs(ref).max() + p[0])
+
+
+@pytest.mark.parametrize("n", [3, 17, 66, 131])
+def test_ray_groups(trained, n):
+    # 81 rays (less than a group of 128) to 1,206 groups (3.97 for each of 304 in flight)
+    from qlens_gb300 import PixelLikelihood, abi
+    xv = (np.arange(n + 1) - n / 2) * (4.0 / n)
+    sie = [{"type": "sple", "params": [1.1, 1.0, 0.0, 0.7, 20.0, 0.01, -0.02]}]
+    halo = [{"type": "nfw", "params": [1e-40, 2.0, 0.8, 10.0, 0.3, 0.2]}]
+    got = []
+    for lenses, precision in ((sie, abi.QLP_FP64), (sie + halo, abi.QLP_MIXED)):
+        pl = PixelLikelihood(xv, xv, np.ones((n, n)), np.ones((n, n), np.uint8), np.ones((1, 1)), covinv=None,
+                             bg_noise=0.1, nsplit=3, src_npixels=(8, 8), regparam=5.0, precision=precision)
+        pl.set_lens_model(lenses)
+        if precision == abi.QLP_MIXED:
+            pl.set_nfw_mode(abi.QLP_NFW_SURROGATE)
+        r = pl.invert_image_surface_brightness_map()
+        got.append(pl.dump(9 * n * n, r)["srcpt"])
+        pl.close()
+    assert np.abs(got[1] - got[0]).max() <= 2e-14 * (np.abs(got[0]).max() + 1.1)
