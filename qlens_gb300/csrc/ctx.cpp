@@ -45,10 +45,7 @@ static std::vector<int> masked_list(const unsigned char* mask, int nx, int ny)
 
 static void free_work(Work& w)
 {
-    void* ptrs[] = {w.spx, w.spy, w.cx, w.cy, w.ccx, w.ccy, w.cell3, w.w3, w.mapped, w.active_index, w.pixmaps,
-                    w.rowidx, w.pixindex, w.rowpix, w.rowptr, w.Lidx, w.Lval, w.cidx, w.cval, w.ccnt, w.Lpsf,
-                    w.dvec, w.cvec, w.D, w.F, w.R, w.s, w.tmp, w.model, w.linv, w.gs, w.out, w.ep,
-                    w.fb_ray, w.fb_xy, w.fb_count, w.F0, w.gpart, w.gpart_cnt, w.cpart, w.sur_eps, w.xlist, w.xcount, w.nfw_xy};
+    void* ptrs[] = {w.base, w.Lpsf, w.F, w.R, w.F0};
     for (void* p : ptrs) if (p) cudaFree(p);
     csc_free(w.csc);
     chol64_free(w.cholF);
@@ -89,31 +86,33 @@ static int alloc_work(qlp_ctx* c, Slot& s, int n_mask, int nsub, int Mcells, int
     const int Mc = round64(std::max(Mcells, 64));
     const size_t n_sub = (size_t)n_mask * nsub;
     const size_t nnz = 3 * n_sub;
-    CK(dalloc(&w.spx, n_sub), "alloc"); CK(dalloc(&w.spy, n_sub), "alloc");
-    CK(dalloc(&w.cx, snx_max + 1), "alloc"); CK(dalloc(&w.cy, sny_max + 1), "alloc");
-    CK(dalloc(&w.ccx, snx_max), "alloc"); CK(dalloc(&w.ccy, sny_max), "alloc");
-    CK(dalloc(&w.cell3, 3 * n_sub), "alloc"); CK(dalloc(&w.w3, 3 * n_sub), "alloc");
-    CK(dalloc(&w.mapped, Mc), "alloc"); CK(dalloc(&w.active_index, Mc), "alloc");
-    CK(dalloc(&w.pixmaps, n_mask), "alloc"); CK(dalloc(&w.rowidx, n_mask), "alloc");
-    CK(dalloc(&w.pixindex, (size_t)c->nx * c->ny), "alloc");
-    CK(dalloc(&w.rowpix, n_mask), "alloc");
-    CK(dalloc(&w.rowptr, n_mask + 1), "alloc");
-    CK(dalloc(&w.Lidx, nnz), "alloc"); CK(dalloc(&w.Lval, nnz), "alloc");
-    CK(dalloc(&w.cidx, nnz), "alloc"); CK(dalloc(&w.cval, nnz), "alloc"); CK(dalloc(&w.ccnt, n_mask), "alloc");
+    Arena ar;
+    ar.add(&w.spx, n_sub); ar.add(&w.spy, n_sub);
+    ar.add(&w.cx, snx_max + 1); ar.add(&w.cy, sny_max + 1);
+    ar.add(&w.ccx, snx_max); ar.add(&w.ccy, sny_max);
+    ar.add(&w.cell3, 3 * n_sub); ar.add(&w.w3, 3 * n_sub);
+    ar.add(&w.mapped, Mc); ar.add(&w.active_index, Mc);
+    ar.add(&w.pixmaps, n_mask); ar.add(&w.rowidx, n_mask);
+    ar.add(&w.pixindex, (size_t)c->nx * c->ny);
+    ar.add(&w.rowpix, n_mask);
+    ar.add(&w.rowptr, n_mask + 1);
+    ar.add(&w.Lidx, nnz); ar.add(&w.Lval, nnz);
+    ar.add(&w.cidx, nnz); ar.add(&w.cval, nnz); ar.add(&w.ccnt, n_mask);
     w.ldL = (n_mask + 31) / 32 * 32;
-    CK(dalloc(&w.dvec, n_mask), "alloc"); CK(dalloc(&w.cvec, n_mask), "alloc");
+    ar.add(&w.dvec, n_mask); ar.add(&w.cvec, n_mask);
     w.ldF = Mc;
-    CK(dalloc(&w.D, Mc), "alloc");
-    CK(dalloc(&w.s, Mc), "alloc"); CK(dalloc(&w.tmp, Mc), "alloc");
-    CK(dalloc(&w.model, n_mask), "alloc");
-    CK(dalloc(&w.gpart, 4 * 1024), "alloc"); CK(dalloc(&w.gpart_cnt, 1024), "alloc");
-    CK(dalloc(&w.cpart, 3 * 1025), "alloc");
-    CK(dalloc(&w.linv, (size_t)Mc * 64), "alloc");
-    CK(dalloc(&w.gs, 1), "alloc"); CK(dalloc(&w.out, 1), "alloc"); CK(dalloc(&w.ep, 1), "alloc");
-    CK(dalloc(&w.fb_ray, n_sub), "alloc"); CK(dalloc(&w.fb_xy, 2 * n_sub), "alloc"); CK(dalloc(&w.fb_count, 1), "alloc");
-    CK(dalloc(&w.sur_eps, n_sub), "alloc");
-    CK(dalloc(&w.xlist, n_sub), "alloc"); CK(dalloc(&w.xcount, 2), "alloc");
-    CK(dalloc(&w.nfw_xy, 2 * n_sub), "alloc");
+    ar.add(&w.D, Mc);
+    ar.add(&w.s, Mc); ar.add(&w.tmp, Mc);
+    ar.add(&w.model, n_mask);
+    ar.add(&w.gpart, 4 * 1024); ar.add(&w.gpart_cnt, 1024);
+    ar.add(&w.cpart, 3 * 1025);
+    ar.add(&w.linv, (size_t)Mc * 64);
+    ar.add(&w.gs, 1); ar.add(&w.out, 1); ar.add(&w.ep, 1);
+    ar.add(&w.fb_ray, n_sub); ar.add(&w.fb_xy, 2 * n_sub); ar.add(&w.fb_count, 1);
+    ar.add(&w.sur_eps, n_sub);
+    ar.add(&w.xlist, n_sub); ar.add(&w.xcount, 2);
+    ar.add(&w.nfw_xy, 2 * n_sub);
+    CK(ar.commit(&w.base), "alloc");
     s.M_cap = Mc;
     s.N_cap = n_mask;
     s.npix_pad = (c->nx + 2 * (c->sd.pnx / 2)) * (c->ny + 2 * (c->sd.pny / 2));
@@ -131,9 +130,9 @@ static int ensure_fp64_mats(Slot& s)
     if (s.fp64_mats) return QLP_OK;
     if (!s.w.Lpsf) CK(dalloc(&s.w.Lpsf, (size_t)s.w.ldL * s.M_cap), "alloc L'");
     if (!s.w.csc.colcnt) {
-        const cudaError_t e = csc_alloc(s.w.csc, s, s.M_cap, true);
-        if (e != cudaSuccess) csc_free(s.w.csc);
-        CK(e, "alloc L by source cell");
+        Arena ar;
+        csc_layout(s.w.csc, s, s.M_cap, true, ar);
+        CK(ar.commit(&s.w.csc.base), "alloc L by source cell");
     }
     if (!s.w.oz) {
         const int r = oz_alloc(&s.w.oz, s.N_cap, s.M_cap);

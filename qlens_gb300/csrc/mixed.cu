@@ -31,6 +31,7 @@ namespace qlpix {
 #define MIXED_SOLVES 5    // solves of one evaluation: one and up to four refinement sweeps
 
 struct MixedWork {
+    void* base = nullptr;    // the allocation that holds all but F0
     double* t = nullptr;     // N (image-plane scratch)
     Csc csc{};               // L by source cell, for k_psf_x and L^T
     float* F0 = nullptr;     // lambda optimisation: X X^T before lambda R (allocated on first use)
@@ -613,49 +614,40 @@ void mixed_free(Slot& c)
 {
     MixedWork* m = mw_of(c);
     if (!m) return;
-    void* ptrs[] = {m->t, m->X_hi, m->X_lo, m->nz, m->F32, m->R32, m->u, m->v, m->r, m->z, m->y, m->img,
-                    m->linvF, m->yf, m->zf, m->flags, m->F0,
-                    m->cf.Lh, m->cf.Ll, m->cf.pexp, m->cf.ih, m->cf.il, m->cf.flags,
-                    m->cr.Lh, m->cr.Ll, m->cr.pexp, m->cr.ih, m->cr.il, m->cr.flags};
+    void* ptrs[] = {m->base, m->F0};
     for (void* p : ptrs) if (p) cudaFree(p);
-    csc_free(m->csc);
     delete m;
     c.mixed = nullptr;
 }
 
 void csc_free(Csc& o)
 {
-    void* ptrs[] = {o.colcnt, o.cursor, o.colrow, o.ent, o.fine, o.col_u, o.src_u, o.colval64, o.pixT, o.tiles,
-                    o.tile_active};
-    for (void* p : ptrs) if (p) cudaFree(p);
+    if (o.base) cudaFree(o.base);
     o = Csc{};
 }
 
-// Workspace of L by source cell for M_cap cells of a slot; fine: the plain path's.
-cudaError_t csc_alloc(Csc& o, const Slot& c, int M_cap, bool fine)
+// L by source cell for M_cap cells of a slot; fine: the plain path's.
+void csc_layout(Csc& o, const Slot& c, int M_cap, bool fine, Arena& ar)
 {
-    cudaError_t e = cudaSuccess;
-    auto A = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes > 0 ? bytes : 16); };
     const int ntile = (c.img_nx + 31) / 32 * ((c.img_ny + PSFX_R - 1) / PSFX_R);
     const size_t nnz = (size_t)3 * c.N_cap * c.nsub_cap;
     o.words = (ntile + 31) / 32;
     o.M_cap = M_cap;
     o.npix_pad = c.npix_pad;
-    A((void**)&o.tiles, sizeof(uint2) * (size_t)M_cap * std::min(ntile, c.N_cap));
-    A((void**)&o.tile_active, sizeof(unsigned) * (o.words + 1));
-    A((void**)&o.colcnt, sizeof(int) * (size_t)(M_cap + 1));
-    A((void**)&o.cursor, sizeof(int) * (size_t)M_cap);
-    A((void**)&o.col_u, sizeof(int) * nnz);
-    A((void**)&o.src_u, sizeof(int) * nnz);
-    A((void**)&o.pixT, sizeof(int2) * (size_t)c.npix_pad);
+    ar.add(&o.tiles, (size_t)M_cap * std::min(ntile, c.N_cap));
+    ar.add(&o.tile_active, o.words + 1);
+    ar.add(&o.colcnt, M_cap + 1);
+    ar.add(&o.cursor, M_cap);
+    ar.add(&o.col_u, nnz);
+    ar.add(&o.src_u, nnz);
+    ar.add(&o.pixT, c.npix_pad);
     if (fine) {
-        A((void**)&o.fine, sizeof(int4) * nnz);
+        ar.add(&o.fine, nnz);
     } else {
-        A((void**)&o.colrow, sizeof(int) * nnz);
-        A((void**)&o.ent, sizeof(int2) * nnz);
-        A((void**)&o.colval64, sizeof(double) * nnz);
+        ar.add(&o.colrow, nnz);
+        ar.add(&o.ent, nnz);
+        ar.add(&o.colval64, nnz);
     }
-    return e;
 }
 
 void csc_clear(const Csc& o, ClearList& l)
@@ -715,8 +707,8 @@ int mixed_init(Slot& c)
     m->K_cap = K_cap;
     m->nkb_cap = K_cap / TC_KB;
     m->ld32 = M_cap;
-    cudaError_t e = cudaSuccess;
-    auto A = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes > 0 ? bytes : 16); };
+    Arena ar;
+    auto A = [&](void** p, size_t bytes) { ar.add(reinterpret_cast<char**>(p), bytes); };
     const size_t xbytes = (m->half ? 2 : 4) * (size_t)M_cap * K_cap;
     A((void**)&m->X_hi, xbytes);
     A((void**)&m->X_lo, xbytes);
@@ -724,7 +716,7 @@ int mixed_init(Slot& c)
     A((void**)&m->F32, sizeof(float) * (size_t)M_cap * M_cap);
     A((void**)&m->R32, sizeof(float) * (size_t)M_cap * M_cap);
     A((void**)&m->img, sizeof(double) * (size_t)c.npix_pad);
-    if (e == cudaSuccess) e = csc_alloc(m->csc, c, M_cap, false);
+    csc_layout(m->csc, c, M_cap, false, ar);
     A((void**)&m->t, sizeof(double) * (size_t)(c.N_cap + 64));
     A((void**)&m->u, sizeof(double) * (size_t)(c.N_cap + 64));
     A((void**)&m->v, sizeof(double) * M_cap);
@@ -745,6 +737,7 @@ int mixed_init(Slot& c)
         A((void**)&f->il, sizeof(float) * (size_t)M_cap * C2);
         A((void**)&f->flags, sizeof(int) * flow128_flags(m->nb));
     }
+    const cudaError_t e = ar.commit(&m->base);
     if (e != cudaSuccess) {
         set_error("%s (%d)", "mixed-precision workspace allocation failed", (int)e);
         return QLP_ERR_NOMEM;

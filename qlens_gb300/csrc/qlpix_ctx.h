@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <string>
+#include <utility>
 #include <vector>
 #include "qlpix_internal.h"
 
@@ -156,7 +157,26 @@ void set_error(const char* fmt, const char* a, int code);
 // mixed.cu
 int mixed_init(Slot& slot);
 void mixed_free(Slot& slot);
-cudaError_t csc_alloc(Csc& o, const Slot& c, int M_cap, bool fine);
+// Buffers that live and die together, in one device allocation (an allocation each,
+// some 70 a slot, was a third of a batch's first pass).
+struct Arena {
+    std::vector<std::pair<void**, size_t>> parts;          // where each part's address goes, its offset
+    size_t bytes = 0;
+    template <typename T>
+    void add(T** p, size_t n)
+    {
+        parts.emplace_back(reinterpret_cast<void**>(p), bytes);
+        bytes += (sizeof(T) * (n > 0 ? n : 1) + 511) / 512 * 512;
+    }
+    cudaError_t commit(void** base) const
+    {
+        const cudaError_t e = cudaMalloc(base, bytes);
+        for (size_t k = 0; e == cudaSuccess && k < parts.size(); k++)
+            *parts[k].first = static_cast<char*>(*base) + parts[k].second;
+        return e;
+    }
+};
+void csc_layout(Csc& o, const Slot& c, int M_cap, bool fine, Arena& ar);
 // launch sequences of one evaluation: the whole of it, or, for the
 // regularisation-parameter optimisation, its lambda-independent part and one
 // lambda trial

@@ -190,11 +190,13 @@ struct Csc {
     unsigned* tile_active;     // bitmap of the image's tiles with active pixels, then the items' count
     int words;                 // words of the bitmap
     int M_cap, npix_pad;
+    void* base;                // the plain path's: the allocation that holds these (else part of another)
     int* ntiles() const { return reinterpret_cast<int*>(tile_active + words); }
 };
 
 // Per-evaluation device workspace (sized for the largest case at creation).
 struct Work {
+    void* base;                        // the allocation that holds all but Lpsf, F, R, F0 and the workspaces
     double* spx;  double* spy;         // n_sub source points
     double* cx;   double* cy;          // snx+1, sny+1 cell corners
     double* ccx;  double* ccy;         // snx, sny cell centres
