@@ -482,13 +482,14 @@ def main():
                      "peak_source": peak_note, "algorithmic_flops_per_launch": flops,
                      "timing": "CUDA events around the SYRK launch of single evaluations after the timed region"}
     if precision != "mixed":
-        # k_syrk64 skips the 16-pixel steps where either tile of L' is zero
-        # (the products it leaves out are zeros): the dense N M^2 count over
-        # its time is a dense-equivalent rate, not a fraction of the pipe
+        # k_oz_syrk skips the 32-pixel stages where either tile of L' is zero
+        # (the products it leaves out are zeros) and runs on the tensor cores: the
+        # dense N M^2 count over its time is a dense-equivalent rate, not a
+        # fraction of the FP64 pipe
         roofline_syrk["frac"] = None
         roofline_syrk["dense_equivalent_frac"] = (achieved / peak) if achieved else None
         roofline_syrk["note"] = ("achieved = the dense contraction's FLOP over the time of a kernel that skips L''s "
-                                 "zero blocks: above the FP64 peak because most products are skipped")
+                                 "zero blocks and forms the others as digit products on the tensor cores")
     # the dominant kernel of the batch: the ray shooting on the NFW surrogate
     # workloads (k_raytrace_sur), else the factorisation of F
     roofline = roofline_syrk
@@ -503,16 +504,15 @@ def main():
                     "algorithmic_flops_per_launch": mlp,
                     "work": "the network's three 128x128 layers per ray (2 x 3 x 128^2 FLOP), %d rays" % n_rays,
                     "limiter": "the network's SIMT epilogues (tanh from the SFU's exp2 and reciprocal, F16 hi/lo "
-                               "split, TMEM loads and stores) at 16 warps per SM: tensor pipe 29%, SFU 26%, FMA 20%, "
-                               "FP64 7% in k_raytrace_sur, top stall the TMEM and ray loads; the FP64 lenses in "
-                               "k_ray_pre at 85% of the FP64 pipe (one ncu capture)",
+                               "split, TMEM loads and stores) at 16 warps per SM; the FP64 lenses in k_ray_pre on "
+                               "the FP64 pipe",
                     "timing": "CUDA events around the ray-shooting stage of single evaluations after the timed "
                               "region"}
     elif precision != "mixed":
-        # the plain path's largest stage: the FP64 blocked Cholesky of F
+        # the plain path's largest stage: the Cholesky of F in digit products
         ch_flop = float(np.mean([r["n_active_src"] ** 3 / 3.0 for r in iso_res]))
         ach = ch_flop / (stage[4] / 1e3) / 1e12 if stage[4] > 0 else None
-        roofline = {"bound": "fp64", "kernel": "FP64 Cholesky of F (k_potrf_t, k_trsm_inv_t, k_chol_update_t)",
+        roofline = {"bound": "fp64", "kernel": "FP64 Cholesky of F (k_chol64)",
                     "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": (ach / peak) if ach else None,
                     "traffic": None, "peak_source": peak_note, "algorithmic_flops_per_launch": ch_flop,
                     "work": "M^3/3 FLOP per factorisation",
@@ -521,7 +521,7 @@ def main():
     elif precision == "mixed":
         ch_flop = float(np.mean([r["n_active_src"] ** 3 / 3.0 for r in iso_res]))
         ach = ch_flop / (stage[4] / 1e3) / 1e12 if stage[4] > 0 else None
-        roofline = {"bound": "tensor", "kernel": "Cholesky of F (k_potrf128, k_chol_tile128, k_chol_upd16)",
+        roofline = {"bound": "tensor", "kernel": "Cholesky of F (k_chol128)",
                     "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": (ach / peak) if ach else None,
                     "traffic": None, "peak_source": peak_note, "algorithmic_flops_per_launch": ch_flop,
                     "work": "M^3/3 FLOP per factorisation",
