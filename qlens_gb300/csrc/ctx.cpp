@@ -397,7 +397,8 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
         return QLP_OK;
     }
     {
-        const int r = mixed ? mixed_init(slot) : ensure_fp64_mats(slot);
+        int r = mixed ? mixed_init(slot) : ensure_fp64_mats(slot);
+        if (r == QLP_OK && !mixed && N_max > 0) r = psf_in_range(sd, Mc);
         if (r != QLP_OK) return r;
         ClearList cl;
         cl.add(w.out, sizeof(EvalOut));
@@ -465,8 +466,7 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             launch_logdet(w.R, w.ldF, Mc, w, 1, slot.side);
             cudaEventRecord(slot.side_join, slot.side);
         }
-        const int rp = launch_psf(sd, w, N_max, Mc, st);
-        if (rp != QLP_OK) return rp;
+        launch_psf(sd, w, N_max, st);
         launch_D(w, Mc, st);
         if (ev) cudaEventRecord(ev[3], st);
         launch_syrk_fp64(sd, w, N_max, Mc, st);

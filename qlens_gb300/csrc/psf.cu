@@ -188,15 +188,18 @@ void launch_rowpix(const StaticData& sd, Work& w, cudaStream_t st)
     count_launches(1);
 }
 
-int launch_psf(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st)
+// The plain path's stated range of PSFs and source grids.
+int psf_in_range(const StaticData& sd, int M_max)
 {
-    if (N_max == 0) return QLP_OK;
-    // the plain path's stated range of PSFs and source grids
     const size_t nT = ((size_t)sd.pnx * sd.pny + 7) / 8 * 8;
-    if (8 * (M_max + nT) + 8 * nT > 227 * 1024) {
-        set_error("%s (%d)", "PSF and source grid too large for the plain path", (int)nT);
-        return QLP_ERR_CUDA;
-    }
+    if (8 * (M_max + nT) + 8 * nT <= 227 * 1024) return QLP_OK;
+    set_error("%s (%d)", "PSF and source grid too large for the plain path", (int)nT);
+    return QLP_ERR_CUDA;
+}
+
+void launch_psf(const StaticData& sd, Work& w, int N_max, cudaStream_t st)
+{
+    if (N_max == 0) return;
     launch_csc(sd, w, w.csc, N_max, w.Lpsf, w.ldL, st);
     const size_t taps = sizeof(int2) * psfx_taps(sd.pnx, sd.pny);
     const bool fixed = sd.psf_fixed && taps <= PSF64_PAD_BYTES;
@@ -205,7 +208,6 @@ int launch_psf(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t
                                             w.csc.ntiles(), w.csc.tiles, w.Lpsf, w.ldL, oz_emax(w.oz), oz_nz(w.oz),
                                             oz_nst(w.oz));
     count_launches(1);
-    return QLP_OK;
 }
 
 }  // namespace qlpix

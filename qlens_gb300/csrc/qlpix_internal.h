@@ -249,7 +249,8 @@ void launch_locate(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream_
 void launch_compact(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream_t st);
 void launch_build_L(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream_t st);
 void launch_rowpix(const StaticData& sd, Work& w, cudaStream_t st);
-int launch_psf(const StaticData& sd, Work& w, int N_max, int M_max, cudaStream_t st);
+int psf_in_range(const StaticData& sd, int M_max);
+void launch_psf(const StaticData& sd, Work& w, int N_max, cudaStream_t st);
 void op_Ls(Work& w, int N_cap, const double* s, double* t, cudaStream_t st);
 void op_conv(const StaticData& sd, Work& w, int N_cap, bool transpose, const double* in, const double* scale_in,
              double* out, double* img, const int2* pixT, cudaStream_t st);

@@ -79,3 +79,24 @@ def test_sums_match_extended_precision(psf):
             tol = (n + 1) * 2.0 ** -53 * mag[i, j] + 2.0 ** -58 * taps
         err = np.abs(got[row, cells] - ref[i, j])
         assert (err <= tol).all(), (psf, row, float(err.max()), float(tol.min()))
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_refused_psf_leaves_the_context_usable(batch):
+    # 131 x 127 taps: past the plain path's range, within the mixed path's
+    from qlens_gb300 import PixelLikelihood, abi
+    nx, pixel = 30, 0.08
+    xv = (np.arange(nx + 1) - nx / 2) * pixel
+    pl = PixelLikelihood(xv, xv, np.ones((nx, nx)), np.ones((nx, nx), np.uint8), _kernel((131, 127)), covinv=None,
+                         bg_noise=0.1, nsplit=1, src_npixels=(6, 6), regparam=5.0, precision=abi.QLP_FP64)
+    pl.set_lens_model([{"type": "sple", "params": [0.6, 1.0, 0.0, 0.75, 30.0, 0.02, -0.01]}])
+    p = np.array([[0.6, 1.0, 0.0, 0.75, 30.0, 0.02, -0.01]] * 2)
+    if batch:
+        with pytest.raises(Exception):
+            pl.eval_batch(p)
+    else:
+        assert pl.invert_image_surface_brightness_map()["status"] != 0
+    pl.set_precision(abi.QLP_MIXED)
+    r = pl.eval_batch(p)[0] if batch else pl.invert_image_surface_brightness_map()
+    assert r["status"] == 0
+    pl.close()
