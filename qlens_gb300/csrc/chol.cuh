@@ -1,5 +1,5 @@
-// chol.cuh -- log det of a Cholesky factor (Cholesky_logdet_lower_packed,
-// pixelgrid.cpp:17201-17210), for the FP64 factor of the plain path and the
+// chol.cuh -- log det R from its Cholesky factor (Cholesky_logdet_lower_packed,
+// pixelgrid.cpp:17201-17210; F's is k_final's), for the FP64 factor of the plain path and the
 // FP32 one of the mixed path; the sum of logarithms is FP64 in both.
 #pragma once
 #include "qlpix_internal.h"
@@ -8,7 +8,7 @@ namespace qlpix {
 
 template <typename T>
 __global__ void __launch_bounds__(1024) k_logdet_t(const T* __restrict__ A, int ld, const GridState* __restrict__ gs,
-                                                   EvalOut* out, int which)
+                                                   EvalOut* out)
 {
     __shared__ double red[32];
     const int M = gs->M;
@@ -20,8 +20,7 @@ __global__ void __launch_bounds__(1024) k_logdet_t(const T* __restrict__ A, int 
     if (threadIdx.x == 0) {
         double t = 0;
         for (int k = 0; k < (int)(blockDim.x >> 5); k++) t += red[k];
-        if (which) out->logdet_R = 2 * t;
-        else out->logdet_F = 2 * t;
+        out->logdet_R = 2 * t;
     }
 }
 

@@ -104,6 +104,7 @@ static int alloc_work(qlp_ctx* c, Slot& s, int n_mask, int nsub, int Mcells, int
     ar.add(&w.D, Mc);
     ar.add(&w.s, Mc); ar.add(&w.tmp, Mc);
     ar.add(&w.model, n_mask);
+    ar.add(&w.fpart, 5 * 32); ar.add(&w.fcount, 1);
     ar.add(&w.gpart, 4 * 1024); ar.add(&w.gpart_cnt, 1024);
     ar.add(&w.cpart, 3 * 1025);
     ar.add(&w.linv, (size_t)Mc * 64);
@@ -113,6 +114,8 @@ static int alloc_work(qlp_ctx* c, Slot& s, int n_mask, int nsub, int Mcells, int
     ar.add(&w.xlist, n_sub); ar.add(&w.xcount, 2);
     ar.add(&w.nfw_xy, 2 * n_sub);
     CK(ar.commit(&w.base), "alloc");
+    CK(cudaMemset(w.fcount, 0, sizeof(int)), "memset");
+    CK(cudaStreamSynchronize(0), "memset");               // the slots' streams do not wait for stream 0
     s.M_cap = Mc;
     s.N_cap = n_mask;
     s.npix_pad = (c->nx + 2 * (c->sd.pnx / 2)) * (c->ny + 2 * (c->sd.pny / 2));
@@ -357,6 +360,14 @@ int factor_ctas(const qlp_ctx* c, int nb)
     return load == 0 ? 148 : load == 1 ? std::max(16, quarter) : quarter;
 }
 
+static void launch_final(Slot& slot, const StaticData& sd, const SrcOpts& so, const double* regp, bool mixed,
+                         cudaStream_t st)
+{
+    int ld = slot.w.ldF;
+    const void* factor = mixed ? (const void*)mixed_factor(slot, ld) : slot.w.F;
+    launch_model_chi2(sd, so, slot.w, sd.n_mask, regp, factor, ld, mixed, st);
+}
+
 // The launch sequence of one evaluation on stream st with the workspace of
 // `slot`; sd / so size the launches (the evaluation's own mask and source
 // grid, or the slot's capacity when the sequence is captured for replay).
@@ -389,10 +400,9 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             launch_copy_square(w.F, w.F0, w.ldF, 8, 64, w.gs, Mc, st);
             launch_regularization(so, w, Mc, regp, REG_F, st);
             launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, Mc, factor_ctas(c, Mc / 64), w.cholF, w.linv, st);
-            launch_logdet(w.F, w.ldF, Mc, w, 0, st);
             launch_solve_fp64(w, Mc, st);
         }
-        launch_model_chi2(sd, so, w, N_max, Mc, regp, st, mixed);
+        launch_final(slot, sd, so, regp, mixed, st);
         if (c->osb_on) launch_outside_sb(sd, so, c->osb, slot.osb, model_has_nfw(c), w, st);
         return QLP_OK;
     }
@@ -463,7 +473,7 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             launch_clear_band(w.R, w.ldF, 8, Mc, 64, (2 * so.snx + 63) / 64 + 2, w.gs, slot.side);
             launch_regularization(so, w, Mc, regp, REG_R, slot.side);
             launch_cholesky_fp64(w.R, w.ldF, Mc, w.gs, 1, 2 * so.snx, 4, w.cholR, nullptr, slot.side);
-            launch_logdet(w.R, w.ldF, Mc, w, 1, slot.side);
+            launch_logdet_R(w.R, w.ldF, w, slot.side);
             cudaEventRecord(slot.side_join, slot.side);
         }
         launch_psf(sd, w, N_max, st);
@@ -479,12 +489,11 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
         }
         launch_regularization(so, w, Mc, regp, REG_F, st);
         launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, Mc, factor_ctas(c, Mc / 64), w.cholF, w.linv, st);
-        launch_logdet(w.F, w.ldF, Mc, w, 0, st);
         launch_solve_fp64(w, Mc, st);
         if (so.regularization) cudaStreamWaitEvent(st, slot.side_join, 0);
     }
     if (ev) cudaEventRecord(ev[5], st);
-    launch_model_chi2(sd, so, w, N_max, Mc, regp, st, mixed);
+    launch_final(slot, sd, so, regp, mixed, st);
     if (c->osb_on) launch_outside_sb(sd, so, c->osb, slot.osb, model_has_nfw(c), w, st);
     if (ev) cudaEventRecord(ev[6], st);
     return QLP_OK;

@@ -239,10 +239,9 @@ void launch_regularization(const SrcOpts& so, Work& w, int M_max, const double* 
 }
 
 // ---- log det of a factor (the factorisations and solves: cholfp64.cu) ----
-void launch_logdet(const double* A, int ld, int M_max, Work& w, int which, cudaStream_t st)
+void launch_logdet_R(const double* A, int ld, Work& w, cudaStream_t st)
 {
-    (void)M_max;
-    k_logdet_t<double><<<1, 1024, 0, st>>>(A, ld, w.gs, w.out, which);
+    k_logdet_t<double><<<1, 1024, 0, st>>>(A, ld, w.gs, w.out);
     count_launches(1);
 }
 
@@ -278,18 +277,29 @@ __global__ void __launch_bounds__(256) k_model(const GridState* __restrict__ gs,
     }
 }
 
-__global__ void __launch_bounds__(1024) k_final(StaticData sd_, SrcOpts so_, const GridState* __restrict__ gs,
-                                                const int* __restrict__ rowidx, const double* __restrict__ model,
-                                                const double* __restrict__ s, const int* __restrict__ ai,
-                                                const double* __restrict__ regp, EvalOut* out)
+// chi^2, s^T R s, log det F from the factor A's diagonal, and the evidence: FINAL_CTAS
+// CTAs sum their shares, and the last of them adds those in a fixed order and puts
+// the result together.  The FP64 pipe bounds the sums (logarithms, the stencil of R):
+// one CTA for each of log det and the rest took 30 + 45 us at 2,934 cells and 11,772
+// pixels, now FINAL_FIG us together.
+#define FINAL_CTAS 32
+#define FINAL_SUMS 5
+__global__ void __launch_bounds__(256) k_final(StaticData sd_, SrcOpts so_, const GridState* __restrict__ gs,
+                                               const int* __restrict__ rowidx, const double* __restrict__ model,
+                                               const double* __restrict__ s, const int* __restrict__ ai,
+                                               const double* __restrict__ regp, const void* __restrict__ A, int ld,
+                                               int fp32, double* __restrict__ part, int* __restrict__ count,
+                                               EvalOut* out)
 {
     const StaticData sd = eval_shape(sd_);
     const SrcOpts so = eval_grid(so_, sd_);
     const double regparam = *regp;
-    __shared__ double red[4][32];
+    __shared__ double red[FINAL_SUMS][8];
+    __shared__ int last;
     const int M = gs->M;
-    double chi = 0, es = 0, chi_act = 0, logc = 0;
-    for (int m = threadIdx.x; m < sd.n_mask; m += blockDim.x) {
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    double chi = 0, es = 0, chi_act = 0, logc = 0, logd = 0;
+    for (int m = first; m < sd.n_mask; m += stride) {
         const int pix = sd.mpix[m];
         const double c = sd.use_noise_map ? sd.covinv[pix] : sd.cov_inverse;
         const int r = rowidx[m];
@@ -300,7 +310,7 @@ __global__ void __launch_bounds__(1024) k_final(StaticData sd_, SrcOpts so_, con
     }
     if (so.regularization && regparam != 0) {
         const int snx = so.snx, sny = so.sny;
-        for (int cidx = threadIdx.x; cidx < snx * sny; cidx += blockDim.x) {
+        for (int cidx = first; cidx < snx * sny; cidx += stride) {
             const int a = ai[cidx];
             if (a < 0) continue;
             const int ci = cidx % snx, cj = cidx / snx;
@@ -317,24 +327,37 @@ __global__ void __launch_bounds__(1024) k_final(StaticData sd_, SrcOpts so_, con
             es += s[a] * rs;
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        chi += __shfl_xor_sync(0xffffffffu, chi, o);
-        es += __shfl_xor_sync(0xffffffffu, es, o);
-        chi_act += __shfl_xor_sync(0xffffffffu, chi_act, o);
-        logc += __shfl_xor_sync(0xffffffffu, logc, o);
+    for (int i = first; i < M; i += stride) {
+        const size_t d = (size_t)i * ld + i;
+        logd += log(fabs(fp32 ? (double)reinterpret_cast<const float*>(A)[d] : reinterpret_cast<const double*>(A)[d]));
     }
-    if ((threadIdx.x & 31) == 0) {
-        red[0][threadIdx.x >> 5] = chi;
-        red[1][threadIdx.x >> 5] = es;
-        red[2][threadIdx.x >> 5] = chi_act;
-        red[3][threadIdx.x >> 5] = logc;
+    double sum[FINAL_SUMS] = {chi, es, chi_act, logc, logd};
+    #pragma unroll
+    for (int k = 0; k < FINAL_SUMS; k++) {
+        for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = sum[k];
     }
     __syncthreads();
+    if (threadIdx.x < FINAL_SUMS) {
+        double t = 0;
+        for (int k = 0; k < 8; k++) t += red[threadIdx.x][k];
+        part[threadIdx.x * FINAL_CTAS + blockIdx.x] = t;
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(count, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    __threadfence();
+    #pragma unroll
+    for (int k = 0; k < FINAL_SUMS; k++) {
+        sum[k] = __ldcg(part + k * FINAL_CTAS + threadIdx.x);
+        for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+    }
     if (threadIdx.x == 0) {
-        double c2 = 0, e2 = 0, ca = 0, lc = 0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) {
-            c2 += red[0][k]; e2 += red[1][k]; ca += red[2][k]; lc += red[3][k];
-        }
+        *count = 0;                                       // for the next evaluation
+        const double c2 = sum[0], e2 = sum[1], ca = sum[2], lc = sum[3];
+        out->logdet_F = 2 * sum[4];
         double regterms = 0, loglike = 0;
         if (so.regularization && M > 0) {
             if (regparam != 0) {
@@ -367,14 +390,14 @@ __global__ void __launch_bounds__(1024) k_final(StaticData sd_, SrcOpts so_, con
     }
 }
 
-void launch_model_chi2(const StaticData& sd, const SrcOpts& so, Work& w, int N_max, int M_max, const double* regp,
-                       cudaStream_t st, bool model_ready)
+void launch_model_chi2(const StaticData& sd, const SrcOpts& so, Work& w, int N_max, const double* regp,
+                       const void* factor, int ld, bool mixed, cudaStream_t st)
 {
-    (void)M_max;
-    if (N_max > 0 && !model_ready) {
+    if (N_max > 0 && !mixed) {
         k_model<<<(N_max + 31) / 32, 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, oz_nz(w.oz), oz_nst(w.oz), w.s, w.model);
     }
-    k_final<<<1, 1024, 0, st>>>(sd, so, w.gs, w.rowidx, w.model, w.s, w.active_index, regp, w.out);
+    k_final<<<FINAL_CTAS, 256, 0, st>>>(sd, so, w.gs, w.rowidx, w.model, w.s, w.active_index, regp, factor, ld,
+                                        mixed ? 1 : 0, w.fpart, w.fcount, w.out);
     count_launches(2);
 }
 

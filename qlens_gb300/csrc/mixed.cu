@@ -744,6 +744,7 @@ int mixed_init(Slot& c)
     }
     cudaMemset(m->X_hi, 0, xbytes);
     cudaMemset(m->X_lo, 0, xbytes);
+    cudaStreamSynchronize(0);                              // the slots' streams do not wait for stream 0
     if (make_map(&m->map_hi, m->X_hi, M_cap, K_cap, m->half) != QLP_OK ||
         make_map(&m->map_lo, m->X_lo, M_cap, K_cap, m->half) != QLP_OK ||
         flow_maps(m->cf, m->cf_maps) != QLP_OK || flow_maps(m->cr, m->cr_maps) != QLP_OK) {
@@ -803,6 +804,12 @@ int mixed_ensure_f0(Slot& slot)
     return QLP_OK;
 }
 
+const float* mixed_factor(Slot& slot, int& ld)
+{
+    ld = mw_of(slot)->ld32;
+    return mw_of(slot)->F32;
+}
+
 // What an evaluation (or one lambda trial) starts from cleared.
 void mixed_clear(Slot& slot, ClearList& l, bool trial)
 {
@@ -859,7 +866,7 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
         k_reg32<<<(so.snx * so.sny + 128 + 255) / 256, 256, 0, slot.side>>>(w.gs, w.active_index, regp, m->F32, m->R32,
                                                                            m->ld32, so.regularization, REG_R);
         cholesky_mixed(m->R32, m->ld32, w.gs, 1, band_R, nullptr, m->cr, m->cr_maps, 2, slot.side);
-        k_logdet_t<float><<<1, 1024, 0, slot.side>>>(m->R32, m->ld32, w.gs, w.out, 1);
+        k_logdet_t<float><<<1, 1024, 0, slot.side>>>(m->R32, m->ld32, w.gs, w.out);
         n += 3;
         cudaEventRecord(slot.side_join, slot.side);
     }
@@ -908,8 +915,6 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
     n++;
     }   // part != PIPE_TRIAL
     cholesky_mixed(m->F32, m->ld32, w.gs, 0, 1 << 20, m->linvF, m->cf, m->cf_maps, factor_ctas(c, m->nb), st);
-    n++;
-    k_logdet_t<float><<<1, 1024, 0, st>>>(m->F32, m->ld32, w.gs, w.out, 0);
     n++;
     if (so.regularization && part == PIPE_ALL) cudaStreamWaitEvent(st, slot.side_join, 0);
     // s = F^-1 D with `refine` FP64 refinement sweeps

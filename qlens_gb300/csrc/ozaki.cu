@@ -249,6 +249,7 @@ int oz_alloc(OzWork** out, int N_cap, int M_cap)
     A((void**)&z->emax, sizeof(int) * z->M128);
     A((void**)&z->nz, (size_t)(z->M128 / 64) * z->nst + 3);
     if (e == cudaSuccess) e = cudaMemset(z->part, 0, pbytes);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);    // the slots' streams do not wait for stream 0
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_oz_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, oz_smem(OZ_S));
     int rc = QLP_OK;

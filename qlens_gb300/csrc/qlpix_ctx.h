@@ -184,6 +184,7 @@ void csc_layout(Csc& o, const Slot& c, int M_cap, bool fine, Arena& ar);
 #define PIPE_PRE 1
 #define PIPE_TRIAL 2
 int mixed_ensure_f0(Slot& slot);
+const float* mixed_factor(Slot& slot, int& ld);
 void mixed_clear(Slot& slot, ClearList& l, bool trial);
 int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, const SrcOpts& so, const double* regp,
                         int part, cudaStream_t st,

@@ -222,6 +222,7 @@ struct Work {
     int ldF;
     double* s;   double* tmp;          // M
     double* model;                     // N
+    double* fpart;  int* fcount;       // k_final's sums by CTA and the CTAs done (0 between evaluations)
     double* gpart;  int* gpart_cnt;    // source-grid bounds: per-block partials (1024 blocks at most)
     int* cpart;                        // compaction: per-block counts (3 x 1025)
     double* linv;                      // per 64 columns: inverse of the diagonal block of F's factor
@@ -293,10 +294,11 @@ void chol64_clear(const Chol64Work* z, ClearList& l);
 void launch_regularization(const SrcOpts& so, Work& w, int M_max, const double* regp, int parts, cudaStream_t st);
 void launch_cholesky_fp64(double* A, int ld, int M_max, GridState* gs, int which, int half_width, int ctas,
                           Chol64Work* z, double* linv, cudaStream_t st);
-void launch_logdet(const double* A, int ld, int M_max, Work& w, int which, cudaStream_t st);
+void launch_logdet_R(const double* A, int ld, Work& w, cudaStream_t st);
 void launch_solve_fp64(Work& w, int M_max, cudaStream_t st);
-void launch_model_chi2(const StaticData& sd, const SrcOpts& so, Work& w, int N_max, int M_max,
-                       const double* regp, cudaStream_t st, bool model_ready = false);
+// factor: F's (its diagonal gives log det F), FP32 on the mixed path
+void launch_model_chi2(const StaticData& sd, const SrcOpts& so, Work& w, int N_max, const double* regp,
+                       const void* factor, int ld, bool mixed, cudaStream_t st);
 void launch_outside_sb(const StaticData& sd, const SrcOpts& so, const OsbStatic& os, const OsbWork& ow, bool nfw,
                        Work& w, cudaStream_t st);
 void init_kernel_attributes();
