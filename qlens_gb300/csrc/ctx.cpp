@@ -99,7 +99,7 @@ static int alloc_work(qlp_ctx* c, Slot& s, int n_mask, int nsub, int Mcells, int
     ar.add(&w.Lidx, nnz); ar.add(&w.Lval, nnz);
     ar.add(&w.cidx, nnz); ar.add(&w.cval, nnz); ar.add(&w.ccnt, n_mask);
     w.ldL = (n_mask + 31) / 32 * 32;
-    ar.add(&w.dvec, n_mask); ar.add(&w.cvec, n_mask);
+    ar.add(&w.dvec, n_mask); ar.add(&w.cvec, n_mask); ar.add(&w.svec, c->sd.use_noise_map ? n_mask : 0);
     w.ldF = Mc;
     ar.add(&w.D, Mc);
     ar.add(&w.s, Mc); ar.add(&w.tmp, Mc);

@@ -23,7 +23,7 @@ namespace qlpix {
 struct OzWork {
     __half* xs = nullptr;              // [OZ_S][M128][Kc] digits of L'^T sqrt(C^-1)
     unsigned long long* part = nullptr; // [tile][hi, lo][64 columns][128 rows], zero between evaluations
-    int* emax = nullptr;               // [M128] largest biased exponent of each source cell's column of L'
+    int* emax = nullptr;               // [M128] largest biased exponent of each source cell's L' (sqrt(C^-1))
     unsigned char* nz = nullptr;       // [M128 / 64][nst] 32-pixel stages where 64 cells have a nonzero
     int M128 = 0, Kc = 0, nst = 0, ntiles = 0;
     CUtensorMap map_a, map_b;
@@ -39,30 +39,14 @@ __device__ __forceinline__ void oz_tile(int t, int& I, int& j)
     j = t - i * (i + 1);
 }
 
-// With a noise map the operand is L' sqrt(C^-1): the exponent of the largest
-// sqrt(C^-1) is added to every cell's bound (an upper bound of the product's).
-__global__ void __launch_bounds__(1024) k_oz_noise_exp(const GridState* __restrict__ gs,
-                                                       const double* __restrict__ cvec, int* __restrict__ emax)
-{
-    __shared__ int top;
-    if (threadIdx.x == 0) top = 0;
-    __syncthreads();
-    int e = 0;
-    for (int r = threadIdx.x; r < gs->N; r += blockDim.x) e = max(e, oz_exponent(sqrt(cvec[r])));
-    atomicMax(&top, e);
-    __syncthreads();
-    const int add = top - 1022;                                // sqrt(C^-1) < 2^add
-    for (int c = threadIdx.x; c < gs->M; c += blockDim.x) {
-        const int m = emax[c];
-        if (m > 0 && m < 2047) emax[c] = (top >= 2047) ? 2047 : min(2046, max(1, m + add));
-    }
-}
-
-// The digits of 64 cells x 32 pixels of L'^T (sqrt(C^-1)), eight pixels a thread.
+// The digits of 64 cells x 32 pixels of L'^T (sqrt(C^-1)), eight pixels a thread.  With a
+// noise map the operand is the product L' sqrt(C^-1) as k_psf64 formed it for the cell's
+// largest exponent (a bound from the image's largest sqrt(C^-1) instead cost a cell on
+// noisier pixels as many of its bits as their noise is larger).
 // Stages without a nonzero in the cells' 128-row block are never loaded by the
 // products, so they are skipped.  14 bytes written per 8 read: memory bound.
 __global__ void __launch_bounds__(256) k_oz_slice(const GridState* __restrict__ gs, const double* __restrict__ L,
-                                                  int ldL, const double* __restrict__ cvec, int use_noise_map,
+                                                  int ldL, const double* __restrict__ svec,
                                                   const int* __restrict__ emax, const unsigned char* __restrict__ nz,
                                                   int nst, int st0, __half* __restrict__ xs, int M128, int Kc)
 {
@@ -86,7 +70,7 @@ __global__ void __launch_bounds__(256) k_oz_slice(const GridState* __restrict__ 
             for (int k = 0; k < 2; k++) {
                 const int r = r0 + u + k;
                 double x = r < N ? (k ? v.y : v.x) : 0.0;
-                if (use_noise_map && x != 0) x *= sqrt(cvec[r]);
+                if (svec && x != 0) x *= svec[r];
                 q[u + k] = oz_bias<OZ_S>(oz_fixed54(x, em));
             }
         }
@@ -287,10 +271,6 @@ void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaS
     OzWork* z = w.oz;
     const int nI = (M_max + OZ_TM - 1) / OZ_TM, tiles = nI * (nI + 1), ncb = 2 * nI;
     int n = 0;
-    if (N_max > 0 && sd.use_noise_map) {
-        k_oz_noise_exp<<<1, 1024, 0, st>>>(w.gs, w.cvec, z->emax);
-        n++;
-    }
     const int nst = (N_max + 31) / 32, per = z->Kc / 32;
     for (int s0 = 0; s0 < nst; s0 += per) {
         const int cnt = std::min(per, nst - s0);
@@ -298,8 +278,8 @@ void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaS
         // but no finer than one read of the accumulators per CTA
         const int split = std::max(1, std::min({(OZ_WANT_CTAS + tiles - 1) / tiles, (cnt + OZ_FLUSH - 1) / OZ_FLUSH,
                                                 64}));
-        k_oz_slice<<<dim3(cnt, ncb), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, w.cvec, sd.use_noise_map, z->emax, z->nz,
-                                                   z->nst, s0, z->xs, z->M128, z->Kc);
+        k_oz_slice<<<dim3(cnt, ncb), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, sd.use_noise_map ? w.svec : nullptr, z->emax,
+                                                   z->nz, z->nst, s0, z->xs, z->M128, z->Kc);
         k_oz_syrk<<<dim3(tiles, split), OZ_THREADS, oz_smem(OZ_S), st>>>(z->map_a, z->map_b, w.gs, z->nz, z->nst, s0,
                                                                    s0 + cnt, z->M128, z->part);
         n += 2;

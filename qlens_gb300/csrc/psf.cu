@@ -48,8 +48,9 @@ __device__ __forceinline__ int exponent_of(double x)
 // L' by image tiles, as k_psf_x builds X: a warp takes a listed (cell, 32 x 8
 // pixels) pair, lane x keeps its column's sums and adds tap x L for every entry
 // whose footprint meets the tile, three wide multiply-adds and a 64-bit load from
-// shared memory a tap.  With the values go each cell's largest biased exponent and
-// the live 32-pixel stages of each 64 cells, for the digits.
+// shared memory a tap.  With the values go each cell's largest biased exponent (with a
+// noise map of L' sqrt(C^-1), the digits' operand) and the live 32-pixel stages of each
+// 64 cells, for the digits.
 // At 24 warps an SM it waits on the chain from an entry to its taps and multiplies
 // (shared memory 21 %, issue 36 % busy).  A warp per image row that scattered tapped
 // rows into shared memory in FP64, a tap after the other, waited on those.  2,934 cells x
@@ -65,7 +66,8 @@ __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* _
                                                const int* __restrict__ colptr, const int4* __restrict__ ent_g,
                                                const int2* __restrict__ pixT, int ntx, const int* __restrict__ count,
                                                const uint2* __restrict__ list, double* __restrict__ L, int ldL,
-                                               int* __restrict__ emax, unsigned char* __restrict__ nz, int nst)
+                                               const double* __restrict__ svec, int* __restrict__ emax,
+                                               unsigned char* __restrict__ nz, int nst)
 {
     extern __shared__ __align__(16) int2 taps64[];  // [pnx + 62][pitch]: column pk + 31, row pl + R - 1
     constexpr int R = PSFX_R;
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* _
                 if (e == 0) continue;
                 L[(size_t)s * ldL + row] = v;
                 nz[(size_t)(s / 64) * nst + row / 32] = 1;
-                top = max(top, e);
+                top = max(top, svec ? exponent_of(v * svec[row]) : e);
             }
         }
         for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
@@ -161,9 +163,9 @@ __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* _
 }
 
 // Active row -> image pixel, the inverse of the compaction's pixindex, and the
-// row's data and C^-1.
+// row's data and C^-1 (svec, or null: its square root).
 __global__ void k_rowpix(StaticData sd_, const int* __restrict__ rowidx, int* __restrict__ rowpix,
-                         double* __restrict__ dvec, double* __restrict__ cvec)
+                         double* __restrict__ dvec, double* __restrict__ cvec, double* __restrict__ svec)
 {
     const StaticData sd = eval_shape(sd_);
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < sd.n_mask; m += gridDim.x * blockDim.x) {
@@ -173,6 +175,7 @@ __global__ void k_rowpix(StaticData sd_, const int* __restrict__ rowidx, int* __
         rowpix[r] = pix;
         dvec[r] = sd.data[pix];
         cvec[r] = sd.use_noise_map ? sd.covinv[pix] : sd.cov_inverse;
+        if (svec) svec[r] = sqrt(cvec[r]);
     }
 }
 
@@ -184,7 +187,8 @@ void psf_init_attributes()
 void launch_rowpix(const StaticData& sd, Work& w, cudaStream_t st)
 {
     if (sd.n_mask == 0) return;
-    k_rowpix<<<(sd.n_mask + 255) / 256, 256, 0, st>>>(sd, w.rowidx, w.rowpix, w.dvec, w.cvec);
+    k_rowpix<<<(sd.n_mask + 255) / 256, 256, 0, st>>>(sd, w.rowidx, w.rowpix, w.dvec, w.cvec,
+                                                        sd.use_noise_map ? w.svec : nullptr);
     count_launches(1);
 }
 
@@ -205,8 +209,8 @@ void launch_psf(const StaticData& sd, Work& w, int N_max, cudaStream_t st)
     const bool fixed = sd.psf_fixed && taps <= PSF64_PAD_BYTES;
     auto k = fixed ? k_psf64<true> : k_psf64<false>;
     k<<<152 * 3, 256, fixed ? taps : 0, st>>>(sd, w.gs, w.csc.colcnt, w.csc.fine, w.csc.pixT, (sd.nx + 31) / 32,
-                                            w.csc.ntiles(), w.csc.tiles, w.Lpsf, w.ldL, oz_emax(w.oz), oz_nz(w.oz),
-                                            oz_nst(w.oz));
+                                            w.csc.ntiles(), w.csc.tiles, w.Lpsf, w.ldL, sd.use_noise_map ? w.svec : nullptr,
+                                            oz_emax(w.oz), oz_nz(w.oz), oz_nst(w.oz));
     count_launches(1);
 }
 

@@ -216,6 +216,7 @@ struct Work {
     Chol64Work* cholF;  Chol64Work* cholR;  // plain path: workspaces of the factorisations (cholfp64.cu)
     int ldL;                           // leading dimension of Lpsf (>= N_max, a multiple of 32)
     double* dvec; double* cvec;        // N: data and C^-1 per active row
+    double* svec;                      // N: sqrt(C^-1) (plain path with a noise map)
     double* D;                         // M
     double* F;                         // M x ldF (lower triangle)
     double* R;                         // M x ldF (lower triangle)
