@@ -1,5 +1,6 @@
 // cholfp64.cu -- the plain path's dense factorisation and solve:
 //   F = L L^T and R = L L^T   k_chol64 (one launch each)
+//   F again, in FP64          k_chol64_plain, where k_chol64 met a pivot <= 0
 //   F s = D                   k_trsv64_fwd, k_trsv64_bwd
 // Reference: Cholesky_dcmp_packed (pixelgrid.cpp:17071-17105; a negative pivot
 // is flagged and sqrt(|d|) used), Cholesky_solve_lower_packed (17230-17246).
@@ -23,7 +24,9 @@
 // pivot cost 1.2 us.  An FP64 factorisation rounds at 2^-53 of the same scale per
 // operation; log det F, log det R and the amplitudes come out as close to an
 // extended-precision factorisation as the FP64 one's (96 to 382 cells, condition
-// numbers 7e2 to 1e9: amplitudes 2e-15 to 2e-11 for both).
+// numbers 7e2 to 1e9: amplitudes 2e-15 to 2e-11 for both).  All this holds for a positive
+// definite matrix; where F is not, its factor outgrows the integers' range, and
+// k_chol64_plain takes over.
 //
 // What bounds it, for one evaluation: the chain of pivot blocks, ~80 us per 64
 // columns -- 46 us the pivots (0.7 us each: 1/sqrt, two barriers, and wide integer
@@ -54,7 +57,9 @@ struct Chol64Work {
     int* rexp = nullptr;           // [M128] E_i
     int* lexp = nullptr;           // [M128] exponents of the inverses' rows
     int* wexp = nullptr;           // [nbc] the inverses' grids
-    int* flags = nullptr;          // ready[nbc][nbc] (column, row block), inverse[nbc], tile counter
+    int* flags = nullptr;          // ready[nbc][nbc] (column, row block), inverse[nbc], tile counter,
+                                   // two solves' [nbc] each, redo (a pivot <= 0), its tile counter
+    double* diag = nullptr;        // F's: [M128] its diagonal, for k_chol64_plain
     int M128 = 0, nbc = 0;
     bool own_ls = false;
     CUtensorMap ls_a, ls_b, li_b;
@@ -152,6 +157,7 @@ struct Diag64 {
     long long brow[C64];       // the pivot's row of the inverse before its division, on 2^-58
     int g[C64];                // the block's own scaling: row and column i times 2^g_i
     int first_bad;             // first negative pivot + 1, 0 none
+    int redo;                  // a pivot that is not positive
     int wide;                  // the inverse left its range: redone in FP64
     int w;                     // it is kept on 2^-(58 - w)
     int top;                   // bits of its largest entry
@@ -185,6 +191,7 @@ __device__ __forceinline__ void diag64_steps(long long (&q)[10], Diag64& s, unsi
             const long long t = tid < 64 ? (i == j ? (d < 0 ? -d : d) : s.col[i] + ((3 * j) >> 2))
                                          : s.brow[i] + ((3 * (j - i)) >> 2);
             int k;
+            if (tid == 0 && (d <= 0 || poison[j])) s.redo = 1;
             if (d < 0) {
                 if (tid == 0 && s.first_bad == 0 && !poison[j]) s.first_bad = j + 1;
                 d = -d;
@@ -317,12 +324,16 @@ __device__ __forceinline__ bool wait_flag(const int* p, GridState* gs, volatile 
 // band: blocks below the diagonal that can be nonzero, even (a tile's second
 // 64 rows reach one further); dense: any number past the matrix.
 // linv: the inverses of the diagonal blocks in FP64 for the solves, or null.
+// redo, diag0 (F; R is positive definite by construction: null): the matrix is kept
+// above its diagonal and in diag0, and *redo set where a pivot is not positive, for
+// k_chol64_plain.
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant__ CUtensorMap ls_a,
                                                          const __grid_constant__ CUtensorMap ls_b,
                                                          const __grid_constant__ CUtensorMap li_b, GridState* gs,
                                                          double* F, int ld, int which, int band, int M128, int nbc,
                                                          __half* ls, __half* li, const int* rexp, int* lexp,
-                                                         int* wexp, int* flags, double* linv)
+                                                         int* wexp, int* flags, double* linv, int* redo,
+                                                         double* diag0)
 {
     extern __shared__ unsigned char smem_raw[];
     __shared__ OzPipe pipe;
@@ -362,7 +373,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
             col_e[threadIdx.x - OZ_TM] = e == C64_POISON ? 0 : e;
             poison[threadIdx.x - OZ_TM] = e == C64_POISON;
         }
-        if (threadIdx.x == 0) dg.first_bad = dg.wide = dg.top = dg.w = 0;
+        if (threadIdx.x == 0) dg.first_bad = dg.redo = dg.wide = dg.top = dg.w = 0;
         __syncthreads();
 
         const int r = 32 * (warp & 3) + lane, h = (warp >> 2) & 1;       // an epilogue thread's row and column half
@@ -393,10 +404,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
             __syncwarp();
         } else {
             const double* src = F + (size_t)row * ld + j * C64 + 32 * h;
+            double* up = F + (size_t)(j * C64 + 32 * h) * ld + row;       // (the diagonal block's: below)
+            const bool keep = redo && row < Mp && (t > 0 || r >= C64);
             #pragma unroll
             for (int c = 0; c < 32; c += 2) {
                 double2 a = make_double2(0.0, 0.0);
                 if (row < Mp) a = *reinterpret_cast<const double2*>(src + c);
+                if (keep) { up[(size_t)c * ld] = a.x; up[(size_t)(c + 1) * ld] = a.y; }
                 const long long v0 = -fx_from_double(a.x, 60 - row_e[r] - col_e[32 * h + c]);
                 const long long v1 = -fx_from_double(a.y, 60 - row_e[r] - col_e[32 * h + c + 1]);
                 hi[c] = v0 >> 24; lo[c] = (uint32_t)v0 << 8;             // v 2^8 = hi 2^32 + lo on 2^-68
@@ -564,6 +578,18 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
             if (t == 0) {
                 // the factor's diagonal block and its inverse in FP64: nothing in
                 // this launch reads them
+                if (redo) {
+                    double a[16];
+                    #pragma unroll
+                    for (int u = 0; u < 16; u++) a[u] = F[(size_t)(j * C64 + u * 4 + (tid >> 6)) * ld + j * C64 + (tid & 63)];
+                    #pragma unroll
+                    for (int u = 0; u < 16; u++) {
+                        const int i = u * 4 + (tid >> 6), c = tid & 63;
+                        if (c < i) F[(size_t)(j * C64 + c) * ld + j * C64 + i] = a[u];
+                        if (c == i) diag0[j * C64 + i] = a[u];
+                    }
+                    if (tid == 0 && dg.redo) *redo = 1;
+                }
                 for (int u = 0; u < 16; u++) {
                     const int i = u * 4 + (tid >> 6), c = tid & 63;
                     if (c <= i) {
@@ -575,7 +601,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
                         linv[(size_t)(j * C64 + i) * C64 + c] =
                             c <= i ? mul_pow2((double)diag_at(SX, i, c), dg.w - 58 + dg.g[c] - col_e[c]) : 0.0;
                 }
-                if (tid == 0 && dg.first_bad) {
+                if (tid == 0 && dg.first_bad && !redo) {
                     int* flag = which ? &gs->not_spd_R : &gs->not_spd_F;
                     if (*flag == 0) *flag = j * C64 + dg.first_bad;
                 }
@@ -613,6 +639,153 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
     __syncwarp();
     oz_end(pipe);
     if (pipe.abort && threadIdx.x == 0) atomicExch(&gs->status, QLP_ERR_TIMEOUT);
+}
+
+// ---------------------------------------------------------------------------
+// F = L L^T in FP64, where k_chol64 met a pivot that is not positive (or a row that
+// holds no finite number): sqrt(|d|) at a negative one, flagged, and no bound on what
+// follows, as the reference goes on.  Left-looking over 64x64 tiles from a counter, as
+// k_chol64, the same flags with the value 2; the matrix comes from above the
+// diagonal and diag0.  Bound by the FP64 pipe (M^3 / 3 multiply-adds at 2 a clock and
+// SM); nothing but the look at *redo for any other matrix.
+// ---------------------------------------------------------------------------
+#define CP_SMEM (2 * C64 * (C64 + 1) * (int)sizeof(double))
+
+// All threads wait (bounded) until *p and *q are 2.
+__device__ __forceinline__ bool wait_redone(const int* p, const int* q, GridState* gs, int* sh)
+{
+    if (threadIdx.x == 0) {
+        const uint64_t t0 = globaltimer();
+        bool ok;
+        while (!(ok = ld_acquire(p) == 2 && ld_acquire(q) == 2)) {
+            if (*(volatile int*)&gs->status == QLP_ERR_TIMEOUT || globaltimer() - t0 > TC_WAIT_NS) break;
+            __nanosleep(64);
+        }
+        if (!ok) atomicExch(&gs->status, QLP_ERR_TIMEOUT);
+        *sh = ok ? 1 : 0;
+    }
+    __syncthreads();
+    const bool ok = *sh != 0;
+    __syncthreads();
+    return ok;
+}
+
+__global__ void __launch_bounds__(256) k_chol64_plain(GridState* gs, double* F, int ld, const double* diag0, int nbc,
+                                                      int* flags, const int* redo, int* counter, double* linv)
+{
+    if (*redo == 0) return;
+    extern __shared__ double cp_smem[];
+    __shared__ double colj[C64];
+    __shared__ int sh, ticket;
+    double (*P)[C64 + 1] = reinterpret_cast<double (*)[C64 + 1]>(cp_smem);
+    double (*Q)[C64 + 1] = reinterpret_cast<double (*)[C64 + 1]>(cp_smem + C64 * (C64 + 1));
+    const int nb = ((gs->M + 63) & ~63) / C64;
+    int* ready = flags;
+    int* inv = flags + (size_t)nbc * nbc;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    int j = 0, base = 0;
+    while (true) {
+        if (tid == 0) ticket = atomicAdd(counter, 1);
+        __syncthreads();
+        const int tk = ticket;
+        __syncthreads();
+        while (j < nb && tk >= base + nb - j) { base += nb - j; j++; }
+        if (j >= nb) return;
+        const int i = j + tk - base;
+        const bool diag = i == j;
+        double acc[4][4];
+        #pragma unroll
+        for (int u = 0; u < 4; u++)
+            #pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const int r = ty * 4 + u, c = tx * 4 + v;
+                acc[u][v] = (diag && r == c) ? diag0[j * C64 + r]
+                            : (diag && r < c) ? 0.0 : F[(size_t)(j * C64 + c) * ld + i * C64 + r];
+            }
+        for (int k = 0; k < j; k++) {
+            const int* rk = ready + (size_t)k * nbc;
+            if (!wait_redone(rk + i, rk + j, gs, &sh)) return;
+            for (int e = tid; e < C64 * C64; e += 256) {
+                const int r = e >> 6, m = e & 63;
+                P[r][m] = __ldcg(F + (size_t)(i * C64 + r) * ld + k * C64 + m);
+                Q[r][m] = __ldcg(F + (size_t)(j * C64 + r) * ld + k * C64 + m);
+            }
+            __syncthreads();
+            #pragma unroll 4
+            for (int m = 0; m < C64; m++) {
+                double a[4], b[4];
+                #pragma unroll
+                for (int u = 0; u < 4; u++) { a[u] = P[ty * 4 + u][m]; b[u] = Q[tx * 4 + u][m]; }
+                #pragma unroll
+                for (int u = 0; u < 4; u++)
+                    #pragma unroll
+                    for (int v = 0; v < 4; v++) acc[u][v] -= a[u] * b[v];
+            }
+            __syncthreads();
+        }
+        #pragma unroll
+        for (int u = 0; u < 4; u++)
+            #pragma unroll
+            for (int v = 0; v < 4; v++) P[ty * 4 + u][tx * 4 + v] = acc[u][v];
+        if (diag) {
+            __syncthreads();
+            for (int p = 0; p < C64; p++) {
+                if (tid >= p && tid < C64) {
+                    const double d = P[p][p], sd = sqrt(fabs(d));
+                    if (tid == p && d < 0) atomicCAS(&gs->not_spd_F, 0, j * C64 + p + 1);
+                    colj[tid] = tid == p ? sd : P[tid][p] / sd;
+                }
+                __syncthreads();
+                for (int r = p + 1 + ty; r < C64; r += 16) {
+                    const double l = colj[r];
+                    for (int c = p + 1 + tx; c <= r; c += 16) P[r][c] -= l * colj[c];
+                }
+                if (tid >= p && tid < C64) P[tid][p] = colj[tid];
+                __syncthreads();
+            }
+            // the inverse, four threads a column
+            const int c = tid >> 2, q = tid & 3;
+            for (int r = 0; r < C64; r++) {
+                double part = 0;
+                if (r > c)
+                    for (int m = c + q; m < r; m += 4) part += P[r][m] * Q[m][c];
+                part += __shfl_xor_sync(0xffffffffu, part, 1);
+                part += __shfl_xor_sync(0xffffffffu, part, 2);
+                if (q == 0) Q[r][c] = r < c ? 0.0 : (r == c ? 1.0 / P[r][r] : -part / P[r][r]);
+                __syncwarp();
+            }
+            __syncthreads();
+            for (int e = tid; e < C64 * C64; e += 256) {
+                const int r = e >> 6, m = e & 63;
+                if (m <= r) F[(size_t)(j * C64 + r) * ld + j * C64 + m] = P[r][m];
+                linv[(size_t)(j * C64 + r) * C64 + m] = Q[r][m];
+            }
+        } else {
+            if (!wait_redone(inv + j, inv + j, gs, &sh)) return;
+            // by substitution (a product with the block's inverse loses digits where the
+            // factor grows), four threads a row
+            for (int e = tid; e < C64 * C64; e += 256) {
+                const int r = e >> 6, m = e & 63;
+                if (m <= r) Q[r][m] = __ldcg(F + (size_t)(j * C64 + r) * ld + j * C64 + m);
+            }
+            __syncthreads();
+            const int r = tid >> 2, q = tid & 3;
+            for (int c = 0; c < C64; c++) {
+                double part = 0;
+                for (int m = q; m < c; m += 4) part += P[r][m] * Q[c][m];
+                part += __shfl_xor_sync(0xffffffffu, part, 1);
+                part += __shfl_xor_sync(0xffffffffu, part, 2);
+                if (q == 0) P[r][c] = (P[r][c] - part) / Q[c][c];
+                __syncwarp();
+            }
+            __syncthreads();
+            for (int e = tid; e < C64 * C64; e += 256)
+                F[(size_t)(i * C64 + (e >> 6)) * ld + j * C64 + (e & 63)] = P[e >> 6][e & 63];
+        }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) st_release(diag ? inv + j : ready + (size_t)j * nbc + i, 2);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -727,13 +900,15 @@ __global__ void __launch_bounds__(256) k_trsv64_bwd(const double* __restrict__ L
 void chol64_free(Chol64Work* z)
 {
     if (!z) return;
-    void* ptrs[] = {z->own_ls ? z->ls : nullptr, z->li, z->rexp, z->lexp, z->wexp, z->flags};
+    void* ptrs[] = {z->own_ls ? z->ls : nullptr, z->li, z->rexp, z->lexp, z->wexp, z->flags, z->diag};
     for (void* p : ptrs) if (p) cudaFree(p);
     delete z;
 }
 
+static size_t chol64_flags(const Chol64Work* z) { return (size_t)z->nbc * z->nbc + 3 * z->nbc + 3; }
+
 // shared: M128 x M128 digits that nothing else uses while this matrix is
-// factored (F: the digits of L', read by then), or null to allocate them.
+// factored (F: the digits of L', read by then), or null to allocate them (R).
 int chol64_alloc(Chol64Work** out, int M_cap, void* shared)
 {
     Chol64Work* z = new Chol64Work();
@@ -749,8 +924,11 @@ int chol64_alloc(Chol64Work** out, int M_cap, void* shared)
     A((void**)&z->rexp, sizeof(int) * z->M128);
     A((void**)&z->lexp, sizeof(int) * z->M128);
     A((void**)&z->wexp, sizeof(int) * z->nbc);
-    A((void**)&z->flags, sizeof(int) * ((size_t)z->nbc * z->nbc + 3 * z->nbc + 1));
+    A((void**)&z->flags, sizeof(int) * chol64_flags(z));
+    if (!z->own_ls) A((void**)&z->diag, sizeof(double) * z->M128);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_chol64, cudaFuncAttributeMaxDynamicSharedMemorySize, oz_smem(CS));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_chol64_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, CP_SMEM);
     int rc = QLP_OK;
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -770,7 +948,7 @@ int chol64_alloc(Chol64Work** out, int M_cap, void* shared)
 // The flags of a factorisation and of one pair of solves.
 void chol64_clear(const Chol64Work* z, ClearList& l)
 {
-    l.add(z->flags, sizeof(int) * ((size_t)z->nbc * z->nbc + 3 * z->nbc + 1));
+    l.add(z->flags, sizeof(int) * chol64_flags(z));
 }
 
 // which: 0 F, 1 R (the not-SPD flag).  half_width: how far below the diagonal
@@ -783,10 +961,15 @@ void launch_cholesky_fp64(double* A, int ld, int M_max, GridState* gs, int which
     const int band = ((std::min(half_width, M_max) + C64 - 1) / C64 + 1) & ~1;
     const int tiles = nb * std::min((nb + 1) / 2, band / 2 + 1);
     k_chol64_prep<<<(M_max + 255) / 256, 256, 0, st>>>(gs, A, ld, z->rexp);
+    int* redo = z->diag ? z->flags + chol64_flags(z) - 2 : nullptr;
     k_chol64<<<std::max(1, std::min(tiles, ctas)), OZ_THREADS, oz_smem(CS), st>>>(
         z->ls_a, z->ls_b, z->li_b, gs, A, ld, which, band, z->M128, z->nbc, z->ls, z->li, z->rexp, z->lexp, z->wexp,
-        z->flags, linv);
+        z->flags, linv, redo, z->diag);
     count_launches(2);
+    if (!redo) return;
+    k_chol64_plain<<<std::max(1, std::min(nb * (nb + 1) / 2, ctas)), 256, CP_SMEM, st>>>(gs, A, ld, z->diag, z->nbc,
+                                                                                    z->flags, redo, redo + 1, linv);
+    count_launches(1);
 }
 
 void launch_solve_fp64(Work& w, int M_max, cudaStream_t st)
