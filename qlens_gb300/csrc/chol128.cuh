@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(C2_THREADS, 1) k_chol128(const __grid_constant
         __syncthreads();
         const int tk = ticket;
         while (j < nb && tk >= base + min(nb - j, band + 1)) { base += min(nb - j, band + 1); j++; }
-        if (j >= nb || f.abort) break;           // uniform: f.abort is raised between the barriers below only
+        if (j >= nb) break;
         const int i = j + tk - base;
         const bool diag = i == j;
         const int k0 = max(0, i - band), nk = j - k0;
@@ -494,8 +494,8 @@ __global__ void __launch_bounds__(C2_THREADS, 1) k_chol128(const __grid_constant
             #pragma unroll 1
             for (int k = 0; k < nk; k++) {
                 const int kc = kc0 + k, b = kc & 1;
-                if (!mbar_wait_bounded(&f.exp_full[b], (kc >> 1) & 1, &f.abort)) break;
-                if (!mbar_wait_bounded(&f.acc_full[b], (kc >> 1) & 1, &f.abort)) break;
+                if (!mbar_wait_warp(&f.exp_full[b], (kc >> 1) & 1, &f.abort)) break;
+                if (!mbar_wait_warp(&f.acc_full[b], (kc >> 1) & 1, &f.abort)) break;
                 tc_fence_after();
                 const int si = 127 - exps[b][0][r];
                 const int* sj = &exps[b][1][64 * h];
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(C2_THREADS, 1) k_chol128(const __grid_constant
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 tc_fence_before();
                 asm volatile("bar.sync 2, 288;" ::: "memory");
-                const bool ok = mbar_wait_bounded(&f.sol[1], nsol & 1, &f.abort);
+                const bool ok = mbar_wait_warp(&f.sol[1], nsol & 1, &f.abort);
                 tc_fence_after();
                 const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(2 * C2 + 64 * h);
                 float mx = 0.f;
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(C2_THREADS, 1) k_chol128(const __grid_constant
             }
             nsol++;
         }
-        __syncthreads();
+        __syncthreads();                          // the one place to leave early: here nobody raises f.abort
         if (f.abort) break;
     }
     if (tid == 32 * (C2_EPI + 1)) mma_commit(&f.done);

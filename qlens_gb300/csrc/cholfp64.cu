@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
         const int tk = ticket;
         auto tiles_of = [&](int c) { return min((nb - c + 1) >> 1, (band >> 1) + 1); };
         while (j < nb && tk >= base + tiles_of(j)) { base += tiles_of(j); j++; }
-        if (j >= nb || pipe.abort) break;        // uniform: pipe.abort is only raised between the barriers below
+        if (j >= nb) break;
         const int t = tk - base, rb = j + 2 * t;
         const int k0 = max(0, rb - band), n = 2 * (j - k0);
         const bool second = rb + 1 < nb;         // the tile's rows 64..127 exist
@@ -632,6 +632,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
         }
         if (solve) f0++;
         if (t > 0) nb_full++;
+        // the one place to leave early: behind a barrier nobody raises pipe.abort until the next one (a
+        // thread that saw it raised by a faster warp's wait would leave the others at their barriers)
         __syncthreads();
         if (pipe.abort) break;
     }

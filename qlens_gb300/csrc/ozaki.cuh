@@ -255,7 +255,7 @@ __device__ __forceinline__ bool oz_accumulate(OzPipe& p, int f0, int n, long lon
     #pragma unroll 1
     for (int f = f0; f < f0 + nf; f++) {
         float v[16];
-        if (!mbar_wait_bounded(&p.acc_full[0], f & 1, &p.abort)) return false;
+        if (!mbar_wait_warp(&p.acc_full[0], f & 1, &p.abort)) return false;
         tc_fence_after();
         #pragma unroll
         for (int h = 0; h < 32; h += 16) {
@@ -270,7 +270,7 @@ __device__ __forceinline__ bool oz_accumulate(OzPipe& p, int f0, int n, long lon
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p.acc_empty[0]);
-        if (!mbar_wait_bounded(&p.acc_full[1], f & 1, &p.abort)) return false;
+        if (!mbar_wait_warp(&p.acc_full[1], f & 1, &p.abort)) return false;
         tc_fence_after();
         #pragma unroll
         for (int h = 0; h < 32; h += 16) {

@@ -68,6 +68,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t phase,
     }
 }
 
+// The same for a whole warp, which goes on together (TMEM loads are warp instructions):
+// true if no lane gave up.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t phase, volatile int* abort_flag)
+{
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, abort_flag));
+}
+
 __device__ __forceinline__ void tma_load_2d(const CUtensorMap* map, uint64_t* bar, void* dst, int x, int y)
 {
     asm volatile(

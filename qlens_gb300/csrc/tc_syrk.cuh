@@ -184,16 +184,17 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
     __syncthreads();
     // ---- epilogue ----
     // Wait for the committed MMAs even after an abort: TMEM is freed below.
-    const bool ok = mbar_wait_bounded(&done_bar, 0, &abort_flag, false);
+    bool ok = mbar_wait_bounded(&done_bar, 0, &abort_flag, false);
     if (abort_flag && threadIdx.x == 0) {
         // let TMA copies that were issued but never consumed land before exit
         for (int it = n_active; it < n_issued; it++)
             mbar_wait_bounded(&full_bar[it % TC_STAGES], (it / TC_STAGES) & 1, &abort_flag, false);
     }
+    ok = __syncthreads_and(ok && !abort_flag);         // the warps' TMEM loads need all their lanes
     tc_fence_after();
     const int row = bi * TC_TILE + warp * 32 + lane;
     float* out = F + (size_t)row * ldF + bj * TC_TILE;
-    if (ok && !abort_flag && n_active > 0) {
+    if (ok && n_active > 0) {
         #pragma unroll 1
         for (int c = 0; c < TC_TILE; c += 32) {
             float v[32];
