@@ -529,7 +529,10 @@ typedef struct {
 int qlp_set_fit_params(qlp_ctx* ctx, const qlp_fit_param* params, int n);
 
 /* -log L of n fit vectors ([n][n_fit]) in one batch (penalised vectors are
- * not evaluated: loglike 1e30, a zeroed result).  out may be NULL. */
+ * not evaluated: loglike 1e30, a zeroed result).  out may be NULL.  If a
+ * bounded device wait ran out in an evaluation (its result's status
+ * QLP_ERR_TIMEOUT), that vector's loglike is 1e30 and the call returns
+ * QLP_ERR_TIMEOUT; the other vectors' values hold. */
 int qlp_fit_loglike_batch(qlp_ctx* ctx, const double* fit_params, int n, double* loglike, qlp_result* out);
 
 /* The host side of one fit vector, no device needed: the transformed values

@@ -672,7 +672,7 @@ static int regopt_wave(qlp_ctx* c, const std::vector<int>& inst, const std::vect
     }
     std::vector<BrentMin> br(k);
     std::vector<double> best(k, INFINITY);
-    std::vector<char> act(k);
+    std::vector<char> act(k), timed_out(k, 0);
     for (int j = 0; j < k; j++) br[j].reset(c->regopt_minlog, c->regopt_maxlog, c->regopt_tol, c->regopt_maxit);
     while (true) {
         bool any = false;
@@ -692,6 +692,7 @@ static int regopt_wave(qlp_ctx* c, const std::vector<int>& inst, const std::vect
         for (int j = 0; j < k; j++) {
             if (!act[j]) continue;
             const double f = c->h_trial[j].f_regopt;
+            timed_out[j] |= c->h_trial[j].status == QLP_ERR_TIMEOUT;
             if (f < best[j]) {
                 best[j] = f;
                 c->h_out[inst[j]] = c->h_trial[j];
@@ -700,7 +701,10 @@ static int regopt_wave(qlp_ctx* c, const std::vector<int>& inst, const std::vect
             br[j].give(f);
         }
     }
-    for (int j = 0; j < k; j++) c->regopt_evals[inst[j]] = br[j].evals();
+    for (int j = 0; j < k; j++) {
+        c->regopt_evals[inst[j]] = br[j].evals();
+        if (timed_out[j]) c->h_out[inst[j]].status = QLP_ERR_TIMEOUT;     // the search went by numbers that mean nothing
+    }
     return QLP_OK;
 }
 

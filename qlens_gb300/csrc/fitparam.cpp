@@ -130,6 +130,7 @@ int fit_loglike_batch(qlp_ctx* c, const double* x, int n, double* loglike, qlp_r
             return rc;
     }
     size_t k = 0;
+    bool timed_out = false;
     for (int i = 0; i < n; i++) {
         qlp_result r;
         memset(&r, 0, sizeof(r));
@@ -137,12 +138,14 @@ int fit_loglike_batch(qlp_ctx* c, const double* x, int n, double* loglike, qlp_r
         if (k < live.size() && live[k] == i) {
             r = res[k++];
             if (r.status == QLP_ERR_ARG) ll = 1e30;            // a lens the model rejects: update_model's penalty
+            else if (r.status == QLP_ERR_TIMEOUT) timed_out = true;       // its numbers mean nothing
             else ll = fit_prior_jacobian(c->fit, x + (size_t)i * nf, &t[(size_t)i * nf], r.m2logev / 2);
         }
         if (out) out[i] = r;
         loglike[i] = ll;
     }
-    return QLP_OK;
+    if (timed_out) set_error("%s (%d)", "a device wait ran out in a fit vector's evaluation", QLP_ERR_TIMEOUT);
+    return timed_out ? QLP_ERR_TIMEOUT : QLP_OK;
 }
 
 int fit_terms(const qlp_fit_param* fp, int n, const double* x, double* t, int* penalised, double* terms)
