@@ -672,7 +672,7 @@ static int regopt_wave(qlp_ctx* c, const std::vector<int>& inst, const std::vect
     }
     std::vector<BrentMin> br(k);
     std::vector<double> best(k, INFINITY);
-    std::vector<char> act(k), timed_out(k, 0);
+    std::vector<char> act(k), have(k, 0), timed_out(k, 0);
     for (int j = 0; j < k; j++) br[j].reset(c->regopt_minlog, c->regopt_maxlog, c->regopt_tol, c->regopt_maxit);
     while (true) {
         bool any = false;
@@ -693,8 +693,9 @@ static int regopt_wave(qlp_ctx* c, const std::vector<int>& inst, const std::vect
             if (!act[j]) continue;
             const double f = c->h_trial[j].f_regopt;
             timed_out[j] |= c->h_trial[j].status == QLP_ERR_TIMEOUT;
-            if (f < best[j]) {
-                best[j] = f;
+            if (f < best[j] || !have[j]) {            // (the first one stands if none has a finite objective)
+                if (f < best[j]) best[j] = f;
+                have[j] = 1;
                 c->h_out[inst[j]] = c->h_trial[j];
                 c->regopt_lam[inst[j]] = c->h_ep[inst[j]].regparam;
             }
