@@ -181,6 +181,27 @@ static int ensure_slot(qlp_ctx* c, int k, int n_mask, int cells, int snx, int sn
                       std::max(sny, s.sny_cap));
 }
 
+// Whether the plain path's L' is summed in fixed point.  Half a unit of the taps and of L
+// has to stay within 2^-51 of the largest tap and L: the sum of a few such errors is then
+// within an FP64 sum's rounding of the cell's largest entries, which F and its factor
+// are relative to.  With a noise map that is L' sqrt(C^-1): an entry that is small for its
+// tap may be the largest by its weight, so the range of sqrt(C^-1) goes off.  pixels: those
+// that any evaluation may use.
+static int psf_fixed_rule(const qlp_ctx* c, const std::vector<int>* lists, int n_lists)
+{
+    if (c->psf_bits < 51) return 0;
+    double lo = INFINITY, hi = 0;
+    for (int k = 0; k < n_lists && c->sd.use_noise_map; k++)
+        for (int p : lists[k]) {
+            const double v = c->covinv[p];
+            if (!(v > 0 && std::isfinite(v))) continue;
+            lo = std::min(lo, v);
+            hi = std::max(hi, v);
+        }
+    const double range = lo < hi ? 0.5 * (log2(hi) - log2(lo)) : 0;
+    return std::min(c->psf_bits, 57) - range >= 51;
+}
+
 int ctx_init(qlp_ctx* c, const qlp_image* im, const qlp_psf* psf, const qlp_srcgrid_opts* opts)
 {
     c->nx = im->npixels_x;
@@ -250,16 +271,14 @@ int ctx_init(qlp_ctx* c, const qlp_image* im, const qlp_psf* psf, const qlp_srcg
             taps += psf->matrix[t] != 0;
         }
         std::vector<int2> pf((size_t)pnx * pny, make_int2(0, 0));
-        sd.psf_fixed = 0;
+        c->psf_bits = 0;
         if (std::isfinite(psum) && psum > 0) {
             frexp(tmax, &emax);
             frexp(psum, &esum);
             sd.psf_t = std::min(30 - emax, 33 - esum);
             sd.psf_w = std::max(4, std::min(30, (int)floor(34.85 - log2((double)taps))));
-            // half a unit within 2^-51 of the largest tap: the sum of a few such
-            // errors stays within an FP64 sum's rounding
-            sd.psf_fixed = log2(tmax) + sd.psf_t + sd.psf_w + 1 >= 51;
-            for (int pl = 0; pl < pny && sd.psf_fixed; pl++)
+            c->psf_bits = std::max(0, (int)floor(log2(tmax) + sd.psf_t + sd.psf_w + 1));
+            for (int pl = 0; pl < pny && c->psf_bits >= 51; pl++)
                 for (int pk = 0; pk < pnx; pk++) {
                     const long long q = llrint(ldexp(psf->matrix[(size_t)pk * pny + pl], sd.psf_t + sd.psf_w));
                     int2& f = pf[(size_t)pl * pnx + pk];
@@ -270,6 +289,8 @@ int ctx_init(qlp_ctx* c, const qlp_image* im, const qlp_psf* psf, const qlp_srcg
         CK(dalloc(&c->d_psf_fine, pf.size()), "alloc");
         CK(cudaMemcpy(c->d_psf_fine, pf.data(), sizeof(int2) * pf.size(), cudaMemcpyHostToDevice), "h2d");
         sd.psf_fine = c->d_psf_fine;
+        if (noise_map) c->covinv = covinv;
+        sd.psf_fixed = psf_fixed_rule(c, &c->mpix, 1);
     }
 
     SrcOpts& so = c->so;
@@ -789,7 +810,11 @@ int ctx_set_masks(qlp_ctx* c, const unsigned char* masks, int n_masks)
         c->mask_cnt.push_back((int)v.size());
         all.insert(all.end(), v.begin(), v.end());
     }
-    // captured graphs stay valid: the mask pointers travel in EvalParams
+    // captured graphs stay valid (the mask pointers travel in EvalParams), but for how L' is summed
+    const std::vector<int> lists[2] = {c->mpix, all};
+    const int fixed = psf_fixed_rule(c, lists, 2);
+    if (fixed != c->sd.psf_fixed) c->graph_gen++;
+    c->sd.psf_fixed = fixed;
     if (c->d_inst_mpix) { cudaFree(c->d_inst_mpix); c->d_inst_mpix = nullptr; }
     CK(dalloc(&c->d_inst_mpix, all.size()), "alloc");
     if (!all.empty())

@@ -187,7 +187,7 @@ __device__ __forceinline__ void csc_store(const Csc& o, int k, int row, double v
 {
     const int pix = rowpix[row], i = pix / ny, j = pix - i * ny;
     if (o.fine) {
-        o.fine[k] = psf64_entry(i, j, v);
+        o.fine[k] = o.raw ? psf64_raw(i, j, v) : psf64_entry(i, j, v);
         return;
     }
     o.colrow[k] = row;

@@ -8,8 +8,9 @@
 // L on the grid 2^-57, the taps to 2^-51 or better of the largest (2^-57 for a
 // Gaussian of 21 x 21), by halves; of a product (th 2^w + tl) (vh 2^29 + vl) only
 // tl vl is left out, below 2^-59 of the largest tap where that is an eighth of their
-// sum.  An FP64 sum rounds at 2^-53 of each product and partial sum.  Other PSFs are
-// summed in FP64.
+// sum.  An FP64 sum rounds at 2^-53 of each product and partial sum.  Other PSFs, and
+// noise maps that weight small entries up past those bounds, are summed in FP64
+// (psf_fixed_rule, ctx.cpp).
 #include "qlpix_ctx.h"
 #include "psf_tiles.cuh"
 
@@ -59,7 +60,7 @@ __device__ __forceinline__ int exponent_of(double x)
 // up to 4,096 cells, 121 taps: 14.2 -> 10.4 ms.  In FP64 these sums alone would take
 // the pipe 250 us.
 // FIXED = false (StaticData::psf_fixed, or bordered taps past PSF64_PAD_BYTES): FP64
-// sums, taps by their bounds from global memory.
+// sums of the FP64 entries, taps by their bounds from global memory.
 #define PSF64_PAD_BYTES (200 * 1024)
 template <bool FIXED>
 __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* __restrict__ gs,
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* _
                 vl = en.z;
             }
             unsigned hit = __ballot_sync(0xffffffffu, dx > -32 && dx < pnx && dy > -R && dy < pny);
-            const unsigned nan = __ballot_sync(0xffffffffu, vh == PSF64_BAD);
+            const unsigned nan = __ballot_sync(0xffffffffu, FIXED && vh == PSF64_BAD);
             for (; hit; hit &= hit - 1) {
                 const int f = __ffs(hit) - 1;
                 const int ox = __shfl_sync(0xffffffffu, dx, f) + lane, oy = __shfl_sync(0xffffffffu, dy, f);
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* _
                         lh[r] += (long long)t.y * eh;
                     }
                 } else if (ox >= 0 && ox < pnx) {
-                    const double v = ((double)eh * 0x1p29 + (double)el) * 0x1p-57;
+                    const double v = __hiloint2double(el, eh);
                     #pragma unroll
                     for (int r = 0; r < R; r++)
                         if (oy + r >= 0 && oy + r < pny) acc[r] = fma(sd.psf[ox * pny + oy + r], v, acc[r]);
@@ -204,9 +205,10 @@ int psf_in_range(const StaticData& sd, int M_max)
 void launch_psf(const StaticData& sd, Work& w, int N_max, cudaStream_t st)
 {
     if (N_max == 0) return;
-    launch_csc(sd, w, w.csc, N_max, w.Lpsf, w.ldL, st);
     const size_t taps = sizeof(int2) * psfx_taps(sd.pnx, sd.pny);
     const bool fixed = sd.psf_fixed && taps <= PSF64_PAD_BYTES;
+    w.csc.raw = fixed ? 0 : 1;
+    launch_csc(sd, w, w.csc, N_max, w.Lpsf, w.ldL, st);
     auto k = fixed ? k_psf64<true> : k_psf64<false>;
     k<<<152 * 3, 256, fixed ? taps : 0, st>>>(sd, w.gs, w.csc.colcnt, w.csc.fine, w.csc.pixT, (sd.nx + 31) / 32,
                                             w.csc.ntiles(), w.csc.tiles, w.Lpsf, w.ldL, sd.use_noise_map ? w.svec : nullptr,

@@ -27,6 +27,12 @@ __device__ __forceinline__ int4 psf64_entry(int i, int j, double v)
     return make_int4(i, (int)(q >> 29), (int)q & 0x1fffffff, j);
 }
 
+// ... and for FP64 sums, L's bits (low, high).
+__device__ __forceinline__ int4 psf64_raw(int i, int j, double v)
+{
+    return make_int4(i, __double2loint(v), __double2hiint(v), j);
+}
+
 __device__ __forceinline__ int ent_col(int2 e) { return e.x >> 16; }
 __device__ __forceinline__ int ent_row(int2 e) { return e.x & 0xffff; }
 __device__ __forceinline__ int ent_col(int4 e) { return e.x; }

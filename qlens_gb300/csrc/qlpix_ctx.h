@@ -86,6 +86,8 @@ struct qlp_ctx {
     double* d_covinv = nullptr;
     double* d_psf = nullptr;
     int2* d_psf_fine = nullptr;    // the plain path's (StaticData::psf_fine)
+    int psf_bits = 0;              // half a unit of its taps is at most 2^-psf_bits of the largest (0: not fixed)
+    std::vector<double> covinv;    // noise map: C^-1 per pixel
     int* d_psf_int = nullptr;      // the PSF on the PSF-to-X fixed-point grid (StaticData::psf_int)
     int* d_mpix = nullptr;
 

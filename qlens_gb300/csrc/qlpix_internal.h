@@ -131,7 +131,7 @@ struct StaticData {            // per-context, uploaded once
     // widest for which a sum of lo times |L| <= 2 (2^29 on its grid) stays within 64 bits
     const int2* psf_fine;
     int psf_t, psf_w;
-    int psf_fixed;             // 0: the taps are summed in FP64 instead (not finite, or below 2^-51 of the largest)
+    int psf_fixed;             // 0: L and the taps are summed in FP64 instead (psf_fixed_rule, ctx.cpp)
     // F16 operands of the mixed path's SYRK: X scaled by 2^x_exp puts its
     // largest possible entry (4 sum|psf| max sqrt(C^-1)) at or below 2^14
     int x_exp;
@@ -182,6 +182,7 @@ struct Csc {
     int* colrow;               // rows, ascending within a column
     int2* ent;                 // (image column << 16 | image row, L on the grid 2^-PSFX_LEXP)
     int4* fine;                // the plain path's entries (psf64_entry), in place of colrow, ent and colval64
+    int raw;                   // these hold L's FP64 bits (psf64_raw), for FP64 sums
     double* colval64;          // FP64 values
     int* col_u;                // rows of each column in atomic (fill) order
     int* src_u;                // their positions in the merged CSR rows
