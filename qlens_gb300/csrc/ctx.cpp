@@ -181,12 +181,12 @@ static int ensure_slot(qlp_ctx* c, int k, int n_mask, int cells, int snx, int sn
                       std::max(sny, s.sny_cap));
 }
 
-// Whether the plain path's L' is summed in fixed point.  Half a unit of the taps and of L
-// has to stay within 2^-51 of the largest tap and L: the sum of a few such errors is then
-// within an FP64 sum's rounding of the cell's largest entries, which F and its factor
-// are relative to.  With a noise map that is L' sqrt(C^-1): an entry that is small for its
-// tap may be the largest by its weight, so the range of sqrt(C^-1) goes off.  pixels: those
-// that any evaluation may use.
+// Whether the plain path's L' is summed in fixed point.  Half a unit of the taps has to
+// stay within 2^-51 of the largest tap, and half a unit of L (2^-58 of the cell's largest)
+// likewise: the sum of a few such errors is then within an FP64 sum's rounding of the cell's
+// largest entries, which F and its factor are relative to.  With a noise map those are of
+// L' sqrt(C^-1), where an entry that is small for its tap may be the largest by its weight,
+// so the range of sqrt(C^-1) goes off.  lists: the pixels that any evaluation may use.
 static int psf_fixed_rule(const qlp_ctx* c, const std::vector<int>* lists, int n_lists)
 {
     if (c->psf_bits < 51) return 0;
@@ -199,7 +199,7 @@ static int psf_fixed_rule(const qlp_ctx* c, const std::vector<int>* lists, int n
             hi = std::max(hi, v);
         }
     const double range = lo < hi ? 0.5 * (log2(hi) - log2(lo)) : 0;
-    return std::min(c->psf_bits, 57) - range >= 51;
+    return std::min(c->psf_bits, 58) - range >= 51;
 }
 
 int ctx_init(qlp_ctx* c, const qlp_image* im, const qlp_psf* psf, const qlp_srcgrid_opts* opts)

@@ -182,12 +182,13 @@ __global__ void k_csc_fill(const GridState* __restrict__ gs, const int* __restri
 
 // Entry k of the sorted columns: as the PSF-to-X build reads it (its pixel and L
 // on its grid) with its row and FP64 value, or (fine) as the plain path's build
-// of L' does.
-__device__ __forceinline__ void csc_store(const Csc& o, int k, int row, double v, const int* __restrict__ rowpix, int ny)
+// of L' does, on the cell's grid (shift).
+__device__ __forceinline__ void csc_store(const Csc& o, int k, int row, double v, const int* __restrict__ rowpix, int ny,
+                                          int shift)
 {
     const int pix = rowpix[row], i = pix / ny, j = pix - i * ny;
     if (o.fine) {
-        o.fine[k] = o.raw ? psf64_raw(i, j, v) : psf64_entry(i, j, v);
+        o.fine[k] = o.raw ? psf64_raw(i, j, v) : psf64_entry(i, j, v, shift);
         return;
     }
     o.colrow[k] = row;
@@ -219,7 +220,7 @@ __device__ __forceinline__ void csc_bitonic_step(int& key, int& pos, int e, int 
 template <int R>
 __device__ __forceinline__ void csc_sort_warp(const int* __restrict__ col_u, const int* __restrict__ src_u,
                                               const double* __restrict__ cval, int b, int n, int lane,
-                                              const Csc& out, const int* __restrict__ rowpix, int ny)
+                                              const Csc& out, const int* __restrict__ rowpix, int ny, int s)
 {
     int key[R], pos[R];
     #pragma unroll
@@ -227,6 +228,15 @@ __device__ __forceinline__ void csc_sort_warp(const int* __restrict__ col_u, con
         const int e = lane + 32 * h;
         key[h] = (e < n) ? col_u[b + e] : INT_MAX;
         pos[h] = (e < n) ? src_u[b + e] : 0;
+    }
+    int shift = 0;
+    if (out.fine) {
+        int top = 0;
+        #pragma unroll
+        for (int h = 0; h < R; h++)
+            if (lane + 32 * h < n) top = max(top, psf64_top(cval[pos[h]]));
+        shift = psf64_shift(__reduce_max_sync(0xffffffffu, top));
+        if (lane == 0) out.shift[s] = shift;
     }
     #pragma unroll
     for (int k = 2; k <= 32 * R; k <<= 1) {
@@ -253,7 +263,7 @@ __device__ __forceinline__ void csc_sort_warp(const int* __restrict__ col_u, con
     #pragma unroll
     for (int h = 0; h < R; h++) {
         const int e = lane + 32 * h;
-        if (e < n) csc_store(out, b + e, key[h], cval[pos[h]], rowpix, ny);
+        if (e < n) csc_store(out, b + e, key[h], cval[pos[h]], rowpix, ny, shift);
     }
 }
 
@@ -268,6 +278,7 @@ __global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ 
     __shared__ unsigned bits[CSC_WORDS];
     __shared__ int below[CSC_WORDS];
     __shared__ int wsum[8];
+    __shared__ int top;
     const int s = blockIdx.x;
     if (s >= gs->M) return;
     const int N = gs->N, b = colptr[s], n = colptr[s + 1] - b;
@@ -277,12 +288,24 @@ __global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ 
     }
     if (n <= CSC_SORT_WARP) {
         if (clear && threadIdx.x < 32) {
-            if (n <= 32) csc_sort_warp<1>(col_u, src_u, cval, b, n, threadIdx.x, out, rowpix, ny);
-            else csc_sort_warp<2>(col_u, src_u, cval, b, n, threadIdx.x, out, rowpix, ny);
+            if (n <= 32) csc_sort_warp<1>(col_u, src_u, cval, b, n, threadIdx.x, out, rowpix, ny, s);
+            else csc_sort_warp<2>(col_u, src_u, cval, b, n, threadIdx.x, out, rowpix, ny, s);
         }
         return;                                           // else k_csc_sort_w's
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int shift = 0;
+    if (out.fine) {
+        if (threadIdx.x == 0) top = 0;
+        __syncthreads();
+        int t = 0;
+        for (int i = threadIdx.x; i < n; i += 256) t = max(t, psf64_top(cval[src_u[b + i]]));
+        t = __reduce_max_sync(0xffffffffu, t);
+        if (lane == 0) atomicMax(&top, t);
+        __syncthreads();
+        shift = psf64_shift(top);
+        if (threadIdx.x == 0) out.shift[s] = shift;
+    }
     int placed = 0;                                       // entries of the passes before
     for (int r0 = 0; r0 < N; r0 += 32 * CSC_WORDS) {
         const int words = min(CSC_WORDS, (N - r0 + 31) / 32);
@@ -322,7 +345,7 @@ __global__ void __launch_bounds__(256) k_csc_sort(const GridState* __restrict__ 
             const unsigned r = (unsigned)(row - r0);
             if (r < 32u * words)
                 csc_store(out, b + below[r >> 5] + __popc(bits[r >> 5] & ((1u << (r & 31)) - 1)), row,
-                          cval[src_u[b + i]], rowpix, ny);
+                          cval[src_u[b + i]], rowpix, ny, shift);
         }
         placed += total;
         __syncthreads();
@@ -339,8 +362,8 @@ __global__ void __launch_bounds__(256, 4) k_csc_sort_w(const GridState* __restri
     const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= gs->M) return;                                // whole warps
     const int b = colptr[s], n = colptr[s + 1] - b;
-    if (n <= 32) csc_sort_warp<1>(col_u, src_u, cval, b, n, lane, out, rowpix, ny);
-    else if (n <= CSC_SORT_WARP) csc_sort_warp<2>(col_u, src_u, cval, b, n, lane, out, rowpix, ny);
+    if (n <= 32) csc_sort_warp<1>(col_u, src_u, cval, b, n, lane, out, rowpix, ny, s);
+    else if (n <= CSC_SORT_WARP) csc_sort_warp<2>(col_u, src_u, cval, b, n, lane, out, rowpix, ny, s);
 }
 
 // out[s] = sum over column s of L of value * w[row]: one warp per column, lane
@@ -643,6 +666,7 @@ void csc_layout(Csc& o, const Slot& c, int M_cap, bool fine, Arena& ar)
     ar.add(&o.pixT, c.npix_pad);
     if (fine) {
         ar.add(&o.fine, nnz);
+        ar.add(&o.shift, M_cap);
     } else {
         ar.add(&o.colrow, nnz);
         ar.add(&o.ent, nnz);

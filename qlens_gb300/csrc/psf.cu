@@ -5,7 +5,7 @@
 //   L'[p][s] = sum over PSF taps (k-major, then l) of psf[k][l] * Ldense[q][s],
 //   q = the active pixel at (i_p + nx/2 - k, j_p + ny/2 - l).
 // The sums are exact in 64-bit fixed point (psf_tiles.cuh, StaticData::psf_fine):
-// L on the grid 2^-57, the taps to 2^-51 or better of the largest (2^-57 for a
+// L to 2^-57 of the power of two below the cell's largest, the taps to 2^-51 or better of the largest (2^-57 for a
 // Gaussian of 21 x 21), by halves; of a product (th 2^w + tl) (vh 2^29 + vl) only
 // tl vl is left out, below 2^-59 of the largest tap where that is an eighth of their
 // sum.  An FP64 sum rounds at 2^-53 of each product and partial sum.  Other PSFs, and
@@ -40,12 +40,6 @@ __device__ __forceinline__ double fixed_to_double(long long s, int k)
     return __longlong_as_double((long long)(b | (s < 0 ? 1ull << 63 : 0)));
 }
 
-__device__ __forceinline__ int exponent_of(double x)
-{
-    const unsigned long long u = (unsigned long long)__double_as_longlong(x) << 1;
-    return u == 0 ? 0 : max(1, (int)(u >> 53));
-}
-
 // L' by image tiles, as k_psf_x builds X: a warp takes a listed (cell, 32 x 8
 // pixels) pair, lane x keeps its column's sums and adds tap x L for every entry
 // whose footprint meets the tile, three wide multiply-adds and a 64-bit load from
@@ -65,7 +59,7 @@ __device__ __forceinline__ int exponent_of(double x)
 template <bool FIXED>
 __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* __restrict__ gs,
                                                const int* __restrict__ colptr, const int4* __restrict__ ent_g,
-                                               const int2* __restrict__ pixT, int ntx, const int* __restrict__ count,
+                                               const int* __restrict__ shift, const int2* __restrict__ pixT, int ntx, const int* __restrict__ count,
                                                const uint2* __restrict__ list, double* __restrict__ L, int ldL,
                                                const double* __restrict__ svec, int* __restrict__ emax,
                                                unsigned char* __restrict__ nz, int nst)
@@ -148,7 +142,7 @@ __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* _
                     // as many of the lower halves' bits as there is room for
                     const int sh = max(0, min(min(20, sd.psf_w), __clzll(hh[r] < 0 ? -hh[r] : hh[r]) - 3));
                     v = fixed_to_double((hh[r] << sh) + (hl[r] >> (29 - sh)) + (lh[r] >> (sd.psf_w - sh)),
-                                        sd.psf_t + 28 + sh);
+                                        sd.psf_t + 28 + sh + shift[s]);
                 }
                 if (bad >> r & 1) v = __longlong_as_double(0x7ff8000000000000ll);
                 const int e = exponent_of(v);
@@ -210,7 +204,8 @@ void launch_psf(const StaticData& sd, Work& w, int N_max, cudaStream_t st)
     w.csc.raw = fixed ? 0 : 1;
     launch_csc(sd, w, w.csc, N_max, w.Lpsf, w.ldL, st);
     auto k = fixed ? k_psf64<true> : k_psf64<false>;
-    k<<<152 * 3, 256, fixed ? taps : 0, st>>>(sd, w.gs, w.csc.colcnt, w.csc.fine, w.csc.pixT, (sd.nx + 31) / 32,
+    k<<<152 * 3, 256, fixed ? taps : 0, st>>>(sd, w.gs, w.csc.colcnt, w.csc.fine, w.csc.shift, w.csc.pixT,
+                                            (sd.nx + 31) / 32,
                                             w.csc.ntiles(), w.csc.tiles, w.Lpsf, w.ldL, sd.use_noise_map ? w.svec : nullptr,
                                             oz_emax(w.oz), oz_nz(w.oz), oz_nst(w.oz));
     count_launches(1);

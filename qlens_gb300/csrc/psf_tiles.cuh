@@ -11,17 +11,34 @@ namespace qlpix {
 __host__ __device__ __forceinline__ int psfx_pitch(int pny) { return (pny + 2 * PSFX_R - 2) | 1; }
 static inline size_t psfx_taps(int pnx, int pny) { return (size_t)(pnx + 62) * psfx_pitch(pny); }
 
-// An entry of the plain path's columns: (image column, hi, lo, image row), L on the
-// grid 2^-57 = hi 2^29 + lo (0 <= lo < 2^29).  |L| <= 2 (a sub-pixel's barycentric weight at the
-// corner of the source grid); anything else, a NaN too, is marked by INT_MIN.
+// The biased exponent of |x| (at least 1), 0 for zero, 2047 for infinities and NaN.
+__device__ __forceinline__ int exponent_of(double x)
+{
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x) << 1;
+    return u == 0 ? 0 : max(1, (int)(u >> 53));
+}
+
+// The grid of a cell whose largest finite L has this biased exponent: that L times 2^shift
+// lies in [1, 2) (a cell that sub-pixels only touch has none but small entries).
+__device__ __forceinline__ int psf64_shift(int top) { return top ? 1023 - top : 0; }
+// ... an entry's part in it
+__device__ __forceinline__ int psf64_top(double v)
+{
+    const int e = exponent_of(v);
+    return e == 2047 ? 0 : e;
+}
+
+// An entry of the plain path's columns: (image column, hi, lo, image row), L on the cell's
+// grid 2^-(57 + shift) = hi 2^29 + lo (0 <= lo < 2^29, |hi| <= 2^29); infinities and NaN are
+// marked by INT_MIN.
 #define PSF64_BAD ((int)0x80000000)
-__device__ __forceinline__ int4 psf64_entry(int i, int j, double v)
+__device__ __forceinline__ int4 psf64_entry(int i, int j, double v, int shift)
 {
     const long long b = __double_as_longlong(v);
     const int e = (int)((b >> 52) & 0x7ff);
-    if (e > 1023 + 1 || (e == 1023 + 1 && (b & 0xfffffffffffffll) > (1ll << 47))) return make_int4(i, PSF64_BAD, 0, j);
+    if (e == 2047) return make_int4(i, PSF64_BAD, 0, j);
     const long long m = (b & 0xfffffffffffffll) | (e ? 1ll << 52 : 0);
-    const int s = max(e, 1) - 1075 + 57;            // m 2^s, s <= 6
+    const int s = max(e, 1) - 1075 + 57 + shift;    // m 2^s, s <= 5
     const long long a = s >= 0 ? m << s : (s > -55 ? (m + (1ll << (-s - 1))) >> -s : 0);
     const long long q = b < 0 ? -a : a;
     return make_int4(i, (int)(q >> 29), (int)q & 0x1fffffff, j);

@@ -182,6 +182,7 @@ struct Csc {
     int* colrow;               // rows, ascending within a column
     int2* ent;                 // (image column << 16 | image row, L on the grid 2^-PSFX_LEXP)
     int4* fine;                // the plain path's entries (psf64_entry), in place of colrow, ent and colval64
+    int* shift;                // ... each cell's grid 2^-(57 + shift) for L
     int raw;                   // these hold L's FP64 bits (psf64_raw), for FP64 sums
     double* colval64;          // FP64 values
     int* col_u;                // rows of each column in atomic (fill) order
