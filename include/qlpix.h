@@ -197,7 +197,10 @@ int qlp_eval(qlp_ctx* ctx, const double* lens_params, double regparam, qlp_resul
  * each on its own stream with its own workspace (default 16, at most 64).
  * More slots hide the sequential parts of each evaluation behind the others
  * at the cost of one workspace per slot (about 0.5 GB for a 200x200 image,
- * 4x4 split and a 64x64 source grid in QLP_MIXED). */
+ * 4x4 split and a 64x64 source grid in QLP_MIXED).  QLP_FP64 takes for N pixels
+ * and M cells 8 N M bytes of L', 16 M^2 of F and R, 8 M^2 of integer sums and
+ * the digits of L' and F's factor, up to 1 GB or 16 M^2 (N = 42,000, M = 4,096:
+ * about 3 GB).  A batch takes as many slots as the device's memory holds. */
 int qlp_set_batch_slots(qlp_ctx* ctx, int slots);
 
 /* on = 1 (default): qlp_eval_batch captures each slot's launch sequence once

@@ -348,7 +348,8 @@ __device__ __forceinline__ bool c2_wait_flag(const int* p, GridState* gs, volati
     return true;
 }
 
-// The factorisation's arrays: the split factor Lh, Ll [rows][rows] with each
+// The factorisation's arrays: the split factor Lh, Ll [rows][128 wb], block column k at k
+// mod wb (all of them, or of a band's rows the band + 1 that are still read), with each
 // column block's row scales pexp[block][rows], the split inverses [rows][128]
 // and the flags: ready[column][row block], inverse[column], tile counter.
 struct Flow128Mem {
@@ -358,7 +359,7 @@ struct Flow128Mem {
     float* ih;
     float* il;
     int* flags;
-    int rows;                                             // M_cap, a multiple of 128
+    int rows, wb;                                         // M_cap, a multiple of 128
 };
 
 __global__ void __launch_bounds__(C2_THREADS, 1) k_chol128(const __grid_constant__ CUtensorMap map_hi,
@@ -434,7 +435,7 @@ __global__ void __launch_bounds__(C2_THREADS, 1) k_chol128(const __grid_constant
                     bulk_load(exps[b][1], pe + j * C2, C2 * 4, &f.exp_full[b]);
                     f.n_exp = kc + 1;
                     for (int half = 0; half < 2 && ok; half++) {
-                        const int it = it0 + 2 * (k - k0) + half, s = it % C2_STAGES, x = k * C2 + half * 64;
+                        const int it = it0 + 2 * (k - k0) + half, s = it % C2_STAGES, x = (k % mem.wb) * C2 + half * 64;
                         if (it >= C2_STAGES)
                             ok = mbar_wait_bounded(&f.empty[s], ((it / C2_STAGES) & 1) ^ 1, &f.abort);
                         if (!ok) break;
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__(C2_THREADS, 1) k_chol128(const __grid_constant
                 const int sc = (mx > 0.f) ? max(-60, min(60, 14 - e)) : 0;
                 if (h == 0) mem.pexp[(size_t)j * mem.rows + row] = sc;
                 const float scf = __int_as_float((127 + sc) << 23);
-                const size_t at16 = (size_t)row * mem.rows + j * C2 + 64 * h;
+                const size_t at16 = (size_t)row * mem.wb * C2 + (j % mem.wb) * C2 + 64 * h;
                 #pragma unroll
                 for (int c = 0; c < 64; c += 8) {
                     uint32_t hw[4], lw[4];

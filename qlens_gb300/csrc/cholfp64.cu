@@ -52,7 +52,7 @@ namespace qlpix {
 #define C64_POISON (1 << 20)       // exponent of a row that holds no finite number: its pivot becomes NaN
 
 struct Chol64Work {
-    __half* ls = nullptr;          // [CS][M128][M128] digits of the factor
+    __half* ls = nullptr;          // [CS][M128][64 wb] digits of the factor, block column k at k mod wb
     __half* li = nullptr;          // [CS][M128][64] digits of the diagonal blocks' inverses
     int* rexp = nullptr;           // [M128] E_i
     int* lexp = nullptr;           // [M128] exponents of the inverses' rows
@@ -60,7 +60,7 @@ struct Chol64Work {
     int* flags = nullptr;          // ready[nbc][nbc] (column, row block), inverse[nbc], tile counter,
                                    // two solves' [nbc] each, redo (a pivot <= 0), its tile counter
     double* diag = nullptr;        // F's: [M128] its diagonal, for k_chol64_plain
-    int M128 = 0, nbc = 0;
+    int M128 = 0, nbc = 0, wb = 0; // wb: block columns kept of a row (all; of a band the band + 2)
     bool own_ls = false;
     CUtensorMap ls_a, ls_b, li_b;
 };
@@ -322,7 +322,9 @@ __device__ __forceinline__ bool wait_flag(const int* p, GridState* gs, volatile 
 }
 
 // band: blocks below the diagonal that can be nonzero, even (a tile's second
-// 64 rows reach one further); dense: any number past the matrix.
+// 64 rows reach one further); dense: any number past the matrix.  Nothing reads a row's
+// block column k once its column k + band + 2 stands, so a band's digits turn round in
+// wb = band + 2 block columns (all of them were 0.27 GB a slot at 4,096 cells, now 17 MB).
 // linv: the inverses of the diagonal blocks in FP64 for the solves, or null.
 // redo, diag0 (F; R is positive definite by construction: null): the matrix is kept
 // above its diagonal and in diag0, and *redo set where a pivot is not positive, for
@@ -330,7 +332,7 @@ __device__ __forceinline__ bool wait_flag(const int* p, GridState* gs, volatile 
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant__ CUtensorMap ls_a,
                                                          const __grid_constant__ CUtensorMap ls_b,
                                                          const __grid_constant__ CUtensorMap li_b, GridState* gs,
-                                                         double* F, int ld, int which, int band, int M128, int nbc,
+                                                         double* F, int ld, int which, int band, int M128, int nbc, int wb,
                                                          __half* ls, __half* li, const int* rexp, int* lexp,
                                                          int* wexp, int* flags, double* linv, int* redo,
                                                          double* diag0)
@@ -392,7 +394,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
                     bool ok = true;
                     for (int half = 0; half < 2 && ok; half++) {
                         const int it = it0 + 2 * (k - k0) + half;
-                        ok = oz_load_stage<CS>(pipe, smem, it, &ls_a, &ls_b, M128, k * C64 + half * OZ_KS, rb * C64, j * C64);
+                        ok = oz_load_stage<CS>(pipe, smem, it, &ls_a, &ls_b, M128, (k % wb) * C64 + half * OZ_KS, rb * C64,
+                                               j * C64);
                         if (ok) pipe.n_issued = it + 1;
                     }
                     if (!ok) break;
@@ -548,7 +551,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
                         const long long x = s > 0 ? (long long)(V >> (s - 1)) : (long long)(V << (min(-s, 60) + 1));
                         hi[c] = min(max((x + 1) >> 1, -(1ll << oz_bits(CS))), 1ll << oz_bits(CS));
                     }
-                    __half* out = ls + (size_t)row * M128 + j * C64 + 32 * h;
+                    __half* out = ls + (size_t)row * wb * C64 + (j % wb) * C64 + 32 * h;
                     unsigned long long b[8];
                     #pragma unroll
                     for (int w = 0; w < 4; w++) {
@@ -556,7 +559,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_chol64(const __grid_constant_
                         for (int c = 0; c < 8; c++) b[c] = oz_bias<CS>(hi[8 * w + c]);
                         #pragma unroll
                         for (int d = 0; d < CS; d++)
-                            *reinterpret_cast<uint4*>(out + (size_t)d * M128 * M128 + 8 * w) = oz_digits8<CS>(b, d);
+                            *reinterpret_cast<uint4*>(out + (size_t)d * M128 * wb * C64 + 8 * w) = oz_digits8<CS>(b, d);
                     }
                 }
                 fence_async();
@@ -909,19 +912,24 @@ void chol64_free(Chol64Work* z)
 
 static size_t chol64_flags(const Chol64Work* z) { return (size_t)z->nbc * z->nbc + 3 * z->nbc + 3; }
 
+// Blocks that a band of half_width entries can reach, rounded up to even.
+static int chol64_band(int half_width, int M) { return ((std::min(half_width, M) + C64 - 1) / C64 + 1) & ~1; }
+
 // shared: M128 x M128 digits that nothing else uses while this matrix is
-// factored (F: the digits of L', read by then), or null to allocate them (R).
-int chol64_alloc(Chol64Work** out, int M_cap, void* shared)
+// factored (F: the digits of L', read by then), or null to allocate them (R: for
+// bands of up to half_width entries).
+int chol64_alloc(Chol64Work** out, int M_cap, void* shared, int half_width)
 {
     Chol64Work* z = new Chol64Work();
     z->M128 = (M_cap + OZ_TM - 1) / OZ_TM * OZ_TM;
     z->nbc = z->M128 / C64;
     z->own_ls = shared == nullptr;
+    z->wb = z->own_ls ? std::min(z->nbc, chol64_band(half_width, M_cap) + 2) : z->nbc;
     z->ls = reinterpret_cast<__half*>(shared);
     cudaError_t e = cudaSuccess;
     auto A = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes); };
     const size_t rows = (size_t)CS * z->M128;
-    if (z->own_ls) A((void**)&z->ls, rows * z->M128 * sizeof(__half));
+    if (z->own_ls) A((void**)&z->ls, rows * z->wb * C64 * sizeof(__half));
     A((void**)&z->li, rows * C64 * sizeof(__half));
     A((void**)&z->rexp, sizeof(int) * z->M128);
     A((void**)&z->lexp, sizeof(int) * z->M128);
@@ -936,8 +944,8 @@ int chol64_alloc(Chol64Work** out, int M_cap, void* shared)
         cudaGetLastError();
         set_error("%s (%d)", "FP64 factorisation workspace", (int)e);
         rc = (e == cudaErrorMemoryAllocation) ? QLP_ERR_NOMEM : QLP_ERR_CUDA;
-    } else if (make_map_box(&z->ls_a, z->ls, rows, z->M128, true, OZ_TM, OZ_KS) != QLP_OK ||
-               make_map_box(&z->ls_b, z->ls, rows, z->M128, true, OZ_TN, OZ_KS) != QLP_OK ||
+    } else if (make_map_box(&z->ls_a, z->ls, rows, z->wb * C64, true, OZ_TM, OZ_KS) != QLP_OK ||
+               make_map_box(&z->ls_b, z->ls, rows, z->wb * C64, true, OZ_TN, OZ_KS) != QLP_OK ||
                make_map_box(&z->li_b, z->li, rows, C64, true, OZ_TN, OZ_KS) != QLP_OK) {
         set_error("%s (%d)", "cuTensorMapEncodeTiled unavailable or failed", 0);
         rc = QLP_ERR_CUDA;
@@ -959,13 +967,12 @@ void launch_cholesky_fp64(double* A, int ld, int M_max, GridState* gs, int which
                           Chol64Work* z, double* linv, cudaStream_t st)
 {
     const int nb = (M_max + C64 - 1) / C64;
-    // blocks that a band of half_width entries can reach, rounded up to even
-    const int band = ((std::min(half_width, M_max) + C64 - 1) / C64 + 1) & ~1;
+    const int band = chol64_band(half_width, M_max);
     const int tiles = nb * std::min((nb + 1) / 2, band / 2 + 1);
     k_chol64_prep<<<(M_max + 255) / 256, 256, 0, st>>>(gs, A, ld, z->rexp);
     int* redo = z->diag ? z->flags + chol64_flags(z) - 2 : nullptr;
     k_chol64<<<std::max(1, std::min(tiles, ctas)), OZ_THREADS, oz_smem(CS), st>>>(
-        z->ls_a, z->ls_b, z->li_b, gs, A, ld, which, band, z->M128, z->nbc, z->ls, z->li, z->rexp, z->lexp, z->wexp,
+        z->ls_a, z->ls_b, z->li_b, gs, A, ld, which, band, z->M128, z->nbc, z->wb, z->ls, z->li, z->rexp, z->lexp, z->wexp,
         z->flags, linv, redo, z->diag);
     count_launches(2);
     if (!redo) return;

@@ -142,11 +142,11 @@ static int ensure_fp64_mats(Slot& s)
         if (r != QLP_OK) return r;
     }
     if (!s.w.cholF) {
-        const int r = chol64_alloc(&s.w.cholF, s.M_cap, oz_buffer(s.w.oz));
+        const int r = chol64_alloc(&s.w.cholF, s.M_cap, oz_buffer(s.w.oz), s.M_cap);
         if (r != QLP_OK) return r;
     }
     if (!s.w.cholR) {
-        const int r = chol64_alloc(&s.w.cholR, s.M_cap, nullptr);
+        const int r = chol64_alloc(&s.w.cholR, s.M_cap, nullptr, 2 * s.snx_cap);
         if (r != QLP_OK) return r;
     }
     if (!s.w.F) CK(dalloc(&s.w.F, (size_t)s.M_cap * s.M_cap), "alloc F");

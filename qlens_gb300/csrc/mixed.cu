@@ -706,12 +706,15 @@ void launch_csc(const StaticData& sd, const Work& w, const Csc& o, int N_cap, do
     count_launches(clear ? 5 : 6);
 }
 
+// R couples a cell to cells at most two grid rows (2 snx active indices) away.
+static int band128_R(int snx) { return (2 * snx - 1) / C2 + 1; }
+
 static size_t flow128_flags(int nb) { return (size_t)nb * nb + nb + 1; }
 
 static int flow_maps(const Flow128Mem& f, CUtensorMap* maps)
 {
     for (int k = 0; k < 2; k++) {
-        int r = make_map(&maps[k], k ? f.Ll : f.Lh, f.rows, f.rows, true);
+        int r = make_map(&maps[k], k ? f.Ll : f.Lh, f.rows, f.wb * C2, true);
         if (r == QLP_OK) r = make_map(&maps[2 + k], k ? f.il : f.ih, f.rows, C2, false);
         if (r != QLP_OK) return r;
     }
@@ -754,8 +757,9 @@ int mixed_init(Slot& c)
     A((void**)&m->flags, sizeof(int) * (size_t)2 * m->nb * MIXED_SOLVES);
     for (Flow128Mem* f : {&m->cf, &m->cr}) {
         f->rows = M_cap;
-        A((void**)&f->Lh, sizeof(__half) * (size_t)M_cap * M_cap);
-        A((void**)&f->Ll, sizeof(__half) * (size_t)M_cap * M_cap);
+        f->wb = f == &m->cr ? std::min(m->nb, band128_R(c.snx_cap) + 1) : m->nb;
+        A((void**)&f->Lh, sizeof(__half) * (size_t)M_cap * f->wb * C2);
+        A((void**)&f->Ll, sizeof(__half) * (size_t)M_cap * f->wb * C2);
         A((void**)&f->pexp, sizeof(int) * (size_t)m->nb * M_cap);
         A((void**)&f->ih, sizeof(float) * (size_t)M_cap * C2);
         A((void**)&f->il, sizeof(float) * (size_t)M_cap * C2);
@@ -880,10 +884,9 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
 
     if (so.regularization) {
         // R hangs on the active cells alone: its factorisation (log det R only)
-        // runs on the slot's second stream beside everything up to the evidence.
-        // R couples a cell to cells at most two grid rows (2 snx active indices)
-        // away, so its factor stays within that band.
-        const int band_R = (2 * so.snx - 1) / C2 + 1;
+        // runs on the slot's second stream beside everything up to the evidence,
+        // within R's band.
+        const int band_R = band128_R(so.snx);
         cudaEventRecord(slot.side_fork, st);
         cudaStreamWaitEvent(slot.side, slot.side_fork, 0);
         launch_clear_band(m->R32, m->ld32, 4, m->M_cap, C2, band_R, w.gs, slot.side);

@@ -288,7 +288,7 @@ int oz_nst(const OzWork* z);
 void csc_free(Csc& o);
 void csc_clear(const Csc& o, ClearList& l);
 void launch_csc(const StaticData& sd, const Work& w, const Csc& o, int N_cap, double* clear, int ld, cudaStream_t st);
-int chol64_alloc(Chol64Work** out, int M_cap, void* shared);
+int chol64_alloc(Chol64Work** out, int M_cap, void* shared, int half_width);
 void chol64_free(Chol64Work* z);
 void chol64_clear(const Chol64Work* z, ClearList& l);
 // parts: REG_F adds lambda R to F, REG_R writes R (both: the plain evaluation)
