@@ -695,13 +695,14 @@ void launch_csc(const StaticData& sd, const Work& w, const Csc& o, int N_cap, do
     if (!clear)
         k_csc_sort_w<<<(o.M_cap + 7) / 8, 256, 0, st>>>(w.gs, o.colcnt, o.col_u, o.src_u, w.cval, o, w.rowpix, sd.ny);
     k_csc_sort<<<o.M_cap, 256, 0, st>>>(w.gs, o.colcnt, o.col_u, o.src_u, w.cval, o, w.rowpix, sd.ny, clear, ld);
-    const size_t wmark = sizeof(unsigned) * o.words;
+    const int span = std::min(o.words, 48 * 1024 / (int)sizeof(unsigned));
+    const size_t wmark = sizeof(unsigned) * span;
     const int tw = (int)std::max<size_t>(1, std::min<size_t>(8, 48 * 1024 / wmark));      // cells a CTA
     if (o.fine)
-        k_psfx_tiles<<<(o.M_cap + tw - 1) / tw, 32 * tw, wmark * tw, st>>>(sd, w.gs, o.colcnt, o.fine, ntx, o.words,
+        k_psfx_tiles<<<(o.M_cap + tw - 1) / tw, 32 * tw, wmark * tw, st>>>(sd, w.gs, o.colcnt, o.fine, ntx, o.words, span,
                                                                           o.tile_active, o.ntiles(), o.tiles);
     else
-        k_psfx_tiles<<<(o.M_cap + tw - 1) / tw, 32 * tw, wmark * tw, st>>>(sd, w.gs, o.colcnt, o.ent, ntx, o.words,
+        k_psfx_tiles<<<(o.M_cap + tw - 1) / tw, 32 * tw, wmark * tw, st>>>(sd, w.gs, o.colcnt, o.ent, ntx, o.words, span,
                                                                           o.tile_active, o.ntiles(), o.tiles);
     count_launches(clear ? 5 : 6);
 }

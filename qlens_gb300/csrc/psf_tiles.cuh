@@ -81,55 +81,61 @@ __device__ __forceinline__ int warp_lower_bound_row(const E* __restrict__ ent, i
 }
 
 // The tiles that each cell's footprints reach: a warp per cell, its bitmap of the
-// image's tiles in shared memory.
+// image's tiles in shared memory, span words at a time (one pass for images of up to
+// 100 million pixels, 48 KB).
 template <typename E>
 __global__ void k_psfx_tiles(StaticData sd, const GridState* __restrict__ gs, const int* __restrict__ colptr,
-                             const E* __restrict__ ent_g, int ntx, int nwords, const unsigned* __restrict__ active,
+                             const E* __restrict__ ent_g, int ntx, int nwords, int span,
+                             const unsigned* __restrict__ active,
                              int* __restrict__ count, uint2* __restrict__ list)
 {
     extern __shared__ unsigned mark_all[];
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, s = blockIdx.x * nw + (threadIdx.x >> 5);
     if (s >= gs->M) return;                                       // whole warps
-    unsigned* mark = mark_all + (threadIdx.x >> 5) * nwords;
+    unsigned* mark = mark_all + (threadIdx.x >> 5) * span;
     const int pnx = sd.pnx, pny = sd.pny, nxh = pnx / 2, nyh = pny / 2;
     const int n = colptr[s + 1] - colptr[s];
     const E* ent = ent_g + colptr[s];
-    for (int i = lane; i < nwords; i += 32) mark[i] = 0;
-    __syncwarp();
-    for (int e0 = 0; e0 < n; e0 += 32) {
-        const E en = ent[min(e0 + lane, n - 1)];
-        const int i0 = ent_col(en) - nxh, j0 = ent_row(en) - nyh;
-        const int c0 = max(i0, 0) >> 5, c1 = (min(i0 + pnx, sd.nx) - 1) >> 5;
-        const int t0 = max(j0, 0) / PSFX_R, t1 = (min(j0 + pny, sd.ny) - 1) / PSFX_R;
-        // neighbours along a row mostly reach the same tiles: only the first marks them
-        const int cc = c0 << 16 | c1, tt = t0 << 16 | t1;
-        const int pc = __shfl_up_sync(0xffffffffu, cc, 1), pt = __shfl_up_sync(0xffffffffu, tt, 1);
-        if (lane > 0 && pc == cc && pt == tt) continue;
-        for (int t = t0; t <= t1; t++) {
-            const int k0 = t * ntx + c0, k1 = t * ntx + c1;
-            for (int w = k0 >> 5; w <= k1 >> 5; w++) {
-                unsigned m = 0xffffffffu;
-                if (w == k0 >> 5) m &= 0xffffffffu << (k0 & 31);
-                if (w == k1 >> 5) m &= 0xffffffffu >> (31 - (k1 & 31));
-                if ((mark[w] & m) != m) atomicOr(&mark[w], m);
+    for (int b0 = 0; b0 < nwords; b0 += span) {
+        const int b1 = min(b0 + span, nwords);
+        for (int i = lane; i < b1 - b0; i += 32) mark[i] = 0;
+        __syncwarp();
+        for (int e0 = 0; e0 < n; e0 += 32) {
+            const E en = ent[min(e0 + lane, n - 1)];
+            const int i0 = ent_col(en) - nxh, j0 = ent_row(en) - nyh;
+            const int c0 = max(i0, 0) >> 5, c1 = (min(i0 + pnx, sd.nx) - 1) >> 5;
+            const int t0 = max(j0, 0) / PSFX_R, t1 = (min(j0 + pny, sd.ny) - 1) / PSFX_R;
+            // neighbours along a row mostly reach the same tiles: only the first marks them
+            const bool same = __shfl_up_sync(0xffffffffu, c0, 1) == c0 & __shfl_up_sync(0xffffffffu, c1, 1) == c1 &
+                              __shfl_up_sync(0xffffffffu, t0, 1) == t0 & __shfl_up_sync(0xffffffffu, t1, 1) == t1;
+            if (lane > 0 && same) continue;
+            for (int t = t0; t <= t1; t++) {
+                const int k0 = t * ntx + c0, k1 = t * ntx + c1;
+                for (int w = max(k0 >> 5, b0); w <= min(k1 >> 5, b1 - 1); w++) {
+                    unsigned m = 0xffffffffu;
+                    if (w == k0 >> 5) m &= 0xffffffffu << (k0 & 31);
+                    if (w == k1 >> 5) m &= 0xffffffffu >> (31 - (k1 & 31));
+                    if ((mark[w - b0] & m) != m) atomicOr(&mark[w - b0], m);
+                }
             }
         }
-    }
-    __syncwarp();
-    for (int w0 = 0; w0 < nwords; w0 += 32) {
-        const int wd = w0 + lane;
-        unsigned bits = wd < nwords ? mark[wd] & active[wd] : 0u;
-        int at = __popc(bits);
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, at, o);
-            if (lane >= o) at += v;
+        __syncwarp();
+        for (int w0 = b0; w0 < b1; w0 += 32) {
+            const int wd = w0 + lane;
+            unsigned bits = wd < b1 ? mark[wd - b0] & active[wd] : 0u;
+            int at = __popc(bits);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, at, o);
+                if (lane >= o) at += v;
+            }
+            const int total = __shfl_sync(0xffffffffu, at, 31);
+            if (total == 0) continue;
+            int base = 0;
+            if (lane == 0) base = atomicAdd(count, total);
+            at += __shfl_sync(0xffffffffu, base, 0) - __popc(bits);
+            for (; bits; bits &= bits - 1) list[at++] = make_uint2(s, 32 * wd + __ffs(bits) - 1);
         }
-        const int total = __shfl_sync(0xffffffffu, at, 31);
-        if (total == 0) continue;
-        int base = 0;
-        if (lane == 0) base = atomicAdd(count, total);
-        at += __shfl_sync(0xffffffffu, base, 0) - __popc(bits);
-        for (; bits; bits &= bits - 1) list[at++] = make_uint2(s, 32 * wd + __ffs(bits) - 1);
+        __syncwarp();
     }
 }
 
