@@ -417,7 +417,8 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             ClearList cl;
             cl.add(&w.gs->not_spd_F, sizeof(int));
             chol64_clear(w.cholF, cl);
-            launch_clear(cl, st);
+            const int r = launch_clear(cl, st);
+            if (r != QLP_OK) return r;
             launch_copy_square(w.F, w.F0, w.ldF, 8, 64, w.gs, Mc, st);
             launch_regularization(so, w, Mc, regp, REG_F, st);
             launch_cholesky_fp64(w.F, w.ldF, Mc, w.gs, 0, Mc, factor_ctas(c, Mc / 64), w.cholF, w.linv, st);
@@ -446,7 +447,8 @@ static int run_pipeline(qlp_ctx* c, Slot& slot, const StaticData& sd_in, const S
             chol64_clear(w.cholF, cl);
             chol64_clear(w.cholR, cl);
         }
-        launch_clear(cl, st);
+        r = launch_clear(cl, st);
+        if (r != QLP_OK) return r;
     }
     if (ev) cudaEventRecord(ev[0], st);
     if (c->nfw_mode == QLP_NFW_SURROGATE && model_has_nfw(c)) {

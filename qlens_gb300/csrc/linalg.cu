@@ -15,7 +15,7 @@
 // padded to a multiple of 64 with an identity block, which leaves log det and
 // the solution unchanged.  Every kernel reads N and M from the device-side
 // GridState, so the launch sequence never waits for the host.
-#include "qlpix_internal.h"
+#include "qlpix_ctx.h"
 #include "chol.cuh"
 
 namespace qlpix {
@@ -76,13 +76,18 @@ __global__ void __launch_bounds__(256) k_clear(ClearList l)
     }
 }
 
-void launch_clear(const ClearList& l, cudaStream_t st)
+int launch_clear(const ClearList& l, cudaStream_t st)
 {
+    if (l.full) {
+        set_error("%s (%d)", "too many buffers to clear", l.n);
+        return QLP_ERR_ARG;
+    }
     size_t words = 0;
     for (int k = 0; k < l.n; k++) words += l.item[k].words;
     const int blocks = (int)((words / 4 + 1023) / 1024);
     k_clear<<<blocks < 1 ? 1 : (blocks > 152 * 2 ? 152 * 2 : blocks), 256, 0, st>>>(l);
     count_launches(1);
+    return QLP_OK;
 }
 
 __global__ void __launch_bounds__(256) k_clear_band(char* __restrict__ A, size_t ld_bytes, int esize, int blk, int back,

@@ -876,7 +876,8 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
         ClearList cl;
         cl.add(&w.gs->not_spd_F, sizeof(int));
         mixed_clear(slot, cl, true);
-        launch_clear(cl, st);
+        rc = launch_clear(cl, st);
+        if (rc != QLP_OK) return rc;
         launch_copy_square(m->F32, m->F0, m->ld32, 4, C2, w.gs, m->M_cap, st);
         k_reg32<<<(so.snx * so.sny + 128 + 255) / 256, 256, 0, st>>>(w.gs, w.active_index, regp, m->F32, m->R32,
                                                                     m->ld32, so.regularization, REG_F);

@@ -261,12 +261,18 @@ void op_conv(const StaticData& sd, Work& w, int N_cap, bool transpose, const dou
 // Buffers that an evaluation starts from cleared, in one kernel (not memset
 // nodes: see issue_eval).
 struct ClearItem { void* p; unsigned words, value; };
+#define CLEAR_MAX 16
 struct ClearList {
-    ClearItem item[16];
+    ClearItem item[CLEAR_MAX];
     int n = 0;
-    void add(void* p, size_t bytes, unsigned value = 0) { item[n++] = ClearItem{p, (unsigned)((bytes + 3) / 4), value}; }
+    bool full = false;                 // one more was asked for: launch_clear refuses the list
+    void add(void* p, size_t bytes, unsigned value = 0)
+    {
+        if (n == CLEAR_MAX) { full = true; return; }
+        item[n++] = ClearItem{p, (unsigned)((bytes + 3) / 4), value};
+    }
 };
-void launch_clear(const ClearList& l, cudaStream_t st);
+int launch_clear(const ClearList& l, cudaStream_t st);
 // columns [blk max(0, i - back), blk (i + 1)) of every row of block row i = row / blk, rows below the padded M
 void launch_clear_band(void* A, int ld, int esize, int rows, int blk, int back, const GridState* gs, cudaStream_t st);
 // the lower triangle of the padded M, in whole blk x blk blocks, from src to dst
