@@ -1,9 +1,9 @@
-// mixed.cu -- mixed-precision inversion: TF32 tensor-core SYRK (3xTF32 split),
+// mixed.cu -- mixed-precision inversion: tensor-core SYRK of F16 hi + lo parts,
 // FP32 Cholesky of F and R, FP64 log det accumulation and FP64 iterative
 // refinement of the source amplitudes.
 //
-//   X      = (P L sqrt(C^-1))^T, built column by column (one source cell
-//            per CTA, exact fixed-point sums), split into TF32 hi + lo  k_psf_x
+//   X      = (P L sqrt(C^-1))^T by image tiles (exact fixed-point
+//            sums), split into F16 hi + lo                       k_psf_x
 //   F32    = X X^T on tcgen05 (block-sparse over pixel blocks)   k_syrk_tc
 //   F32   += lambda R, R32 = R                                  k_reg32
 //   L_F L_F^T = F32, L_R L_R^T = R32 (FP32 blocked Cholesky)    chol128.cuh
@@ -12,8 +12,8 @@
 //   s = F32^-1 D, then `refine` times: r = D - L^T P^T C^-1 P L s - lambda R s (FP64),
 //                                       s += F32^-1 r
 //   model = P L s                             (FP64, for chi^2)
-// The plain FP64 path (linalg.cu) computes the same quantities entirely in
-// FP64; the mixed path's deviation from it is measured by the tests.
+// The plain FP64 path (linalg.cu, psf.cu, ozaki.cu, cholfp64.cu) computes the same
+// quantities at FP64 accuracy; the mixed path's deviation from it is measured by the tests.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <climits>
@@ -35,9 +35,8 @@ struct MixedWork {
     double* t = nullptr;     // N (image-plane scratch)
     Csc csc{};               // L by source cell, for k_psf_x and L^T
     float* F0 = nullptr;     // lambda optimisation: X X^T before lambda R (allocated on first use)
-    void* X_hi = nullptr;    // F16 (or TF32 in FP32 storage) parts of X
-    void* X_lo = nullptr;
-    bool half = true;        // X in F16 for the kind::f16 SYRK
+    __half* X_hi = nullptr;  // F16 parts of X
+    __half* X_lo = nullptr;
     int K_cap = 0;           // columns of X (image pixels), multiple of 32
     int M_cap = 0;           // rows of X, multiple of 128
     unsigned char* nz = nullptr;
@@ -65,18 +64,18 @@ struct MixedWork {
 
 static MixedWork* mw_of(Slot& s) { return reinterpret_cast<MixedWork*>(s.mixed); }
 
-// 128-row boxes of 128 bytes (32 FP32 or 64 F16 values), 128-byte swizzle
+// 128-row boxes of 128 bytes (64 F16 or 32 FP32 values), 128-byte swizzle
 static int make_map(CUtensorMap* map, void* base, int rows, int cols, bool half)
 {
     return make_map_box(map, base, rows, cols, half, TC_TILE, half ? 64 : 32);
 }
 
 // ---------------------------------------------------------------------------
-// X = (P L sqrt(C^-1))^T as TF32 hi + lo, and the nonzero flags of its
+// X = (P L sqrt(C^-1))^T as F16 hi + lo, and the nonzero flags of its
 // 128-cell x 32-pixel blocks.
 //
 // Row s of X is the PSF-convolved image of source cell s: every pixel q that
-// sees s (column s of the pre-PSF L) spreads L[q][s] over its PSF neighbours
+// sees s (column s of the pre-PSF L) contributes L[q][s] to its PSF neighbours
 // p with weight psf[k][l] (the transpose of QLens's gather,
 // pixelgrid.cpp:14126-14168); the sum at p is then scaled by sqrt(C^-1) of p.
 // The sums are 64-bit fixed point, so they are exact and independent of the
@@ -85,31 +84,18 @@ static int make_map(CUtensorMap* map, void* base, int rows, int cols, bool half)
 // grid 2^-PSFX_LEXP (2^-28: 4e-9 absolute, far below FP32 resolution of the
 // entries) -- one wide multiply per tap.  No dense L' is stored.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float to_tf32(float f)
-{
-    uint32_t u;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(f));
-    return __uint_as_float(u);
-}
 
-// One entry of X split into hi + lo: TF32 parts in FP32 storage, or F16 parts
-// of v scaled by xs (a power of two that puts X's largest entry near 2^14,
-// undone exactly by the SYRK).  Returns whether either part is nonzero.
-__device__ __forceinline__ bool store_x(void* Xh, void* Xl, size_t idx, float v, float xs, bool half)
+// One entry of X split into F16 hi + lo parts of v scaled by xs (a power of two that
+// puts X's largest entry near 2^14, undone exactly by the SYRK).  Returns whether
+// either part is nonzero.
+__device__ __forceinline__ bool store_x(__half* Xh, __half* Xl, size_t idx, float v, float xs)
 {
-    if (half) {
-        const float vs = v * xs;
-        const __half h = __float2half_rn(vs);
-        const __half l = __float2half_rn(vs - __half2float(h));
-        reinterpret_cast<__half*>(Xh)[idx] = h;
-        reinterpret_cast<__half*>(Xl)[idx] = l;
-        return __half2float(h) != 0.0f || __half2float(l) != 0.0f;
-    }
-    const float h = to_tf32(v);
-    const float l = to_tf32(v - h);
-    reinterpret_cast<float*>(Xh)[idx] = h;
-    reinterpret_cast<float*>(Xl)[idx] = l;
-    return h != 0.0f || l != 0.0f;
+    const float vs = v * xs;
+    const __half h = __float2half_rn(vs);
+    const __half l = __float2half_rn(vs - __half2float(h));
+    Xh[idx] = h;
+    Xl[idx] = l;
+    return __half2float(h) != 0.0f || __half2float(l) != 0.0f;
 }
 
 // column counts of the merged pre-PSF L, the image tiles with active pixels, and the
@@ -431,8 +417,8 @@ template <bool PAD>
 __global__ void __launch_bounds__(512) k_psf_x(StaticData sd, const int* __restrict__ colptr,
                                                const int2* __restrict__ ent_g, const int2* __restrict__ pixT, int ntx,
                                                const int* __restrict__ count, const uint2* __restrict__ list,
-                                               void* __restrict__ Xh, void* __restrict__ Xl, float xs, int half,
-                                               int K_cap, unsigned char* __restrict__ nz, int nkb_cap)
+                                               __half* __restrict__ Xh, __half* __restrict__ Xl, float xs, int K_cap,
+                                               unsigned char* __restrict__ nz, int nkb_cap)
 {
     extern __shared__ __align__(16) int taps[];  // [pnx + 62][pitch]: column pk + 31, row pl + R - 1
     constexpr int R = PSFX_R;
@@ -493,7 +479,7 @@ __global__ void __launch_bounds__(512) k_psf_x(StaticData sd, const int* __restr
             const int2 pt = pixT[(size_t)(y0 + r + nyh) * nxp + x + nxh];
             if (pt.x < 0 || acc[r] == 0) continue;
             const float v = (ll2f_rn_int(acc[r]) * inv) * __int_as_float(pt.y);
-            if (store_x(Xh, Xl, (size_t)s * K_cap + pt.x, v, xs, half))
+            if (store_x(Xh, Xl, (size_t)s * K_cap + pt.x, v, xs))
                 nz[(size_t)(s / TC_TILE) * nkb_cap + pt.x / TC_KB] = 1;
         }
     }
@@ -503,7 +489,7 @@ __global__ void __launch_bounds__(512) k_psf_x(StaticData sd, const int* __restr
 // X moved ~480 MB at 4,096 cells x 58,000 pixels).
 __global__ void __launch_bounds__(256) k_x_clean(StaticData sd, const int2* __restrict__ pixT, int ntx,
                                                  const int* __restrict__ count, const uint2* __restrict__ list,
-                                                 void* __restrict__ Xh, void* __restrict__ Xl, int half, int K_cap)
+                                                 __half* __restrict__ Xh, __half* __restrict__ Xl, int K_cap)
 {
     const int lane = threadIdx.x & 31, items = *count;
     const int nxh = sd.pnx / 2, nyh = sd.pny / 2, nxp = sd.nx + 2 * nxh;
@@ -519,13 +505,8 @@ __global__ void __launch_bounds__(256) k_x_clean(StaticData sd, const int2* __re
         for (int r = 0; r < PSFX_R; r++) {
             if (row[r] < 0) continue;
             const size_t idx = (size_t)item.x * K_cap + row[r];
-            if (half) {
-                reinterpret_cast<__half*>(Xh)[idx] = __float2half_rn(0.0f);
-                reinterpret_cast<__half*>(Xl)[idx] = __float2half_rn(0.0f);
-            } else {
-                reinterpret_cast<float*>(Xh)[idx] = 0.0f;
-                reinterpret_cast<float*>(Xl)[idx] = 0.0f;
-            }
+            Xh[idx] = __float2half_rn(0.0f);
+            Xl[idx] = __float2half_rn(0.0f);
         }
     }
 }
@@ -737,7 +718,7 @@ int mixed_init(Slot& c)
     m->ld32 = M_cap;
     Arena ar;
     auto A = [&](void** p, size_t bytes) { ar.add(reinterpret_cast<char**>(p), bytes); };
-    const size_t xbytes = (m->half ? 2 : 4) * (size_t)M_cap * K_cap;
+    const size_t xbytes = sizeof(__half) * (size_t)M_cap * K_cap;
     A((void**)&m->X_hi, xbytes);
     A((void**)&m->X_lo, xbytes);
     A((void**)&m->nz, (size_t)(M_cap / TC_TILE) * m->nkb_cap + 3);
@@ -774,8 +755,8 @@ int mixed_init(Slot& c)
     cudaMemset(m->X_hi, 0, xbytes);
     cudaMemset(m->X_lo, 0, xbytes);
     cudaStreamSynchronize(0);                              // the slots' streams do not wait for stream 0
-    if (make_map(&m->map_hi, m->X_hi, M_cap, K_cap, m->half) != QLP_OK ||
-        make_map(&m->map_lo, m->X_lo, M_cap, K_cap, m->half) != QLP_OK ||
+    if (make_map(&m->map_hi, m->X_hi, M_cap, K_cap, true) != QLP_OK ||
+        make_map(&m->map_lo, m->X_lo, M_cap, K_cap, true) != QLP_OK ||
         flow_maps(m->cf, m->cf_maps) != QLP_OK || flow_maps(m->cr, m->cr_maps) != QLP_OK) {
         set_error("%s (%d)", "cuTensorMapEncodeTiled unavailable or failed", 0);
         return QLP_ERR_CUDA;
@@ -792,8 +773,7 @@ int mixed_init(Slot& c)
         opt((const void*)k_psf_x<true>, 227 * 1024);
         opt((const void*)k_psf_x<false>, 227 * 1024);
         opt((const void*)k_chol128, C2_SMEM);
-        opt((const void*)k_syrk_tc<false>, TC_SMEM);
-        opt((const void*)k_syrk_tc<true>, TC_SMEM);
+        opt((const void*)k_syrk_tc, TC_SMEM);
         if (ea != cudaSuccess) {
             set_error("%s (%d)", "shared-memory opt-in failed", (int)ea);
             return QLP_ERR_CUDA;
@@ -905,7 +885,7 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
     k_LTw_csc<<<ltw_blocks, 256, 0, st>>>(w.gs, m->csc.colcnt, m->csc.colrow, m->csc.colval64, m->t, w.D);
     n++;
     // X = (P L sqrt(C^-1))^T and its block flags, from L by source cell
-    const float xs = m->half ? ldexpf(1.0f, sd.x_exp) : 1.0f;     // F16 scale of X
+    const float xs = ldexpf(1.0f, sd.x_exp);                      // F16 scale of X
     const int ntx = (sd.nx + 31) / 32;
     const int* ntiles = m->csc.ntiles();
     {
@@ -914,22 +894,17 @@ int run_inversion_mixed(const qlp_ctx* c, Slot& slot, const StaticData& sd, cons
         const bool pad = taps <= PSFX_PAD_BYTES;
         auto k = pad ? k_psf_x<true> : k_psf_x<false>;
         k<<<152 * 1024 / pt, pt, pad ? taps : 0, st>>>(sd, m->csc.colcnt, m->csc.ent, m->csc.pixT, ntx, ntiles, m->csc.tiles, m->X_hi,
-                                                       m->X_lo, xs, m->half ? 1 : 0, m->K_cap, m->nz, m->nkb_cap);
+                                                       m->X_lo, xs, m->K_cap, m->nz, m->nkb_cap);
         n++;
     }
     if (ev) cudaEventRecord(ev[3], st);
     {
         const int nt = m->M_cap / TC_TILE;
-        if (m->half)
-            k_syrk_tc<true><<<nt * (nt + 1) / 2, 128, TC_SMEM, st>>>(m->map_hi, m->map_lo, w.gs, m->nz, m->nkb_cap,
-                                                                      m->F32, m->ld32, ldexpf(1.0f, -2 * sd.x_exp));
-        else
-            k_syrk_tc<false><<<nt * (nt + 1) / 2, 128, TC_SMEM, st>>>(m->map_hi, m->map_lo, w.gs, m->nz,
-                                                                       m->nkb_cap, m->F32, m->ld32, 1.0f);
+        k_syrk_tc<<<nt * (nt + 1) / 2, 128, TC_SMEM, st>>>(m->map_hi, m->map_lo, w.gs, m->nz, m->nkb_cap, m->F32,
+                                                           m->ld32, ldexpf(1.0f, -2 * sd.x_exp));
         n++;
         // X back to all zero for the next evaluation
-        k_x_clean<<<152 * 8, 256, 0, st>>>(sd, m->csc.pixT, ntx, ntiles, m->csc.tiles, m->X_hi, m->X_lo, m->half ? 1 : 0,
-                                           m->K_cap);
+        k_x_clean<<<152 * 8, 256, 0, st>>>(sd, m->csc.pixT, ntx, ntiles, m->csc.tiles, m->X_hi, m->X_lo, m->K_cap);
         n++;
     }
     if (ev) cudaEventRecord(ev[4], st);

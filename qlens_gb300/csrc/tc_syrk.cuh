@@ -2,20 +2,18 @@
 //
 // X is L'^T scaled by sqrt(C^-1): M_cap rows (source cells) x K_cap columns
 // (image pixels), K contiguous, split into a rounded high part and a rounded
-// remainder so that hi*hi + hi*lo + lo*hi carries ~22 bits.  Two operand
-// types, one kernel: TF32 (FP32 storage, kind::tf32, K = 8 per MMA, 32 pixels
-// per 128-byte stage row) or F16 (kind::f16 at twice the tensor rate, K = 16
-// per MMA, 64 pixels per stage row; X scaled by a power of two so that its
-// largest entry is near 2^14, undone exactly in the epilogue).  Both have 11
-// significant bits per part.  One CTA computes one 128x128 tile of the lower
-// triangle of F:
+// remainder so that hi*hi + hi*lo + lo*hi carries ~22 bits.  The parts are F16
+// (kind::f16, K = 16 per MMA, 64 pixels per 128-byte stage row): as many
+// significant bits as TF32 at twice the tensor rate, X scaled by a power of two so
+// that its largest entry is near 2^14, undone exactly in the epilogue.  One CTA
+// computes one 128x128 tile of the lower triangle of F:
 //   warp 0 / lane 0  TMA producer: 128-row boxes of 128 B (128 B swizzle) of
 //                    X_hi, X_lo for the tile's row block and column block
 //                    into a 3-stage shared-memory ring;
 //   warp 1 / lane 0  MMA issuer, 4 k-steps of tcgen05.mma.cta_group::1 per stage
-//                    into FP32 accumulators in TMEM: F16 hi*(hi, lo) as one
+//                    into FP32 accumulators in TMEM: hi*(hi, lo) as one
 //                    N = 256 product (lo's rows follow hi's in shared memory) and
-//                    lo*hi into the second half, TF32 three N = 128 products;
+//                    lo*hi into the second half;
 //   all 4 warps      epilogue: tcgen05.ld 32x32b.x32, the halves added, FP32
 //                    stores to F.
 // Block sparsity: a stage is processed only if both the row block and the
@@ -41,16 +39,14 @@ namespace qlpix {
 
 // grid: one CTA per lower-triangle 128x128 tile of the M_cap x M_cap output.
 // nzflags[rb * nkb_cap + kb] != 0 when rows [128 rb, 128 rb + 128) of X have a
-// nonzero in columns [32 kb, 32 kb + 32).  HALF: F16 operands (64 pixels per
-// stage: flags 2 kb and 2 kb + 1); fscale multiplies the result (2^-2s for X
-// scaled by 2^s).
-template <bool HALF>
+// nonzero in columns [32 kb, 32 kb + 32) (a stage's 64 pixels: flags 2 kb and
+// 2 kb + 1); fscale multiplies the result (2^-2s for X scaled by 2^s).
 __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUtensorMap map_hi,
                                                     const __grid_constant__ CUtensorMap map_lo,
                                                     GridState* gs, const unsigned char* __restrict__ nzflags,
                                                     int nkb_cap, float* __restrict__ F, int ldF, float fscale)
 {
-    constexpr int KPS = HALF ? 2 * TC_KB : TC_KB;      // pixels per stage (128 bytes of a row)
+    constexpr int KPS = 2 * TC_KB;                     // pixels per stage (128 bytes of a row)
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t full_bar[TC_STAGES];
     __shared__ uint64_t empty_bar[TC_STAGES];
@@ -93,7 +89,7 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
     __syncwarp();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(HALF ? 256 : 128)
+                     "r"(2 * TC_TILE)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -106,8 +102,7 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
     const unsigned char* fj = nzflags + (size_t)bj * nkb_cap;
     // stage kb has work when both blocks have a nonzero among its pixels
     auto live = [&](int kb) -> bool {
-        if (HALF) return (fi[2 * kb] | fi[2 * kb + 1]) && (fj[2 * kb] | fj[2 * kb + 1]);
-        return fi[kb] && fj[kb];
+        return (fi[2 * kb] | fi[2 * kb + 1]) && (fj[2 * kb] | fj[2 * kb + 1]);
     };
 
     int it_p = 0, it_m = 0;                            // stages loaded (warp 0), multiplied (warp 1)
@@ -146,7 +141,7 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
             n_issued = it_p;
         } else if (warp == 1 && lane == 0) {
             // ---- MMA issuer ----
-            const uint32_t idesc = HALF ? idesc_f16_128x128() : idesc_tf32_128x128();
+            const uint32_t idesc = idesc_f16_128x128();
             const uint32_t idesc2 = idesc_f16(128, 256);
             for (int u = 0; u < n; u++, it_m++) {
                 const int s = it_m % TC_STAGES;
@@ -156,22 +151,15 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
                 const uint64_t a_hi = sdesc_sw128(smem_u32(st));
                 const uint64_t a_lo = sdesc_sw128(smem_u32(st + TC_TILE_BYTES));
                 const uint64_t b_hi = sdesc_sw128(smem_u32(st + 2 * TC_TILE_BYTES));
-                const uint64_t b_lo = sdesc_sw128(smem_u32(st + 3 * TC_TILE_BYTES));
                 #pragma unroll
                 for (int kk = 0; kk < 4; kk++) {
-                    // one MMA takes 32 bytes along K: 8 TF32 or 16 F16 values
+                    // one MMA takes 32 bytes along K: 16 F16 values
                     const uint64_t off = (uint64_t)((kk * 32) >> 4);
                     const uint32_t acc = (it_m > 0 || kk > 0) ? 1u : 0u;
-                    if (HALF) {
-                        // b_lo's rows follow b_hi's: hi*hi and hi*lo are one N = 256
-                        // product, side by side in TMEM; lo*hi joins hi*lo
-                        mma_f16(tmem, a_hi + off, b_hi + off, idesc2, acc);
-                        mma_f16(tmem + TC_TILE, a_lo + off, b_hi + off, idesc, 1u);
-                    } else {
-                        mma_tf32(tmem, a_hi + off, b_hi + off, idesc, acc);
-                        mma_tf32(tmem, a_hi + off, b_lo + off, idesc, 1u);
-                        mma_tf32(tmem, a_lo + off, b_hi + off, idesc, 1u);
-                    }
+                    // B's lo rows follow its hi rows: hi*hi and hi*lo are one N = 256
+                    // product, side by side in TMEM; lo*hi joins hi*lo
+                    mma_f16(tmem, a_hi + off, b_hi + off, idesc2, acc);
+                    mma_f16(tmem + TC_TILE, a_lo + off, b_hi + off, idesc, 1u);
                 }
                 mma_commit(&empty_bar[s]);
             }
@@ -200,12 +188,10 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
             float v[32];
             const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c;
             tmem_ld_32cols(taddr, v);
-            if (HALF) {
-                float lo[32];
-                tmem_ld_32cols(taddr + TC_TILE, lo);
-                #pragma unroll
-                for (int i = 0; i < 32; i++) v[i] += lo[i];
-            }
+            float lo[32];
+            tmem_ld_32cols(taddr + TC_TILE, lo);
+            #pragma unroll
+            for (int i = 0; i < 32; i++) v[i] += lo[i];
             #pragma unroll
             for (int i = 0; i < 32; i += 4)
                 *reinterpret_cast<float4*>(out + c + i) =
@@ -219,7 +205,7 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
     if (abort_flag && threadIdx.x == 0) atomicExch(&gs->status, QLP_ERR_TIMEOUT);
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(HALF ? 256 : 128) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TC_TILE) : "memory");
     }
 }
 
