@@ -422,19 +422,20 @@ static cudaError_t st_chain(const SurTrain& T, cudaStream_t s)
 
 // Forward and backward pass: the gradients' parts, and with lpart the loss's.
 // RT: a CTA's time goes with RT + 1 (the weights' copies, the output layer), so
-// the one with the fewest waves x (RT + 1) -- 7 for 16,384 rows: 147 CTAs on 152
-// SMs, 130 us a step (8, as many waves, 136; 4, two waves, 147).
+// the one of 2 to 8 with the fewest waves x (RT + 1) -- 7 for 16,384 rows: 147 CTAs on
+// 152 SMs, 130 us a step (8, as many waves, 136; 4, two waves, 147).  With 2, 4, 7 and 8
+// alone 10,240 rows took 111 us (5 rows: 92), 12,288 120 (6: 110), 24,000 275 (5: 192).
 static cudaError_t st_fwd_bwd(const SurTrain& T, int sms, int mse_blocks, cudaStream_t s)
 {
-    const int rts[4] = {2, 4, 7, 8};
+    static cudaError_t (*const chain[7])(const SurTrain&, cudaStream_t) = {st_chain<2>, st_chain<3>, st_chain<4>, st_chain<5>,
+                                                                           st_chain<6>, st_chain<7>, st_chain<8>};
     int rt = 8;
     long best = 1L << 60;
-    for (int r : rts) {
+    for (int r = 2; r <= 8; r++) {
         const long tiles = (T.bs + 16 * r - 1) / (16 * r), cost = (tiles + sms - 1) / sms * (r + 1);
         if (cost < best) { best = cost; rt = r; }
     }
-    cudaError_t e = rt == 2 ? st_chain<2>(T, s) : rt == 4 ? st_chain<4>(T, s) : rt == 7 ? st_chain<7>(T, s)
-                                                                                      : st_chain<8>(T, s);
+    cudaError_t e = chain[rt - 2](T, s);
     if (e != cudaSuccess) return e;
     if (T.lpart)
         k_sur_mse<<<mse_blocks, 256, 0, s>>>(T.bs, T.act + 5 * (size_t)T.bs * SUR_H, T.t, T.w,
