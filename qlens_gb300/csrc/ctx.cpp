@@ -193,7 +193,7 @@ static int psf_fixed_rule(const qlp_ctx* c, const std::vector<int>* lists, int n
     double lo = INFINITY, hi = 0;
     for (int k = 0; k < n_lists && c->sd.use_noise_map; k++)
         for (int p : lists[k]) {
-            const double v = c->covinv[p];
+            const double v = fabs(c->covinv[p]);
             if (!(v > 0 && std::isfinite(v))) continue;
             lo = std::min(lo, v);
             hi = std::max(hi, v);
@@ -242,6 +242,7 @@ int ctx_init(qlp_ctx* c, const qlp_image* im, const qlp_psf* psf, const qlp_srcg
     if (c->psfx_mode < 0) c->psfx_mode = (psf->nx * psf->ny >= 500) ? 1 : 0;
     sd.use_noise_map = noise_map ? 1 : 0;
     sd.cov_inverse = cov_inverse;
+    sd.neg_noise = noise_map && std::any_of(covinv.begin(), covinv.end(), [](double v) { return v < 0; });
     c->bg_noise = im->background_pixel_noise;
     sd.xvals = c->d_xvals; sd.yvals = c->d_yvals; sd.data = c->d_data; sd.covinv = c->d_covinv;
     sd.mpix = c->d_mpix; sd.psf = c->d_psf;

@@ -42,11 +42,12 @@ __device__ __forceinline__ void oz_tile(int t, int& I, int& j)
 // The digits of 64 cells x 32 pixels of L'^T (sqrt(C^-1)), eight pixels a thread.  With a
 // noise map the operand is the product L' sqrt(C^-1) as k_psf64 formed it for the cell's
 // largest exponent (a bound from the image's largest sqrt(C^-1) instead cost a cell on
-// noisier pixels as many of its bits as their noise is larger).
+// noisier pixels as many of its bits as their noise is larger).  sign: the pixels with
+// this sign of C^-1.
 // Stages without a nonzero in the cells' 128-row block are never loaded by the
 // products, so they are skipped.  14 bytes written per 8 read: memory bound.
 __global__ void __launch_bounds__(256) k_oz_slice(const GridState* __restrict__ gs, const double* __restrict__ L,
-                                                  int ldL, const double* __restrict__ svec,
+                                                  int ldL, const double* __restrict__ svec, int sign,
                                                   const int* __restrict__ emax, const unsigned char* __restrict__ nz,
                                                   int nst, int st0, __half* __restrict__ xs, int M128, int Kc)
 {
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(256) k_oz_slice(const GridState* __restrict__ 
             for (int k = 0; k < 2; k++) {
                 const int r = r0 + u + k;
                 double x = r < N ? (k ? v.y : v.x) : 0.0;
-                if (svec && x != 0) x *= svec[r];
+                if (svec && x != 0) x = (svec[r] < 0) == (sign < 0) ? x * fabs(svec[r]) : 0.0;
                 q[u + k] = oz_bias<OZ_S>(oz_fixed54(x, em));
             }
         }
@@ -91,12 +92,13 @@ __global__ void __launch_bounds__(256) k_oz_slice(const GridState* __restrict__ 
 // 0.48 -> 0.05 ms, everything of launch_syrk_fp64 included.
 // The digit products of one tile over its share of the chunk's live stages
 // (both blocks have a nonzero among the stage's 32 pixels): grid (tiles,
-// splits).  The tile's integers are added into `part` by 64-bit reductions, lanes
-// along the rows.
+// splits).  The tile's integers are added into `part` (sign < 0: taken off) by 64-bit
+// reductions, lanes along the rows.
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_syrk(const __grid_constant__ CUtensorMap map_a,
                                                           const __grid_constant__ CUtensorMap map_b, GridState* gs,
                                                           const unsigned char* __restrict__ nz, int nst, int st0,
-                                                          int st1, int M128, unsigned long long* __restrict__ part)
+                                                          int st1, int M128, unsigned long long* __restrict__ part,
+                                                          int sign)
 {
     extern __shared__ unsigned char smem_raw[];
     __shared__ OzPipe pipe;
@@ -168,8 +170,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_syrk(const __grid_constant
                                   (warp & 3) * 32 + lane;
         #pragma unroll
         for (int c = 0; c < 32; c++) {
-            atomicAdd(out + c * OZ_TM, (unsigned long long)hi[c]);
-            atomicAdd(out + OZ_TM * OZ_TN + c * OZ_TM, (unsigned long long)lo[c]);
+            atomicAdd(out + c * OZ_TM, (unsigned long long)(sign < 0 ? -hi[c] : hi[c]));
+            atomicAdd(out + OZ_TM * OZ_TN + c * OZ_TM,
+                      sign < 0 ? 0ull - (unsigned long long)lo[c] : (unsigned long long)lo[c]);
         }
     }
 }
@@ -278,11 +281,14 @@ void launch_syrk_fp64(const StaticData& sd, Work& w, int N_max, int M_max, cudaS
         // but no finer than one read of the accumulators per CTA
         const int split = std::max(1, std::min({(OZ_WANT_CTAS + tiles - 1) / tiles, (cnt + OZ_FLUSH - 1) / OZ_FLUSH,
                                                 64}));
-        k_oz_slice<<<dim3(cnt, ncb), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, sd.use_noise_map ? w.svec : nullptr, z->emax,
-                                                   z->nz, z->nst, s0, z->xs, z->M128, z->Kc);
-        k_oz_syrk<<<dim3(tiles, split), OZ_THREADS, oz_smem(OZ_S), st>>>(z->map_a, z->map_b, w.gs, z->nz, z->nst, s0,
-                                                                   s0 + cnt, z->M128, z->part);
-        n += 2;
+        // (a noise map with negative C^-1, no one's noise but taken: those pixels in a turn of their own)
+        for (int sign = 1; sign >= (sd.neg_noise ? -1 : 1); sign -= 2) {
+            k_oz_slice<<<dim3(cnt, ncb), 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, sd.use_noise_map ? w.svec : nullptr, sign,
+                                                       z->emax, z->nz, z->nst, s0, z->xs, z->M128, z->Kc);
+            k_oz_syrk<<<dim3(tiles, split), OZ_THREADS, oz_smem(OZ_S), st>>>(z->map_a, z->map_b, w.gs, z->nz, z->nst,
+                                                                       s0, s0 + cnt, z->M128, z->part, sign);
+            n += 2;
+        }
     }
     k_oz_finish<<<2 * tiles, 256, 0, st>>>(w.gs, z->part, z->emax, sd.use_noise_map ? 1.0 : sd.cov_inverse, w.F,
                                            w.ldF);

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256) k_psf64(StaticData sd, const GridState* _
 }
 
 // Active row -> image pixel, the inverse of the compaction's pixindex, and the
-// row's data and C^-1 (svec, or null: its square root).
+// row's data and C^-1 (svec, or null: the root of its size, with its sign).
 __global__ void k_rowpix(StaticData sd_, const int* __restrict__ rowidx, int* __restrict__ rowpix,
                          double* __restrict__ dvec, double* __restrict__ cvec, double* __restrict__ svec)
 {
@@ -170,7 +170,7 @@ __global__ void k_rowpix(StaticData sd_, const int* __restrict__ rowidx, int* __
         rowpix[r] = pix;
         dvec[r] = sd.data[pix];
         cvec[r] = sd.use_noise_map ? sd.covinv[pix] : sd.cov_inverse;
-        if (svec) svec[r] = sqrt(cvec[r]);
+        if (svec) svec[r] = cvec[r] < 0 ? -sqrt(-cvec[r]) : sqrt(cvec[r]);
     }
 }
 

@@ -109,6 +109,7 @@ struct StaticData {            // per-context, uploaded once
     int n_sub;                 // n_mask * nsub
     int pnx, pny;              // PSF size
     int use_noise_map;
+    int neg_noise;             // some C^-1 is negative
     double cov_inverse;        // uniform 1/sigma^2 when !use_noise_map
     int noise_term;            // add the pixel-noise normalisation to -2 log(evidence)
     const double* xvals;       // nx+1
@@ -218,7 +219,7 @@ struct Work {
     Chol64Work* cholF;  Chol64Work* cholR;  // plain path: workspaces of the factorisations (cholfp64.cu)
     int ldL;                           // leading dimension of Lpsf (>= N_max, a multiple of 32)
     double* dvec; double* cvec;        // N: data and C^-1 per active row
-    double* svec;                      // N: sqrt(C^-1) (plain path with a noise map)
+    double* svec;                      // N: sqrt|C^-1| with C^-1's sign (plain path with a noise map)
     double* D;                         // M
     double* F;                         // M x ldF (lower triangle)
     double* R;                         // M x ldF (lower triangle)
