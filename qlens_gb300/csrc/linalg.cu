@@ -400,10 +400,11 @@ void launch_model_chi2(const StaticData& sd, const SrcOpts& so, Work& w, int N_m
 {
     if (N_max > 0 && !mixed) {
         k_model<<<(N_max + 31) / 32, 256, 0, st>>>(w.gs, w.Lpsf, w.ldL, oz_nz(w.oz), oz_nst(w.oz), w.s, w.model);
+        count_launches(1);
     }
     k_final<<<FINAL_CTAS, 256, 0, st>>>(sd, so, w.gs, w.rowidx, w.model, w.s, w.active_index, regp, factor, ld,
                                         mixed ? 1 : 0, w.fpart, w.fcount, w.out);
-    count_launches(2);
+    count_launches(1);
 }
 
 }  // namespace qlpix
