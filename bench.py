@@ -53,7 +53,7 @@ MLP_FLOP_PER_RAY = 2 * 3 * 128 * 128
 # DRAM bytes (read + written) of one evaluation's ray-shooting stage on the
 # workload, from one ncu capture of its kernels (dram__bytes_read.sum +
 # dram__bytes_write.sum of k_ray_pre and k_raytrace_sur<true>)
-RAYSUR_TRAFFIC = {"cfg5": (255488 + 2560) + (22348032 + 24320)}
+RAYSUR_TRAFFIC = {"cfg5": (284928 + 20992) + (22062336 + 0)}
 SYRK_TRAFFIC = {}
 UNIT = "evals/s"
 
@@ -481,15 +481,16 @@ def main():
                      "traffic": SYRK_TRAFFIC.get(args.config) if precision == "mixed" else None,
                      "peak_source": peak_note, "algorithmic_flops_per_launch": flops,
                      "timing": "CUDA events around the SYRK launch of single evaluations after the timed region"}
+    # both kernels skip the 32- and 64-pixel stages where either tile is zero (the
+    # products they leave out are zeros), and the plain path's runs as digit
+    # products on the tensor cores: the dense N M^2 count over their time is a
+    # dense-equivalent rate, not a fraction of a pipe
+    roofline_syrk["frac"] = None
+    roofline_syrk["dense_equivalent_frac"] = (achieved / peak) if achieved else None
+    roofline_syrk["note"] = ("achieved = the dense contraction's FLOP over the time of a kernel that skips the zero "
+                             "blocks of its operand")
     if precision != "mixed":
-        # k_oz_syrk skips the 32-pixel stages where either tile of L' is zero
-        # (the products it leaves out are zeros) and runs on the tensor cores: the
-        # dense N M^2 count over its time is a dense-equivalent rate, not a
-        # fraction of the FP64 pipe
-        roofline_syrk["frac"] = None
-        roofline_syrk["dense_equivalent_frac"] = (achieved / peak) if achieved else None
-        roofline_syrk["note"] = ("achieved = the dense contraction's FLOP over the time of a kernel that skips L''s "
-                                 "zero blocks and forms the others as digit products on the tensor cores")
+        roofline_syrk["note"] += " and forms the others as digit products on the tensor cores"
     # the dominant kernel of the batch: the ray shooting on the NFW surrogate
     # workloads (k_raytrace_sur), else the factorisation of F
     roofline = roofline_syrk

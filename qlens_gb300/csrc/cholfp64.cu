@@ -28,8 +28,8 @@
 // definite matrix; where F is not, its factor outgrows the integers' range, and
 // k_chol64_plain takes over.
 //
-// What bounds it, for one evaluation: the chain of pivot blocks, ~80 us per 64
-// columns -- 46 us the pivots (0.7 us each: 1/sqrt, two barriers, and wide integer
+// What bounds it, for one evaluation (tensor pipe 5 %, DRAM nothing): the chain of pivot
+// blocks, ~80 us per 64 columns -- 46 us the pivots (0.7 us each: 1/sqrt, two barriers, and wide integer
 // multiplies at a quarter of the plain rate), 6 us the inverse's digits, 8 us the
 // product below the block, 20 us the way to the next diagonal tile through flags
 // and global memory.  2,934 cells: F and R and the solves 43.3 -> 4.2 ms, 738
@@ -97,8 +97,7 @@ __device__ __forceinline__ int fx_scale4(long long d) { return max(0, (__clzll(d
 
 // Products of 62-bit numbers by 31-bit halves a = ah 2^31 + al (al >= 0): three
 // wide multiplies; al bl is left out, so a product comes out 3/4 of its unit low
-// on average.  (The compiler's 64x64 -> 128 multiply is ~40 instructions, no
-// faster per product than the FP64 pipe.)
+// on average.
 __device__ __forceinline__ int fx_hi(long long a) { return (int)(a >> 31); }
 __device__ __forceinline__ int fx_lo(long long a) { return (int)a & 0x7fffffff; }
 

@@ -375,7 +375,8 @@ static int load_of(const qlp_ctx* c) { return c->in_flight <= 1 ? 0 : c->in_flig
 // within its pivot block's time: a quarter of the block columns, and at least 16
 // while the SMs do for it.  (FP64, four optimising lambda: 35.7 ms with a
 // quarter, 32.6 with 12, 30.4 with 16, 31.1 with 37.  Mixed, 32 at 4,096 cells: 24.9 ms with 8,
-// 30.3 with 37.)
+// 30.3 with 37.  Not measured far below 25 block columns, where a quarter is few: 12 of them
+// with 9 or more in flight get 3 CTAs each.)
 int factor_ctas(const qlp_ctx* c, int nb)
 {
     const int quarter = std::max(2, (nb + 3) / 4), load = load_of(c);

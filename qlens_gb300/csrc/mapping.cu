@@ -417,7 +417,7 @@ void launch_compact(const StaticData& sd, const SrcOpts& so, Work& w, cudaStream
 // mapped sub-pixels in sub-cell order, 3 entries each.  The same thread also
 // writes the row with duplicate source indices merged (summed in CSR order,
 // i.e. exactly the row of convert_Lmatrix_to_dense, pixelgrid.cpp:13734-13739),
-// which the PSF kernel gathers from.
+// which both paths put together by source cell (launch_csc).
 // ---------------------------------------------------------------------------
 #define BUILD_L_MAXD 192      // entries of one row merged in shared memory (3 per sub-pixel, up to 8x8 split)
 #define BUILD_L_THREADS 32

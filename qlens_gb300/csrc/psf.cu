@@ -187,7 +187,9 @@ void launch_rowpix(const StaticData& sd, Work& w, cudaStream_t st)
     count_launches(1);
 }
 
-// The plain path's stated range of PSFs and source grids.
+// The plain path's stated range of PSFs and source grids: calls past it were refused by its
+// first kernel, which held a row of L' and the taps in shared memory, and stay refused
+// (k_psf64 itself would take them).
 int psf_in_range(const StaticData& sd, int M_max)
 {
     const size_t nT = ((size_t)sd.pnx * sd.pny + 7) / 8 * 8;
