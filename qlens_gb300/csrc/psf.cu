@@ -51,8 +51,8 @@ __device__ __forceinline__ double fixed_to_double(long long s, int k)
 // rows into shared memory in FP64, a tap after the other, waited on those.  2,934 cells x
 // 11,772 pixels, 441 taps: 1,940 -> 146 us (and 46 us for the entries by cell and
 // the clearing of L'); 738 x 6,220, 49 taps: 101 -> 38 us; 16 uneven evaluations at
-// up to 4,096 cells, 121 taps: 14.2 -> 10.4 ms.  In FP64 these sums alone would take
-// the pipe 250 us.
+// up to 4,096 cells, 121 taps: 14.2 -> 10.4 ms.  In FP64 (below)
+// the first takes 0.14 ms more.
 // FIXED = false (StaticData::psf_fixed, or bordered taps past PSF64_PAD_BYTES): FP64
 // sums of the FP64 entries, taps by their bounds from global memory.
 #define PSF64_PAD_BYTES (200 * 1024)
